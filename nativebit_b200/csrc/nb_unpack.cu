@@ -8,15 +8,10 @@
 #include <cuda_bf16.h>
 
 #include "nb_common.cuh"
+#include "nb_device.cuh"
 #include "nb_host.h"
 
 namespace nb {
-
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t c) {
-  uint32_t d;
-  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-  return d;
-}
 
 __device__ __forceinline__ uint32_t stream_index(const uint8_t* __restrict__ p, int64_t n_bytes, int64_t i, int bits) {
   const int64_t bit = i * bits;
@@ -65,10 +60,32 @@ __global__ void unpack_generic_kernel(const uint8_t* __restrict__ packed, int64_
 }
 
 // ---- pack ---------------------------------------------------------------------------------
-// One thread writes one output byte: it ORs the (at most 5) indices that overlap the byte.
-__global__ void pack_kernel(const uint8_t* __restrict__ idx, int64_t count, int bits, int64_t n_bytes,
+// Fast path, the inverse of unpack32_kernel: one thread turns 32 indices (two 16-byte loads) into `BITS` words.  HBM-bound:
+// 17.7 M indices to 3 bits in 6.7 us (24.3 MB); one thread per output byte took 40 us, on 64-bit index arithmetic.
+template <int BITS>
+__global__ void pack32_kernel(const uint4* __restrict__ idx, int64_t n_chunks, uint32_t* __restrict__ out) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n_chunks) return;
+  const uint4 a = idx[2 * c], b = idx[2 * c + 1];
+  const uint32_t in[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  uint32_t w[BITS];
+#pragma unroll
+  for (int i = 0; i < BITS; ++i) w[i] = 0;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    const uint32_t f = (in[j >> 2] >> (8 * (j & 3))) & ((1u << BITS) - 1u);
+    const int wi = (j * BITS) >> 5, sh = (j * BITS) & 31;
+    w[wi] |= f << sh;
+    if (sh + BITS > 32 && wi + 1 < BITS) w[wi + 1] |= f >> (32 - sh);
+  }
+#pragma unroll
+  for (int i = 0; i < BITS; ++i) out[c * BITS + i] = w[i];
+}
+
+// The rest, and unaligned buffers: one thread writes one output byte, ORing the (at most 5) indices that overlap it.
+__global__ void pack_kernel(const uint8_t* __restrict__ idx, int64_t count, int bits, int64_t first, int64_t n_bytes,
                             uint8_t* __restrict__ out) {
-  const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t b = first + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n_bytes) return;
   const int64_t lo_bit = b * 8, hi_bit = lo_bit + 8;
   const uint32_t mask = (1u << bits) - 1u;
@@ -82,51 +99,103 @@ __global__ void pack_kernel(const uint8_t* __restrict__ idx, int64_t count, int 
 }
 
 // ---- dequant ------------------------------------------------------------------------------
-template <typename T> __device__ __forceinline__ T from_half_bits(uint32_t h16);
-template <> __device__ __forceinline__ __half from_half_bits<__half>(uint32_t h) { return __ushort_as_half((unsigned short)h); }
-template <> __device__ __forceinline__ float from_half_bits<float>(uint32_t h) { return __half2float(__ushort_as_half((unsigned short)h)); }
-template <> __device__ __forceinline__ __nv_bfloat16 from_half_bits<__nv_bfloat16>(uint32_t h) {
-  return __float2bfloat16_rn(__half2float(__ushort_as_half((unsigned short)h)));
+// Fast path (fp16 codebook, block_size % 8 == 0, aligned): a thread dequantises the consecutive weights of ONE 16-byte
+// store, so that a warp's stores are one contiguous run (a thread with 32 weights of its own left every store 64 or 128
+// bytes from its neighbour's: 12.1 us for 6912 x 2560 to fp16 and 34.7 us to fp32, which take 6.7 and 12.2 us at the copy
+// rate).  The 3- or 2-bit fields are spread to the nibbles of one selector word; the block's table, as byte planes, answers
+// four lookups with two byte permutes.  A thread takes kDqPer stores a block stride apart and requests all inputs first.
+constexpr int kDqPer = 4, kDqThreads = 256;
+
+template <int BITS> __device__ __forceinline__ uint32_t load_selectors(const uint32_t* __restrict__ packed, int64_t c) {
+  if (BITS == 4) return packed[c];
+  if (BITS == 2) {
+    uint32_t v = reinterpret_cast<const uint16_t*>(packed)[c];
+    v = (v | (v << 8)) & 0x00FF00FFu;
+    v = (v | (v << 4)) & 0x0F0F0F0Fu;
+    return (v | (v << 2)) & 0x33333333u;
+  }
+  const int64_t bit = c * 24, wi = bit >> 5;
+  const int sh = (int)(bit & 31);                      // 0, 8, 16 or 24
+  const uint32_t lo = packed[wi], hi = sh > 8 ? packed[wi + 1] : 0u;
+  uint32_t v = __funnelshift_r(lo, hi, sh) & 0xFFFFFFu;
+  v = (v & 0xFFFu) | ((v & 0xFFF000u) << 4);           // twelve bits per half word
+  v = (v & 0x003F003Fu) | ((v & 0x0FC00FC0u) << 2);    // six per byte
+  return (v & 0x07070707u) | ((v & 0x38383838u) << 1); // three per nibble
 }
 
-// Fast path (fp16 codebook, block_size % 32 == 0, aligned): one thread dequantises 32
-// consecutive weights of one block.  The 2^BITS entry table lives in registers as a low-byte
-// plane and a high-byte plane; each lookup is two byte-permutes.
+// Four lookups (eight for 16-bit types) as one 16-byte store.
+template <int BITS> __device__ __forceinline__ void store16(__half* dst, uint32_t sel, const uint32_t (&T)[BITS == 4 ? 8 : 4]) {
+  uint32_t h[4];
+  lookup4<BITS>(sel, T, h[0], h[1]);
+  lookup4<BITS>(sel >> 16, T, h[2], h[3]);
+  *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
+}
+template <int BITS> __device__ __forceinline__ void store16(__nv_bfloat16* dst, uint32_t sel, const uint32_t (&T)[BITS == 4 ? 8 : 4]) {
+  uint32_t h[4];
+  lookup4<BITS>(sel, T, h[0], h[1]);
+  lookup4<BITS>(sel >> 16, T, h[2], h[3]);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h[j]));
+    const __nv_bfloat162 b = __floats2bfloat162_rn(f.x, f.y);
+    h[j] = *reinterpret_cast<const uint32_t*>(&b);
+  }
+  *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
+}
+template <int BITS> __device__ __forceinline__ void store16(float* dst, uint32_t sel, const uint32_t (&T)[BITS == 4 ? 8 : 4]) {
+  uint32_t h[2];
+  lookup4<BITS>(sel, T, h[0], h[1]);
+  const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&h[0])), b = __half22float2(*reinterpret_cast<const __half2*>(&h[1]));
+  *reinterpret_cast<float4*>(dst) = make_float4(a.x, a.y, b.x, b.y);
+}
+
 template <int BITS, typename OutT>
-__global__ void dequant32_kernel(const uint32_t* __restrict__ packed, const __half* __restrict__ codebook,
-                                 int64_t n_chunks, int block_size, OutT* __restrict__ out) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n_chunks) return;
-  uint32_t w[BITS];
+__global__ void __launch_bounds__(kDqThreads) dequant16b_kernel(const uint32_t* __restrict__ packed, const __half* __restrict__ codebook,
+                                                              int64_t n_stores, int chunks_per_block, int shift, OutT* __restrict__ out) {
+  constexpr int kT = BITS == 4 ? 8 : 4;
+  constexpr bool kHalves = sizeof(OutT) == 4;          // a store takes half of a chunk of eight
+  const int64_t i0 = (int64_t)blockIdx.x * (kDqThreads * kDqPer) + threadIdx.x;
+  uint32_t sel[kDqPer], e[kDqPer][kT];
 #pragma unroll
-  for (int i = 0; i < BITS; ++i) w[i] = packed[c * BITS + i];
-  const int64_t block = (c * 32) / block_size;
-  uint32_t lo0, lo1, hi0, hi1;
-  if (BITS == 3) {
-    const uint4 e = *reinterpret_cast<const uint4*>(codebook + block * 8);
-    lo0 = prmt(e.x, e.y, 0x6420); lo1 = prmt(e.z, e.w, 0x6420);
-    hi0 = prmt(e.x, e.y, 0x7531); hi1 = prmt(e.z, e.w, 0x7531);
-  } else {
-    const uint2 e = *reinterpret_cast<const uint2*>(codebook + block * 4);
-    lo0 = prmt(e.x, e.y, 0x6420); hi0 = prmt(e.x, e.y, 0x7531);
-    lo1 = 0; hi1 = 0;
+  for (int u = 0; u < kDqPer; ++u) {
+    const int64_t i = i0 + u * kDqThreads, c = kHalves ? i >> 1 : i;
+    sel[u] = 0;
+#pragma unroll
+    for (int j = 0; j < kT; ++j) e[u][j] = 0;
+    if (i < n_stores) {
+      sel[u] = load_selectors<BITS>(packed, c);
+      if (kHalves && (i & 1)) sel[u] >>= 16;
+      const int64_t block = shift >= 0 ? c >> shift : c / chunks_per_block;
+      const uint8_t* row = reinterpret_cast<const uint8_t*>(codebook) + block * (2 << BITS);
+      if (BITS == 2) {
+        const uint2 v = *reinterpret_cast<const uint2*>(row);
+        e[u][0] = v.x; e[u][1] = v.y;
+      } else {
+#pragma unroll
+        for (int j = 0; j < kT / 4; ++j) {
+          const uint4 v = reinterpret_cast<const uint4*>(row)[j];
+          e[u][4 * j] = v.x; e[u][4 * j + 1] = v.y; e[u][4 * j + 2] = v.z; e[u][4 * j + 3] = v.w;
+        }
+      }
+    }
   }
-  alignas(16) OutT v[32];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    const int bit = j * BITS;
-    const int wi = bit >> 5, sh = bit & 31;
-    uint32_t f = w[wi] >> sh;
-    if (sh + BITS > 32 && wi + 1 < BITS) f |= w[wi + 1] << (32 - sh);
-    f &= (1u << BITS) - 1u;
-    const uint32_t h = (prmt(lo0, lo1, f) & 0xFFu) | ((prmt(hi0, hi1, f) & 0xFFu) << 8);
-    v[j] = from_half_bits<OutT>(h);
+  for (int u = 0; u < kDqPer; ++u) {
+    const int64_t i = i0 + u * kDqThreads;
+    if (i >= n_stores) return;
+    uint32_t T[kT];
+    if (BITS == 2) {
+      T[0] = prmt(e[u][0], e[u][1], 0x6420); T[2] = prmt(e[u][0], e[u][1], 0x7531);
+      T[1] = T[2]; T[3] = T[0];
+    } else {
+#pragma unroll
+      for (int j = 0; j < kT; j += 4) {
+        T[j + 0] = prmt(e[u][j], e[u][j + 1], 0x6420); T[j + 1] = prmt(e[u][j + 2], e[u][j + 3], 0x6420);
+        T[j + 2] = prmt(e[u][j], e[u][j + 1], 0x7531); T[j + 3] = prmt(e[u][j + 2], e[u][j + 3], 0x7531);
+      }
+    }
+    store16<BITS>(out + i * (16 / sizeof(OutT)), sel[u], T);
   }
-  // 16-byte stores (out + 32*c is 16-byte aligned for 2- and 4-byte element types)
-  const uint4* src = reinterpret_cast<const uint4*>(v);
-  uint4* dst = reinterpret_cast<uint4*>(out + c * 32);
-#pragma unroll
-  for (int j = 0; j < (int)(32 * sizeof(OutT) / 16); ++j) dst[j] = src[j];
 }
 
 template <typename CbT, typename OutT>
@@ -158,6 +227,106 @@ __global__ void quantize_kernel(const float* __restrict__ w, int64_t total, int6
   idx[i] = (uint8_t)arg;
 }
 
+// The same for four consecutive weights per thread (one block's: block_size % 4 == 0), kQPer runs per thread with all their
+// loads first; with PACK the indices leave as the packed stream, 32 of them gathered by the shuffles of eight lanes.
+// 64-bit index arithmetic and single-byte stores held the general kernel at 92 us for 6912 x 2560 weights; what bounds
+// this one is the argmin itself, three operations of the half-rate pipe per entry and weight (floor 20 us).
+constexpr int kQPer = 4, kQThreads = 256;
+
+template <typename CbT, int NE> __device__ __forceinline__ void load_entries(const CbT* cb, float (&c)[NE]);
+template <> __device__ __forceinline__ void load_entries<float, 4>(const float* cb, float (&c)[4]) {
+  const float4 v = *reinterpret_cast<const float4*>(cb);
+  c[0] = v.x; c[1] = v.y; c[2] = v.z; c[3] = v.w;
+}
+template <> __device__ __forceinline__ void load_entries<float, 8>(const float* cb, float (&c)[8]) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float4 v = reinterpret_cast<const float4*>(cb)[i];
+    c[4 * i] = v.x; c[4 * i + 1] = v.y; c[4 * i + 2] = v.z; c[4 * i + 3] = v.w;
+  }
+}
+template <> __device__ __forceinline__ void load_entries<float, 16>(const float* cb, float (&c)[16]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float4 v = reinterpret_cast<const float4*>(cb)[i];
+    c[4 * i] = v.x; c[4 * i + 1] = v.y; c[4 * i + 2] = v.z; c[4 * i + 3] = v.w;
+  }
+}
+
+template <int BITS, bool PACK>
+__global__ void __launch_bounds__(kQThreads) quantize4_kernel(const float* __restrict__ w, int64_t total, int64_t padded,
+                                                              const float* __restrict__ codebook, int block4, int shift,
+                                                              uint32_t* __restrict__ out) {
+  constexpr int NE = 1 << BITS;
+  const int64_t i0 = (int64_t)blockIdx.x * (kQThreads * kQPer) + threadIdx.x;      // in units of four weights
+  const int lane = threadIdx.x & 31;
+  float v[kQPer][4];
+#pragma unroll
+  for (int u = 0; u < kQPer; ++u) {
+    const int64_t i = i0 + u * kQThreads;
+    if (4 * i + 4 <= total) {
+      const float4 x = reinterpret_cast<const float4*>(w)[i];
+      v[u][0] = x.x; v[u][1] = x.y; v[u][2] = x.z; v[u][3] = x.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[u][j] = 4 * i + j < total ? w[4 * i + j] : 0.f;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kQPer; ++u) {
+    const int64_t i = i0 + u * kQThreads;
+    const bool in = 4 * i < padded;
+    uint32_t arg[4] = {0u, 0u, 0u, 0u};
+    if (in) {
+      float c[NE];
+      load_entries<float, NE>(codebook + (shift >= 0 ? i >> shift : i / block4) * NE, c);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float best = fabsf(v[u][j] - c[0]);
+#pragma unroll
+        for (int e = 1; e < NE; ++e) {
+          const float d = fabsf(v[u][j] - c[e]);
+          if (d < best) { best = d; arg[j] = e; }
+        }
+      }
+    }
+    if (!PACK) {
+      if (in) out[i] = arg[0] | (arg[1] << 8) | (arg[2] << 16) | (arg[3] << 24);
+    } else {
+      // two lanes hold 8 indices = 8 * BITS bits; at 3 bits even lane 2 q < 6 of eight writes word q: bits 32 q .. 32 q + 31 of
+      // the four pairs of 24, which lie in its own pair and the next
+      const uint32_t f = arg[0] | (arg[1] << BITS) | (arg[2] << (2 * BITS)) | (arg[3] << (3 * BITS));
+      const uint32_t pair = f | (__shfl_down_sync(0xffffffffu, f, 1) << (4 * BITS));      // of the even lanes
+      const uint32_t next = __shfl_down_sync(0xffffffffu, pair, 2);
+      const int q = (lane & 7) >> 1;
+      if (!in || (lane & 1)) continue;
+      uint32_t* dst = out + (i >> 3) * BITS;
+      if (BITS == 4) dst[q] = pair;
+      else if (BITS == 2) { if (!(q & 1)) dst[q >> 1] = pair | (next << 16); }
+      else if (q < 3) dst[q] = __funnelshift_r(pair | (next << 24), next >> 8, 8 * q);
+    }
+  }
+}
+
+// Whether the four-wide kernels take these arguments: fp32 entries (the exporter's), 2 to 4 bits, four weights per load
+// and four indices per store (a packed word holds 32 indices of whole blocks).
+static bool quantize4_fits(const float* w, const void* codebook, int cb_dtype, int n_entries, int block_size, const void* out, bool pack) {
+  return cb_dtype == NB_F32 && (n_entries == 4 || n_entries == 8 || n_entries == 16) && block_size % (pack ? 32 : 4) == 0 && (uintptr_t)w % 16 == 0 &&
+         (uintptr_t)codebook % 16 == 0 && (uintptr_t)out % 4 == 0;
+}
+
+template <bool PACK>
+static int launch_quantize4(const float* w, int64_t total, int64_t padded, const float* codebook, int n_entries, int block_size, void* out,
+                            cudaStream_t st) {
+  const int block4 = block_size / 4, shift = (block4 & (block4 - 1)) ? -1 : __builtin_ctz(block4);
+  const unsigned grid = (unsigned)((padded / 4 + kQThreads * kQPer - 1) / (kQThreads * kQPer));
+  uint32_t* o = (uint32_t*)out;
+  if (n_entries == 4) quantize4_kernel<2, PACK><<<grid, kQThreads, 0, st>>>(w, total, padded, codebook, block4, shift, o);
+  else if (n_entries == 8) quantize4_kernel<3, PACK><<<grid, kQThreads, 0, st>>>(w, total, padded, codebook, block4, shift, o);
+  else quantize4_kernel<4, PACK><<<grid, kQThreads, 0, st>>>(w, total, padded, codebook, block4, shift, o);
+  return check_launch();
+}
+
 template <typename OutT>
 static int dequant_dispatch(const uint8_t* packed, const void* codebook, int cb_dtype, int bits, int block_size,
                             int64_t total, OutT* out, cudaStream_t st) {
@@ -165,15 +334,19 @@ static int dequant_dispatch(const uint8_t* packed, const void* codebook, int cb_
   const int64_t n_bytes = packed_bytes(n_blocks * block_size, bits);
   int64_t done = 0;
   const bool aligned = ((uintptr_t)packed % 4 == 0) && ((uintptr_t)out % 16 == 0) && ((uintptr_t)codebook % 16 == 0);
-  if (cb_dtype == NB_F16 && (bits == 2 || bits == 3) && block_size % 32 == 0 && aligned) {
-    const int64_t chunks = total / 32;
+  if (cb_dtype == NB_F16 && block_size % 8 == 0 && aligned) {
+    const int64_t chunks = total / 32 * 4;             // whole packed words
+    const int per_block = block_size / 8;
+    const int shift = (per_block & (per_block - 1)) ? -1 : __builtin_ctz(per_block);
     if (chunks > 0) {
-      const unsigned grid = (unsigned)((chunks + 127) / 128);
-      if (bits == 3)
-        dequant32_kernel<3, OutT><<<grid, 128, 0, st>>>((const uint32_t*)packed, (const __half*)codebook, chunks, block_size, out);
-      else
-        dequant32_kernel<2, OutT><<<grid, 128, 0, st>>>((const uint32_t*)packed, (const __half*)codebook, chunks, block_size, out);
-      done = chunks * 32;
+      const int64_t stores = chunks * 8 / (int64_t)(16 / sizeof(OutT));
+      const unsigned grid = (unsigned)((stores + kDqThreads * kDqPer - 1) / (kDqThreads * kDqPer));
+      const uint32_t* pw = (const uint32_t*)packed;
+      const __half* cb = (const __half*)codebook;
+      if (bits == 3) dequant16b_kernel<3, OutT><<<grid, kDqThreads, 0, st>>>(pw, cb, stores, per_block, shift, out);
+      else if (bits == 2) dequant16b_kernel<2, OutT><<<grid, kDqThreads, 0, st>>>(pw, cb, stores, per_block, shift, out);
+      else dequant16b_kernel<4, OutT><<<grid, kDqThreads, 0, st>>>(pw, cb, stores, per_block, shift, out);
+      done = chunks * 8;
     }
   }
   if (done < total) {
@@ -219,9 +392,19 @@ extern "C" int nb_pack(const uint8_t* idx, int bits, int64_t count, uint8_t* pac
   if (!idx || !packed_out || count < 0 || (bits != 2 && bits != 3 && bits != 4)) return NB_ERR_ARG;
   if (count == 0) return NB_OK;
   if (int rc = check_device()) return rc;
+  cudaStream_t st = (cudaStream_t)stream;
   const int64_t n_bytes = packed_bytes(count, bits);
-  const unsigned grid = (unsigned)((n_bytes + 255) / 256);
-  pack_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(idx, count, bits, n_bytes, packed_out);
+  int64_t done = 0;                                    // bytes
+  if ((uintptr_t)idx % 16 == 0 && (uintptr_t)packed_out % 4 == 0 && count >= 32) {
+    const int64_t chunks = count / 32;
+    const unsigned grid = (unsigned)((chunks + 127) / 128);
+    if (bits == 2) pack32_kernel<2><<<grid, 128, 0, st>>>((const uint4*)idx, chunks, (uint32_t*)packed_out);
+    if (bits == 3) pack32_kernel<3><<<grid, 128, 0, st>>>((const uint4*)idx, chunks, (uint32_t*)packed_out);
+    if (bits == 4) pack32_kernel<4><<<grid, 128, 0, st>>>((const uint4*)idx, chunks, (uint32_t*)packed_out);
+    done = chunks * 4 * bits;
+  }
+  if (done < n_bytes)
+    pack_kernel<<<(unsigned)((n_bytes - done + 255) / 256), 256, 0, st>>>(idx, count, bits, done, n_bytes, packed_out);
   return check_launch();
 }
 
@@ -247,10 +430,21 @@ extern "C" int nb_quantize(const float* w, int64_t total, const void* codebook, 
   if (cb_dtype != NB_F16 && cb_dtype != NB_F32) return NB_ERR_ARG;
   if (int rc = check_device()) return rc;
   const int64_t padded = (total + block_size - 1) / block_size * block_size;
+  if (quantize4_fits(w, codebook, cb_dtype, n_entries, block_size, idx_out, false))
+    return launch_quantize4<false>(w, total, padded, (const float*)codebook, n_entries, block_size, idx_out, (cudaStream_t)stream);
   const unsigned grid = (unsigned)((padded + 255) / 256);
   if (cb_dtype == NB_F16)
     quantize_kernel<__half><<<grid, 256, 0, (cudaStream_t)stream>>>(w, total, padded, (const __half*)codebook, n_entries, block_size, idx_out);
   else
     quantize_kernel<float><<<grid, 256, 0, (cudaStream_t)stream>>>(w, total, padded, (const float*)codebook, n_entries, block_size, idx_out);
   return check_launch();
+}
+
+extern "C" int nb_quantize_pack(const float* w, int64_t total, const void* codebook, int cb_dtype, int bits, int block_size,
+                                uint8_t* packed_out, void* stream) {
+  if (!w || !codebook || !packed_out || total <= 0 || block_size <= 0 || (bits != 2 && bits != 3 && bits != 4)) return NB_ERR_ARG;
+  if (!quantize4_fits(w, codebook, cb_dtype, 1 << bits, block_size, packed_out, true)) return NB_ERR_SHAPE;
+  if (int rc = check_device()) return rc;
+  const int64_t padded = (total + block_size - 1) / block_size * block_size;
+  return launch_quantize4<true>(w, total, padded, (const float*)codebook, 1 << bits, block_size, packed_out, (cudaStream_t)stream);
 }

@@ -81,20 +81,38 @@ def dequant(packed: torch.Tensor, codebook: torch.Tensor, bits: int, block_size:
     return out
 
 
-def quantize(weight: torch.Tensor, codebook: torch.Tensor, block_size: int) -> torch.Tensor:
-    """Nearest-entry indices (num_blocks * block_size,) uint8 of a dense fp32 weight
-    (nativebit/pack.py:176-199, inference/pack.py:21-35)."""
+def _quantize_args(weight: torch.Tensor, codebook: torch.Tensor, block_size: int) -> int:
+    """Checks the arguments of the nearest-entry search; returns the number of codebook blocks."""
     _need_cuda(weight, codebook)
     if weight.dtype != torch.float32 or codebook.dtype not in (torch.float16, torch.float32):
         raise RuntimeError("quantize needs an fp32 weight and an fp16/fp32 codebook")
-    total = weight.numel()
-    nb, ne = codebook.shape
-    if nb != (total + block_size - 1) // block_size:
-        raise RuntimeError(f"codebook has {nb} blocks, the weight needs {(total + block_size - 1) // block_size}")
+    nb = codebook.shape[0]
+    if nb != (weight.numel() + block_size - 1) // block_size:
+        raise RuntimeError(f"codebook has {nb} blocks, the weight needs {(weight.numel() + block_size - 1) // block_size}")
+    return nb
+
+
+def quantize(weight: torch.Tensor, codebook: torch.Tensor, block_size: int) -> torch.Tensor:
+    """Nearest-entry indices (num_blocks * block_size,) uint8 of a dense fp32 weight
+    (nativebit/pack.py:176-199, inference/pack.py:21-35)."""
+    nb = _quantize_args(weight, codebook, block_size)
     out = torch.empty(nb * block_size, dtype=torch.uint8, device=weight.device)
     with torch.cuda.device(weight.device):
-        _lib.check(_lib.lib().nb_quantize(weight.data_ptr(), total, codebook.data_ptr(), _DTYPE[codebook.dtype], ne, block_size,
-                                          out.data_ptr(), _stream()), "nb_quantize")
+        _lib.check(_lib.lib().nb_quantize(weight.data_ptr(), weight.numel(), codebook.data_ptr(), _DTYPE[codebook.dtype], codebook.shape[1],
+                                          block_size, out.data_ptr(), _stream()), "nb_quantize")
+    return out
+
+
+def quantize_pack(weight: torch.Tensor, codebook: torch.Tensor, block_size: int, bits: int) -> torch.Tensor:
+    """pack(quantize(weight, codebook, block_size), bits); one kernel where it takes the arguments (nb_quantize_pack)."""
+    nb = _quantize_args(weight, codebook, block_size)
+    if (block_size % 32 or codebook.dtype != torch.float32 or codebook.shape[1] != 1 << bits or weight.data_ptr() % 16
+            or codebook.data_ptr() % 16):
+        return pack(quantize(weight, codebook, block_size), bits)
+    out = torch.empty(packed_nbytes(nb * block_size, bits), dtype=torch.uint8, device=weight.device)
+    with torch.cuda.device(weight.device):
+        _lib.check(_lib.lib().nb_quantize_pack(weight.data_ptr(), weight.numel(), codebook.data_ptr(), _DTYPE[codebook.dtype], bits,
+                                               block_size, out.data_ptr(), _stream()), "nb_quantize_pack")
     return out
 
 

@@ -73,8 +73,8 @@ def pack_linear(weight: torch.Tensor, codebook: torch.Tensor, block_size: int = 
     bits = max(1, (codebook.shape[1] - 1).bit_length())
     if bits not in (2, 3, 4):
         raise RuntimeError(f"codebooks of {codebook.shape[1]} entries are not supported")
-    idx = _compute_indices(weight, codebook, block_size, weight.numel())
-    return PackedLinear(ops.pack(idx, bits), codebook.half().contiguous(), weight.shape[0], weight.shape[1], bits=bits,
+    packed = ops.quantize_pack(weight.contiguous().float(), codebook.contiguous(), block_size, bits)
+    return PackedLinear(packed, codebook.half().contiguous(), weight.shape[0], weight.shape[1], bits=bits,
                         block_size=block_size)
 
 

@@ -365,3 +365,32 @@ def test_quantize_matches_reference_argmin(dev, golden):
     idx2 = ops.quantize(w2, cb2, 8).cpu().numpy()
     ref2 = np.abs(np.pad(w2.cpu().numpy(), (0, 6))[:, None] - cb2.cpu().numpy()[0][None, :]).argmin(1)
     assert np.array_equal(idx2, ref2)
+
+
+@pytest.mark.parametrize("bits", [2, 3, 4])
+@pytest.mark.parametrize("total,block", [(1, 32), (31, 32), (32, 32), (127, 128), (4096, 96), (4101, 128), (70_003, 64), (40_000, 8), (1003, 12)])
+def test_quantize_pack_dequant_edges_of_the_wide_kernels(dev, bits, total, block):
+    """The four-, eight- and 32-wide kernels against the oracle's argmin and the reference's byte layout: padded last
+    blocks, ties, blocks that are no power of two, counts that are no multiple of a word, unaligned buffers."""
+    from nativebit_b200 import ops
+    rng = np.random.default_rng(total * 8 + bits)
+    blocks = -(-total // block)
+    cb = np.sort(rng.standard_normal((blocks, 1 << bits)).astype(np.float32), axis=1)
+    cb[::3, 1] = cb[::3, 0]                                        # ties go to the first entry
+    w = rng.standard_normal(total).astype(np.float32)
+    padded = np.zeros(blocks * block, np.float32)
+    padded[:total] = w
+    ref = np.abs(padded.reshape(blocks, block, 1) - cb[:, None, :]).argmin(-1).astype(np.uint8).reshape(-1)
+    wd, cd = _cu(w, dev), _cu(cb, dev)
+    idx = ops.quantize(wd, cd, block)
+    assert np.array_equal(idx.cpu().numpy(), ref)
+    packed = ops.quantize_pack(wd, cd, block, bits)
+    off = torch.zeros(ref.size + 1, dtype=torch.uint8, device=dev)
+    off[1:] = idx
+    general = ops.pack(off[1:], bits)                              # an unaligned source takes the byte kernel
+    assert torch.equal(ops.pack(idx, bits), general) and torch.equal(packed, general)
+    assert torch.equal(ops.unpack(packed, bits, ref.size), idx)
+    half = cd.half()
+    want = torch.gather(half, 1, torch.from_numpy(ref.astype(np.int64)).to(dev).view(blocks, block)).view(-1)[:total].view(1, total)
+    for dtype in (torch.float16, torch.bfloat16, torch.float32):
+        assert torch.equal(ops.dequant(packed, half, bits, block, (1, total), dtype), want.to(dtype))
