@@ -10,6 +10,7 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <type_traits>
 
 #include "nb_common.cuh"
 #include "nb_host.h"
@@ -297,150 +298,240 @@ static int launch_attention(int B, int H, int hd, int ctx, cudaStream_t st, Args
   return record_cuda_error(cudaLaunchKernelEx(&cfg, decode_attention_kernel, args...));
 }
 
-// Causal attention of a prompt (or a chunk of one that continues a cache of pos0 keys) in ONE launch per layer:
-// RoPE on q and k, cache write, softmax(q k^T / sqrt(hd)) v over keys 0 .. pos0 + t for query t
-// (inference/generate_torch.py:41-60 RoPE, :86-97 cache write and masked attention).  grid (ceil(T / 16), H, B):
-// a CTA owns 16 queries of one head; it walks the keys in chunks of 32, staging a chunk of K and V in shared
-// memory — from the cache below pos0, from qkv (rotating k on the way) from pos0 on, so no CTA reads what
-// another one writes in this launch — and keeps a running maximum, denominator and numerator per query.  The
-// CTA whose queries sit at positions [q0, q0 + 16) is the one that writes those positions' k and v to the cache.
-// Eight threads share a query: for the scores each takes every eighth key of the chunk, for the values four head
-// dimensions out of every 32.  Everything is fp32.  head_dim a multiple of 4, <= 128.
-constexpr int kPQ = 16, kPK = 32, kPThreads = 128;
+// The pairs (x, y) and (z, w) turned by their angles.
+__device__ __forceinline__ float4 turn_pairs(float4 x, float2 c, float2 s) {
+  return make_float4(x.x * c.x - x.y * s.x, x.y * c.x + x.x * s.x, x.z * c.y - x.w * s.y, x.w * c.y + x.z * s.y);
+}
 
-__global__ void __launch_bounds__(kPThreads) prefill_attention_kernel(
-    const float* __restrict__ qkv, const float* __restrict__ cos2, const float* __restrict__ sin2, float* __restrict__ k_cache,
-    float* __restrict__ v_cache, float* __restrict__ out, int T, int H, int hd, int ctx, int pos0, int out_stride, int out_offset,
+// Causal attention of a prompt (or a chunk of one that continues a cache of pos0 keys), two launches per layer: the first
+// rotates the chunk's keys into the cache and copies its values there, the second is softmax(q k^T / sqrt(hd)) v over the
+// cached keys 0 .. pos0 + t for query t (inference/generate_torch.py:41-60 RoPE, :86-97 cache write and masked attention).
+// (Rotating the keys wherever they are read needs one launch, but every CTA then waits for its loads: 381 us against the
+// 337 us of both launches, 8 sequences of 512 tokens, 32 heads of 80.)
+__global__ void __launch_bounds__(256) prompt_keys_kernel(const float* __restrict__ qkv, const float* __restrict__ cos2,
+                                                          const float* __restrict__ sin2, float* __restrict__ k_cache,
+                                                          float* __restrict__ v_cache, int T, int H, int hd, int ctx, int pos0) {
+  const int t = blockIdx.x, b = blockIdx.y, quarter = hd >> 2;
+  const float* row = qkv + (size_t)(b * T + t) * 3 * H * hd + H * hd;
+  for (int i = threadIdx.x; i < H * quarter; i += 256) {
+    const int h = i / quarter, d = (i - h * quarter) * 4;
+    const float4 k = *reinterpret_cast<const float4*>(row + 4 * i), v = *reinterpret_cast<const float4*>(row + H * hd + 4 * i);
+    const size_t ri = (size_t)(pos0 + t) * hd + d, at = ((size_t)b * H + h) * (size_t)ctx * hd + ri;
+    *reinterpret_cast<float4*>(k_cache + at) = turn_pairs(k, make_float2(cos2[ri], cos2[ri + 2]), make_float2(sin2[ri], sin2[ri + 2]));
+    *reinterpret_cast<float4*>(v_cache + at) = v;
+  }
+}
+
+// grid (H, B, ceil(T / BQ)): a CTA owns BQ = 8 R queries of one head (all heads' longest rows first); it walks the cached keys
+// in chunks of PK staged in shared memory by asynchronous copies — a chunk's values arrive while its scores are formed, the
+// next chunk's keys while the values are added — and keeps a running maximum, denominator and numerator per query.
+//
+// Everything is fp32 multiply-adds, so the floor is the fp32 pipe (74 TFLOP/s); what decides is how many operands a
+// multiply-add costs.  Scores: a thread owns R queries x PK / 16 keys, and every 16-byte load feeds packed two-wide
+// multiply-adds along the head dimension (12 loads per 64 of them at R = 8).  Values: the same thread owns its R queries x
+// 2 * NP head dimensions (pairs 16 apart) for every second four keys — eight lanes of a half-warp take the even fours, eight
+// the odd ones, and the halves meet once at the end — so the weights cross shared memory inside a half-warp only.
+// head_dim a multiple of 4, <= 128; NP pairs per thread cover 16 * NP >= head_dim.  Two CTAs share an SM: PK is 64 where
+// their tiles fit, else 32.
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+
+__device__ __forceinline__ void copy16_or_zero(float* dst, const float* src, bool there) {   // asynchronous, global -> shared
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
+
+template <int R, int PK, int NP>
+__global__ void __launch_bounds__(128, 2) prefill_attention_kernel(
+    const float* __restrict__ qkv, const float* __restrict__ cos2, const float* __restrict__ sin2, const float* __restrict__ k_cache,
+    const float* __restrict__ v_cache, float* __restrict__ out, int T, int H, int hd, int ctx, int pos0, int out_stride, int out_offset,
     float scale) {
+  constexpr int NT = 128, BQ = 8 * R, KI = PK / 16, kPStride = PK + 4;
   extern __shared__ __align__(16) float psm[];
   const int hdp = hd + 4;                       // row stride: 16-byte aligned, eight consecutive rows on different banks
-  float* q_s = psm;                             // [kPQ][hdp]
-  float* k_s = q_s + kPQ * hdp;                 // [kPK][hdp]
-  float* v_s = k_s + kPK * hdp;                 // [kPK][hdp]
-  float* p_s = v_s + kPK * hdp;                 // [kPQ][kPK + 1]
-  const int tid = threadIdx.x, q0 = blockIdx.x * kPQ, h = blockIdx.y, b = blockIdx.z;
-  const int row3 = 3 * H * hd, half = hd >> 1, quarter = hd >> 2;
+  float* q_s = psm;                             // [BQ][hdp]
+  float* k_s = q_s + BQ * hdp;                  // [PK][hdp]
+  float* v_s = k_s + PK * hdp;                  // [PK][hdp], and 2 * 16 floats that the last row's spare pairs read
+  float* p_s = v_s + PK * hdp + 32;             // [BQ][kPStride]
+  const int tid = threadIdx.x, h = blockIdx.x, b = blockIdx.y, q0 = ((int)gridDim.z - 1 - (int)blockIdx.z) * BQ;
+  const int row3 = 3 * H * hd, quarter = hd >> 2, rcp = 65536 / quarter + 1;      // i / quarter = i * rcp >> 16 for i < 2048
   const size_t cbase = ((size_t)b * H + h) * (size_t)ctx * hd;
-
   // this tile's queries, rotated (rows past the prompt's end repeat its last query and are not written)
-  for (int i = tid; i < kPQ * half; i += kPThreads) {
-    const int r = i / half, d = (i - r * half) * 2;
-    const int t = min(q0 + r, T - 1);
-    const float2 x = *reinterpret_cast<const float2*>(qkv + (size_t)(b * T + t) * row3 + h * hd + d);
+#pragma unroll 2
+  for (int i = tid; i < BQ * quarter; i += NT) {
+    const int r = (i * rcp) >> 16, d = (i - r * quarter) * 4, t = min(q0 + r, T - 1);
     const size_t ri = (size_t)(pos0 + t) * hd + d;
-    const float c = cos2[ri], s = sin2[ri];
-    q_s[r * hdp + d] = x.x * c - x.y * s;
-    q_s[r * hdp + d + 1] = x.y * c + x.x * s;
+    *reinterpret_cast<float4*>(q_s + r * hdp + d) = turn_pairs(*reinterpret_cast<const float4*>(qkv + (size_t)(b * T + t) * row3 + h * hd + d),
+                                                               make_float2(cos2[ri], cos2[ri + 2]), make_float2(sin2[ri], sin2[ri + 2]));
   }
 
-  const int qi = tid >> 3, sub = tid & 7;
-  const int my_pos = pos0 + min(q0 + qi, T - 1);
-  const int kmax = pos0 + min(q0 + kPQ - 1, T - 1);      // last key any query of this tile may see
-  float m = -INFINITY, l = 0.f;
-  float4 acc[4];
+  const int ty = tid >> 4, tx = tid & 15;       // scores: queries R ty .. + R - 1, keys tx + 16 i
+  const int upper = (tid >> 3) & 1, tx2 = tid & 7;      // values: the same queries, one half of the keys, dimensions 2 tx2 + 16 i and the next
+  const int kmax = pos0 + min(q0 + BQ - 1, T - 1);      // last key any query of this tile may see
+  float m[R], l[R];
+  unsigned long long acc[R][NP];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int r = 0; r < R; ++r) {
+    m[r] = -INFINITY;
+    l[r] = 0.f;
+#pragma unroll
+    for (int i = 0; i < NP; ++i) acc[r][i] = 0ull;
+  }
 
-  for (int kc = 0; kc <= kmax; kc += kPK) {
-    for (int i = tid; i < kPK * half; i += kPThreads) {
-      const int j = i / half, d = (i - j * half) * 2, p = kc + j;
-      float2 r = make_float2(0.f, 0.f);
-      if (p <= kmax) {
-        if (p < pos0) {
-          r = *reinterpret_cast<const float2*>(k_cache + cbase + (size_t)p * hd + d);
-        } else {
-          const int t = p - pos0;
-          const float2 x = *reinterpret_cast<const float2*>(qkv + (size_t)(b * T + t) * row3 + (H + h) * hd + d);
-          const size_t ri = (size_t)p * hd + d;
-          const float c = cos2[ri], s = sin2[ri];
-          r.x = x.x * c - x.y * s;
-          r.y = x.y * c + x.x * s;
-          if (t >= q0) *reinterpret_cast<float2*>(k_cache + cbase + (size_t)p * hd + d) = r;
-        }
-      }
-      k_s[j * hdp + d] = r.x;
-      k_s[j * hdp + d + 1] = r.y;
+  auto stage = [&](float* dst, const float* cache, int kc) {       // keys or values kc .. kc + PK - 1, zeros past kmax
+    const float* src = cache + cbase + (size_t)kc * hd;
+    const int there = (kmax - kc + 1) * quarter;
+    for (int i = tid; i < PK * quarter; i += NT) {
+      const int j = (i * rcp) >> 16;
+      copy16_or_zero(dst + i * 4 + j * 4, src + (i < there ? i * 4 : 0), i < there);
     }
-    for (int i = tid; i < kPK * quarter; i += kPThreads) {
-      const int j = i / quarter, d = (i - j * quarter) * 4, p = kc + j;
-      float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (p <= kmax) {
-        if (p < pos0) {
-          r = *reinterpret_cast<const float4*>(v_cache + cbase + (size_t)p * hd + d);
-        } else {
-          const int t = p - pos0;
-          r = *reinterpret_cast<const float4*>(qkv + (size_t)(b * T + t) * row3 + (2 * H + h) * hd + d);
-          if (t >= q0) *reinterpret_cast<float4*>(v_cache + cbase + (size_t)p * hd + d) = r;
-        }
-      }
-      *reinterpret_cast<float4*>(v_s + j * hdp + d) = r;
-    }
-    __syncthreads();
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  stage(k_s, k_cache, 0);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  stage(v_s, v_cache, 0);
 
-    // scores of keys sub, sub + 8, sub + 16, sub + 24 of the chunk against query qi
-    float sc[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int kc = 0; kc <= kmax; kc += PK) {
+    float s[R][KI];
     {
-      const float4* qr = reinterpret_cast<const float4*>(q_s + qi * hdp);
-      const float4* kr = reinterpret_cast<const float4*>(k_s + sub * hdp);
-      const int kstep = 8 * hdp / 4;
-      for (int d4 = 0; d4 < quarter; ++d4) {
-        const float4 x = qr[d4];
+      unsigned long long sum[R][KI];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 y = kr[i * kstep + d4];
-          sc[i] += x.x * y.x + x.y * y.y + x.z * y.z + x.w * y.w;
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int i = 0; i < KI; ++i) sum[r][i] = 0ull;
+      const float* qr = q_s + ty * R * hdp;
+      const float* kr = k_s + tx * hdp;
+#pragma unroll 1
+      for (int d = 0; d < hd; d += 4) {
+        ulonglong2 y[KI];
+#pragma unroll
+        for (int i = 0; i < KI; ++i) y[i] = *reinterpret_cast<const ulonglong2*>(kr + 16 * i * hdp + d);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(qr + r * hdp + d);
+#pragma unroll
+          for (int i = 0; i < KI; ++i) { fma2(sum[r][i], x.x, y[i].x); fma2(sum[r][i], x.y, y[i].y); }
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int i = 0; i < KI; ++i) {
+          const float2 e = unpack2(sum[r][i]);
+          s[r][i] = (e.x + e.y) * scale;
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                            // this chunk's values are here, and nobody reads its keys any more
+    if (kc + PK <= kmax) stage(k_s, k_cache, kc + PK);
+    if (kc + PK - 1 > pos0 + q0) {              // some query of the tile does not see all keys of the chunk
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int my_pos = pos0 + min(q0 + R * ty + r, T - 1);
+#pragma unroll
+        for (int i = 0; i < KI; ++i)
+          if (kc + tx + 16 * i > my_pos) s[r][i] = -INFINITY;
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      float cm = s[r][0];
+#pragma unroll
+      for (int i = 1; i < KI; ++i) cm = fmaxf(cm, s[r][i]);
+#pragma unroll
+      for (int o = 1; o < 16; o <<= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
+      const float m_new = fmaxf(m[r], cm);      // finite from the first chunk on: key 0 is visible to every query
+      const float corr = expf(m[r] - m_new);
+      m[r] = m_new;
+      float ps = 0.f;
+#pragma unroll
+      for (int i = 0; i < KI; ++i) {
+        const float e = expf(s[r][i] - m_new);
+        p_s[(R * ty + r) * kPStride + tx + 16 * i] = e;
+        ps += e;
+      }
+      l[r] = l[r] * corr + ps;                  // this thread's keys; the sixteen parts meet at the end
+      const unsigned long long c2 = pack2(corr, corr);
+#pragma unroll
+      for (int i = 0; i < NP; ++i) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[r][i]) : "l"(c2));
+    }
+    __syncwarp();                               // the sixteen threads of a query are lanes of one warp
+    const float* pr = p_s + R * ty * kPStride;
+    const float* vr = v_s + 2 * tx2;
+    const int jn = min(PK, kmax - kc + 1);      // the weights past it are zero
+#pragma unroll 1
+    for (int j = upper * 4; j < jn; j += 8) {
+      float4 w[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) w[r] = *reinterpret_cast<const float4*>(pr + r * kPStride + j);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        unsigned long long y[NP];
+#pragma unroll
+        for (int i = 0; i < NP; ++i) y[i] = *reinterpret_cast<const unsigned long long*>(vr + (j + e) * hdp + 16 * i);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float x = e == 0 ? w[r].x : e == 1 ? w[r].y : e == 2 ? w[r].z : w[r].w;
+          const unsigned long long x2 = pack2(x, x);
+#pragma unroll
+          for (int i = 0; i < NP; ++i) fma2(acc[r][i], x2, y[i]);
         }
       }
     }
-    float cm = -INFINITY;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                            // the next chunk's keys are here, and nobody reads these values any more
+    if (kc + PK <= kmax) stage(v_s, v_cache, kc + PK);
+  }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      sc[i] = (kc + sub + 8 * i <= my_pos) ? sc[i] * scale : -INFINITY;
-      cm = fmaxf(cm, sc[i]);
+  for (int r = 0; r < R; ++r) {
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) l[r] += __shfl_xor_sync(0xffffffffu, l[r], o);
+    const float inv = 1.f / l[r];
+    const int t = q0 + R * ty + r;
+    float* o = out + (size_t)(b * T + t) * out_stride + out_offset + h * hd + 2 * tx2;
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {              // the two halves of the keys
+      float2 v = unpack2(acc[r][i]);
+      v.x += __shfl_xor_sync(0xffffffffu, v.x, 8);
+      v.y += __shfl_xor_sync(0xffffffffu, v.y, 8);
+      if (t < T && upper == (r & 1) && 2 * tx2 + 16 * i < hd) *reinterpret_cast<float2*>(o + 16 * i) = make_float2(v.x * inv, v.y * inv);
     }
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
-    const float m_new = fmaxf(m, cm);           // finite from the first chunk on: key 0 is visible to every query
-    const float corr = expf(m - m_new);
-    float ps = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float pr = expf(sc[i] - m_new);
-      p_s[qi * (kPK + 1) + sub + 8 * i] = pr;
-      ps += pr;
-    }
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) ps += __shfl_xor_sync(0xffffffffu, ps, o);
-    l = l * corr + ps;
-    m = m_new;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { acc[i].x *= corr; acc[i].y *= corr; acc[i].z *= corr; acc[i].w *= corr; }
-    __syncwarp();                               // the eight threads of a query are lanes of one warp
+  }
+}
 
-    // numerator: head dimensions sub*4 + 32*i of query qi
-    const float* pr = p_s + qi * (kPK + 1);
-#pragma unroll 4
-    for (int j = 0; j < kPK; ++j) {
-      const float w = pr[j];
-      const float* vr = v_s + j * hdp + sub * 4;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (sub * 4 + 32 * i < hd) {
-          const float4 v = *reinterpret_cast<const float4*>(vr + 32 * i);
-          acc[i].x += w * v.x; acc[i].y += w * v.y; acc[i].z += w * v.z; acc[i].w += w * v.w;
-        }
-      }
-    }
-    __syncthreads();                            // before the next chunk overwrites K, V and the weights
+template <int R, int NP, typename... Args>
+static int launch_prefill_attention(int B, int T, int H, int hd, cudaStream_t st, Args... args) {
+  constexpr int BQ = 8 * R, PK = NP > 5 && R == 8 ? 32 : 64;
+  const size_t smem = (size_t)((BQ + 2 * PK) * (hd + 4) + 32 + BQ * (PK + 4)) * sizeof(float);      // <= 95 KB
+  static bool attr_done[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!attr_done[dev & 63]) {
+    if (cudaError_t e = cudaFuncSetAttribute(prefill_attention_kernel<R, PK, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024))
+      return record_cuda_error(e);
+    attr_done[dev & 63] = true;
   }
-  if (q0 + qi < T) {
-    const float inv = 1.f / l;
-    float* o = out + (size_t)(b * T + q0 + qi) * out_stride + out_offset + h * hd + sub * 4;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (sub * 4 + 32 * i < hd)
-        *reinterpret_cast<float4*>(o + 32 * i) = make_float4(acc[i].x * inv, acc[i].y * inv, acc[i].z * inv, acc[i].w * inv);
-  }
+  prefill_attention_kernel<R, PK, NP><<<dim3(H, B, (T + BQ - 1) / BQ), 128, smem, st>>>(args...);
+  return record_cuda_error(cudaGetLastError());
+}
+
+// Tiles of 64 queries stage every key half as often as tiles of 32; short or few prompts take the latter, which puts
+// twice as many SMs to work on them.
+template <int NP, typename... Args>
+static int prefill_attention_tile(int B, int T, int H, int hd, cudaStream_t st, Args... args) {
+  if ((long long)B * H * ((T + 63) / 64) < 2 * sm_count()) return launch_prefill_attention<4, NP>(B, T, H, hd, st, args...);
+  return launch_prefill_attention<8, NP>(B, T, H, hd, st, args...);
 }
 
 // The tied LM head of one sequence as a matvec over the bf16 embedding table, with the final residual add + RMSNorm
@@ -747,11 +838,17 @@ extern "C" int nb_prefill_attention(const float* qkv, int B, int T, int H, int h
     return NB_ERR_ALIGN;
   if (H > 65535 || B > 65535) return NB_ERR_SHAPE;
   if (int rc = check_device()) return rc;
-  const int hdp = hd + 4;
-  const size_t smem = (size_t)((kPQ + 2 * kPK) * hdp + kPQ * (kPK + 1)) * sizeof(float);      // <= 44 KB
-  prefill_attention_kernel<<<dim3((T + kPQ - 1) / kPQ, H, B), kPThreads, smem, (cudaStream_t)stream>>>(
-      qkv, cos2, sin2, k_cache, v_cache, out, T, H, hd, ctx, pos0, out_stride, out_offset, 1.0f / sqrtf((float)hd));
-  return record_cuda_error(cudaGetLastError());
+  const float scale = 1.0f / sqrtf((float)hd);
+  prompt_keys_kernel<<<dim3(T, B), 256, 0, (cudaStream_t)stream>>>(qkv, cos2, sin2, k_cache, v_cache, T, H, hd, ctx, pos0);
+  if (int rc = check_launch()) return rc;
+  auto run = [&](auto pairs) {
+    return prefill_attention_tile<decltype(pairs)::value>(B, T, H, hd, (cudaStream_t)stream, qkv, cos2, sin2, (const float*)k_cache,
+                                                          (const float*)v_cache, out, T, H, hd, ctx, pos0, out_stride, out_offset, scale);
+  };
+  if (hd <= 32) return run(std::integral_constant<int, 2>{});
+  if (hd <= 64) return run(std::integral_constant<int, 4>{});
+  if (hd <= 80) return run(std::integral_constant<int, 5>{});
+  return run(std::integral_constant<int, 8>{});
 }
 
 extern "C" size_t nb_lm_head_scratch_bytes(void) { return (size_t)kHeadMaxCtas * 8; }

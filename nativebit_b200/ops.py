@@ -433,7 +433,7 @@ def decode_attention_rope(qkv, cos2, sin2, pos, k_cache, v_cache, out, out_offse
 
 def prefill_attention(qkv: torch.Tensor, T: int, cos2, sin2, pos0: int, k_cache, v_cache, out: torch.Tensor,
                       out_offset: int = 0) -> None:
-    """RoPE + cache write + causal attention of a T-token prompt chunk per sequence in one launch.
+    """RoPE + cache write + causal attention of a T-token prompt chunk per sequence.
     qkv (B*T, 3*H*hd) fp32 contiguous; caches (B, H, ctx, hd) fp32; out (B*T, >= out_offset + H*hd) fp32."""
     b, h, ctx, hd = k_cache.shape
     for t in (qkv, k_cache, v_cache, out, cos2, sin2):
