@@ -58,6 +58,17 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
                ::"r"(s2u(dst)), "l"(map), "r"(s2u(bar)), "r"(x), "r"(y) : "memory");
 }
 
+// True in one lane of a converged warp.  The roles that issue MMAs and copies are entered through this and not through
+// `lane == 0`: behind elect.sync the compiler knows that a single lane is active and needs no detour to bring descriptors
+// and addresses into uniform registers.  Entered by lane number, every tcgen05.mma cost its issuing thread 54 - 86 clocks, and
+// a k-step of the pair's 256 x 256 x 64 tile (0.27 us of tensor time) up to 0.43 us (8192 x 2560 x 6912: 299 us, 201 us entered
+// this way).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r != 0;
+}
+
 // Shared-memory matrix descriptor of a K-major tile with 128-byte swizzle: rows of 128 bytes, groups
 // of 8 rows 1024 bytes apart (stride byte offset), descriptor version 1, layout type SWIZZLE_128B.
 __device__ __forceinline__ uint64_t smem_desc_sw128(const void* p) {

@@ -134,3 +134,28 @@ def test_dequant_then_gemm_with_fp32_activations(built_lib, m, n, k):
     assert ops.prefill_status(dev) == 0
     assert (y.double() - ref).abs().max() <= 2e-5 * ref.abs().max()
     assert yl.dtype == torch.float32 and (yl.double() - ref).abs().max() <= 2e-5 * ref.abs().max()
+
+
+@pytest.mark.parametrize("m,n,k", [(127, 33, 64), (129, 100, 64), (257, 264, 192), (640, 1031, 448), (2305, 130, 128), (4200, 777, 128)])
+def test_gemm_tiles_at_the_edges(built_lib, m, n, k):
+    """The plain tensor-core kernel alone and in pairs of CTAs: rows and columns one past a tile, more row tiles than a group,
+    odd widths that cannot be stored sixteen bytes at a time, and the two terms of fp32 activations side by side."""
+    from nativebit_b200 import ops
+    dev = _dev()
+    g = torch.Generator(device=dev).manual_seed(m + n + k)
+    x = torch.randn(m, k, device=dev, generator=g)
+    w = (torch.randn(n, k, device=dev, generator=g) * 0.05).bfloat16()
+    xb = x.bfloat16()
+    ref = xb.double() @ w.double().T
+    for out_dtype, tol in ((torch.float32, 2e-5), (torch.bfloat16, 2.0 ** -8)):                # bf16 output: half an ulp
+        y = ops.gemm_bf16(xb, w, out_dtype=out_dtype)
+        torch.cuda.synchronize()
+        assert (y.double() - ref).abs().max() <= tol * ref.abs().max()
+    if k % 128 == 0:
+        packed, cb, _ = o.make_packed_linear(n, k, 3, seed=m)
+        W = torch.from_numpy(o.dequant_packed(packed, cb.astype(np.float32), n, k, 3)).to(dev)
+        y = ops.gemm_prefill(x, torch.from_numpy(packed).to(dev), torch.from_numpy(cb).to(dev), 3, 128, n, k, out_dtype=torch.float32)
+        torch.cuda.synchronize()
+        ref = x.double() @ W.double().T
+        assert (y.double() - ref).abs().max() <= 2e-5 * ref.abs().max()
+    assert ops.prefill_status(dev) == 0
