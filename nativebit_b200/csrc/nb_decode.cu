@@ -13,6 +13,7 @@
 #include <type_traits>
 
 #include "nb_common.cuh"
+#include "nb_device.cuh"
 #include "nb_host.h"
 #include "nb_launch.cuh"
 #include "../../include/nativebit_b200_layered.h"
@@ -270,6 +271,157 @@ __global__ void __launch_bounds__(kAttnWarps * 32) decode_attention_kernel(
   cluster.sync();  // the exchange buffers stay alive until rank 0 has read them
 }
 
+// The same with one CTA per (head, batch), for calls whose heads alone fill the GPU (taken where the kernel above would split
+// a head over one or two CTAs; where it splits over four or eight, splitting wins).  Bound by the bytes of the cached
+// keys and values.  A warp takes eight keys at a time, every fourth such chunk: its keys and values travel through the warp's
+// own ring of asynchronous copies (two chunks ahead, no registers held), and scores, running maximum, denominator and numerator
+// stay in the warp until one merge at the end, so no barrier separates the scores from the values.  The row this step writes
+// never comes from the cache: warp 0 starts from it.  A decode step of the 2.2B model at 512 keys, per layer: 8 sequences
+// 92 -> 81 us, 32 sequences of 100 keys 113 -> 108 us.
+constexpr int kWideWarps = 4, kWideKeys = 8, kWideD = 3;
+static size_t wide_smem_floats(int hd) { return (size_t)kWideWarps * kWideD * 2 * kWideKeys * hd + (size_t)(3 + kWideWarps) * hd; }
+
+__global__ void __launch_bounds__(kWideWarps * 32) decode_attention_wide_kernel(
+    const float* __restrict__ q, float* k_cache, float* v_cache, const long long* __restrict__ pos_ptr, float* __restrict__ out,
+    int H, int hd, int ctx, int out_stride, int out_offset, const float* __restrict__ qkv, const float* __restrict__ cos2,
+    const float* __restrict__ sin2) {
+  extern __shared__ __align__(16) float sm[];  // per warp kWideD stages of keys | values, then q | key | value of this step | outputs
+  __shared__ float s_m[kWideWarps], s_l[kWideWarps];
+  const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  asm volatile("griddepcontrol.launch_dependents;");
+  // as above: position and older rows do not depend on the launch before this one
+  long long pos = *pos_ptr;
+  if (pos < 0) return;
+  if (pos >= ctx) pos = ctx - 1;
+  const int n = (int)pos, hd4 = hd >> 2, n_chunks = (n + kWideKeys - 1) / kWideKeys;
+  const size_t head = (size_t)b * H + h;
+  float* kb = k_cache + head * ctx * hd;
+  float* vb = v_cache + head * ctx * hd;
+  const int half = kWideKeys * hd, stage_floats = 2 * half;
+  float* ring = sm + warp * kWideD * stage_floats;
+  float* qs = sm + kWideWarps * kWideD * stage_floats;
+  float *ks = qs + hd, *vs = ks + hd, *part = vs + hd;
+  int rq = warp, rq_stage = 0;
+  auto request = [&]() {      // the warp's next chunk, a contiguous span of each cache
+    if (rq < n_chunks) {
+      const int k0 = rq * kWideKeys, n4 = min(kWideKeys, n - k0) * hd4;
+      float4* dst = reinterpret_cast<float4*>(ring + rq_stage * stage_floats);
+      const float4* ksrc = reinterpret_cast<const float4*>(kb + (size_t)k0 * hd);
+      const float4* vsrc = reinterpret_cast<const float4*>(vb + (size_t)k0 * hd);
+      for (int i = lane; i < n4; i += 32) cp_async16(dst + i, ksrc + i);
+      for (int i = lane; i < n4; i += 32) cp_async16(dst + kWideKeys * hd4 + i, vsrc + i);
+      rq += kWideWarps;
+    }
+    if (++rq_stage == kWideD) rq_stage = 0;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll 1
+  for (int i = 0; i < kWideD - 1; ++i) request();
+  float c_pre = 0.f, s_pre = 0.f;
+  if (qkv && tid < hd) { c_pre = cos2[pos * hd + tid]; s_pre = sin2[pos * hd + tid]; }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (tid < hd) {             // head_dim <= 128 threads
+    if (qkv) {
+      const float* qh = qkv + (size_t)b * 3 * H * hd + h * hd;
+      const float* kh = qh + H * hd;
+      const int j = tid ^ 1;
+      const float sign = (tid & 1) ? 1.f : -1.f;   // rot = (-x2, x1) on interleaved pairs
+      const float k = kh[tid] * c_pre + sign * kh[j] * s_pre, v = kh[H * hd + tid];
+      qs[tid] = (qh[tid] * c_pre + sign * qh[j] * s_pre) * rsqrtf((float)hd);
+      ks[tid] = k;
+      vs[tid] = v;
+      kb[(size_t)pos * hd + tid] = k;
+      vb[(size_t)pos * hd + tid] = v;
+    } else {
+      qs[tid] = q[head * hd + tid] * rsqrtf((float)hd);
+      ks[tid] = kb[(size_t)pos * hd + tid];
+      vs[tid] = vb[(size_t)pos * hd + tid];
+    }
+  }
+  __syncthreads();
+
+  const int kq = lane >> 2, t = lane & 3;
+  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 qv[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) qv[i] = t + 4 * i < hd4 ? reinterpret_cast<const float4*>(qs)[t + 4 * i] : zero4;
+  float mx = -FLT_MAX, sum = 0.f;
+  float4 acc = zero4;
+  if (warp == 0) {
+    float s = 0.f;
+    if (lane < hd4) {
+      const float4 a = reinterpret_cast<const float4*>(qs)[lane], c = reinterpret_cast<const float4*>(ks)[lane];
+      s = a.x * c.x + a.y * c.y + a.z * c.z + a.w * c.w;
+      acc = reinterpret_cast<const float4*>(vs)[lane];
+    }
+    mx = warp_sum(s);
+    sum = 1.f;
+  }
+  int stage = 0;
+#pragma unroll 1
+  for (int c = warp; c < n_chunks; c += kWideWarps) {
+    request();
+    asm volatile("cp.async.wait_group %0;" ::"n"(kWideD - 1) : "memory");
+    __syncwarp();
+    const float* kst = ring + stage * stage_floats;
+    const int cnt = min(kWideKeys, n - c * kWideKeys);
+    float s = 0.f;
+    if (kq < cnt) {
+      const float4* krow = reinterpret_cast<const float4*>(kst + kq * hd);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (t + 4 * i < hd4) {
+          const float4 kv = krow[t + 4 * i];
+          s += qv[i].x * kv.x + qv[i].y * kv.y + qv[i].z * kv.z + qv[i].w * kv.w;
+        }
+    }
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if (kq >= cnt) s = -FLT_MAX;
+    float m_new = fmaxf(mx, s);
+    m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 4));
+    m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 8));
+    m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 16));
+    const float e = kq < cnt ? __expf(s - m_new) : 0.f;
+    const float keep = __expf(mx - m_new);
+    mx = m_new;
+    float e_sum = e;
+    e_sum += __shfl_xor_sync(0xffffffffu, e_sum, 4);
+    e_sum += __shfl_xor_sync(0xffffffffu, e_sum, 8);
+    e_sum += __shfl_xor_sync(0xffffffffu, e_sum, 16);
+    sum = sum * keep + e_sum;
+    acc.x *= keep; acc.y *= keep; acc.z *= keep; acc.w *= keep;
+    const float4* vst = reinterpret_cast<const float4*>(kst + half);
+#pragma unroll
+    for (int u = 0; u < kWideKeys; ++u) {
+      const float pj = __shfl_sync(0xffffffffu, e, 4 * u);
+      if (u < cnt && lane < hd4) {
+        const float4 vv = vst[u * hd4 + lane];
+        acc.x += pj * vv.x; acc.y += pj * vv.y; acc.z += pj * vv.z; acc.w += pj * vv.w;
+      }
+    }
+    if (++stage == kWideD) stage = 0;
+    __syncwarp();             // every lane is done with this stage before it is requested again
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  if (lane < hd4) reinterpret_cast<float4*>(part + warp * hd)[lane] = acc;
+  if (lane == 0) { s_m[warp] = mx; s_l[warp] = sum; }
+  __syncthreads();
+  if (tid < hd) {             // a warp without keys has maximum -FLT_MAX: its weight is exp(-inf) = 0
+    float m_all = s_m[0];
+#pragma unroll
+    for (int w = 1; w < kWideWarps; ++w) m_all = fmaxf(m_all, s_m[w]);
+    float num = 0.f, den = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWideWarps; ++w) {
+      const float e = __expf(s_m[w] - m_all);
+      num += e * part[w * hd + tid];
+      den += e * s_l[w];
+    }
+    out[(size_t)b * out_stride + out_offset + h * hd + tid] = num / den;
+  }
+}
+
 // Cluster size: enough CTAs for a few waves of the GPU, at most 8 per head.
 static int attn_split(int B, int H) {
   const int want = 592 / std::max(1, B * H);
@@ -281,6 +433,18 @@ static int launch_attention(int B, int H, int hd, int ctx, cudaStream_t st, Args
   const int S = attn_split(B, H);
   const size_t smem = attn_smem_floats(ctx, hd, S) * sizeof(float);
   if (smem > 48 * 1024) return NB_ERR_SHAPE;
+  if (S <= 2) {     // more heads than SMs: no split is needed to occupy the GPU
+    static bool done[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!done[dev & 63]) {
+      if (cudaError_t e = cudaFuncSetAttribute(decode_attention_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)(wide_smem_floats(128) * sizeof(float))))
+        return record_cuda_error(e);
+      done[dev & 63] = true;
+    }
+    return launch_pdl(decode_attention_wide_kernel, dim3(H, B), dim3(kWideWarps * 32), wide_smem_floats(hd) * sizeof(float), st, args...);
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(H, B, S);
   cfg.blockDim = dim3(kAttnWarps * 32);

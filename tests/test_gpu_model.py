@@ -373,3 +373,36 @@ def test_full_size_decoder_against_dense_oracle_teacher_forced(built_lib):
 def test_prefill_attention_edges_of_its_tiles(built_lib, B, T, H, hd, ctx, pos0):
     """One query or key past a tile, both query tiles (few and many CTAs), every number of head dimensions per thread."""
     test_prefill_attention_against_torch(built_lib, B, T, H, hd, ctx, pos0, H * hd, 0)
+
+
+@pytest.mark.parametrize("B,H,hd,ctx", [(40, 4, 128, 300), (149, 1, 4, 40), (10, 16, 36, 97)])
+def test_decode_attention_one_cta_per_head(built_lib, B, H, hd, ctx):
+    """More heads than SMs: one CTA per head.  Positions around the chunks of eight keys that its four warps take in turn; with
+    the rotation folded in, the row of this step comes from the projection and is written to the cache."""
+    from nativebit_b200 import ops
+    from nativebit_b200.generate import apply_rope, precompute_rope
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(B + hd)
+    cos2, sin2 = precompute_rope(hd, ctx, 10000.0, dev)
+    k = torch.randn(B, H, ctx, hd, device=dev, generator=g)
+    v = torch.randn(B, H, ctx, hd, device=dev, generator=g)
+    for p_ in sorted({0, 1, 7, 8, 9, 31, 32, 33, ctx - 1} & set(range(ctx))):
+        pos = torch.tensor([p_], device=dev)
+        q = torch.randn(B, H, hd, device=dev, generator=g)
+        qkv = torch.randn(B, 3, H, hd, device=dev, generator=g)
+        out, rot = torch.zeros(B, H * hd, device=dev), torch.full((B, H * hd + 8), 7.0, device=dev)
+        k2, v2 = k.clone(), v.clone()
+        ops.decode_attention(q, k, v, pos, out, 0)
+        ops.decode_attention_rope(qkv.view(B, -1), cos2, sin2, pos, k2, v2, rot, 4)
+        torch.cuda.synchronize()
+
+        def turned(x):
+            return apply_rope(x[:, :, None], cos2[p_:p_ + 1], sin2[p_:p_ + 1])[:, :, 0]
+        k_want, v_want = k.clone(), v.clone()
+        k_want[:, :, p_], v_want[:, :, p_] = turned(qkv[:, 1]), qkv[:, 2]
+        assert torch.equal(v2, v_want) and (k2 - k_want).abs().max() <= 1e-6 * k_want.abs().max()
+        for got, qq, kk, vv in ((out, q, k, v), (rot[:, 4:-4], turned(qkv[:, 0]), k_want, v_want)):
+            sc = torch.einsum("bhd,bhjd->bhj", qq.double(), kk[:, :, :p_ + 1].double()) / hd ** 0.5
+            ref = torch.einsum("bhj,bhjd->bhd", torch.softmax(sc, -1), vv[:, :, :p_ + 1].double()).reshape(B, H * hd)
+            assert (got.double() - ref).abs().max() <= 2e-5 * ref.abs().max(), p_          # fp32 sums, __expf
+        assert (rot[:, :4] == 7.0).all() and (rot[:, -4:] == 7.0).all()
