@@ -12,21 +12,29 @@
 // lookups per 512 tensor-core clocks, a quarter of the SM's byte-permute throughput.
 //
 // Weights are read in the stream layout (nb_stream_pack: per 16 rows x 128 weights, every lane-group's
-// indices as nibbles in position order + the rows' byte-plane lookup tables), straight from L2 into
-// registers.  Persistent kernel, one CTA per SM, 704 threads:
+// indices as nibbles in position order + the rows' byte-plane lookup tables).  Persistent kernel, one CTA per SM, 736 threads:
 //   warp 0       one lane issues the TMA loads (cp.async.bulk.tensor.2d, 128-byte swizzle, no multicast)
 //                of the BN x 64 activation slab of every k-step into a ring of stages;
-//   warp 1       allocates tensor memory; one lane waits on the stage's "full" barrier (eight producer warps'
+//   warp 1       allocates tensor memory; one lane waits on the stage's "full" barrier (four producer warps'
 //                arrivals + the TMA bytes) and issues four tcgen05.mma (128 x BN x 16, fp16 x fp16 -> fp32)
 //                per stage, then tcgen05.commit on the stage's "empty" barrier;
 //   warps 2-5    epilogue: each warp owns one 32-lane quadrant of tensor memory (32 output features),
 //                reads a finished accumulator with tcgen05.ld and stores Y (transposed: lanes run along
 //                N, so a warp's store of one token covers 32 consecutive outputs);
-//   warps 6-21   dequant producers, two groups of 8 warps that take turns at the k-steps (filling a stage is
-//                a chain of dependent steps, so two stages are filled at a time): thread (row, half) of the
-//                128 x 64 weight tile loads four selector words and the row's table (prefetched one of its
-//                k-steps ahead), looks 32 weights up with byte permutes and writes them as four 16-byte
-//                chunks into the 128-byte-swizzled stage.
+//   warps 6-21   dequant producers, four groups of 4 warps that take turns at the k-steps (filling a stage is a chain of about
+//                1200 clocks, most of it waits and barriers, so four are filled at a time): a warp owns two of the eight row
+//                tiles of the 128 x 64 weight tile, a thread (row, half) of both reads four selector words and the row's
+//                table from a raw stage, looks 32 weights up with byte permutes and, once the stage is free, writes them as
+//                four 16-byte chunks into its 128-byte swizzle;
+//   warp 22      one lane issues the TMA loads of the raw weights, the eight row tiles of a k-block (two k-steps) at once,
+//                into a ring of its own.  (Producers that load through registers wait at every proxy fence until their
+//                own prefetches have landed: a k-step then took half a memory latency, 0.40 - 0.45 us, whatever BN was and
+//                however far ahead they loaded.)
+// The kernel starts while the launch that converts the activations still runs (programmatic dependent launch): only warp 0
+// waits for it, the producers fill the first stages meanwhile.
+// From a graph over cold weights, before -> now (us): 17 fp32 rows x 7680 x 2560 16.9 -> 13.2, 129 rows 25.2 -> 20.7, 400 rows
+// 45.1 -> 34.5; 17 rows x 13824 x 2560 22.7 -> 17.3; 400 rows x 2560 x 6912 52.6 -> 39.5.  A decode step of 32 sequences, per layer
+// 108 -> 91.
 // Two accumulators in tensor memory let the epilogue of one tile overlap the MMAs of the next.  Every
 // mbarrier wait is bounded; on a timeout the waiter raises a shared abort flag, writes NB_ERR_TIMEOUT
 // to the status word and all roles fall through to the exit, where tensor memory is freed.
@@ -41,23 +49,39 @@
 #include "nb_common.cuh"
 #include "nb_device.cuh"
 #include "nb_host.h"
+#include "nb_launch.cuh"
 #include "nb_umma.cuh"
 
 namespace nb {
 
 constexpr int kFM = 128;                  // output features per tile (the MMA's M)
 constexpr int kFK = 64;                   // k per stage
-constexpr int kFProducerWarp0 = 6, kFProducerWarps = 8;   // warps per producer group
-constexpr int kFGroups = 2;                                // groups take turns at the k-steps
-constexpr int kFThreads = (kFProducerWarp0 + kFGroups * kFProducerWarps) * 32;
+constexpr int kFProducerWarp0 = 6, kFProducerWarps = 4;   // warps per producer group
+constexpr int kFGroups = 4;                                // groups take turns at the k-steps
+constexpr int kFRawWarp = kFProducerWarp0 + kFGroups * kFProducerWarps;
+constexpr int kFThreads = (kFRawWarp + 1) * 32;
 constexpr int kFABytes = kFM * kFK * 2;   // 16 KB of weights per stage
-constexpr int kFRing = 192 * 1024;
 constexpr int kFMaxStages = 8;
-constexpr int kFSmem = kFRing + 1024 + 512;
+constexpr int kFRawBytes = 8 * 1536;       // raw weights: eight row tiles of a k-block at 4 bits
+constexpr int kFMaxRaw = 4;
+constexpr int kFOperands = 176 * 1024 + kFMaxRaw * kFRawBytes;      // operand stages and raw stages
+constexpr int kFSmem = kFOperands + 1024 + 512;
+static_assert(kFSmem <= 227 * 1024, "shared memory of a CTA");
 
+// Operand stages are at least as many as producer groups at every BN: past 224 columns two raw stages give way to the fourth
+// (a step then takes 512 clocks of the tensor cores, time enough for a raw stage to be filled again).  The raw stages are an
+// even number, so that a group, which takes every second k-block, meets each of its stages every turn.
+__host__ __device__ constexpr int fused_raw_stages(int bn) { return bn > 224 ? 2 : kFMaxRaw; }
+__host__ __device__ constexpr int fused_ring(int bn) { return bn > 224 ? 192 * 1024 : 176 * 1024; }
 __host__ __device__ constexpr int fused_stages(int bn) {
-  return kFRing / (kFABytes + bn * kFK * 2) < kFMaxStages ? kFRing / (kFABytes + bn * kFK * 2) : kFMaxStages;
+  return fused_ring(bn) / (kFABytes + bn * kFK * 2) < kFMaxStages ? fused_ring(bn) / (kFABytes + bn * kFK * 2) : kFMaxStages;
 }
+constexpr bool enough_stages() {
+  for (int bn = 16; bn <= 256; bn += 16)
+    if (fused_stages(bn) < kFGroups || fused_ring(bn) + fused_raw_stages(bn) * kFRawBytes > kFOperands) return false;
+  return true;
+}
+static_assert(enough_stages(), "stages per producer group");
 
 #ifdef NB_FUSED_TRACE
 __device__ long long g_ftrace[8][512];
@@ -71,34 +95,45 @@ template <int BITS> struct FusedFmt {
   static constexpr int kUnitBytes = 1024 + 16 * kTabBytes;   // the stream layout's unit (nb_stream.cu)
 };
 
+// k-steps of one of ks splits: whole k-blocks, as the raw weights arrive
+__host__ __device__ constexpr int split_steps(int KT, int ks) { return (KT / 2 + ks - 1) / ks * 2; }
+
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+               ::"r"(s2u(dst)), "l"(map), "r"(s2u(bar)), "r"(x), "r"(y), "r"(z) : "memory");
+}
+
 template <int BITS>
 __global__ void __launch_bounds__(kFThreads, 1)
-gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const uint8_t* __restrict__ w_stream, void* __restrict__ y, int y_dtype,
+gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, void* __restrict__ y, int y_dtype,
                   int M, int N, int K, int BN, int m_tiles, int w_tiles, int pair, int ks, float* __restrict__ partial, int* status) {
   using F = FusedFmt<BITS>;
   constexpr int kT = BITS == 4 ? 8 : 4;
-  const int S = fused_stages(BN);
+  const int S = fused_stages(BN), R = fused_raw_stages(BN);
   const int b_bytes = BN * kFK * 2;           // multiple of 1024 because BN is a multiple of 16
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* sA = smem;                         // weights
   uint8_t* sB = smem + S * kFABytes;          // activations
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kFRing);   // a stage's weights (8 producer warps) AND activations (TMA bytes)
+  uint8_t* sW = smem + fused_ring(BN);        // raw weights
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kFOperands);   // a stage's weights (4 producer warps) AND activations (TMA bytes)
   uint64_t* empty = full + kFMaxStages;
   uint64_t* acc_full = empty + kFMaxStages;   // [2] MMA -> epilogue
   uint64_t* acc_empty = acc_full + 2;         // [2] epilogue -> MMA
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* raw_full = acc_empty + 2;
+  uint64_t* raw_empty = raw_full + kFMaxRaw;   // the two producer groups of a k-block have read it
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(raw_empty + kFMaxRaw);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int KT = K / kFK, bpr = K / kBlock;
-  const int KTs = (KT + ks - 1) / ks;           // k-steps per k split (the last split may be shorter, never empty)
+  const int KT = K / kFK;
+  const int KTs = split_steps(KT, ks);          // k-steps per k split (the last split may be shorter, never empty)
   const int n_total = m_tiles * w_tiles * ks;   // work item t: k split t % ks of output tile t / ks
-  const int rows_padded = ((N + 15) >> 4) << 4;   // rows the stream layout holds (zero rows past N)
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) { bar_init(&full[s], kFProducerWarps + 1); bar_init(&empty[s], 1); }
     for (int b = 0; b < 2; ++b) { bar_init(&acc_full[b], 1); bar_init(&acc_empty[b], 4); }
+    for (int r = 0; r < R; ++r) { bar_init(&raw_full[r], 1); bar_init(&raw_empty[r], 2 * kFProducerWarps); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -115,8 +150,10 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const uint8_t* __re
   // weight tile; with ks > 1 the k range of an output tile is cut into ks parts whose fp32 results go to
   // `partial` and are added in k order by a second kernel (short inputs would otherwise leave most SMs idle
   // behind a long serial chain of k-steps)
+  if (ks > 1) asm volatile("griddepcontrol.launch_dependents;");      // the summing kernel: it waits for this one's end
   if (warp == 0) {
-    if (lane == 0) {  // ---- TMA producer of the activation slabs
+    if (elect_one()) {  // ---- TMA producer of the activation slabs
+      asm volatile("griddepcontrol.wait;" ::: "memory");      // the fp16 operand is the launch before's result, the weights are not
       int s = 0;
       uint32_t phase = 0;
       for (int t = blockIdx.x; t < n_total; t += gridDim.x) {
@@ -135,7 +172,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const uint8_t* __re
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {  // ---- MMA issuer
+    if (elect_one()) {  // ---- MMA issuer
       // instruction descriptor: fp32 accumulate (bit 4), A and B fp16 (format 0 at bits 7 and 10), both K-major,
       // N = BN (tokens), M = 128 (features)
       const uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kFM >> 4) << 24);
@@ -223,70 +260,84 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const uint8_t* __re
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s2u(&acc_empty[buf])) : "memory");
     }
-  } else {
-    // ---- dequant producers: thread (row, half) writes 32 weights = 64 bytes of row `row` of the stage
-    const int p = threadIdx.x - kFProducerWarp0 * 32;
-    const int grp = p >> 8, pp = p & 255;                // group `grp` fills the k-steps kt with kt % kFGroups == grp
-    const int row = pp & 127, q2 = pp >> 7;
-    const int r16 = row & 15, g = r16 & 7, hrow = r16 >> 3;
-    const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
-    uint32_t step0 = 0;                                  // k-steps of all earlier work items: stage = step % S, phase = (step / S) & 1
-    for (int t = blockIdx.x; t < n_total; t += gridDim.x) {
-      const int n0 = ((t / ks) / m_tiles) * kFM;
-      const int k_lo = (t % ks) * KTs, k_hi = min(KT, k_lo + KTs);
-      const int grow = n0 + row;
-      const bool valid = grow < rows_padded;
-      const uint8_t* urow = w_stream + (size_t)(grow >> 4) * bpr * F::kUnitBytes;   // the row tile's units
-      // k-step kt covers positions 64*(kt&1) .. +63 of k-block kt>>1: this thread's lane group is t = 2*(kt&1) + q2
-      auto load = [&](int kt, uint4& sel, uint4 (&tab)[kT / 4]) {
-        sel = zero4;
-#pragma unroll
-        for (int j = 0; j < kT / 4; ++j) tab[j] = zero4;
-        if (valid && kt < k_hi) {
-          const uint8_t* u = urow + (size_t)(kt >> 1) * F::kUnitBytes;
-          const int lane_u = g * 4 + 2 * (kt & 1) + q2;
-          sel = __ldg(reinterpret_cast<const uint4*>(u + hrow * 512 + lane_u * 16));
-#pragma unroll
-          for (int j = 0; j < kT / 4; ++j) tab[j] = __ldg(reinterpret_cast<const uint4*>(u + 1024 + r16 * F::kTabBytes + 16 * j));
-        }
-      };
-      uint4 sel, tab[kT / 4];
-      load(k_lo + grp, sel, tab);
+  } else if (warp == kFRawWarp) {
+    if (elect_one()) {  // ---- TMA producer of the raw weights: row tiles past the matrix arrive as zeros
+      int r = 0;
+      uint32_t phase = 0;
       bool ok = true;
-      for (int kt = k_lo + grp; kt < k_hi; kt += kFGroups) {
-        uint4 sel_n, tab_n[kT / 4];
-        load(kt + kFGroups, sel_n, tab_n);               // this group's next k-step, in flight while this one is unpacked
-        const uint32_t step = step0 + (uint32_t)(kt - k_lo);
-        const int s = (int)(step % (uint32_t)S);
-        const uint32_t phase = (step / (uint32_t)S) & 1u;
-        if (pp == 0) FTRACE(3, kt);
-        ok = bar_wait<20>(&empty[s], phase ^ 1, abort_flag, status);
-        if (!ok) break;
-        if (pp == 0) FTRACE(4, kt);
-        uint32_t T[kT];
-#pragma unroll
-        for (int j = 0; j < kT / 4; ++j) { T[4 * j] = tab[j].x; T[4 * j + 1] = tab[j].y; T[4 * j + 2] = tab[j].z; T[4 * j + 3] = tab[j].w; }
-        const uint32_t words[4] = {sel.x, sel.y, sel.z, sel.w};
-        // row `row` of a K-major tile with 128-byte swizzle: 16-byte chunk c sits at chunk c ^ (row & 7)
-        uint8_t* rbase = sA + s * kFABytes + (row >> 3) * 1024 + (row & 7) * 128;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          uint32_t a, b, c, d;
-          lookup4<BITS>(words[j], T, a, b);              // positions 8j .. 8j+3
-          lookup4<BITS>(words[j] >> 16, T, c, d);        // positions 8j+4 .. 8j+7
-          const int chunk = (4 * q2 + j) ^ (row & 7);
-          *reinterpret_cast<uint4*>(rbase + chunk * 16) = make_uint4(a, b, c, d);
+      for (int t = blockIdx.x; t < n_total && ok; t += gridDim.x) {
+        const int rt0 = ((t / ks) / m_tiles) * (kFM / 16);
+        const int k_lo = (t % ks) * KTs, k_hi = min(KT, k_lo + KTs);
+        for (int kb = k_lo >> 1; kb < k_hi >> 1; ++kb) {
+          ok = bar_wait(&raw_empty[r], phase ^ 1, abort_flag, status);
+          if (!ok) break;
+          bar_expect_tx(&raw_full[r], 8u * F::kUnitBytes);
+          tma_load_3d(sW + r * kFRawBytes, &map_w, &raw_full[r], 0, kb, rt0);
+          if (++r == R) { r = 0; phase ^= 1; }
         }
+      }
+    }
+  } else {
+    // ---- dequant producers: thread (row, half) writes 32 weights = 64 bytes of row `row` of the stage.  A warp's lanes are
+    // (row, half) with the halves side by side: eight lanes' chunks fall into eight different bank groups
+    const int w = warp - kFProducerWarp0;
+    const int grp = w / kFProducerWarps, rt0 = 2 * (w % kFProducerWarps);      // group `grp` fills the steps st with st % 4 == grp
+    const int r16 = lane >> 1, q2 = lane & 1, g = r16 & 7, hrow = r16 >> 3;
+    const uint8_t* raw0 = sW + rt0 * F::kUnitBytes;
+    // positions 64 * (grp & 1) .. + 63 of a k-block: this thread's lane group of the unit is 2 * (grp & 1) + q2
+    const int sel_off = hrow * 512 + (g * 4 + 2 * (grp & 1) + q2) * 16, tab_off = 1024 + r16 * F::kTabBytes;
+    // row r of a K-major tile with 128-byte swizzle: 16-byte chunk c sits at chunk c ^ (r & 7); a row tile is 2 KB
+    uint8_t* const rbase = sA + rt0 * 2048 + hrow * 1024 + g * 128;
+    uint32_t step0 = 0;                                  // k-steps of all earlier work items (even): stage = step % S, phase = (step / S) & 1
+    bool ok = true;
+    for (int t = blockIdx.x; t < n_total && ok; t += gridDim.x) {
+      const int k_lo = (t % ks) * KTs, steps = min(KT, k_lo + KTs) - k_lo;
+      const uint32_t end = step0 + (uint32_t)steps;
+      uint32_t st = step0 + (((uint32_t)grp - step0) & (kFGroups - 1));           // the group's first step of this item
+      int s = (int)(st % (uint32_t)S);
+      uint32_t phase = (st / (uint32_t)S) & 1u;
+      for (; st < end; st += kFGroups) {
+        const uint32_t kb = st >> 1;                     // k-blocks since the start: the group's are every second one
+        const int r = (int)(kb & (uint32_t)(R - 1));
+        if (rt0 == 0 && lane == 0) FTRACE(3, k_lo + (int)(st - step0));
+        ok = bar_wait<20>(&raw_full[r], kb / (uint32_t)R & 1u, abort_flag, status);
+        if (!ok) break;
+        uint4 out[2][4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint8_t* u = raw0 + r * kFRawBytes + h * F::kUnitBytes;
+          const uint4 sel = *reinterpret_cast<const uint4*>(u + sel_off);
+          uint32_t T[kT];
+#pragma unroll
+          for (int j = 0; j < kT / 4; ++j) {
+            const uint4 v = *reinterpret_cast<const uint4*>(u + tab_off + 16 * j);
+            T[4 * j] = v.x; T[4 * j + 1] = v.y; T[4 * j + 2] = v.z; T[4 * j + 3] = v.w;
+          }
+          const uint32_t words[4] = {sel.x, sel.y, sel.z, sel.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            lookup4<BITS>(words[j], T, out[h][j].x, out[h][j].y);              // positions 8j .. 8j+3
+            lookup4<BITS>(words[j] >> 16, T, out[h][j].z, out[h][j].w);        // positions 8j+4 .. 8j+7
+          }
+        }
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s2u(&raw_empty[r])) : "memory");
+        // (a parity tells a phase from its neighbours only: with at least as many stages as groups, the wait for this group's step
+        // before implies that the stage is at most one use behind)
+        ok = bar_wait<20>(&empty[s], phase ^ 1u, abort_flag, status);
+        if (!ok) break;
+        if (rt0 == 0 && lane == 0) FTRACE(4, k_lo + (int)(st - step0));
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(rbase + s * kFABytes + h * 2048 + (((4 * q2 + j) ^ g) << 4)) = out[h][j];
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy stores -> visible to the tensor core
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s2u(&full[s])) : "memory");
-        if (pp == 0) FTRACE(5, kt);
-        sel = sel_n;
-#pragma unroll
-        for (int j = 0; j < kT / 4; ++j) tab[j] = tab_n[j];
+        if (rt0 == 0 && lane == 0) FTRACE(5, k_lo + (int)(st - step0));
+        for (s += kFGroups; s >= S; s -= S) phase ^= 1u;
       }
-      if (!ok) break;
-      step0 += (uint32_t)(k_hi - k_lo);
+      step0 += (uint32_t)steps;
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -299,6 +350,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const uint8_t* __re
 
 // bf16 -> fp16, eight elements per thread, saturating to +-65504 (exact for magnitudes 6.1e-5 .. 65504).
 __global__ void __launch_bounds__(256) bf16_to_f16_kernel2(const uint4* __restrict__ in, uint4* __restrict__ out, size_t n8) {
+  asm volatile("griddepcontrol.launch_dependents;");
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n8) return;
   const uint4 v = in[i];
@@ -328,7 +380,7 @@ static FusedPlan plan_fused(int rows, int N, int K, int sms) {
   for (int bn = bn_hi; bn >= bn_lo; bn -= 16) {
     const long tiles = (long)w_tiles * ((rows + bn - 1) / bn);
     for (int ks = 1; ks <= 8; ++ks) {
-      const int kts = (KT + ks - 1) / ks;
+      const int kts = split_steps(KT, ks);
       if (ks > 1 && (kts < 4 || (long)(ks - 1) * kts >= KT)) continue;
       const long waves = (tiles * ks + sms - 1) / sms;
       // the second kernel reads ks slabs of rows x N floats at roughly 3 KB per clock
@@ -344,6 +396,7 @@ static FusedPlan plan_fused(int rows, int N, int K, int sms) {
 __global__ void __launch_bounds__(256) splitk_sum_kernel(const float* __restrict__ partial, int ks, size_t slab, void* __restrict__ y,
                                                          int y_dtype, size_t n4) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (i >= n4) return;
   float4 acc = reinterpret_cast<const float4*>(partial)[i];
   for (int z = 1; z < ks; ++z) {
@@ -357,6 +410,24 @@ __global__ void __launch_bounds__(256) splitk_sum_kernel(const float* __restrict
   } else {
     reinterpret_cast<float4*>(y)[i] = acc;
   }
+}
+
+// The stream layout as (row tiles, k-blocks, units of 8-byte elements) with boxes of eight row tiles of one k-block.
+static int make_map_units(CUtensorMap* map, const void* base, int unit_bytes, int bpr, int row_tiles) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) { set_last_error("cuTensorMapEncodeTiled is not available from the driver"); return NB_ERR_LAUNCH; }
+  const cuuint64_t dims[3] = {(cuuint64_t)unit_bytes / 8, (cuuint64_t)bpr, (cuuint64_t)row_tiles};
+  const cuuint64_t strides[2] = {(cuuint64_t)unit_bytes, (cuuint64_t)bpr * unit_bytes};
+  const cuuint32_t box[3] = {(cuuint32_t)unit_bytes / 8, 1, 8}, estr[3] = {1, 1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_INT64, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    char msg[96];
+    std::snprintf(msg, sizeof(msg), "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
+    set_last_error(msg);
+    return NB_ERR_LAUNCH;
+  }
+  return NB_OK;
 }
 
 // (rows, cols) row-major 16-bit matrix -> tensor map with a (box_rows x 64) box and 128-byte swizzle.
@@ -414,8 +485,9 @@ extern "C" int nb_gemm_prefill_fused(const void* x, int x_dtype, int M, const ui
   const int sms = sm_count();
   const FusedPlan plan = plan_fused(rows, N, K, sms);
   const int bn = plan.bn;
-  CUtensorMap mx;
+  CUtensorMap mx, mw;
   if (int rc = make_map_f16(&mx, xh, rows, K, bn)) return rc;
+  if (int rc = make_map_units(&mw, w_stream, bits == 4 ? FusedFmt<4>::kUnitBytes : FusedFmt<3>::kUnitBytes, K / kBlock, (N + 15) / 16)) return rc;
   const int m_tiles = (rows + bn - 1) / bn, w_tiles = (N + kFM - 1) / kFM;
   int ks = plan.ks;
   if (ks > 1 && (N % 4 != 0 || (uintptr_t)y % 16)) ks = 1;       // the summing kernel writes four outputs at a time
@@ -430,14 +502,23 @@ extern "C" int nb_gemm_prefill_fused(const void* x, int x_dtype, int M, const ui
     if (cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem)) return record_cuda_error(e);
     attr_done[dev & 63][bits] = true;
   }
-  if (bits == 3) gemm_fused_kernel<3><<<grid, kFThreads, kFSmem, st>>>(mx, w_stream, y, y_dtype, rows, N, K, bn, m_tiles, w_tiles, pair, ks, partial, status);
-  else if (bits == 2) gemm_fused_kernel<2><<<grid, kFThreads, kFSmem, st>>>(mx, w_stream, y, y_dtype, rows, N, K, bn, m_tiles, w_tiles, pair, ks, partial, status);
-  else gemm_fused_kernel<4><<<grid, kFThreads, kFSmem, st>>>(mx, w_stream, y, y_dtype, rows, N, K, bn, m_tiles, w_tiles, pair, ks, partial, status);
-  if (int rc = check_launch()) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kFThreads);
+  cfg.dynamicSmemBytes = kFSmem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  // ahead of its turn only behind this call's own conversion: whatever wrote the weights has then ended
+  cfg.numAttrs = xh != x ? 1 : 0;
+  int y_tag = y_dtype, rows_arg = rows, n_arg = N, k_arg = K, bn_arg = bn, m_t = m_tiles, w_t = w_tiles, pair_arg = pair;
+  void* args[] = {&mx, &mw, &y, &y_tag, &rows_arg, &n_arg, &k_arg, &bn_arg, &m_t, &w_t, &pair_arg, &ks, &partial, &status};
+  if (cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args)) return record_cuda_error(e);
   if (ks > 1) {
     const size_t n4 = (size_t)M * N / 4;
-    splitk_sum_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(partial, ks, (size_t)M * N, y, y_dtype, n4);
-    return check_launch();
+    return launch_pdl(splitk_sum_kernel, dim3((unsigned)((n4 + 255) / 256)), dim3(256), 0, st, partial, ks, (size_t)M * N, y, y_dtype, n4);
   }
   return NB_OK;
 }

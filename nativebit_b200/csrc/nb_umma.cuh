@@ -125,6 +125,7 @@ inline int make_map(CUtensorMap* map, const void* base, int rows, int cols, int 
 // fp32 -> two fp16 terms per element, hi = fp16(x) (saturating) and lo = fp16(x - hi), written as rows 2i and
 // 2i+1 of a (2M, K) fp16 matrix: x = hi + lo to about 22 significant bits.  Eight elements per thread.
 static __global__ void __launch_bounds__(256) f32_to_f16_pair_kernel(const float4* __restrict__ in, uint4* __restrict__ out, int M, int K) {
+  asm volatile("griddepcontrol.launch_dependents;");        // the GEMM behind it waits before it reads
   const int k8 = K >> 3;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)M * k8) return;
