@@ -11,7 +11,7 @@ import re
 
 from .build import LIB_PATH, library_path
 
-NB_F32, NB_F16, NB_BF16 = 0, 1, 2
+NB_F32, NB_F16, NB_BF16, NB_F16_TERMS = 0, 1, 2, 8
 
 _INCLUDE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "include")
 _HEADERS = {"packed": "nativebit_b200.h", "layered": "nativebit_b200_layered.h"}
@@ -46,6 +46,8 @@ _SIGNATURES = {
                                        _c.c_void_p, _c.c_int, _c.c_int, _c.c_void_p]),
     "nb_decode_attention_rope": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_int,
                                             _c.c_int, _c.c_int, _c.c_int, _c.c_void_p, _c.c_int, _c.c_int, _c.c_void_p]),
+    "nb_add_rmsnorm_terms": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_float, _c.c_void_p, _c.c_int, _c.c_int, _c.c_void_p]),
+    "nb_silu_mul_terms": (_c.c_int, [_c.c_void_p, _c.c_int, _c.c_int, _c.c_void_p, _c.c_void_p]),
     "nb_silu_mul": (_c.c_int, [_c.c_void_p, _c.c_int, _c.c_int, _c.c_void_p, _c.c_void_p]),
     "nb_lm_head_scratch_bytes": (_c.c_size_t, []),
     "nb_lm_head": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_float, _c.c_void_p, _c.c_int, _c.c_int, _c.c_float,

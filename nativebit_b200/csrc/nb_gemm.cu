@@ -487,7 +487,7 @@ extern "C" int nb_gemm_prefill(const void* x, int x_dtype, int M, const uint8_t*
                                int block_size, int N, int K, void* y, int y_dtype, void* workspace, size_t workspace_bytes,
                                void* stream) {
   if (!x || !packed || !codebook || !y) return NB_ERR_ARG;
-  if (x_dtype != NB_BF16 && x_dtype != NB_F16 && x_dtype != NB_F32) return NB_ERR_ARG;
+  if (x_dtype != NB_BF16 && x_dtype != NB_F16 && x_dtype != NB_F32 && x_dtype != NB_F16_TERMS) return NB_ERR_ARG;
   if (!workspace || workspace_bytes < nb_prefill_workspace_bytes(M, N, K)) return NB_ERR_WORKSPACE;
   if ((uintptr_t)workspace % 256) return NB_ERR_ALIGN;
   if (K % kBK != 0 || K % block_size != 0) return NB_ERR_SHAPE;
@@ -495,7 +495,8 @@ extern "C" int nb_gemm_prefill(const void* x, int x_dtype, int M, const uint8_t*
   uint8_t* w = reinterpret_cast<uint8_t*>(workspace) + 256;
   uint8_t* xh = w + (((size_t)N * K * 2 + 255) & ~(size_t)255);
   if (int rc = nb_dequant(packed, codebook, cb_dtype, bits, block_size, N, K, w, NB_F16, stream)) return rc;
-  if (x_dtype == NB_F16) return gemm_16bit(x, w, 1, M, N, K, y, y_dtype, reinterpret_cast<int*>(workspace), stream);
+  if (x_dtype == NB_F16 || x_dtype == NB_F16_TERMS)
+    return gemm_16bit(x, w, 1, M, N, K, y, y_dtype, reinterpret_cast<int*>(workspace), stream, x_dtype == NB_F16_TERMS);
   const size_t n8 = (size_t)M * K / 8;  // K % 64 == 0
   if (x_dtype == NB_F32) {  // two fp16 terms per element; rows 2i and 2i + 1 of the kernel's result are one row of 2K here
     f32_to_f16_pair_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(reinterpret_cast<const float4*>(x),

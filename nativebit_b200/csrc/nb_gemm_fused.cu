@@ -459,7 +459,7 @@ extern "C" size_t nb_prefill_fused_workspace_bytes(int M, int N, int K) {
 extern "C" int nb_gemm_prefill_fused(const void* x, int x_dtype, int M, const uint8_t* w_stream, int bits, int N, int K, void* y,
                                      int y_dtype, void* workspace, size_t workspace_bytes, void* stream) {
   if (!x || !w_stream || !y || M < 1 || N < 1 || K < 1) return NB_ERR_ARG;
-  if (x_dtype != NB_BF16 && x_dtype != NB_F16 && x_dtype != NB_F32) return NB_ERR_ARG;
+  if (x_dtype != NB_BF16 && x_dtype != NB_F16 && x_dtype != NB_F32 && x_dtype != NB_F16_TERMS) return NB_ERR_ARG;
   if (y_dtype != NB_BF16 && y_dtype != NB_F32) return NB_ERR_ARG;
   if (bits != 2 && bits != 3 && bits != 4) return NB_ERR_SHAPE;
   if (K % kBlock != 0) return NB_ERR_SHAPE;
@@ -468,7 +468,7 @@ extern "C" int nb_gemm_prefill_fused(const void* x, int x_dtype, int M, const ui
   if (int rc = check_device()) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   const void* xh = x;
-  const int pair = x_dtype == NB_F32 ? 1 : 0;
+  const int pair = x_dtype == NB_F32 || x_dtype == NB_F16_TERMS ? 1 : 0;
   const int rows = pair ? 2 * M : M;              // rows of the fp16 operand
   uint8_t* dst = reinterpret_cast<uint8_t*>(workspace) + 256;
   if (x_dtype == NB_BF16) {

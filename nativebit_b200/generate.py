@@ -168,6 +168,28 @@ class PackedGPT(torch.nn.Module):
             x.add_(delta)
         return rms_norm(x, weight, eps)
 
+    def _norm_linear(self, x: torch.Tensor, delta, weight: torch.Tensor, eps: float, lin: PackedLinear) -> torch.Tensor:
+        """lin(rmsnorm(x += delta) * weight), fp32; many rows travel as the GEMM's two fp16 terms instead of fp32."""
+        C, rows = x.shape[-1], x.numel() // x.shape[-1]
+        if (lin.takes_terms(rows) and x.is_cuda and x.dtype == torch.float32 and x.is_contiguous() and C <= 4096 and weight.dtype == torch.float32
+                and (delta is None or (delta.dtype == torch.float32 and delta.is_contiguous()))):
+            terms = torch.empty(2 * rows, C, dtype=torch.float16, device=x.device)
+            ops.add_rmsnorm_terms(x.view(rows, C), None if delta is None else delta.view(rows, C), weight, eps, terms)
+            return lin.forward_terms(terms).view(*x.shape[:-1], -1)
+        return lin(self._add_norm(x, delta, weight, eps)).float().contiguous()
+
+    @staticmethod
+    def _silu_linear(gu: torch.Tensor, lin: PackedLinear) -> torch.Tensor:
+        """lin(silu(gate) * up), fp32, for gu (rows, 2F) = [gate | up]."""
+        rows, F_ = gu.shape[0], gu.shape[1] // 2
+        if gu.is_cuda and gu.is_contiguous() and lin.takes_terms(rows) and rows <= 65535:
+            terms = torch.empty(2 * rows, F_, dtype=torch.float16, device=gu.device)
+            ops.silu_mul_terms(gu, terms)
+            return lin.forward_terms(terms)
+        act = torch.empty(rows, F_, dtype=torch.float32, device=gu.device)
+        ops.silu_mul(gu, act)
+        return lin(act).float()
+
     def _finish_block(self, x, blk, attn_out):
         """attn_out (B, T, Hl*hd) -> residual adds of out_proj and the SwiGLU FFN."""
         if attn_out.shape[-1] != self.o_cols:  # pad to the whole codebook blocks covering this rank's columns
@@ -221,17 +243,15 @@ class PackedGPT(torch.nn.Module):
                 # residual adds ride in the norm kernels, the last one of a block is still pending when the block ends
                 k_buf, v_buf, cache_len = kv_caches[i]
                 eps = self.config.norm_eps
-                qkv = blk.qkv(self._add_norm(x, delta, blk.ln1, eps)).float().contiguous()
+                qkv = self._norm_linear(x, delta, blk.ln1, eps, blk.qkv)
                 cols = self.heads_local * self.config.head_dim
                 out = (x.new_empty if cols == self.o_cols else x.new_zeros)(B, T, self.o_cols)
                 ops.prefill_attention(qkv.view(B * T, -1), T, self.cos2, self.sin2, int(cache_len), k_buf, v_buf,
                                       out.view(B * T, -1), self.o_col0 if cols != self.o_cols else 0)
                 new_caches.append((k_buf, v_buf, cache_len + T))
                 d1 = self._all_reduce(blk.out_proj(out).float())
-                gu = blk.gate_up(self._add_norm(x, d1, blk.ln2, eps)).float().contiguous()
-                act = torch.empty(B, T, gu.shape[-1] // 2, dtype=torch.float32, device=gu.device)
-                ops.silu_mul(gu.view(B * T, -1), act.view(B * T, -1))
-                delta = self._all_reduce(blk.down(act).float())
+                gu = self._norm_linear(x, d1, blk.ln2, eps, blk.gate_up)
+                delta = self._all_reduce(self._silu_linear(gu.view(B * T, -1), blk.down).view(B, T, -1))
                 continue
             if delta is not None:
                 x, delta = x + delta, None
@@ -384,6 +404,14 @@ class DecodeSession(Session):
             self.bgu = torch.zeros(B, blk.gate_up.out_features, **f32)
             self.bhm = torch.zeros(B, blk.down.in_features, **f32)
             self.bd = torch.zeros(B, cfg.n_embd, **f32)
+            self.bterms = torch.empty(2 * B * max(cfg.n_embd, blk.down.in_features) if B > 16 else 0, dtype=torch.float16, device=dev)
+
+    def _terms_of(self, lin: PackedLinear) -> torch.Tensor | None:
+        """Room for the rows of this linear as two fp16 terms, if the step hands them over so."""
+        return self.bterms[:2 * self.B * lin.in_features].view(2 * self.B, -1) if lin.takes_terms(self.B) and lin.in_features % 4 == 0 else None
+
+    def _terms_into(self, lin: PackedLinear, terms: torch.Tensor, out: torch.Tensor) -> None:
+        ops.gemm_prefill_fused(terms, lin.stream_weight(), lin.bits, lin.out_features, lin.in_features, out=out, terms=True)
 
     def _linear_into(self, lin: PackedLinear, x: torch.Tensor, out: torch.Tensor) -> None:
         """out = lin(x) for a batch of rows: up to 16 through the fused GEMV, more through the tensor-core
@@ -436,6 +464,9 @@ class DecodeSession(Session):
             elif fold:
                 ops.gemv_fused(ops.PRO_ADD_RMSNORM, xa, *args, out, delta=delta, norm_weight=w, eps=eps, x_out=xb)
                 xa, xb = xb, xa
+            elif (terms := self._terms_of(lin)) is not None and lin.in_features <= 4096:
+                ops.add_rmsnorm_terms(xa, delta, w, eps, terms)
+                self._terms_into(lin, terms, out)
             else:
                 ops.add_rmsnorm(xa, delta, w, eps, self.bh)
                 self._linear_into(lin, self.bh, out)
@@ -459,6 +490,9 @@ class DecodeSession(Session):
                 ops.gemv_stream_rows(prologue, x, lin.stream_weight(), lin.bits, lin.out_features, lin.in_features, out)
             elif prologue == ops.PRO_SILU_MUL and fold:
                 ops.gemv_fused(prologue, x, *args, out)
+            elif prologue == ops.PRO_SILU_MUL and (terms := self._terms_of(lin)) is not None:
+                ops.silu_mul_terms(x, terms)
+                self._terms_into(lin, terms, out)
             elif prologue == ops.PRO_SILU_MUL:
                 ops.silu_mul(x, self.bhm)
                 self._linear_into(lin, self.bhm, out)

@@ -8,7 +8,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from ._lib import NB_BF16, NB_F16, NB_F32
+from ._lib import NB_BF16, NB_F16, NB_F16_TERMS, NB_F32
 
 _DTYPE = {torch.float32: NB_F32, torch.float16: NB_F16, torch.bfloat16: NB_BF16}
 
@@ -326,7 +326,7 @@ def prefill_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
 
 
 def gemm_prefill(x: torch.Tensor, packed: torch.Tensor, codebook: torch.Tensor, bits: int, block_size: int,
-                 n: int, k: int, out_dtype: torch.dtype = torch.bfloat16, out: torch.Tensor | None = None) -> torch.Tensor:
+                 n: int, k: int, out_dtype: torch.dtype = torch.bfloat16, out: torch.Tensor | None = None, terms: bool = False) -> torch.Tensor:
     """y (M, n) = x (M, k) @ W.T on the tcgen05 tensor cores: W is dequantised once into the workspace, then
     the plain tensor-core kernel multiplies.  x bf16, fp16 or fp32; the library carries fp32 activations as two
     fp16 terms per element (about 22 significant bits, as in the GEMV) in adjacent operand rows and adds their
@@ -336,10 +336,12 @@ def gemm_prefill(x: torch.Tensor, packed: torch.Tensor, codebook: torch.Tensor, 
         raise RuntimeError(f"x must be a bf16, fp16 or fp32 (M, {k}) tensor; got {x.dtype} {tuple(x.shape)}")
     if not x.is_contiguous():
         x = x.contiguous()
-    m = x.shape[0]
+    m = x.shape[0] // 2 if terms else x.shape[0]
+    if terms and (x.dtype != torch.float16 or x.shape[0] % 2):
+        raise RuntimeError(f"terms must be an fp16 (2M, {k}) tensor; got {x.dtype} {tuple(x.shape)}")
     if out_dtype is None:
-        out_dtype = out.dtype if out is not None else x.dtype
-    if out is None and out_dtype == torch.float16:     # the kernel writes bf16 or fp32
+        out_dtype = out.dtype if out is not None else torch.float32 if terms else x.dtype
+    if out is None and out_dtype == torch.float16 and not terms:     # the kernel writes bf16 or fp32
         return gemm_prefill(x, packed, codebook, bits, block_size, n, k, out_dtype=torch.float32).half()
     if out is None:
         out = torch.empty(m, n, dtype=out_dtype, device=x.device)
@@ -347,17 +349,18 @@ def gemm_prefill(x: torch.Tensor, packed: torch.Tensor, codebook: torch.Tensor, 
     with torch.cuda.device(x.device):
         need = l.nb_prefill_workspace_bytes(m, n, k)
         ws = prefill_workspace(x.device, need)
-        _lib.check(l.nb_gemm_prefill(x.data_ptr(), _DTYPE[x.dtype], m, packed.data_ptr(), codebook.data_ptr(), _DTYPE[codebook.dtype], bits,
+        _lib.check(l.nb_gemm_prefill(x.data_ptr(), NB_F16_TERMS if terms else _DTYPE[x.dtype], m, packed.data_ptr(), codebook.data_ptr(), _DTYPE[codebook.dtype], bits,
                                      block_size, n, k, out.data_ptr(), _DTYPE[out.dtype], ws.data_ptr(), ws.numel(),
                                      _stream()), "nb_gemm_prefill")
     return out
 
 
 def gemm_prefill_fused(x: torch.Tensor, w_stream: torch.Tensor, bits: int, n: int, k: int,
-                       out_dtype: torch.dtype | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
+                       out_dtype: torch.dtype | None = None, out: torch.Tensor | None = None, terms: bool = False) -> torch.Tensor:
     """y (M, n) = x (M, k) @ W.T with the dequantisation fused into the tcgen05 kernel; w_stream is the
     stream-layout copy of the packed weight (stream.stream_pack).  x fp16, bf16 or fp32; the library carries
-    fp32 activations as two fp16 terms per element (rows 2i, 2i+1 of the operand) and adds their results."""
+    fp32 activations as two fp16 terms per element (rows 2i, 2i+1 of the operand) and adds their results.  terms: x is
+    (2M, k) fp16, those rows themselves."""
     _need_cuda(x, w_stream)
     if x.dim() != 2 or x.shape[1] != k:
         raise RuntimeError(f"x must be an (M, {k}) tensor; got {tuple(x.shape)}")
@@ -365,18 +368,20 @@ def gemm_prefill_fused(x: torch.Tensor, w_stream: torch.Tensor, bits: int, n: in
         raise RuntimeError(f"unsupported activation dtype {x.dtype}")
     if not x.is_contiguous():
         x = x.contiguous()
+    if terms and (x.dtype != torch.float16 or x.shape[0] % 2):
+        raise RuntimeError(f"terms must be an fp16 (2M, {k}) tensor; got {x.dtype} {tuple(x.shape)}")
     if out_dtype is None:
-        out_dtype = out.dtype if out is not None else x.dtype
-    if out is None and out_dtype == torch.float16:     # the kernel writes bf16 or fp32
+        out_dtype = out.dtype if out is not None else torch.float32 if terms else x.dtype
+    if out is None and out_dtype == torch.float16 and not terms:     # the kernel writes bf16 or fp32
         return gemm_prefill_fused(x, w_stream, bits, n, k, out_dtype=torch.float32).half()
-    m = x.shape[0]
+    m = x.shape[0] // 2 if terms else x.shape[0]
     if out is None:
         out = torch.empty(m, n, dtype=out_dtype, device=x.device)
     l = _lib.lib()
     with torch.cuda.device(x.device):
         need = int(l.nb_prefill_fused_workspace_bytes(m, n, k))
         ws = prefill_workspace(x.device, need)
-        _lib.check(l.nb_gemm_prefill_fused(x.data_ptr(), _DTYPE[x.dtype], m, w_stream.data_ptr(), bits, n, k, out.data_ptr(),
+        _lib.check(l.nb_gemm_prefill_fused(x.data_ptr(), NB_F16_TERMS if terms else _DTYPE[x.dtype], m, w_stream.data_ptr(), bits, n, k, out.data_ptr(),
                                            _DTYPE[out.dtype], ws.data_ptr(), ws.numel(), _stream()), "nb_gemm_prefill_fused")
     return out
 
@@ -499,3 +504,22 @@ def softcap_argmax(logits: torch.Tensor, cap: float, logits_out: torch.Tensor, t
 
 def silu_mul(gu: torch.Tensor, out: torch.Tensor) -> None:
     _lib.check(_lib.lib().nb_silu_mul(gu.data_ptr(), gu.shape[0], out.shape[1], out.data_ptr(), _stream()), "nb_silu_mul")
+
+
+def add_rmsnorm_terms(x: torch.Tensor, delta: torch.Tensor | None, w: torch.Tensor, eps: float, out: torch.Tensor) -> None:
+    """x (B, C) fp32 += delta; out (2B, C) fp16 = the two terms of every row of rmsnorm(x) * w, the prefill GEMMs' operand."""
+    for t in (x, out) if delta is None else (x, delta, out):
+        if not t.is_cuda or not t.is_contiguous():
+            raise RuntimeError("add_rmsnorm_terms needs contiguous CUDA tensors")
+    if x.dtype != torch.float32 or out.dtype != torch.float16 or out.numel() != 2 * x.numel() or (delta is not None and delta.shape != x.shape):
+        raise RuntimeError("add_rmsnorm_terms: x (B, C) fp32, delta alike, out (2B, C) fp16")
+    _lib.check(_lib.lib().nb_add_rmsnorm_terms(x.data_ptr(), 0 if delta is None else delta.data_ptr(), w.data_ptr(), eps, out.data_ptr(),
+                                               x.shape[0], x.shape[1], _stream()), "nb_add_rmsnorm_terms")
+
+
+def silu_mul_terms(gu: torch.Tensor, out: torch.Tensor) -> None:
+    """out (2B, F) fp16 = the two terms of silu(gate) * up for gu (B, 2F) fp32 = [gate | up]."""
+    if (gu.dtype != torch.float32 or out.dtype != torch.float16 or not gu.is_contiguous() or not out.is_contiguous()
+            or out.numel() != gu.numel()):
+        raise RuntimeError("silu_mul_terms: gu (B, 2F) fp32, out (2B, F) fp16, both contiguous")
+    _lib.check(_lib.lib().nb_silu_mul_terms(gu.data_ptr(), gu.shape[0], gu.shape[1] // 2, out.data_ptr(), _stream()), "nb_silu_mul_terms")

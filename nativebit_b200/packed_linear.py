@@ -118,6 +118,17 @@ class PackedLinear(torch.nn.Module):
                         (self.out_features, self.in_features), dtype=wdt)
         return x_flat @ w.T
 
+    def takes_terms(self, rows: int) -> bool:
+        """Whether `forward_terms` takes this many rows: those that forward would split into two fp16 terms itself."""
+        return rows > GEMV_MAX_M and self.block_size == BS and self.in_features % BS == 0 and self.bits in (2, 3, 4)
+
+    def forward_terms(self, terms, out=None):
+        """fp32 (M, out_features) of M fp32 rows given as their two fp16 terms, (2M, in_features); see ops.add_rmsnorm_terms."""
+        if terms.shape[0] > FUSED_MAX_ROWS:
+            return ops.gemm_prefill(terms, self.packed_indices, self.codebook, self.bits, self.block_size, self.out_features, self.in_features,
+                                    out_dtype=torch.float32, out=out, terms=True)
+        return ops.gemm_prefill_fused(terms, self.stream_weight(), self.bits, self.out_features, self.in_features, out=out, terms=True)
+
     def dequantized_weight(self, dtype=torch.float32):
         """The dense (out_features, in_features) weight; bit-exact gather of the codebook values."""
         return ops.dequant(self.packed_indices, self.codebook, self.bits, self.block_size,

@@ -159,3 +159,37 @@ def test_gemm_tiles_at_the_edges(built_lib, m, n, k):
         ref = x.double() @ W.double().T
         assert (y.double() - ref).abs().max() <= 2e-5 * ref.abs().max()
     assert ops.prefill_status(dev) == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(17, 200, 256), (64, 1000, 640), (513, 384, 4096), (700, 130, 128)])
+def test_operands_as_two_terms(built_lib, m, n, k):
+    """The norm and the SwiGLU that write the GEMMs' two fp16 terms, and both GEMMs on them, against the fp64 values: as exact
+    as from fp32 rows; the residual is updated in place."""
+    import nativebit_b200 as nbt
+    from nativebit_b200 import ops
+    dev = _dev()
+    packed, cb, _ = o.make_packed_linear(n, k, 3, seed=m)
+    lin = nbt.PackedLinear(torch.from_numpy(packed).to(dev), torch.from_numpy(cb).to(dev), n, k)
+    W = torch.from_numpy(o.dequant_packed(packed, cb.astype(np.float32), n, k, 3)).to(dev).double()
+    g = torch.Generator(device=dev).manual_seed(m)
+    x, d, gu = (torch.randn(m, c, device=dev, generator=g) for c in (k, k, 2 * k))
+    w = 1.0 + 0.1 * torch.randn(k, device=dev, generator=g)
+    terms = torch.empty(2 * m, k, dtype=torch.float16, device=dev)
+    for delta in (d, None):
+        xc = x.clone()
+        ops.add_rmsnorm_terms(xc, delta, w, 1e-6, terms)
+        v = x.double() + (0 if delta is None else delta.double())
+        want = v / torch.sqrt((v * v).mean(1, keepdim=True) + 1e-6) * w.double()
+        assert torch.equal(xc, x if delta is None else x + delta)
+        got = terms.double().view(m, 2, k).sum(1)
+        assert (got - want).abs().max() <= 2e-6 * want.abs().max()               # 22 bits and the norm's fp32 sums
+    y = lin.forward_terms(terms)
+    ref = want @ W.T
+    assert (y.double() - ref).abs().max() <= 2e-5 * ref.abs().max()
+    ops.silu_mul_terms(gu, terms)
+    gate, up = gu.double().split(k, 1)
+    want = gate * torch.sigmoid(gate) * up
+    assert (terms.double().view(m, 2, k).sum(1) - want).abs().max() <= 2e-6 * want.abs().max()     # __expf
+    y, ref = lin.forward_terms(terms), want @ W.T
+    torch.cuda.synchronize()
+    assert (y.double() - ref).abs().max() <= 2e-5 * ref.abs().max() and ops.prefill_status(dev) == 0
