@@ -207,6 +207,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
       int s = 0;           // ring position and its phase bit, carried across tiles
       uint32_t phase = 0;
       bool ok = true;
+      asm volatile("griddepcontrol.wait;" ::: "memory");      // barriers and tensor memory were set up beside the launch before
       for (int t = first; t < n_total && ok; t += step) {
         int mt, nt;
         gemm_tile(p, t, mt, nt);
@@ -414,13 +415,15 @@ static int launch_gemm(const void* x, int ldx, const void* w, int ldw, int K, bo
   cfg.blockDim = dim3(192);
   cfg.dynamicSmemBytes = GemmCfg::kSmem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = plan.cg;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   void* args[] = {&mx, &mw, &p};
   return record_cuda_error(cudaLaunchKernelExC(&cfg, fn, args));
 }
@@ -438,6 +441,7 @@ extern "C" size_t nb_prefill_workspace_bytes(int M, int N, int K) {
 namespace nb {
 // bf16 -> fp16, eight elements per thread, saturating to +-65504.
 __global__ void __launch_bounds__(256) bf16_to_f16_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, size_t n8) {
+  asm volatile("griddepcontrol.launch_dependents;");        // the GEMM behind it waits before it reads
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n8) return;
   const uint4 v = in[i];

@@ -511,8 +511,9 @@ extern "C" int nb_gemm_prefill_fused(const void* x, int x_dtype, int M, const ui
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  // ahead of its turn only behind this call's own conversion: whatever wrote the weights has then ended
-  cfg.numAttrs = xh != x ? 1 : 0;
+  // ahead of its turn only where the launch before wrote the activations, this call's own conversion or the kernel that wrote
+  // the terms: whatever wrote the weights has then ended
+  cfg.numAttrs = xh != x || x_dtype == NB_F16_TERMS ? 1 : 0;
   int y_tag = y_dtype, rows_arg = rows, n_arg = N, k_arg = K, bn_arg = bn, m_t = m_tiles, w_t = w_tiles, pair_arg = pair;
   void* args[] = {&mx, &mw, &y, &y_tag, &rows_arg, &n_arg, &k_arg, &bn_arg, &m_t, &w_t, &pair_arg, &ks, &partial, &status};
   if (cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args)) return record_cuda_error(e);

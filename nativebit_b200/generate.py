@@ -410,8 +410,9 @@ class DecodeSession(Session):
         """Room for the rows of this linear as two fp16 terms, if the step hands them over so."""
         return self.bterms[:2 * self.B * lin.in_features].view(2 * self.B, -1) if lin.takes_terms(self.B) and lin.in_features % 4 == 0 else None
 
-    def _terms_into(self, lin: PackedLinear, terms: torch.Tensor, out: torch.Tensor) -> None:
-        ops.gemm_prefill_fused(terms, lin.stream_weight(), lin.bits, lin.out_features, lin.in_features, out=out, terms=True)
+    def _terms_into(self, lin: PackedLinear, w: torch.Tensor, terms: torch.Tensor, out: torch.Tensor) -> None:
+        """w: lin.stream_weight(), asked for before the launch that wrote the terms."""
+        ops.gemm_prefill_fused(terms, w, lin.bits, lin.out_features, lin.in_features, out=out, terms=True)
 
     def _linear_into(self, lin: PackedLinear, x: torch.Tensor, out: torch.Tensor) -> None:
         """out = lin(x) for a batch of rows: up to 16 through the fused GEMV, more through the tensor-core
@@ -465,8 +466,9 @@ class DecodeSession(Session):
                 ops.gemv_fused(ops.PRO_ADD_RMSNORM, xa, *args, out, delta=delta, norm_weight=w, eps=eps, x_out=xb)
                 xa, xb = xb, xa
             elif (terms := self._terms_of(lin)) is not None and lin.in_features <= 4096:
+                packed = lin.stream_weight()
                 ops.add_rmsnorm_terms(xa, delta, w, eps, terms)
-                self._terms_into(lin, terms, out)
+                self._terms_into(lin, packed, terms, out)
             else:
                 ops.add_rmsnorm(xa, delta, w, eps, self.bh)
                 self._linear_into(lin, self.bh, out)
@@ -491,8 +493,9 @@ class DecodeSession(Session):
             elif prologue == ops.PRO_SILU_MUL and fold:
                 ops.gemv_fused(prologue, x, *args, out)
             elif prologue == ops.PRO_SILU_MUL and (terms := self._terms_of(lin)) is not None:
+                packed = lin.stream_weight()
                 ops.silu_mul_terms(x, terms)
-                self._terms_into(lin, terms, out)
+                self._terms_into(lin, packed, terms, out)
             elif prologue == ops.PRO_SILU_MUL:
                 ops.silu_mul(x, self.bhm)
                 self._linear_into(lin, self.bhm, out)

@@ -127,6 +127,9 @@ class PackedLinear(torch.nn.Module):
         if terms.shape[0] > FUSED_MAX_ROWS:
             return ops.gemm_prefill(terms, self.packed_indices, self.codebook, self.bits, self.block_size, self.out_features, self.in_features,
                                     out_dtype=torch.float32, out=out, terms=True)
+        if getattr(self, "_wstream", None) is None:
+            self.stream_weight()
+            terms = terms.clone()           # a launch between the packing and the GEMM, which starts beside the launch before it
         return ops.gemm_prefill_fused(terms, self.stream_weight(), self.bits, self.out_features, self.in_features, out=out, terms=True)
 
     def dequantized_weight(self, dtype=torch.float32):
