@@ -488,6 +488,9 @@ class DecodeSession(Session):
             if self.tile_gemv:
                 ops.gemv_stream(prologue, x, lin.stream_weight(), lin.bits, lin.out_features, lin.in_features, out,
                                 single_term=self.single_term)
+            elif self.tile_rows and prologue == ops.PRO_NONE and self.B > 2 * ops.gemv_stream_max_rows(lin.bits, lin.in_features):
+                # three launches over the same weights (8 rows of 6912: 25 us) take longer than the tensor-core kernel (14 us)
+                ops.gemm_prefill_fused(x, lin.stream_weight(), lin.bits, lin.out_features, lin.in_features, out=out)
             elif self.tile_rows:
                 ops.gemv_stream_rows(prologue, x, lin.stream_weight(), lin.bits, lin.out_features, lin.in_features, out)
             elif prologue == ops.PRO_SILU_MUL and fold:
