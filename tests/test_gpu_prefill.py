@@ -193,3 +193,20 @@ def test_operands_as_two_terms(built_lib, m, n, k):
     y, ref = lin.forward_terms(terms), want @ W.T
     torch.cuda.synchronize()
     assert (y.double() - ref).abs().max() <= 2e-5 * ref.abs().max() and ops.prefill_status(dev) == 0
+
+
+@pytest.mark.parametrize("bits,m,n,k", [(3, 240, 19000, 384), (4, 256, 19100, 128), (2, 100, 19000, 640), (3, 33, 19000, 384)])
+def test_fused_dequant_gemm_many_tiles_per_cta(built_lib, bits, m, n, k):
+    """More tiles than SMs with an odd number of k-blocks: the rings of operand and raw stages carry on from tile to tile out of
+    step with each other, with two raw stages (more than 224 columns) and with four."""
+    from nativebit_b200 import ops, stream as S
+    dev = _dev()
+    packed, cb, _ = o.make_packed_linear(n, k, bits, seed=m)
+    w = S.stream_pack(torch.from_numpy(packed).to(dev), torch.from_numpy(cb).to(dev), bits, n, k)
+    x = torch.from_numpy(o.make_activation(m, k, seed=m)).to(dev).bfloat16()
+    y = ops.gemm_prefill_fused(x, w, bits, n, k, out_dtype=torch.float32)
+    torch.cuda.synchronize()
+    W = torch.from_numpy(o.dequant_packed(packed, cb.astype(np.float32), n, k, bits)).to(dev)
+    ref = x.double() @ W.double().T
+    assert ops.prefill_status(dev) == 0
+    assert (y.double() - ref).abs().max() <= 2e-5 * ref.abs().max()
