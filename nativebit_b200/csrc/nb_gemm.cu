@@ -143,16 +143,15 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// a / (1 + e^-x) to the last bit or two without the division's branches, which run the 16 pairs of a chunk one after the
-// other (2 x 10 us per 128 x 160 tile, more than the tile's products): the reciprocal by one Newton step, the quotient by its
-// residual.  e^87 keeps the divisor finite, an infinite quotient its value.
+// a / (1 + e^-x) without the branches of a full-range division, which run the 16 pairs of a chunk one after the other (2 x 10 us
+// per 128 x 160 tile, more than the tile's products).  With e = e^-|x| the divisor 1 + e lies in [1, 2], well inside the range
+// of __fdividef (2 ulp), for every x: a gate far below zero gives zero, one of -inf NaN, as the plain quotient does.
+// One step of iterative refinement (the residual of the quotient over the same divisor, Wilkinson 1963) takes the two ulps
+// off; a residual that is zero or no number (infinite quotients) leaves the quotient with its sign.
 __device__ __forceinline__ float times_sigmoid(float a, float x) {
-  const float d = 1.0f + __expf(fminf(-x, 87.0f));
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-  r = fmaf(fmaf(-d, r, 1.0f), r, r);
-  const float q = a * r;
-  return fabsf(q) <= FLT_MAX ? fmaf(fmaf(-d, q, a), r, q) : q;
+  const float e = __expf(-fabsf(x)), d = 1.0f + e, n = x < 0.0f ? a * e : a;
+  const float q = __fdividef(n, d), c = __fdividef(fmaf(-d, q, n), d);
+  return fabsf(c) > 0.0f ? q + c : q;
 }
 
 // silu(gate) * up, or the clamped form (alpha, limit)

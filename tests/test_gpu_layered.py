@@ -86,6 +86,43 @@ def test_linear(dev, m, n, k, dtype):
         close(act[:, :n // 2], ref, max(TOL[dtype], 1e-5))
 
 
+@pytest.mark.parametrize("m", [3, 130])
+@pytest.mark.parametrize("clamped", [False, True])
+def test_gated_epilogue_over_all_gates(dev, m, clamped):
+    """The tensor-core epilogue's sigmoid quotient against 64 bits from -200 to 200, and against the plain quotient of the
+    fp32 product where gates are huge, infinite or no number: the products are zero, the biases are the gates."""
+    from nativebit_b200 import layer_ops as L
+    act = L.Act(L.ACT_CLAMPED_GLU_PAIRS, 1.702, 150.0) if clamped else L.SWIGLU
+    far = [s * v for v in (86.9, 87.0, 87.1, 88.0, 1e30, 1e36, 3.3e38, float("inf")) for s in (-1, 1)] + [float("nan")]
+    gate = torch.cat((torch.linspace(-200, 200, 4001), torch.tensor(far))).to(dev)
+    bias = torch.stack((gate, torch.full_like(gate, 1.5)), 1).flatten()
+    n, k = bias.numel(), 64
+    w = torch.zeros(n, k, dtype=BF16, device=dev)
+    got = {}
+    for x_dtype, out_dtype in ((BF16, F32), (BF16, BF16), (F32, F32)):
+        x = torch.ones(m, k, dtype=x_dtype, device=dev)
+        out = L.rows_empty(m, n // 2, out_dtype, dev)
+        L.linear(x, w, k, n, out, bias=bias, act=act)
+        assert (torch.isnan(out[:, :n // 2]) == torch.isnan(out[0, :n // 2])).all()
+        got[x_dtype, out_dtype] = out[m - 1, :n // 2].double()
+    assert int(L.linear_status(dev).item()) == 0
+    g = torch.fmin(gate, torch.tensor(150.0, device=dev)).double() if clamped else gate.double()
+    z, up = (1.702 * g, 2.5) if clamped else (g, 1.5)
+    want = g / (1 + torch.exp(-z)) * up
+    want = torch.where(want.abs() > 3.4e38, torch.sign(want) * float("inf"), want)             # past fp32
+    y, plain = got[BF16, F32], got[F32, F32]
+    assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.equal(torch.isnan(plain), torch.isnan(want))
+    ok = ~torch.isnan(want) & ~torch.isinf(want)
+    assert torch.equal(y[torch.isinf(want)], want[torch.isinf(want)])
+    # __expf: 2 + 1.173 |z| ulp; the products, the sum and the quotient half an ulp each; 1e-35: results among the subnormals
+    limit = (5.0 + 1.2 * z.abs().clamp(max=200)) * 2.0 ** -23 * want.abs() + 1e-35
+    assert ((y - want).abs() <= limit)[ok].all()
+    near = ok & (z.abs() < 1)                                       # the quotient itself, where e^z is all but exact
+    assert ((y - want).abs() <= 5 * 2.0 ** -23 * want.abs())[near].all()
+    b = got[BF16, BF16]
+    assert torch.equal(torch.isnan(b), torch.isnan(want)) and ((b - want).abs() <= 2.0 ** -8 * want.abs() + 1e-35)[ok].all()
+
+
 @pytest.mark.parametrize("n,k", [(1, 8), (6, 50), (131, 72), (148, 256), (150, 257), (700, 264), (4000, 1000), (3001, 2560), (64, 7000)])
 def test_matvec(dev, n, k):
     from nativebit_b200 import layer_ops as L
