@@ -5,6 +5,8 @@ libnativebit_b200.so.  Every function requires CUDA tensors and raises otherwise
 """
 from __future__ import annotations
 
+from typing import NamedTuple
+
 import torch
 
 from . import _lib
@@ -120,13 +122,35 @@ _workspaces: dict = {}
 _ws_need: dict = {}
 
 
+def _scratch_key(device: torch.device) -> tuple:
+    return (device.index if device.index is not None else torch.cuda.current_device(), _stream())
+
+
+def _grown(ws: torch.Tensor | None, nbytes: int, device: torch.device) -> torch.Tensor:
+    """A zeroed workspace in place of `ws`.  At least twice as large: holders of captured graphs keep the ones it replaces
+    (`scratch`), which together then take no more than the last."""
+    return torch.zeros(max(nbytes, 0 if ws is None else 2 * ws.numel()), dtype=torch.uint8, device=device)
+
+
+class Scratch(NamedTuple):
+    """The workspaces of one stream (None: not needed yet)."""
+    gemv: torch.Tensor | None
+    prefill: torch.Tensor | None
+
+
+def scratch(device: torch.device) -> Scratch:
+    """The workspaces that launches on torch's current stream use now.  A launch that needs more replaces them, and a CUDA
+    graph holds their addresses only: whoever captures one keeps this beside it for as long as the graph is replayed."""
+    key = _scratch_key(device)
+    return Scratch(_workspaces.get(key), _prefill_ws.get(key))
+
+
 def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     """Zero-initialised scratch for split-K launches, one per (device, stream), grown on demand."""
-    key = (device.index if device.index is not None else torch.cuda.current_device(), _stream())
+    key = _scratch_key(device)
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < nbytes:
-        ws = torch.zeros(max(nbytes, 4 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
+        ws = _workspaces[key] = _grown(ws, max(nbytes, 4 << 20), device)
     return ws
 
 
@@ -316,12 +340,11 @@ _prefill_ws: dict = {}
 
 
 def prefill_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    """Scratch for the dequantised bf16 weight of the prefill GEMM, one per (device, stream)."""
-    key = (device.index if device.index is not None else torch.cuda.current_device(), _stream())
+    """Scratch of the prefill GEMMs (fp16 operand, dequantised weight, k-split sums), one per (device, stream), grown on demand."""
+    key = _scratch_key(device)
     ws = _prefill_ws.get(key)
     if ws is None or ws.numel() < nbytes:
-        ws = torch.zeros(nbytes, dtype=torch.uint8, device=device)
-        _prefill_ws[key] = ws
+        ws = _prefill_ws[key] = _grown(ws, nbytes, device)
     return ws
 
 
@@ -388,8 +411,7 @@ def gemm_prefill_fused(x: torch.Tensor, w_stream: torch.Tensor, bits: int, n: in
 
 def prefill_status(device) -> int:
     """Status word of the prefill workspace of the current stream (0, or NB_ERR_TIMEOUT); synchronises."""
-    key = (torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device(), _stream())
-    ws = _prefill_ws.get(key)
+    ws = _prefill_ws.get(_scratch_key(torch.device(device)))
     return 0 if ws is None else int(ws[:4].view(torch.int32).item())
 
 

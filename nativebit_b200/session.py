@@ -9,6 +9,8 @@ from __future__ import annotations
 
 import torch
 
+from . import ops
+
 
 class Session:
     def __init__(self, model, batch_size: int, context_len: int, vocab_size: int, device, use_graph: bool = True):
@@ -22,6 +24,7 @@ class Session:
         self.graph = None
         self._prefill_graphs = {}             # prompt length -> (captured prefill, its static input)
         self.stream = torch.cuda.Stream(device=device) if torch.device(device).type == "cuda" else None
+        self._scratch = []                    # the workspaces that the captured graphs were captured with
 
     # ---- what a model family provides
     def _prefill_body(self, prompt: torch.Tensor) -> None:
@@ -46,6 +49,13 @@ class Session:
         """Raises if a bounded wait inside one of the kernels ever ran out."""
 
     # ---- the loop
+    def _keep_scratch(self) -> None:
+        """Right after a capture, on its stream: the graph's workspaces live as long as the session, also when a longer prompt
+        replaces them for the launches that follow."""
+        held = ops.scratch(torch.device(self.dev))
+        if not any(all(a is b for a, b in zip(held, s)) for s in self._scratch):
+            self._scratch.append(held)
+
     def reset(self) -> None:
         """Back to an empty sequence: the cache and state of the one before are given back."""
         self.pos.zero_()
@@ -74,6 +84,7 @@ class Session:
                     g = torch.cuda.CUDAGraph()
                     with torch.cuda.graph(g, stream=self.stream):
                         self._prefill_body(static_in)
+                    self._keep_scratch()
                 cur.wait_stream(self.stream)
                 self._prefill_graphs[T] = (g, static_in)
             else:
@@ -128,6 +139,7 @@ class Session:
                 self.graph = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(self.graph, stream=self.stream):
                     self._step_body()
+                self._keep_scratch()
                 # the capture does not execute: state is unchanged; stale cache slots past `pos` are masked
             torch.cuda.current_stream().wait_stream(self.stream)
         self.graph.replay()

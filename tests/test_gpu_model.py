@@ -406,3 +406,29 @@ def test_decode_attention_one_cta_per_head(built_lib, B, H, hd, ctx):
             ref = torch.einsum("bhj,bhjd->bhd", torch.softmax(sc, -1), vv[:, :, :p_ + 1].double()).reshape(B, H * hd)
             assert (got.double() - ref).abs().max() <= 2e-5 * ref.abs().max(), p_          # fp32 sums, __expf
         assert (rot[:, :4] == 7.0).all() and (rot[:, -4:] == 7.0).all()
+
+
+@pytest.mark.parametrize("B", [8, 20])
+def test_captured_steps_outlive_a_longer_prompt(built_lib, B):
+    """A step is captured, then a longer prompt makes the session's stream replace its workspace: the step replays on the one
+    it was captured with, and its logits equal the eager session's."""
+    from nativebit_b200 import generate as G, ops
+    dev = torch.device("cuda:0")
+    cfg = G.ModelConfig(vocab_size=512, n_layers=2, n_embd=512, n_head=4, ffn_hidden=6912, context_len=256)
+    model = G.PackedGPT.random_init(cfg, seed=5, device=dev)
+    toks = torch.randint(0, cfg.vocab_size, (B, 130), generator=torch.Generator().manual_seed(B)).to(dev)
+    a, b = G.DecodeSession(model, B), G.DecodeSession(model, B, use_graph=False)
+    for s in (a, b):
+        s.prefill(toks[:, :3])
+        s.step()
+    with torch.cuda.stream(a.stream):
+        before = ops.scratch(dev).prefill
+    a.prefill(toks); b.prefill(toks)
+    with torch.cuda.stream(a.stream):
+        after = ops.scratch(dev).prefill
+    assert after is not before and any(h.prefill is before for h in a._scratch) and any(h.prefill is after for h in a._scratch)
+    for _ in range(3):
+        a.step(); b.step()
+        assert torch.equal(a.logits, b.logits) and torch.equal(a.token, b.token)
+    a.prefill(toks[:, :3]); b.prefill(toks[:, :3])                  # the prompt's graph of before, on the workspace of before
+    assert torch.equal(a.logits, b.logits)

@@ -217,3 +217,63 @@ def test_layered_argument_checks_need_no_gpu(layered_lib):
     assert l.nb_latent_attention(ctypes.byref(_lib.LatentAttentionArgs(**{**t, "vdim": 300})), None) == 3
     assert l.nb_latent_attention(ctypes.byref(_lib.LatentAttentionArgs(**{**t, "rot": 3})), None) == 1
     assert l.nb_argmax(None, 1, 8, fake, None, None) == 1
+
+
+def test_sessions_keep_the_workspaces_of_their_graphs(monkeypatch):
+    """A captured step holds its workspace by address: when a later call on the session's stream needs more, the one the
+    graph was captured with lives on with the session, and the replacements add up to little more than the last."""
+    import contextlib
+    import gc
+    import weakref
+    import torch
+    from nativebit_b200 import ops
+    from nativebit_b200.session import Session
+    dev = torch.device("cpu", 0)
+
+    class Stream:
+        def wait_stream(self, other): pass
+        def synchronize(self): pass
+
+    class Graph:
+        def replay(self): pass
+    for name, fake in (("current_stream", lambda *a: Stream()), ("stream", lambda s: contextlib.nullcontext()), ("CUDAGraph", Graph),
+                       ("graph", lambda g, stream: contextlib.nullcontext())):
+        monkeypatch.setattr(torch.cuda, name, fake)
+    monkeypatch.setattr(ops, "_stream", lambda: 12345)
+    monkeypatch.setattr(ops, "_prefill_ws", {})
+    monkeypatch.setattr(ops, "_workspaces", {})
+    used = []
+
+    class Steps(Session):
+        def _step_body(self):
+            used.append((weakref.ref(ops.prefill_workspace(dev, 1000)), weakref.ref(ops.workspace(dev, 1 << 10))))
+    s = Steps(None, 1, 16, 8, dev)
+    s.stream = Stream()
+    s.step()
+    for need in range(2000, 100000, 1000):
+        ops.prefill_workspace(dev, need)
+        ops.workspace(dev, need << 10)
+    gc.collect()
+    assert ops._prefill_ws[0, 12345].numel() >= 99000 and all(ref() is not None for ref in used[-1])
+    assert ops._prefill_ws[0, 12345].numel() < 2 * 99000
+    s.step()
+    del s
+    gc.collect()
+    assert all(ref() is None for ref in used[-1])
+
+
+def test_session_scratch_is_bounded_over_ascending_prompts(monkeypatch):
+    """One workspace per captured prompt length, each a little longer than the one before: held ones add up to a small multiple
+    of the largest need."""
+    import torch
+    from nativebit_b200 import ops
+    from nativebit_b200.session import Session
+    dev = torch.device("cpu", 0)
+    monkeypatch.setattr(ops, "_stream", lambda: 12345)
+    monkeypatch.setattr(ops, "_prefill_ws", {})
+    monkeypatch.setattr(ops, "_workspaces", {})
+    s = Session(None, 1, 16, 8, dev)
+    for need in range(1000, 100000, 1000):
+        ops.prefill_workspace(dev, need)
+        s._keep_scratch()
+    assert sum(h.prefill.numel() for h in s._scratch) <= 4 * 99000
