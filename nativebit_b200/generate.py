@@ -581,11 +581,12 @@ class DecodeSession(Session):
         tensor-parallel exchange that never arrived).  Reads device status words: synchronises."""
         if self.prog is not None and self.prog.status() != 0:
             raise RuntimeError("nb_stream_run: a bounded wait ran out (status NB_ERR_TIMEOUT in the program state)")
+        held = list(self._scratch)               # what the graphs replay on, and the workspaces of the streams the steps ran on
         for st in ((self.stream, torch.cuda.current_stream(self.dev)) if self.use_graph else (torch.cuda.current_stream(self.dev),)):
-            with torch.cuda.stream(st):          # the workspace of the stream the steps ran on
-                ws = ops.workspace(self.model.embedding.device, 0)
-            if ops.workspace_status(ws) != 0:
-                raise RuntimeError("nb_gemv: a bounded wait ran out (status NB_ERR_TIMEOUT in the workspace)")
+            with torch.cuda.stream(st):
+                held.append(ops.scratch(self.model.embedding.device))
+        for name in sum((ops.timed_out(h) for h in held), []):
+            raise RuntimeError(f"{name}: a bounded wait ran out (status NB_ERR_TIMEOUT in the workspace)")
         for name in ("oneshot", "head_ar", "exchange"):
             obj = getattr(self.model, name, None)
             if obj is not None and int(obj.status.item()) != 0:

@@ -122,6 +122,10 @@ _workspaces: dict = {}
 _ws_need: dict = {}
 
 
+def _status_word(ws: torch.Tensor, at: int) -> int:
+    return int(ws[at:at + 4].view(torch.int32).item())
+
+
 def _scratch_key(device: torch.device) -> tuple:
     return (device.index if device.index is not None else torch.cuda.current_device(), _stream())
 
@@ -156,7 +160,13 @@ def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
 
 def workspace_status(ws: torch.Tensor) -> int:
     """The status word of a GEMV workspace (0, or NB_ERR_TIMEOUT = 6 if a bounded wait ran out); synchronises."""
-    return int(ws[4095 * 4:4096 * 4].view(torch.int32).item())
+    return _status_word(ws, 4095 * 4)
+
+
+def timed_out(held: Scratch) -> list[str]:
+    """The kernels of which a bounded wait ran out on these workspaces; synchronises."""
+    found = ["nb_gemv"] if held.gemv is not None and workspace_status(held.gemv) else []
+    return found + (["nb_gemm_prefill"] if held.prefill is not None and _status_word(held.prefill, 0) else [])
 
 
 def gemv_workspace_bytes(m: int, n: int, k: int, bits: int, block_size: int) -> int:
@@ -412,7 +422,7 @@ def gemm_prefill_fused(x: torch.Tensor, w_stream: torch.Tensor, bits: int, n: in
 def prefill_status(device) -> int:
     """Status word of the prefill workspace of the current stream (0, or NB_ERR_TIMEOUT); synchronises."""
     ws = _prefill_ws.get(_scratch_key(torch.device(device)))
-    return 0 if ws is None else int(ws[:4].view(torch.int32).item())
+    return 0 if ws is None else _status_word(ws, 0)
 
 
 def gemm_bf16(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16) -> torch.Tensor:

@@ -365,6 +365,29 @@ def test_batched_decode_step_on_the_rows_kernel_equals_the_workspace_kernels(bui
     assert torch.equal(toks_g, toks_e)
 
 
+@pytest.mark.parametrize("B,tensor_cores", [(6, False), (7, True), (8, True)])
+def test_batched_step_with_a_wide_down_projection(built_lib, B, tensor_cores):
+    """Shared memory holds three rows of 6912: from seven sequences on the down projection goes to the tensor-core kernel.  Against
+    the session on nb_gemv_fused, eager and from a graph."""
+    from nativebit_b200 import generate as G, ops
+    dev = _dev()
+    cfg = G.ModelConfig(vocab_size=512, n_layers=2, n_embd=512, n_head=4, ffn_hidden=6912, context_len=64)
+    assert (B > 2 * ops.gemv_stream_max_rows(cfg.bits, cfg.ffn_hidden)) == tensor_cores
+    model = G.PackedGPT.random_init(cfg, seed=5, device=dev)
+    prompt = torch.randint(0, cfg.vocab_size, (B, 7), generator=torch.Generator().manual_seed(B)).to(dev)
+    a, g = G.DecodeSession(model, B, use_graph=False), G.DecodeSession(model, B)
+    b = G.DecodeSession(model, B, use_graph=False, tile_gemv=False)
+    for s in (a, g, b):
+        s.prefill(prompt)
+    for _ in range(6):
+        for s in (a, g, b):
+            s.step()
+        assert torch.equal(a.token, b.token) and torch.equal(a.logits, g.logits)
+        assert (a.logits - b.logits).abs().max() <= 1e-4 * b.logits.abs().max()
+    for s in (a, g, b):
+        s.check()
+
+
 @pytest.mark.parametrize("bits,n,k,m", [(3, 7680, 2560, 8), (3, 2560, 6912, 3), (3, 13824, 2560, 5), (3, 1000, 640, 2), (2, 2560, 2560, 7),
                                         (4, 512, 1280, 4), (3, 320, 384, 8), (3, 40, 7168, 1), (3, 2560, 6912, 8)])
 def test_chain_gemv_rows(built_lib, bits, n, k, m):

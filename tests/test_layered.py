@@ -277,3 +277,37 @@ def test_session_scratch_is_bounded_over_ascending_prompts(monkeypatch):
         ops.prefill_workspace(dev, need)
         s._keep_scratch()
     assert sum(h.prefill.numel() for h in s._scratch) <= 4 * 99000
+
+
+@pytest.mark.parametrize("where", ["current", "session", "replaced"])
+@pytest.mark.parametrize("kind,word", [("prefill", 0), ("gemv", 4095)])
+def test_check_reads_every_workspace_of_the_session(monkeypatch, where, kind, word):
+    """A bounded wait that ran out in the tensor-core kernel or in the matvec is reported, whichever of the session's
+    workspaces its status word is in."""
+    import contextlib
+    import types
+    import torch
+    from nativebit_b200 import generate as G, ops
+    dev, at = torch.device("cpu", 0), [1]
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: 1)
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext(at.__setitem__(0, s)))
+    monkeypatch.setattr(ops, "_stream", lambda: at[0])
+    monkeypatch.setattr(ops, "_prefill_ws", {})
+    monkeypatch.setattr(ops, "_workspaces", {})
+    s = G.DecodeSession.__new__(G.DecodeSession)
+    s.prog, s.use_graph, s.stream, s.dev, s._scratch = None, True, 2, dev, []
+    s.model = types.SimpleNamespace(embedding=types.SimpleNamespace(device=dev))
+
+    def grow(stream, n):
+        at[0] = stream
+        ops.prefill_workspace(dev, n), ops.workspace(dev, n << 10)
+    grow(1, 1000), grow(2, 1000)
+    s._keep_scratch()
+    s.check()
+    at[0] = 1 if where == "current" else 2
+    held = ops.scratch(dev)
+    if where == "replaced":
+        grow(2, 9000)
+    getattr(held, kind)[4 * word:4 * word + 4].view(torch.int32).fill_(6)
+    with pytest.raises(RuntimeError, match="nb_gemm_prefill" if kind == "prefill" else "nb_gemv"):
+        s.check()
