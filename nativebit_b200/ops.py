@@ -393,7 +393,8 @@ def gemm_prefill_fused(x: torch.Tensor, w_stream: torch.Tensor, bits: int, n: in
     """y (M, n) = x (M, k) @ W.T with the dequantisation fused into the tcgen05 kernel; w_stream is the
     stream-layout copy of the packed weight (stream.stream_pack).  x fp16, bf16 or fp32; the library carries
     fp32 activations as two fp16 terms per element (rows 2i, 2i+1 of the operand) and adds their results.  terms: x is
-    (2M, k) fp16, those rows themselves."""
+    (2M, k) fp16, those rows themselves; the kernel then starts beside the launch before it on the stream, which may have
+    written x but not w_stream (a weight packed just now needs another launch in between)."""
     _need_cuda(x, w_stream)
     if x.dim() != 2 or x.shape[1] != k:
         raise RuntimeError(f"x must be an (M, {k}) tensor; got {tuple(x.shape)}")
@@ -540,18 +541,22 @@ def silu_mul(gu: torch.Tensor, out: torch.Tensor) -> None:
 
 def add_rmsnorm_terms(x: torch.Tensor, delta: torch.Tensor | None, w: torch.Tensor, eps: float, out: torch.Tensor) -> None:
     """x (B, C) fp32 += delta; out (2B, C) fp16 = the two terms of every row of rmsnorm(x) * w, the prefill GEMMs' operand."""
-    for t in (x, out) if delta is None else (x, delta, out):
-        if not t.is_cuda or not t.is_contiguous():
-            raise RuntimeError("add_rmsnorm_terms needs contiguous CUDA tensors")
-    if x.dtype != torch.float32 or out.dtype != torch.float16 or out.numel() != 2 * x.numel() or (delta is not None and delta.shape != x.shape):
-        raise RuntimeError("add_rmsnorm_terms: x (B, C) fp32, delta alike, out (2B, C) fp16")
+    _need_cuda(*(t for t in (x, delta, w, out) if t is not None))
+    if x.dtype != torch.float32 or x.dim() != 2 or (delta is not None and (delta.dtype != torch.float32 or delta.shape != x.shape)):
+        raise RuntimeError("add_rmsnorm_terms: x (B, C) must be fp32, delta alike")
+    if w.dtype != torch.float32 or w.numel() != x.shape[1]:
+        raise RuntimeError(f"add_rmsnorm_terms: w must be {x.shape[1]} fp32 values; got {w.dtype} {tuple(w.shape)}")
+    if out.dtype != torch.float16 or out.numel() != 2 * x.numel() or out.shape[-1] != x.shape[1]:
+        raise RuntimeError(f"add_rmsnorm_terms: out must be fp16 {(2 * x.shape[0], x.shape[1])}; got {out.dtype} {tuple(out.shape)}")
     _lib.check(_lib.lib().nb_add_rmsnorm_terms(x.data_ptr(), 0 if delta is None else delta.data_ptr(), w.data_ptr(), eps, out.data_ptr(),
                                                x.shape[0], x.shape[1], _stream()), "nb_add_rmsnorm_terms")
 
 
 def silu_mul_terms(gu: torch.Tensor, out: torch.Tensor) -> None:
     """out (2B, F) fp16 = the two terms of silu(gate) * up for gu (B, 2F) fp32 = [gate | up]."""
-    if (gu.dtype != torch.float32 or out.dtype != torch.float16 or not gu.is_contiguous() or not out.is_contiguous()
-            or out.numel() != gu.numel()):
-        raise RuntimeError("silu_mul_terms: gu (B, 2F) fp32, out (2B, F) fp16, both contiguous")
+    _need_cuda(gu, out)
+    if gu.dtype != torch.float32 or gu.dim() != 2 or gu.shape[1] % 2:
+        raise RuntimeError(f"silu_mul_terms: gu must be fp32 (B, 2F); got {gu.dtype} {tuple(gu.shape)}")
+    if out.dtype != torch.float16 or out.numel() != gu.numel() or out.shape[-1] != gu.shape[1] // 2:
+        raise RuntimeError(f"silu_mul_terms: out must be fp16 {(2 * gu.shape[0], gu.shape[1] // 2)}; got {out.dtype} {tuple(out.shape)}")
     _lib.check(_lib.lib().nb_silu_mul_terms(gu.data_ptr(), gu.shape[0], gu.shape[1] // 2, out.data_ptr(), _stream()), "nb_silu_mul_terms")

@@ -104,7 +104,7 @@ class PackedLinear(torch.nn.Module):
         """M > 16 rows on the tcgen05 kernels (exact fp16 weights; bf16 and fp16 activations as given, fp32
         carried as two fp16 terms; fp32 accumulation; result in x's dtype): one pass over the packed weights,
         dequantised inside the kernel, up to FUSED_MAX_ROWS rows; dequantise-once + GEMM beyond."""
-        if self.in_features % BS == 0 and self.bits in (2, 3, 4):
+        if self._tensor_cores():
             rows = x_flat.shape[0] * (2 if x_flat.dtype == torch.float32 else 1)
             if rows > FUSED_MAX_ROWS:
                 # long inputs: dequantising W once into a scratch copy (12 us for 6912 x 2560) and running the plain
@@ -118,12 +118,17 @@ class PackedLinear(torch.nn.Module):
                         (self.out_features, self.in_features), dtype=wdt)
         return x_flat @ w.T
 
+    def _tensor_cores(self) -> bool:
+        return self.block_size == BS and self.in_features % BS == 0 and self.bits in (2, 3, 4)
+
     def takes_terms(self, rows: int) -> bool:
-        """Whether `forward_terms` takes this many rows: those that forward would split into two fp16 terms itself."""
-        return rows > GEMV_MAX_M and self.block_size == BS and self.in_features % BS == 0 and self.bits in (2, 3, 4)
+        """Whether forward would split this many fp32 rows into two fp16 terms itself, so that `forward_terms` may take them."""
+        return rows > GEMV_MAX_M and self._tensor_cores()
 
     def forward_terms(self, terms, out=None):
         """fp32 (M, out_features) of M fp32 rows given as their two fp16 terms, (2M, in_features); see ops.add_rmsnorm_terms."""
+        if not self._tensor_cores():
+            raise RuntimeError(f"forward_terms needs 2 to 4 bits, blocks of {BS} and a multiple of {BS} columns: {self.extra_repr()}")
         if terms.shape[0] > FUSED_MAX_ROWS:
             return ops.gemm_prefill(terms, self.packed_indices, self.codebook, self.bits, self.block_size, self.out_features, self.in_features,
                                     out_dtype=torch.float32, out=out, terms=True)

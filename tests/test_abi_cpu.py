@@ -87,6 +87,33 @@ def test_python_wrappers_refuse_cpu_tensors(built_lib):
         lin(torch.zeros(1, 128))
 
 
+def test_operand_terms_wrappers_check_their_tensors(monkeypatch):
+    """Nothing but what the kernels take reaches them: device, dtypes, rows and lengths of the two-term operand's writers."""
+    import torch
+    import nativebit_b200 as nbt
+    from nativebit_b200 import ops
+
+    class OnGpu(torch.Tensor):
+        is_cuda = True
+
+    def t(*shape, dtype=torch.float32):
+        return torch.zeros(*shape, dtype=dtype).as_subclass(OnGpu)
+    monkeypatch.setattr(ops._lib, "lib", lambda: pytest.fail("reached the kernel"))
+    half = torch.float16
+    for gu, out in ((torch.zeros(4, 64), torch.zeros(8, 32, dtype=half)), (t(4, 64), torch.zeros(8, 32, dtype=half)), (t(4, 64), t(4, 64, dtype=half)),
+                    (t(4, 64), t(8, 32)), (t(4, 64).t(), t(8, 32, dtype=half)), (t(256), t(8, 32, dtype=half)), (t(4, 64), t(6, 32, dtype=half))):
+        with pytest.raises(RuntimeError):
+            ops.silu_mul_terms(gu, out)
+    x, w, out = t(4, 64), t(64), t(8, 64, dtype=half)
+    for args in ((x, None, torch.zeros(64), out), (x, None, w[:60], out), (x, None, w.half(), out), (x, None, t(128)[::2], out), (x, x.half(), w, out),
+                 (x, None, w, t(4, 128, dtype=half)), (torch.zeros(4, 64), None, w, out), (x, torch.zeros(4, 64), w, out), (x, t(8, 32), w, out)):
+        with pytest.raises(RuntimeError):
+            ops.add_rmsnorm_terms(args[0], args[1], args[2], 1e-6, args[3])
+    lin = nbt.PackedLinear(torch.zeros(48 * 16, dtype=torch.uint8), torch.zeros(256, 8, dtype=half), 16, 128, block_size=8)
+    with pytest.raises(RuntimeError, match="blocks of 128"):
+        lin.forward_terms(t(40, 128, dtype=half))
+
+
 def test_fused_and_exchange_argument_checks(built_lib):
     """Argument validation of the prologue / tensor-parallel entry points runs before any device call."""
     from nativebit_b200 import _lib
