@@ -171,8 +171,8 @@ class PackedGPT(torch.nn.Module):
     def _norm_linear(self, x: torch.Tensor, delta, weight: torch.Tensor, eps: float, lin: PackedLinear) -> torch.Tensor:
         """lin(rmsnorm(x += delta) * weight), fp32; many rows travel as the GEMM's two fp16 terms instead of fp32."""
         C, rows = x.shape[-1], x.numel() // x.shape[-1]
-        if (lin.takes_terms(rows) and x.is_cuda and x.dtype == torch.float32 and x.is_contiguous() and C <= 4096 and weight.dtype == torch.float32
-                and (delta is None or (delta.dtype == torch.float32 and delta.is_contiguous()))):
+        if (isinstance(lin, PackedLinear) and lin.takes_terms(rows) and x.is_cuda and x.dtype == torch.float32 and x.is_contiguous()
+                and C <= 4096 and weight.dtype == torch.float32 and (delta is None or (delta.dtype == torch.float32 and delta.is_contiguous()))):
             terms = torch.empty(2 * rows, C, dtype=torch.float16, device=x.device)
             ops.add_rmsnorm_terms(x.view(rows, C), None if delta is None else delta.view(rows, C), weight, eps, terms)
             return lin.forward_terms(terms).view(*x.shape[:-1], -1)
@@ -180,14 +180,14 @@ class PackedGPT(torch.nn.Module):
 
     @staticmethod
     def _silu_linear(gu: torch.Tensor, lin: PackedLinear) -> torch.Tensor:
-        """lin(silu(gate) * up), fp32, for gu (rows, 2F) = [gate | up]."""
-        rows, F_ = gu.shape[0], gu.shape[1] // 2
-        if gu.is_cuda and gu.is_contiguous() and lin.takes_terms(rows) and rows <= 65535:
-            terms = torch.empty(2 * rows, F_, dtype=torch.float16, device=gu.device)
-            ops.silu_mul_terms(gu, terms)
-            return lin.forward_terms(terms)
-        act = torch.empty(rows, F_, dtype=torch.float32, device=gu.device)
-        ops.silu_mul(gu, act)
+        """lin(silu(gate) * up), fp32, for contiguous gu (..., 2F) = [gate | up]."""
+        shape, rows = (*gu.shape[:-1], gu.shape[-1] // 2), gu.numel() // gu.shape[-1]
+        if isinstance(lin, PackedLinear) and lin.takes_terms(rows) and rows <= 65535:
+            terms = torch.empty(2 * rows, shape[-1], dtype=torch.float16, device=gu.device)
+            ops.silu_mul_terms(gu.view(rows, -1), terms)
+            return lin.forward_terms(terms).view(*shape[:-1], -1)
+        act = torch.empty(shape, dtype=torch.float32, device=gu.device)
+        ops.silu_mul(gu.view(rows, -1), act.view(rows, -1))
         return lin(act).float()
 
     def _finish_block(self, x, blk, attn_out):
@@ -251,7 +251,7 @@ class PackedGPT(torch.nn.Module):
                 new_caches.append((k_buf, v_buf, cache_len + T))
                 d1 = self._all_reduce(blk.out_proj(out).float())
                 gu = self._norm_linear(x, d1, blk.ln2, eps, blk.gate_up)
-                delta = self._all_reduce(self._silu_linear(gu.view(B * T, -1), blk.down).view(B, T, -1))
+                delta = self._all_reduce(self._silu_linear(gu, blk.down))
                 continue
             if delta is not None:
                 x, delta = x + delta, None

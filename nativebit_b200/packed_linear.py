@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import numpy as np
 import torch
+from torch.nn.modules import module as _module
 
 from . import ops
 
@@ -122,8 +123,11 @@ class PackedLinear(torch.nn.Module):
         return self.block_size == BS and self.in_features % BS == 0 and self.bits in (2, 3, 4)
 
     def takes_terms(self, rows: int) -> bool:
-        """Whether forward would split this many fp32 rows into two fp16 terms itself, so that `forward_terms` may take them."""
-        return rows > GEMV_MAX_M and self._tensor_cores()
+        """Whether a call would split this many fp32 rows into two fp16 terms itself and nobody else looks at them, so that
+        `forward_terms` may take their place: no hooks, no forward of a subclass or of this instance."""
+        seen = (self._forward_pre_hooks or self._forward_hooks or _module._global_forward_pre_hooks or _module._global_forward_hooks
+                or "forward" in self.__dict__ or type(self).forward is not PackedLinear.forward)
+        return rows > GEMV_MAX_M and self._tensor_cores() and not seen
 
     def forward_terms(self, terms, out=None):
         """fp32 (M, out_features) of M fp32 rows given as their two fp16 terms, (2M, in_features); see ops.add_rmsnorm_terms."""

@@ -432,3 +432,37 @@ def test_captured_steps_outlive_a_longer_prompt(built_lib, B):
         assert torch.equal(a.logits, b.logits) and torch.equal(a.token, b.token)
     a.prefill(toks[:, :3]); b.prefill(toks[:, :3])                  # the prompt's graph of before, on the workspace of before
     assert torch.equal(a.logits, b.logits)
+
+
+def test_prompt_calls_the_linears_that_others_look_at(built_lib):
+    """Linears with hooks, of a subclass or of another kind are called as modules with (B, T, C) activations; the logits are those
+    of the prompt whose activations go straight into the GEMMs' operand."""
+    from nativebit_b200 import generate as G
+    from nativebit_b200.packed_linear import PackedLinear
+    dev = torch.device("cuda:0")
+    cfg = G.ModelConfig(vocab_size=512, n_layers=2, n_embd=512, n_head=4, ffn_hidden=1408, context_len=64)
+    toks = torch.randint(0, cfg.vocab_size, (2, 30), generator=torch.Generator().manual_seed(0)).to(dev)
+
+    def logits(model):
+        return model(toks, kv_caches=G.init_kv_cache(model, 2, dev))[0]
+    model = G.PackedGPT.random_init(cfg, seed=5, device=dev)
+    want, seen = logits(model), []
+
+    class Sub(PackedLinear):
+        def forward(self, x):
+            seen.append(("sub", tuple(x.shape)))
+            return super().forward(x)
+    hooks = [model.blocks[0].qkv.register_forward_pre_hook(lambda m, args: seen.append(("qkv", tuple(args[0].shape)))),
+             model.blocks[1].down.register_forward_hook(lambda m, args, y: seen.append(("down", tuple(args[0].shape))))]
+    model.blocks[0].down.__class__ = Sub
+    old = model.blocks[1].gate_up
+    dense = torch.nn.Linear(old.in_features, old.out_features, bias=False, device=dev)
+    dense.weight.data = old.dequantized_weight()
+    model.blocks[1].gate_up = dense
+    got = logits(model)
+    assert seen == [("qkv", (2, 30, 512)), ("sub", (2, 30, 1408)), ("down", (2, 30, 1408))]
+    assert (got - want).abs().max() <= 1e-4 * want.abs().max()                # one product by the library in fp32
+    for h in hooks:
+        h.remove()
+    model.blocks[0].down.__class__, model.blocks[1].gate_up = PackedLinear, old
+    assert torch.equal(logits(model), want)
