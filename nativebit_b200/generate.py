@@ -171,8 +171,7 @@ class PackedGPT(torch.nn.Module):
     def _norm_linear(self, x: torch.Tensor, delta, weight: torch.Tensor, eps: float, lin: PackedLinear) -> torch.Tensor:
         """lin(rmsnorm(x += delta) * weight), fp32; many rows travel as the GEMM's two fp16 terms instead of fp32."""
         C, rows = x.shape[-1], x.numel() // x.shape[-1]
-        if (isinstance(lin, PackedLinear) and lin.takes_terms(rows) and x.is_cuda and x.dtype == torch.float32 and x.is_contiguous()
-                and C <= 4096 and weight.dtype == torch.float32 and (delta is None or (delta.dtype == torch.float32 and delta.is_contiguous()))):
+        if isinstance(lin, PackedLinear) and lin.takes_terms(rows) and x.is_cuda and ops.rmsnorm_terms_fits(x, delta, weight):
             terms = torch.empty(2 * rows, C, dtype=torch.float16, device=x.device)
             ops.add_rmsnorm_terms(x.view(rows, C), None if delta is None else delta.view(rows, C), weight, eps, terms)
             return lin.forward_terms(terms).view(*x.shape[:-1], -1)
@@ -182,7 +181,7 @@ class PackedGPT(torch.nn.Module):
     def _silu_linear(gu: torch.Tensor, lin: PackedLinear) -> torch.Tensor:
         """lin(silu(gate) * up), fp32, for contiguous gu (..., 2F) = [gate | up]."""
         shape, rows = (*gu.shape[:-1], gu.shape[-1] // 2), gu.numel() // gu.shape[-1]
-        if isinstance(lin, PackedLinear) and lin.takes_terms(rows) and rows <= 65535:
+        if isinstance(lin, PackedLinear) and lin.takes_terms(rows) and rows <= 65535 and gu.data_ptr() % 16 == 0:
             terms = torch.empty(2 * rows, shape[-1], dtype=torch.float16, device=gu.device)
             ops.silu_mul_terms(gu.view(rows, -1), terms)
             return lin.forward_terms(terms).view(*shape[:-1], -1)
@@ -465,7 +464,7 @@ class DecodeSession(Session):
             elif fold:
                 ops.gemv_fused(ops.PRO_ADD_RMSNORM, xa, *args, out, delta=delta, norm_weight=w, eps=eps, x_out=xb)
                 xa, xb = xb, xa
-            elif (terms := self._terms_of(lin)) is not None and lin.in_features <= 4096:
+            elif (terms := self._terms_of(lin)) is not None and ops.rmsnorm_terms_fits(xa, delta, w):
                 packed = lin.stream_weight()
                 ops.add_rmsnorm_terms(xa, delta, w, eps, terms)
                 self._terms_into(lin, packed, terms, out)

@@ -539,6 +539,13 @@ def silu_mul(gu: torch.Tensor, out: torch.Tensor) -> None:
     _lib.check(_lib.lib().nb_silu_mul(gu.data_ptr(), gu.shape[0], out.shape[1], out.data_ptr(), _stream()), "nb_silu_mul")
 
 
+def rmsnorm_terms_fits(x: torch.Tensor, delta: torch.Tensor | None, w: torch.Tensor) -> bool:
+    """Whether add_rmsnorm_terms takes these rows (..., C): four values at a time, so that a norm's weight that is a view at an
+    odd place of a larger buffer needs add_rmsnorm instead."""
+    return x.shape[-1] <= 4096 and x.shape[-1] % 4 == 0 and all(
+        t is None or (t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0) for t in (x, delta, w))
+
+
 def add_rmsnorm_terms(x: torch.Tensor, delta: torch.Tensor | None, w: torch.Tensor, eps: float, out: torch.Tensor) -> None:
     """x (B, C) fp32 += delta; out (2B, C) fp16 = the two terms of every row of rmsnorm(x) * w, the prefill GEMMs' operand."""
     _need_cuda(*(t for t in (x, delta, w, out) if t is not None))

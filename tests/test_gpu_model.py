@@ -466,3 +466,29 @@ def test_prompt_calls_the_linears_that_others_look_at(built_lib):
         h.remove()
     model.blocks[0].down.__class__, model.blocks[1].gate_up = PackedLinear, old
     assert torch.equal(logits(model), want)
+
+
+def test_norm_weights_at_any_place_of_a_buffer(built_lib):
+    """Norm weights that are views at odd places of one buffer: prompts and steps of more than 16 rows give the same logits as with
+    weights of their own."""
+    from nativebit_b200 import generate as G
+    dev = torch.device("cuda:0")
+    cfg = G.ModelConfig(vocab_size=512, n_layers=2, n_embd=512, n_head=4, ffn_hidden=1408, context_len=64)
+    toks = torch.randint(0, cfg.vocab_size, (20, 5), generator=torch.Generator().manual_seed(0)).to(dev)
+    got = []
+    for at in (0, 1):
+        model = G.PackedGPT.random_init(cfg, seed=5, device=dev)
+        for blk in model.blocks:
+            for name in ("ln1", "ln2"):
+                buf = 1.0 + 0.1 * torch.randn(cfg.n_embd + 4, device=dev, generator=torch.Generator(device=dev).manual_seed(1))
+                w = buf[:cfg.n_embd]
+                if at:
+                    w = torch.cat((buf[:at], w))[at:]
+                    assert w.data_ptr() % 16
+                setattr(blk, name, w)
+        s = G.DecodeSession(model, 20, use_graph=False)
+        first = s.prefill(toks).clone()
+        s.step()
+        got.append((first, s.logits.clone()))
+    for a, b in zip(*got):
+        assert (a - b).abs().max() <= 2e-5 * a.abs().max()                       # another order of the norm's sum
