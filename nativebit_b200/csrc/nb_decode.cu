@@ -551,6 +551,16 @@ __global__ void __launch_bounds__(256) prompt_keys_kernel(const float* __restric
 // the odd ones, and the halves meet once at the end — so the weights cross shared memory inside a half-warp only.
 // head_dim a multiple of 4, <= 128; NP pairs per thread cover 16 * NP >= head_dim.  Two CTAs share an SM: PK is 64 where
 // their tiles fit, else 32.
+constexpr int prompt_pairs(int hd) { return hd <= 32 ? 2 : hd <= 64 ? 4 : hd <= 80 ? 5 : 8; }
+// Floats behind the values that the spare pairs of the last row read (and nobody uses): all 16 * NP dimensions of that row
+// end before the weights, which other warps are writing.
+constexpr int kPromptSpare = 40;
+constexpr bool prompt_spare_covers() {
+  for (int hd = 4; hd <= 128; hd += 4)
+    if (16 * prompt_pairs(hd) > hd + 4 + kPromptSpare) return false;
+  return true;
+}
+static_assert(prompt_spare_covers() && kPromptSpare % 4 == 0, "spare pairs of the last value row");
 __device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
@@ -579,8 +589,8 @@ __global__ void __launch_bounds__(128, 2) prefill_attention_kernel(
   const int hdp = hd + 4;                       // row stride: 16-byte aligned, eight consecutive rows on different banks
   float* q_s = psm;                             // [BQ][hdp]
   float* k_s = q_s + BQ * hdp;                  // [PK][hdp]
-  float* v_s = k_s + PK * hdp;                  // [PK][hdp], and 2 * 16 floats that the last row's spare pairs read
-  float* p_s = v_s + PK * hdp + 32;             // [BQ][kPStride]
+  float* v_s = k_s + PK * hdp;                  // [PK][hdp]
+  float* p_s = v_s + PK * hdp + kPromptSpare;   // [BQ][kPStride]
   const int tid = threadIdx.x, h = blockIdx.x, b = blockIdx.y, q0 = ((int)gridDim.z - 1 - (int)blockIdx.z) * BQ;
   const int row3 = 3 * H * hd, quarter = hd >> 2, rcp = 65536 / quarter + 1;      // i / quarter = i * rcp >> 16 for i < 2048
   const size_t cbase = ((size_t)b * H + h) * (size_t)ctx * hd;
@@ -731,7 +741,7 @@ __global__ void __launch_bounds__(128, 2) prefill_attention_kernel(
 template <int R, int NP, typename... Args>
 static int launch_prefill_attention(int B, int T, int H, int hd, cudaStream_t st, Args... args) {
   constexpr int BQ = 8 * R, PK = NP > 5 && R == 8 ? 32 : 64;
-  const size_t smem = (size_t)((BQ + 2 * PK) * (hd + 4) + 32 + BQ * (PK + 4)) * sizeof(float);      // <= 95 KB
+  const size_t smem = (size_t)((BQ + 2 * PK) * (hd + 4) + kPromptSpare + BQ * (PK + 4)) * sizeof(float);      // <= 92 KB
   static bool attr_done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1077,10 +1087,12 @@ extern "C" int nb_prefill_attention(const float* qkv, int B, int T, int H, int h
     return prefill_attention_tile<decltype(pairs)::value>(B, T, H, hd, (cudaStream_t)stream, qkv, cos2, sin2, (const float*)k_cache,
                                                           (const float*)v_cache, out, T, H, hd, ctx, pos0, out_stride, out_offset, scale);
   };
-  if (hd <= 32) return run(std::integral_constant<int, 2>{});
-  if (hd <= 64) return run(std::integral_constant<int, 4>{});
-  if (hd <= 80) return run(std::integral_constant<int, 5>{});
-  return run(std::integral_constant<int, 8>{});
+  switch (prompt_pairs(hd)) {
+    case 2: return run(std::integral_constant<int, 2>{});
+    case 4: return run(std::integral_constant<int, 4>{});
+    case 5: return run(std::integral_constant<int, 5>{});
+    default: return run(std::integral_constant<int, 8>{});
+  }
 }
 
 extern "C" size_t nb_lm_head_scratch_bytes(void) { return (size_t)kHeadMaxCtas * 8; }
