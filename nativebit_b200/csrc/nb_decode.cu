@@ -524,11 +524,13 @@ __device__ __forceinline__ float4 turn_pairs(float4 x, float2 c, float2 s) {
 // Causal attention of a prompt (or a chunk of one that continues a cache of pos0 keys), two launches per layer: the first
 // rotates the chunk's keys into the cache and copies its values there, the second is softmax(q k^T / sqrt(hd)) v over the
 // cached keys 0 .. pos0 + t for query t (inference/generate_torch.py:41-60 RoPE, :86-97 cache write and masked attention).
+// The second starts beside the first and turns its queries meanwhile.
 // (Rotating the keys wherever they are read needs one launch, but every CTA then waits for its loads: 381 us against the
 // 337 us of both launches, 8 sequences of 512 tokens, 32 heads of 80.)
 __global__ void __launch_bounds__(256) prompt_keys_kernel(const float* __restrict__ qkv, const float* __restrict__ cos2,
                                                           const float* __restrict__ sin2, float* __restrict__ k_cache,
                                                           float* __restrict__ v_cache, int T, int H, int hd, int ctx, int pos0) {
+  asm volatile("griddepcontrol.launch_dependents;");        // the attention behind it turns its queries meanwhile
   const int t = blockIdx.x, b = blockIdx.y, quarter = hd >> 2;
   const float* row = qkv + (size_t)(b * T + t) * 3 * H * hd + H * hd;
   for (int i = threadIdx.x; i < H * quarter; i += 256) {
@@ -550,7 +552,7 @@ __global__ void __launch_bounds__(256) prompt_keys_kernel(const float* __restric
 // 2 * NP head dimensions (pairs 16 apart) for every second four keys — eight lanes of a half-warp take the even fours, eight
 // the odd ones, and the halves meet once at the end — so the weights cross shared memory inside a half-warp only.
 // head_dim a multiple of 4, <= 128; NP pairs per thread cover 16 * NP >= head_dim.  Two CTAs share an SM: PK is 64 where
-// their tiles fit, else 32.
+// their tiles fit, else 32 (and for tiles of 16 queries, which are taken where 32 keys are all there are).
 constexpr int prompt_pairs(int hd) { return hd <= 32 ? 2 : hd <= 64 ? 4 : hd <= 80 ? 5 : 8; }
 // Floats behind the values that the spare pairs of the last row read (and nobody uses): all 16 * NP dimensions of that row
 // end before the weights, which other warps are writing.
@@ -603,6 +605,7 @@ __global__ void __launch_bounds__(128, 2) prefill_attention_kernel(
                                                                make_float2(cos2[ri], cos2[ri + 2]), make_float2(sin2[ri], sin2[ri + 2]));
   }
 
+  asm volatile("griddepcontrol.wait;" ::: "memory");      // the chunk's keys and values are in the caches
   const int ty = tid >> 4, tx = tid & 15;       // scores: queries R ty .. + R - 1, keys tx + 16 i
   const int upper = (tid >> 3) & 1, tx2 = tid & 7;      // values: the same queries, one half of the keys, dimensions 2 tx2 + 16 i and the next
   const int kmax = pos0 + min(q0 + BQ - 1, T - 1);      // last key any query of this tile may see
@@ -740,7 +743,7 @@ __global__ void __launch_bounds__(128, 2) prefill_attention_kernel(
 
 template <int R, int NP, typename... Args>
 static int launch_prefill_attention(int B, int T, int H, int hd, cudaStream_t st, Args... args) {
-  constexpr int BQ = 8 * R, PK = NP > 5 && R == 8 ? 32 : 64;
+  constexpr int BQ = 8 * R, PK = R == 2 || (NP > 5 && R == 8) ? 32 : 64;
   const size_t smem = (size_t)((BQ + 2 * PK) * (hd + 4) + kPromptSpare + BQ * (PK + 4)) * sizeof(float);      // <= 92 KB
   static bool attr_done[64] = {};
   int dev = 0;
@@ -750,15 +753,17 @@ static int launch_prefill_attention(int B, int T, int H, int hd, cudaStream_t st
       return record_cuda_error(e);
     attr_done[dev & 63] = true;
   }
-  prefill_attention_kernel<R, PK, NP><<<dim3(H, B, (T + BQ - 1) / BQ), 128, smem, st>>>(args...);
-  return record_cuda_error(cudaGetLastError());
+  return launch_pdl(prefill_attention_kernel<R, PK, NP>, dim3(H, B, (T + BQ - 1) / BQ), dim3(128), smem, st, args...);
 }
 
 // Tiles of 64 queries stage every key half as often as tiles of 32; short or few prompts take the latter, which puts
-// twice as many SMs to work on them.
+// twice as many SMs to work on them, and very short ones (one chunk of 32 keys in all) tiles of 16, whose padding and shared
+// memory are half of that again.  32 sequences x 32 heads of 80, 64 / 32 / 16 queries: 5 tokens 36.9 / 25.1 / 14.9 us,
+// 17 tokens 42.0 / 29.9 us; one sequence, 5 tokens 8.7 / 7.7 / 5.9 us.
 template <int NP, typename... Args>
-static int prefill_attention_tile(int B, int T, int H, int hd, cudaStream_t st, Args... args) {
-  if ((long long)B * H * ((T + 63) / 64) < 2 * sm_count()) return launch_prefill_attention<4, NP>(B, T, H, hd, st, args...);
+static int prefill_attention_tile(int B, int T, int H, int hd, int pos0, cudaStream_t st, Args... args) {
+  if (T <= 16 && pos0 + T <= 32) return launch_prefill_attention<2, NP>(B, T, H, hd, st, args...);
+  if (T <= 32 || (long long)B * H * ((T + 63) / 64) < 2 * sm_count()) return launch_prefill_attention<4, NP>(B, T, H, hd, st, args...);
   return launch_prefill_attention<8, NP>(B, T, H, hd, st, args...);
 }
 
@@ -1084,7 +1089,7 @@ extern "C" int nb_prefill_attention(const float* qkv, int B, int T, int H, int h
   prompt_keys_kernel<<<dim3(T, B), 256, 0, (cudaStream_t)stream>>>(qkv, cos2, sin2, k_cache, v_cache, T, H, hd, ctx, pos0);
   if (int rc = check_launch()) return rc;
   auto run = [&](auto pairs) {
-    return prefill_attention_tile<decltype(pairs)::value>(B, T, H, hd, (cudaStream_t)stream, qkv, cos2, sin2, (const float*)k_cache,
+    return prefill_attention_tile<decltype(pairs)::value>(B, T, H, hd, pos0, (cudaStream_t)stream, qkv, cos2, sin2, (const float*)k_cache,
                                                           (const float*)v_cache, out, T, H, hd, ctx, pos0, out_stride, out_offset, scale);
   };
   switch (prompt_pairs(hd)) {

@@ -369,9 +369,11 @@ def test_full_size_decoder_against_dense_oracle_teacher_forced(built_lib):
 
 
 @pytest.mark.parametrize("B,T,H,hd,ctx,pos0", [(1, 33, 2, 20, 64, 0), (1, 95, 3, 36, 160, 63), (1, 65, 2, 84, 80, 1), (5, 65, 60, 20, 70, 0),
-                                               (3, 129, 50, 64, 130, 0), (4, 64, 80, 80, 100, 31), (5, 63, 60, 84, 64, 1), (2, 130, 50, 128, 140, 5), (1, 70, 3, 88, 80, 3)])
+                                               (3, 129, 50, 64, 130, 0), (4, 64, 80, 80, 100, 31), (5, 63, 60, 84, 64, 1), (2, 130, 50, 128, 140, 5), (1, 70, 3, 88, 80, 3),
+                                               (40, 5, 32, 80, 64, 0), (1, 1, 3, 20, 8, 0), (3, 16, 5, 128, 40, 16), (3, 16, 5, 128, 40, 17),
+                                               (2, 17, 60, 64, 40, 0), (5, 32, 60, 36, 33, 1)])
 def test_prefill_attention_edges_of_its_tiles(built_lib, B, T, H, hd, ctx, pos0):
-    """One query or key past a tile, both query tiles (few and many CTAs), every number of head dimensions per thread."""
+    """One query or key past a tile, the three query tiles (very short, few or many CTAs), every number of head dimensions per thread."""
     test_prefill_attention_against_torch(built_lib, B, T, H, hd, ctx, pos0, H * hd, 0)
 
 
