@@ -25,6 +25,12 @@ __host__ __device__ inline int64_t packed_bytes(int64_t count, int bits) {
   return bits == 3 ? 3 * ((count + 7) / 8) : (count * bits + 7) / 8;
 }
 
+// Quotient of a place by a block's size: a shift for powers of two (`shift` >= 0), else in 32 bits where they hold the place.
+__device__ __forceinline__ int64_t block_of(int64_t i, int size, int shift) {
+  return shift >= 0 ? i >> shift : i <= 0xFFFFFFFFll ? (int64_t)((uint32_t)i / (uint32_t)size) : i / size;
+}
+static int shift_of(int size) { return (size & (size - 1)) ? -1 : __builtin_ctz(size); }
+
 // ---- unpack -------------------------------------------------------------------------------
 // Fast path: one thread turns `BITS` aligned 32-bit words into 32 indices (two 16-byte stores).
 template <int BITS>
@@ -60,12 +66,29 @@ __global__ void unpack_generic_kernel(const uint8_t* __restrict__ packed, int64_
 }
 
 // ---- pack ---------------------------------------------------------------------------------
+// Output byte b: the (at most 5) indices that overlap it.
+__device__ __forceinline__ uint8_t pack_byte(const uint8_t* __restrict__ idx, int64_t count, int bits, int64_t b) {
+  const int64_t lo_bit = b * 8, hi_bit = lo_bit + 8;
+  const uint32_t mask = (1u << bits) - 1u;
+  uint32_t v = 0;
+  for (int64_t i = lo_bit / bits; i * bits < hi_bit; ++i) {
+    const uint32_t f = (i < count) ? (idx[i] & mask) : 0u;
+    const int64_t sh = i * bits - lo_bit;
+    v |= sh >= 0 ? (f << sh) : (f >> (-sh));
+  }
+  return (uint8_t)v;
+}
+
 // Fast path, the inverse of unpack32_kernel: one thread turns 32 indices (two 16-byte loads) into `BITS` words.  HBM-bound:
 // 17.7 M indices to 3 bits in 6.7 us (24.3 MB); one thread per output byte took 40 us, on 64-bit index arithmetic.
 template <int BITS>
-__global__ void pack32_kernel(const uint4* __restrict__ idx, int64_t n_chunks, uint32_t* __restrict__ out) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n_chunks) return;
+__global__ void pack32_kernel(const uint4* __restrict__ idx, int64_t count, int64_t n_bytes, uint32_t* __restrict__ out) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, n_chunks = count >> 5;
+  if (c >= n_chunks) {                                 // the bytes of the last, partial chunk (at most 16)
+    const int64_t b = n_chunks * (4 * BITS) + (c - n_chunks);
+    if (b < n_bytes) reinterpret_cast<uint8_t*>(out)[b] = pack_byte(reinterpret_cast<const uint8_t*>(idx), count, BITS, b);
+    return;
+  }
   const uint4 a = idx[2 * c], b = idx[2 * c + 1];
   const uint32_t in[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
   uint32_t w[BITS];
@@ -82,20 +105,10 @@ __global__ void pack32_kernel(const uint4* __restrict__ idx, int64_t n_chunks, u
   for (int i = 0; i < BITS; ++i) out[c * BITS + i] = w[i];
 }
 
-// The rest, and unaligned buffers: one thread writes one output byte, ORing the (at most 5) indices that overlap it.
-__global__ void pack_kernel(const uint8_t* __restrict__ idx, int64_t count, int bits, int64_t first, int64_t n_bytes,
-                            uint8_t* __restrict__ out) {
-  const int64_t b = first + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n_bytes) return;
-  const int64_t lo_bit = b * 8, hi_bit = lo_bit + 8;
-  const uint32_t mask = (1u << bits) - 1u;
-  uint32_t v = 0;
-  for (int64_t i = lo_bit / bits; i * bits < hi_bit; ++i) {
-    const uint32_t f = (i < count) ? (idx[i] & mask) : 0u;
-    const int64_t sh = i * bits - lo_bit;
-    v |= sh >= 0 ? (f << sh) : (f >> (-sh));
-  }
-  out[b] = (uint8_t)v;
+// Unaligned buffers and less than a chunk: one thread writes one output byte.
+__global__ void pack_kernel(const uint8_t* __restrict__ idx, int64_t count, int bits, int64_t n_bytes, uint8_t* __restrict__ out) {
+  const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < n_bytes) out[b] = pack_byte(idx, count, bits, b);
 }
 
 // ---- dequant ------------------------------------------------------------------------------
@@ -103,8 +116,10 @@ __global__ void pack_kernel(const uint8_t* __restrict__ idx, int64_t count, int 
 // store, so that a warp's stores are one contiguous run (a thread with 32 weights of its own left every store 64 or 128
 // bytes from its neighbour's: 12.1 us for 6912 x 2560 to fp16 and 34.7 us to fp32, which take 6.7 and 12.2 us at the copy
 // rate).  The 3- or 2-bit fields are spread to the nibbles of one selector word; the block's table, as byte planes, answers
-// four lookups with two byte permutes.  A thread takes kDqPer stores a block stride apart and requests all inputs first.
-constexpr int kDqPer = 4, kDqThreads = 256;
+// four lookups with two byte permutes.  A thread takes PER stores a block stride apart and requests all inputs first: four where
+// that leaves every SM four CTAs (6912 x 2560 over six block sizes, three widths and three types 1237 us in sum, 1305 with one),
+// else one, as small matrices wait for one thread's chain of loads and not for memory (1024 x 1024 211 -> 183 us in sum).
+constexpr int kDqRuns = 4, kDqThreads = 256;
 
 template <int BITS> __device__ __forceinline__ uint32_t load_selectors(const uint32_t* __restrict__ packed, int64_t c) {
   if (BITS == 4) return packed[c];
@@ -149,15 +164,16 @@ template <int BITS> __device__ __forceinline__ void store16(float* dst, uint32_t
   *reinterpret_cast<float4*>(dst) = make_float4(a.x, a.y, b.x, b.y);
 }
 
-template <int BITS, typename OutT>
+template <int BITS, int PER, typename OutT>
 __global__ void __launch_bounds__(kDqThreads) dequant16b_kernel(const uint32_t* __restrict__ packed, const __half* __restrict__ codebook,
-                                                              int64_t n_stores, int chunks_per_block, int shift, OutT* __restrict__ out) {
+                                                               int64_t n_stores, int64_t n_bytes, int64_t total, int block_size, int shift,
+                                                               OutT* __restrict__ out) {
   constexpr int kT = BITS == 4 ? 8 : 4;
   constexpr bool kHalves = sizeof(OutT) == 4;          // a store takes half of a chunk of eight
-  const int64_t i0 = (int64_t)blockIdx.x * (kDqThreads * kDqPer) + threadIdx.x;
-  uint32_t sel[kDqPer], e[kDqPer][kT];
+  const int64_t i0 = (int64_t)blockIdx.x * (kDqThreads * PER) + threadIdx.x;
+  uint32_t sel[PER], e[PER][kT];
 #pragma unroll
-  for (int u = 0; u < kDqPer; ++u) {
+  for (int u = 0; u < PER; ++u) {
     const int64_t i = i0 + u * kDqThreads, c = kHalves ? i >> 1 : i;
     sel[u] = 0;
 #pragma unroll
@@ -165,7 +181,7 @@ __global__ void __launch_bounds__(kDqThreads) dequant16b_kernel(const uint32_t* 
     if (i < n_stores) {
       sel[u] = load_selectors<BITS>(packed, c);
       if (kHalves && (i & 1)) sel[u] >>= 16;
-      const int64_t block = shift >= 0 ? c >> shift : c / chunks_per_block;
+      const int64_t block = block_of(c, block_size >> 3, shift);
       const uint8_t* row = reinterpret_cast<const uint8_t*>(codebook) + block * (2 << BITS);
       if (BITS == 2) {
         const uint2 v = *reinterpret_cast<const uint2*>(row);
@@ -179,10 +195,10 @@ __global__ void __launch_bounds__(kDqThreads) dequant16b_kernel(const uint32_t* 
       }
     }
   }
+  int64_t i = i0;
 #pragma unroll
-  for (int u = 0; u < kDqPer; ++u) {
-    const int64_t i = i0 + u * kDqThreads;
-    if (i >= n_stores) return;
+  for (int u = 0; u < PER; ++u, i += kDqThreads) {
+    if (i >= n_stores) break;
     uint32_t T[kT];
     if (BITS == 2) {
       T[0] = prmt(e[u][0], e[u][1], 0x6420); T[2] = prmt(e[u][0], e[u][1], 0x7531);
@@ -196,12 +212,18 @@ __global__ void __launch_bounds__(kDqThreads) dequant16b_kernel(const uint32_t* 
     }
     store16<BITS>(out + i * (16 / sizeof(OutT)), sel[u], T);
   }
+  // fewer than 32 weights behind the last whole packed word, one for each of the threads without a store
+  const int64_t one = n_stores * (16 / (int)sizeof(OutT)) + (i - n_stores);
+  if (i >= n_stores && i < i0 + PER * kDqThreads && one < total) {
+    const uint32_t at = stream_index(reinterpret_cast<const uint8_t*>(packed), n_bytes, one, BITS);
+    out[one] = (OutT)(float)codebook[block_of(one, block_size, -1) * (1 << BITS) + at];
+  }
 }
 
 template <typename CbT, typename OutT>
 __global__ void dequant_generic_kernel(const uint8_t* __restrict__ packed, int64_t n_bytes, const CbT* __restrict__ codebook,
-                                       int bits, int block_size, int64_t first, int64_t total, OutT* __restrict__ out) {
-  const int64_t i = first + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+                                       int bits, int block_size, int64_t total, OutT* __restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const uint32_t e = stream_index(packed, n_bytes, i, bits);
   const float v = (float)codebook[(i / block_size) * (1 << bits) + e];
@@ -227,11 +249,11 @@ __global__ void quantize_kernel(const float* __restrict__ w, int64_t total, int6
   idx[i] = (uint8_t)arg;
 }
 
-// The same for four consecutive weights per thread (one block's: block_size % 4 == 0), kQPer runs per thread with all their
-// loads first; with PACK the indices leave as the packed stream, 32 of them gathered by the shuffles of eight lanes.
-// 64-bit index arithmetic and single-byte stores held the general kernel at 92 us for 6912 x 2560 weights; what bounds
-// this one is the argmin itself, three operations of the half-rate pipe per entry and weight (floor 20 us).
-constexpr int kQPer = 4, kQThreads = 256;
+// The same for four consecutive weights per thread (one block's: block_size % 4 == 0); with PACK the indices leave as the packed
+// stream, 32 of them gathered by the shuffles of eight lanes.  64-bit index arithmetic and single-byte stores held the general
+// kernel at 92 us for 6912 x 2560 weights; what bounds this one is the argmin itself, three operations of the half-rate pipe
+// per entry and weight (floor 20 us).  (Four such runs per thread take 1 % longer there and 4.4 instead of 2.6 us for 100 x 100.)
+constexpr int kQThreads = 256;
 
 template <typename CbT, int NE> __device__ __forceinline__ void load_entries(const CbT* cb, float (&c)[NE]);
 template <> __device__ __forceinline__ void load_entries<float, 4>(const float* cb, float (&c)[4]) {
@@ -258,53 +280,45 @@ __global__ void __launch_bounds__(kQThreads) quantize4_kernel(const float* __res
                                                               const float* __restrict__ codebook, int block4, int shift,
                                                               uint32_t* __restrict__ out) {
   constexpr int NE = 1 << BITS;
-  const int64_t i0 = (int64_t)blockIdx.x * (kQThreads * kQPer) + threadIdx.x;      // in units of four weights
+  const int64_t i = (int64_t)blockIdx.x * kQThreads + threadIdx.x;      // in units of four weights
   const int lane = threadIdx.x & 31;
-  float v[kQPer][4];
+  const bool in = 4 * i < padded;
+  float v[4];
+  if (4 * i + 4 <= total) {
+    const float4 x = reinterpret_cast<const float4*>(w)[i];
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+  } else {
 #pragma unroll
-  for (int u = 0; u < kQPer; ++u) {
-    const int64_t i = i0 + u * kQThreads;
-    if (4 * i + 4 <= total) {
-      const float4 x = reinterpret_cast<const float4*>(w)[i];
-      v[u][0] = x.x; v[u][1] = x.y; v[u][2] = x.z; v[u][3] = x.w;
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) v[u][j] = 4 * i + j < total ? w[4 * i + j] : 0.f;
-    }
+    for (int j = 0; j < 4; ++j) v[j] = 4 * i + j < total ? w[4 * i + j] : 0.f;
   }
+  uint32_t arg[4] = {0u, 0u, 0u, 0u};
+  if (in) {
+    float c[NE];
+    load_entries<float, NE>(codebook + block_of(i, block4, shift) * NE, c);
 #pragma unroll
-  for (int u = 0; u < kQPer; ++u) {
-    const int64_t i = i0 + u * kQThreads;
-    const bool in = 4 * i < padded;
-    uint32_t arg[4] = {0u, 0u, 0u, 0u};
-    if (in) {
-      float c[NE];
-      load_entries<float, NE>(codebook + (shift >= 0 ? i >> shift : i / block4) * NE, c);
+    for (int j = 0; j < 4; ++j) {
+      float best = fabsf(v[j] - c[0]);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float best = fabsf(v[u][j] - c[0]);
-#pragma unroll
-        for (int e = 1; e < NE; ++e) {
-          const float d = fabsf(v[u][j] - c[e]);
-          if (d < best) { best = d; arg[j] = e; }
-        }
+      for (int e = 1; e < NE; ++e) {
+        const float d = fabsf(v[j] - c[e]);
+        if (d < best) { best = d; arg[j] = e; }
       }
     }
-    if (!PACK) {
-      if (in) out[i] = arg[0] | (arg[1] << 8) | (arg[2] << 16) | (arg[3] << 24);
-    } else {
-      // two lanes hold 8 indices = 8 * BITS bits; at 3 bits even lane 2 q < 6 of eight writes word q: bits 32 q .. 32 q + 31 of
-      // the four pairs of 24, which lie in its own pair and the next
-      const uint32_t f = arg[0] | (arg[1] << BITS) | (arg[2] << (2 * BITS)) | (arg[3] << (3 * BITS));
-      const uint32_t pair = f | (__shfl_down_sync(0xffffffffu, f, 1) << (4 * BITS));      // of the even lanes
-      const uint32_t next = __shfl_down_sync(0xffffffffu, pair, 2);
-      const int q = (lane & 7) >> 1;
-      if (!in || (lane & 1)) continue;
-      uint32_t* dst = out + (i >> 3) * BITS;
-      if (BITS == 4) dst[q] = pair;
-      else if (BITS == 2) { if (!(q & 1)) dst[q >> 1] = pair | (next << 16); }
-      else if (q < 3) dst[q] = __funnelshift_r(pair | (next << 24), next >> 8, 8 * q);
-    }
+  }
+  if (!PACK) {
+    if (in) out[i] = arg[0] | (arg[1] << 8) | (arg[2] << 16) | (arg[3] << 24);
+  } else {
+    // two lanes hold 8 indices = 8 * BITS bits; at 3 bits even lane 2 q < 6 of eight writes word q: bits 32 q .. 32 q + 31 of
+    // the four pairs of 24, which lie in its own pair and the next
+    const uint32_t f = arg[0] | (arg[1] << BITS) | (arg[2] << (2 * BITS)) | (arg[3] << (3 * BITS));
+    const uint32_t pair = f | (__shfl_down_sync(0xffffffffu, f, 1) << (4 * BITS));      // of the even lanes
+    const uint32_t next = __shfl_down_sync(0xffffffffu, pair, 2);
+    const int q = (lane & 7) >> 1;
+    if (!in || (lane & 1)) return;
+    uint32_t* dst = out + (i >> 3) * BITS;
+    if (BITS == 4) dst[q] = pair;
+    else if (BITS == 2) { if (!(q & 1)) dst[q >> 1] = pair | (next << 16); }
+    else if (q < 3) dst[q] = __funnelshift_r(pair | (next << 24), next >> 8, 8 * q);
   }
 }
 
@@ -318,8 +332,8 @@ static bool quantize4_fits(const float* w, const void* codebook, int cb_dtype, i
 template <bool PACK>
 static int launch_quantize4(const float* w, int64_t total, int64_t padded, const float* codebook, int n_entries, int block_size, void* out,
                             cudaStream_t st) {
-  const int block4 = block_size / 4, shift = (block4 & (block4 - 1)) ? -1 : __builtin_ctz(block4);
-  const unsigned grid = (unsigned)((padded / 4 + kQThreads * kQPer - 1) / (kQThreads * kQPer));
+  const int block4 = block_size / 4, shift = shift_of(block4);
+  const unsigned grid = (unsigned)((padded / 4 + kQThreads - 1) / kQThreads);
   uint32_t* o = (uint32_t*)out;
   if (n_entries == 4) quantize4_kernel<2, PACK><<<grid, kQThreads, 0, st>>>(w, total, padded, codebook, block4, shift, o);
   else if (n_entries == 8) quantize4_kernel<3, PACK><<<grid, kQThreads, 0, st>>>(w, total, padded, codebook, block4, shift, o);
@@ -332,31 +346,28 @@ static int dequant_dispatch(const uint8_t* packed, const void* codebook, int cb_
                             int64_t total, OutT* out, cudaStream_t st) {
   const int64_t n_blocks = (total + block_size - 1) / block_size;
   const int64_t n_bytes = packed_bytes(n_blocks * block_size, bits);
-  int64_t done = 0;
   const bool aligned = ((uintptr_t)packed % 4 == 0) && ((uintptr_t)out % 16 == 0) && ((uintptr_t)codebook % 16 == 0);
   if (cb_dtype == NB_F16 && block_size % 8 == 0 && aligned) {
-    const int64_t chunks = total / 32 * 4;             // whole packed words
-    const int per_block = block_size / 8;
-    const int shift = (per_block & (per_block - 1)) ? -1 : __builtin_ctz(per_block);
-    if (chunks > 0) {
-      const int64_t stores = chunks * 8 / (int64_t)(16 / sizeof(OutT));
-      const unsigned grid = (unsigned)((stores + kDqThreads * kDqPer - 1) / (kDqThreads * kDqPer));
-      const uint32_t* pw = (const uint32_t*)packed;
-      const __half* cb = (const __half*)codebook;
-      if (bits == 3) dequant16b_kernel<3, OutT><<<grid, kDqThreads, 0, st>>>(pw, cb, stores, per_block, shift, out);
-      else if (bits == 2) dequant16b_kernel<2, OutT><<<grid, kDqThreads, 0, st>>>(pw, cb, stores, per_block, shift, out);
-      else dequant16b_kernel<4, OutT><<<grid, kDqThreads, 0, st>>>(pw, cb, stores, per_block, shift, out);
-      done = chunks * 8;
+    const int64_t stores = total / 32 * 32 / (int64_t)(16 / sizeof(OutT));      // whole packed words
+    if (stores > 0) {
+      const int shift = shift_of(block_size / 8);
+      const bool several = stores >= (int64_t)kDqRuns * kDqThreads * 4 * sm_count();
+      const int64_t per = kDqThreads * (several ? kDqRuns : 1);
+      auto run = [&](auto kernel) {
+        kernel<<<(unsigned)((stores + 31 + per - 1) / per), kDqThreads, 0, st>>>((const uint32_t*)packed, (const __half*)codebook, stores, n_bytes, total,
+                                                                            block_size, shift, out);
+        return check_launch();
+      };
+      if (bits == 3) return several ? run(dequant16b_kernel<3, kDqRuns, OutT>) : run(dequant16b_kernel<3, 1, OutT>);
+      if (bits == 2) return several ? run(dequant16b_kernel<2, kDqRuns, OutT>) : run(dequant16b_kernel<2, 1, OutT>);
+      return several ? run(dequant16b_kernel<4, kDqRuns, OutT>) : run(dequant16b_kernel<4, 1, OutT>);
     }
   }
-  if (done < total) {
-    const int64_t rest = total - done;
-    const unsigned grid = (unsigned)((rest + 255) / 256);
-    if (cb_dtype == NB_F16)
-      dequant_generic_kernel<__half, OutT><<<grid, 256, 0, st>>>(packed, n_bytes, (const __half*)codebook, bits, block_size, done, total, out);
-    else
-      dequant_generic_kernel<float, OutT><<<grid, 256, 0, st>>>(packed, n_bytes, (const float*)codebook, bits, block_size, done, total, out);
-  }
+  const unsigned grid = (unsigned)((total + 255) / 256);
+  if (cb_dtype == NB_F16)
+    dequant_generic_kernel<__half, OutT><<<grid, 256, 0, st>>>(packed, n_bytes, (const __half*)codebook, bits, block_size, total, out);
+  else
+    dequant_generic_kernel<float, OutT><<<grid, 256, 0, st>>>(packed, n_bytes, (const float*)codebook, bits, block_size, total, out);
   return check_launch();
 }
 
@@ -394,17 +405,14 @@ extern "C" int nb_pack(const uint8_t* idx, int bits, int64_t count, uint8_t* pac
   if (int rc = check_device()) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t n_bytes = packed_bytes(count, bits);
-  int64_t done = 0;                                    // bytes
   if ((uintptr_t)idx % 16 == 0 && (uintptr_t)packed_out % 4 == 0 && count >= 32) {
-    const int64_t chunks = count / 32;
-    const unsigned grid = (unsigned)((chunks + 127) / 128);
-    if (bits == 2) pack32_kernel<2><<<grid, 128, 0, st>>>((const uint4*)idx, chunks, (uint32_t*)packed_out);
-    if (bits == 3) pack32_kernel<3><<<grid, 128, 0, st>>>((const uint4*)idx, chunks, (uint32_t*)packed_out);
-    if (bits == 4) pack32_kernel<4><<<grid, 128, 0, st>>>((const uint4*)idx, chunks, (uint32_t*)packed_out);
-    done = chunks * 4 * bits;
+    const unsigned grid = (unsigned)((count / 32 + 16 + 127) / 128);
+    if (bits == 2) pack32_kernel<2><<<grid, 128, 0, st>>>((const uint4*)idx, count, n_bytes, (uint32_t*)packed_out);
+    if (bits == 3) pack32_kernel<3><<<grid, 128, 0, st>>>((const uint4*)idx, count, n_bytes, (uint32_t*)packed_out);
+    if (bits == 4) pack32_kernel<4><<<grid, 128, 0, st>>>((const uint4*)idx, count, n_bytes, (uint32_t*)packed_out);
+  } else {
+    pack_kernel<<<(unsigned)((n_bytes + 255) / 256), 256, 0, st>>>(idx, count, bits, n_bytes, packed_out);
   }
-  if (done < n_bytes)
-    pack_kernel<<<(unsigned)((n_bytes - done + 255) / 256), 256, 0, st>>>(idx, count, bits, done, n_bytes, packed_out);
   return check_launch();
 }
 

@@ -368,7 +368,8 @@ def test_quantize_matches_reference_argmin(dev, golden):
 
 
 @pytest.mark.parametrize("bits", [2, 3, 4])
-@pytest.mark.parametrize("total,block", [(1, 32), (31, 32), (32, 32), (127, 128), (4096, 96), (4101, 128), (70_003, 64), (40_000, 8), (1003, 12)])
+@pytest.mark.parametrize("total,block", [(1, 32), (31, 32), (32, 32), (127, 128), (4096, 96), (4101, 128), (70_003, 64), (40_000, 8), (1003, 12),
+                                         (4_900_007, 96)])
 def test_quantize_pack_dequant_edges_of_the_wide_kernels(dev, bits, total, block):
     """The four-, eight- and 32-wide kernels against the oracle's argmin and the reference's byte layout: padded last
     blocks, ties, blocks that are no power of two, counts that are no multiple of a word, unaligned buffers."""
