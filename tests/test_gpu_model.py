@@ -494,3 +494,17 @@ def test_norm_weights_at_any_place_of_a_buffer(built_lib):
         got.append((first, s.logits.clone()))
     for a, b in zip(*got):
         assert (a - b).abs().max() <= 2e-5 * a.abs().max()                       # another order of the norm's sum
+
+
+@pytest.mark.parametrize("B,F", [(1, 4), (16, 102), (17, 6912), (1000, 100), (4096, 100), (900, 260), (129, 1408), (70_000, 8)])
+def test_silu_mul_one_and_four_values_per_thread(built_lib, B, F):
+    """Both widths of the kernel and its CTAs narrower than, as wide as and wider than a row, against 64 bits."""
+    from nativebit_b200 import ops
+    dev = torch.device("cuda:0")
+    gu = 4 * torch.randn(B, 2 * F, device=dev, generator=torch.Generator(device=dev).manual_seed(B))
+    out = torch.full((B + 1, F), 7.0, device=dev)
+    ops.silu_mul(gu, out[:B])
+    gate, up = gu.double().split(F, 1)
+    ref = gate / (1 + torch.exp(-gate)) * up
+    assert ((out[:B].double() - ref).abs() <= 40 * 2.0 ** -23 * ref.abs() + 1e-30).all()          # __expf: 2 + 1.2 |x| ulp, |x| < 25
+    assert (out[B] == 7.0).all()
