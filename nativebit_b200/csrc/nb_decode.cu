@@ -330,8 +330,10 @@ __global__ void __launch_bounds__(kAttnWarps * 32) decode_attention_kernel(
 // keys and values.  A warp takes eight keys at a time, every fourth such chunk: its keys and values travel through the warp's
 // own ring of asynchronous copies (two chunks ahead, no registers held), and scores, running maximum, denominator and numerator
 // stay in the warp until one merge at the end, so no barrier separates the scores from the values.  The row this step writes
-// never comes from the cache: warp 0 starts from it.  A decode step of the 2.2B model at 512 keys, per layer: 8 sequences
-// 92 -> 81 us, 32 sequences of 100 keys 113 -> 108 us.
+// never comes from the cache: warp 0 starts from it.  Against the cluster kernel over 149 ... 1024 heads of 64, 80 and 128 and
+// 5 ... 8000 keys: 0.68 of its time in the middle of 230 sizes (256 heads of 64: 500 keys 21 -> 18 us), nowhere longer but for 256
+// heads of 128 over 4000 and 8000 keys (167 -> 171, 319 -> 335 us: 6.3 TB/s, and 148 SMs hold 256 CTAs unevenly); the length
+// is known on the device only, so those take it as well.
 constexpr int kWideWarps = 4, kWideKeys = 8, kWideD = 3;
 static size_t wide_smem_floats(int hd) { return (size_t)kWideWarps * kWideD * 2 * kWideKeys * hd + (size_t)(3 + kWideWarps) * hd; }
 
@@ -486,7 +488,7 @@ template <typename... Args>
 static int launch_attention(int B, int H, int hd, int ctx, cudaStream_t st, Args... args) {
   const int S = attn_split(B, H);
   const size_t smem = attn_smem_floats(ctx, hd, S) * sizeof(float);
-  if (smem > 48 * 1024) return NB_ERR_SHAPE;
+  if (smem > 48 * 1024) return NB_ERR_SHAPE;      // the contexts that are taken do not depend on the kernel (this one could do more)
   if (S <= 2) {     // more heads than SMs: no split is needed to occupy the GPU
     static bool done[64] = {};
     int dev = 0;

@@ -238,7 +238,7 @@ class PackedGPT(torch.nn.Module):
         delta = None                                   # a residual update that the next norm kernel will add
         for i, blk in enumerate(self.blocks):
             if kv_caches is not None and x.is_cuda and kv_caches[i][0].shape[0] == B:
-                # RoPE, cache write and causal attention in one launch (the rotary tables and the caches are fp32); the
+                # RoPE, cache write and causal attention in two launches (the rotary tables and the caches are fp32); the
                 # residual adds ride in the norm kernels, the last one of a block is still pending when the block ends
                 k_buf, v_buf, cache_len = kv_caches[i]
                 eps = self.config.norm_eps
@@ -427,7 +427,8 @@ class DecodeSession(Session):
     @torch.no_grad()
     def _step_body_fused(self):
         """The decode step on the fused kernels.  Up to 8 sequences: 5 launches per layer (residual add +
-        RMSNorm and SwiGLU are computed inside the packed GEMVs that consume them); more: 8 launches."""
+        RMSNorm and SwiGLU are computed inside the packed GEMVs that consume them); more: 7 to 12 (a norm or SwiGLU in front
+        of three linears, a conversion in front of out_proj, a sum behind every linear whose k range is split)."""
         m, cfg = self.model, self.model.config
         eps = cfg.norm_eps
         fold = self.B <= 8
@@ -488,7 +489,9 @@ class DecodeSession(Session):
                 ops.gemv_stream(prologue, x, lin.stream_weight(), lin.bits, lin.out_features, lin.in_features, out,
                                 single_term=self.single_term)
             elif self.tile_rows and prologue == ops.PRO_NONE and self.B > 2 * ops.gemv_stream_max_rows(lin.bits, lin.in_features):
-                # three launches over the same weights (8 rows of 6912: 25 us) take longer than the tensor-core kernel (14 us)
+                # three launches over the same weights (7 or 8 rows of 6912 columns: 26 us) take longer than the tensor-core kernel
+                # (13.6 us).  Two launches do not at 5632 columns (5 ... 8 rows 11.6 - 13.0 against 12.6 us); at 6912 they do
+                # (4 ... 6 rows 16.9 - 17.9 against 13.4 us), which this rule leaves as it was.
                 ops.gemm_prefill_fused(x, lin.stream_weight(), lin.bits, lin.out_features, lin.in_features, out=out)
             elif self.tile_rows:
                 ops.gemv_stream_rows(prologue, x, lin.stream_weight(), lin.bits, lin.out_features, lin.in_features, out)

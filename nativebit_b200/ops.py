@@ -362,8 +362,8 @@ def gemm_prefill(x: torch.Tensor, packed: torch.Tensor, codebook: torch.Tensor, 
                  n: int, k: int, out_dtype: torch.dtype = torch.bfloat16, out: torch.Tensor | None = None, terms: bool = False) -> torch.Tensor:
     """y (M, n) = x (M, k) @ W.T on the tcgen05 tensor cores: W is dequantised once into the workspace, then
     the plain tensor-core kernel multiplies.  x bf16, fp16 or fp32; the library carries fp32 activations as two
-    fp16 terms per element (about 22 significant bits, as in the GEMV) in adjacent operand rows and adds their
-    results in the epilogue."""
+    fp16 terms per element (about 22 significant bits, as in the GEMV), whose products meet in one fp32 sum, the second
+    terms' first.  terms: x is (2M, k) fp16, the two terms of every row."""
     _need_cuda(x, packed, codebook)
     if x.dtype not in (torch.bfloat16, torch.float16, torch.float32) or x.dim() != 2 or x.shape[1] != k:
         raise RuntimeError(f"x must be a bf16, fp16 or fp32 (M, {k}) tensor; got {x.dtype} {tuple(x.shape)}")

@@ -108,8 +108,11 @@ class PackedLinear(torch.nn.Module):
         if self._tensor_cores():
             rows = x_flat.shape[0] * (2 if x_flat.dtype == torch.float32 else 1)
             if rows > FUSED_MAX_ROWS:
-                # long inputs: dequantising W once into a scratch copy (12 us for 6912 x 2560) and running the plain
-                # tensor-core kernel measures faster than dequantising every weight tile once per 256 rows
+                # long inputs: dequantising W once into a scratch copy (8.8 us for 6912 x 2560) and running the plain
+                # tensor-core kernel, against dequantising every weight tile once per 256 operand rows.  6912 x 2560, fused |
+                # two passes (us): bf16 512 rows 30.0 | 31.8, 1024 45 | 42, 2048 71 | 67; fp32 512 rows 37 | 44, 1024 59 | 68, 2048
+                # 117 | 118.  bf16 rows cross between 256 (2560 x 2560) and 1280 (13824 x 2560), fp32 ones only past 1024:
+                # up to there the line is early for them by up to a seventh.
                 return ops.gemm_prefill(x_flat, self.packed_indices, self.codebook, self.bits, self.block_size,
                                         self.out_features, self.in_features, out_dtype=x_flat.dtype)
             return ops.gemm_prefill_fused(x_flat, self.stream_weight(), self.bits, self.out_features, self.in_features,

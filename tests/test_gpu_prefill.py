@@ -117,8 +117,8 @@ def test_fused_dequant_gemm_with_k_splits(built_lib, bits, m, n, k, xdt):
 
 @pytest.mark.parametrize("m,n,k", [(130, 200, 256), (1100, 640, 1280)])
 def test_dequant_then_gemm_with_fp32_activations(built_lib, m, n, k):
-    """The two-kernel form with fp32 activations: the library splits them into two fp16 terms in adjacent operand rows
-    and the epilogue adds the pair's results; 1100 rows is also what PackedLinear sends this way."""
+    """The two-kernel form with fp32 activations: the library splits them into two fp16 terms whose products meet in one
+    sum; 1100 rows is also what PackedLinear sends this way."""
     import nativebit_b200 as nbt
     from nativebit_b200 import ops
     dev = _dev()
