@@ -332,9 +332,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
           fill += 32;
         }
         if (fill < 32 && c + 1 < chunks) continue;
-        // store the rows, `fill` words each: eight lanes per 128-byte line
+        // store the rows, `fill` words each: eight lanes per 128-byte line, all eight stores of a lane independent of each other (one
+        // after the other behind their reads: 8192 rows x 200 columns x 520 deep 9.7 us, now 8.7; 16384 x 2560 x 64 57.9, now 38.7)
         __syncwarp();
-        const int per_row = fill >> 2;
+        if (vec && fill == 32 && rows == 32 && col + 32 * per_word <= n_out) {
+          const size_t hop = (size_t)4 * p.ldy * esize;
+          const uint32_t* src = st + (lane >> 3) * Cfg::kEpiRow + 4 * (lane & 7);
+          uint8_t* dst = reinterpret_cast<uint8_t*>(p.y) + ((size_t)(m0 + (lane >> 3)) * p.ldy + col + (lane & 7) * 4 * per_word) * esize;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(dst + j * hop) = *reinterpret_cast<const uint4*>(src + j * 4 * Cfg::kEpiRow);
+          __syncwarp();
+          col += fill * per_word;
+          fill = 0;
+          continue;
+        }
+        const int per_row = fill >> 2;                // the edges: any number of rows, columns and words per row
         for (int i = lane; i < rows * per_row; i += 32) {
           const int rr = per_row == 8 ? i >> 3 : i / per_row, v = i - rr * per_row;
           const int m = m0 + rr, o = col + v * 4 * per_word;
@@ -371,20 +383,25 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
   }
 }
 
-// CTAs per tile and tile width: the plan with the fewest estimated clocks, waves * clocks per k-step.  A step costs 2 * BN
-// clocks of the tensor cores and a part that does not depend on BN (loads and issue), a pair's at least what its loads take.
-// Ties go to the pair and to the wider tile, which reads X fewer times.  (8192 x 2560 x 2560: 160 columns in 7 waves 77 us,
-// 256 in 5 waves 95 us; 128 x 2560 x 2560: 32 columns on 80 SMs 11.3 us, 128 on 20 SMs 12.9 us.)
-static int step_clocks(int cg, int bn) { return cg == 2 ? std::max(2 * bn + 100, 330) : 2 * bn + 250; }
+// CTAs per tile and tile width: the plan with the fewest estimated clocks.  A k-step takes the tensor cores' 2 * BN clocks, a
+// quarter more in practice, and a part that does not depend on BN, and at least what its loads and issue take; a tile's
+// epilogue 1200 and 12 per column, of which only what outlasts the next tile's k-steps and the last tile's show; a pair 2500
+// more than a lone CTA for setting up and meeting.  Ties go to the pair and to the wider tile, which reads X fewer times.  The
+// figures are fitted to all plans of 324 shapes (1 ... 16384 rows, 20 ... 13824 columns, 16 ... 6912 deep): 1 % above the best
+// plan's time in the mean.  (1500 x 2560 x 960: a lone 224 12.5 us, a pair of 224 14.1; 1 x 6912 x 2560: 64 columns 12.3, 256
+// 17.2; 8192 x 2560 x 2560: 160 columns in 7 waves 77, 256 in 5 waves 95; 128 x 2560 x 2560: 32 columns on 80 SMs 11.3, 128 on
+// 20 SMs 12.9.)
 struct GemmPlan { int cg, bn; };
-static GemmPlan plan_gemm(int M, int N, int sms) {
+static int step_clocks(int cg, int bn) { return cg == 2 ? std::max(bn * 5 / 2 + 100, 470) : std::max(bn * 5 / 2 + 150, 480); }
+static GemmPlan plan_gemm(int M, int N, int k_steps, int sms) {
   GemmPlan best{1, 32};
   double best_cost = 1e30;
   for (int cg = M > kBM && sms > 1 ? 2 : 1; cg >= 1; --cg) {
     const long m_tiles = (M + kBM * cg - 1) / (kBM * cg);
     for (int bn = N >= 256 ? 256 : (N + 31) / 32 * 32; bn >= 32; bn -= 32) {
-      const long tiles = m_tiles * ((N + bn - 1) / bn), slots = sms / cg;
-      const double cost = (double)((tiles + slots - 1) / slots) * step_clocks(cg, bn);
+      const long tiles = m_tiles * ((N + bn - 1) / bn), slots = sms / cg, waves = (tiles + slots - 1) / slots;
+      const double steps = (double)k_steps * step_clocks(cg, bn), epilogue = 1200.0 + 12.0 * bn;
+      const double cost = waves * steps + epilogue + (waves - 1) * std::max(0.0, epilogue - steps) + (cg == 2 ? 2500 : 0);
       if (cost < best_cost * 0.999) { best_cost = cost; best = GemmPlan{cg, bn}; }
     }
   }
@@ -393,12 +410,12 @@ static GemmPlan plan_gemm(int M, int N, int sms) {
 
 // X (M rows, `ldx` apart; two: a row's two fp16 terms side by side) times W (N, K).
 static int launch_gemm(const void* x, int ldx, const void* w, int ldw, int K, bool two, GemmArgs p, cudaStream_t st) {
-  const GemmPlan plan = plan_gemm(p.M, p.N, sm_count());
+  p.w_steps = (K + kBK - 1) / kBK;
+  p.k_steps = two ? 2 * p.w_steps : p.w_steps;
+  const GemmPlan plan = plan_gemm(p.M, p.N, p.k_steps, sm_count());
   p.BN = plan.bn;
   p.m_tiles = (p.M + kBM * plan.cg - 1) / (kBM * plan.cg);
   p.n_tiles = (p.N + p.BN - 1) / p.BN;
-  p.w_steps = (K + kBK - 1) / kBK;
-  p.k_steps = two ? 2 * p.w_steps : p.w_steps;
   // rows past X's last are not copied as zeros, which takes longer than copying them: one row x 6912 x 2560, 64 columns per CTA,
   // 20.0 us with a box of 128 rows, 12.3 with one of 8
   const int x_rows = std::min(kBM, (p.M + 7) / 8 * 8);
@@ -420,14 +437,14 @@ static int launch_gemm(const void* x, int ldx, const void* w, int ldw, int K, bo
   cfg.dynamicSmemBytes = GemmCfg::kSmem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = plan.cg;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = plan.cg;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = plan.cg;                              // a CTA alone needs no cluster
   void* args[] = {&mx, &mw, &p};
   return record_cuda_error(cudaLaunchKernelExC(&cfg, fn, args));
 }
