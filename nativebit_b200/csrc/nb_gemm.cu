@@ -459,24 +459,6 @@ extern "C" size_t nb_prefill_workspace_bytes(int M, int N, int K) {
   return 256 + (((size_t)N * K * 2 + 255) & ~(size_t)255) + (size_t)2 * M * K * 2;
 }
 
-namespace nb {
-// bf16 -> fp16, eight elements per thread, saturating to +-65504.
-__global__ void __launch_bounds__(256) bf16_to_f16_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, size_t n8) {
-  asm volatile("griddepcontrol.launch_dependents;");        // the GEMM behind it waits before it reads
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n8) return;
-  const uint4 v = in[i];
-  const uint32_t u[4] = {v.x, v.y, v.z, v.w};
-  uint32_t r[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float a = __uint_as_float(u[j] << 16), b = __uint_as_float(u[j] & 0xFFFF0000u);
-    asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(r[j]) : "f"(b), "f"(a));
-  }
-  out[i] = make_uint4(r[0], r[1], r[2], r[3]);
-}
-}  // namespace nb
-
 // x (M, K) times w (N, K), both bf16 or both fp16 (f16).  The tensor maps copy 2-byte elements either way.  two: x is (M, 2K),
 // a row's two fp16 terms side by side.
 static int gemm_16bit(const void* x, const void* w, int f16, int M, int N, int K, void* y, int y_dtype, int* status, void* stream,

@@ -83,13 +83,6 @@ constexpr bool enough_stages() {
 }
 static_assert(enough_stages(), "stages per producer group");
 
-#ifdef NB_FUSED_TRACE
-__device__ long long g_ftrace[8][512];
-#define FTRACE(role, kt) do { if (blockIdx.x == 0 && (kt) < 512) g_ftrace[role][kt] = clock64(); } while (0)
-#else
-#define FTRACE(role, kt) do {} while (0)
-#endif
-
 template <int BITS> struct FusedFmt {
   static constexpr int kTabBytes = BITS == 4 ? 32 : 16;
   static constexpr int kUnitBytes = 1024 + 16 * kTabBytes;   // the stream layout's unit (nb_stream.cu)
@@ -163,7 +156,6 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         for (int kt = k_lo; kt < k_hi; ++kt) {
           ok = bar_wait(&empty[s], phase ^ 1, abort_flag, status);
           if (!ok) break;
-          FTRACE(0, kt);
           bar_expect_tx(&full[s], (uint32_t)b_bytes);
           tma_load_2d(sB + s * b_bytes, &map_x, &full[s], kt * kFK, m0);
           if (++s == S) { s = 0; phase ^= 1; }
@@ -188,7 +180,6 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         for (int kt = k_lo; kt < k_hi && ok; ++kt) {
           ok = bar_wait(&full[s], phase, abort_flag, status);
           if (!ok) break;
-          FTRACE(2, kt);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           // the stage's descriptors: the start-address field counts 16-byte units, so a stage further on is an add
           const uint64_t da = desc_a0 + (uint64_t)(s * (kFABytes >> 4)), db = desc_b0 + (uint64_t)(s * (b_bytes >> 4));
@@ -299,7 +290,6 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       for (; st < end; st += kFGroups) {
         const uint32_t kb = st >> 1;                     // k-blocks since the start: the group's are every second one
         const int r = (int)(kb & (uint32_t)(R - 1));
-        if (rt0 == 0 && lane == 0) FTRACE(3, k_lo + (int)(st - step0));
         ok = bar_wait<20>(&raw_full[r], kb / (uint32_t)R & 1u, abort_flag, status);
         if (!ok) break;
         uint4 out[2][4];
@@ -326,7 +316,6 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         // before implies that the stage is at most one use behind)
         ok = bar_wait<20>(&empty[s], phase ^ 1u, abort_flag, status);
         if (!ok) break;
-        if (rt0 == 0 && lane == 0) FTRACE(4, k_lo + (int)(st - step0));
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -334,7 +323,6 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy stores -> visible to the tensor core
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s2u(&full[s])) : "memory");
-        if (rt0 == 0 && lane == 0) FTRACE(5, k_lo + (int)(st - step0));
         for (s += kFGroups; s >= S; s -= S) phase ^= 1u;
       }
       step0 += (uint32_t)steps;
@@ -346,19 +334,6 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
   }
-}
-
-// bf16 -> fp16, eight elements per thread, saturating to +-65504 (exact for magnitudes 6.1e-5 .. 65504).
-__global__ void __launch_bounds__(256) bf16_to_f16_kernel2(const uint4* __restrict__ in, uint4* __restrict__ out, size_t n8) {
-  asm volatile("griddepcontrol.launch_dependents;");
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n8) return;
-  const uint4 v = in[i];
-  const uint32_t u[4] = {v.x, v.y, v.z, v.w};
-  uint32_t r[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) r[j] = f32x2_to_f16x2_sat(__uint_as_float(u[j] << 16), __uint_as_float(u[j] & 0xFFFF0000u));
-  out[i] = make_uint4(r[0], r[1], r[2], r[3]);
 }
 
 // Tile plan of one call: token-tile width BN (a multiple of 16 up to 256) and number of k splits.  A k-step of a work
@@ -414,34 +389,15 @@ __global__ void __launch_bounds__(256) splitk_sum_kernel(const float* __restrict
 
 // The stream layout as (row tiles, k-blocks, units of 8-byte elements) with boxes of eight row tiles of one k-block.
 static int make_map_units(CUtensorMap* map, const void* base, int unit_bytes, int bpr, int row_tiles) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) { set_last_error("cuTensorMapEncodeTiled is not available from the driver"); return NB_ERR_LAUNCH; }
   const cuuint64_t dims[3] = {(cuuint64_t)unit_bytes / 8, (cuuint64_t)bpr, (cuuint64_t)row_tiles};
   const cuuint64_t strides[2] = {(cuuint64_t)unit_bytes, (cuuint64_t)bpr * unit_bytes};
-  const cuuint32_t box[3] = {(cuuint32_t)unit_bytes / 8, 1, 8}, estr[3] = {1, 1, 1};
-  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_INT64, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    char msg[96];
-    std::snprintf(msg, sizeof(msg), "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
-    set_last_error(msg);
-    return NB_ERR_LAUNCH;
-  }
-  return NB_OK;
-}
-
-// (rows, cols) row-major 16-bit matrix -> tensor map with a (box_rows x 64) box and 128-byte swizzle.
-static int make_map_f16(CUtensorMap* map, const void* base, int rows, int cols, int box_rows) {
-  return make_map(map, base, rows, cols, box_rows);   // element size and swizzle are those of the bf16 maps
+  const cuuint32_t box[3] = {(cuuint32_t)unit_bytes / 8, 1, 8};
+  return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_INT64, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 }  // namespace nb
 
 using namespace nb;
-
-#ifdef NB_FUSED_TRACE
-extern "C" int nb_fused_trace_read(long long* host) { return (int)cudaMemcpyFromSymbol(host, g_ftrace, sizeof(g_ftrace)); }
-#endif
 
 // Workspace: [256 B status][fp16 operand rows x K][k-split slabs: ks x (M x N) floats]; sized for the worse of the
 // one-term (bf16 / fp16) and two-term (fp32) forms of M activation rows.
@@ -473,7 +429,7 @@ extern "C" int nb_gemm_prefill_fused(const void* x, int x_dtype, int M, const ui
   uint8_t* dst = reinterpret_cast<uint8_t*>(workspace) + 256;
   if (x_dtype == NB_BF16) {
     const size_t n8 = (size_t)M * K / 8;
-    bf16_to_f16_kernel2<<<(unsigned)((n8 + 255) / 256), 256, 0, st>>>(reinterpret_cast<const uint4*>(x), reinterpret_cast<uint4*>(dst), n8);
+    bf16_to_f16_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, st>>>(reinterpret_cast<const uint4*>(x), reinterpret_cast<uint4*>(dst), n8);
     if (int rc = check_launch()) return rc;
     xh = dst;
   } else if (x_dtype == NB_F32) {
@@ -486,7 +442,7 @@ extern "C" int nb_gemm_prefill_fused(const void* x, int x_dtype, int M, const ui
   const FusedPlan plan = plan_fused(rows, N, K, sms);
   const int bn = plan.bn;
   CUtensorMap mx, mw;
-  if (int rc = make_map_f16(&mx, xh, rows, K, bn)) return rc;
+  if (int rc = make_map(&mx, xh, rows, K, bn)) return rc;
   if (int rc = make_map_units(&mw, w_stream, bits == 4 ? FusedFmt<4>::kUnitBytes : FusedFmt<3>::kUnitBytes, K / kBlock, (N + 15) / 16)) return rc;
   const int m_tiles = (rows + bn - 1) / bn, w_tiles = (N + kFM - 1) / kFM;
   int ks = plan.ks;

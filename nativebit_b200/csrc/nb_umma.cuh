@@ -61,8 +61,7 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
 // True in one lane of a converged warp.  The roles that issue MMAs and copies are entered through this and not through
 // `lane == 0`: behind elect.sync the compiler knows that a single lane is active and needs no detour to bring descriptors
 // and addresses into uniform registers.  Entered by lane number, every tcgen05.mma cost its issuing thread 54 - 86 clocks, and
-// a k-step of the pair's 256 x 256 x 64 tile (0.27 us of tensor time) up to 0.43 us (8192 x 2560 x 6912: 299 us, 201 us entered
-// this way).
+// a k-step of the pair's 256 x 256 x 64 tile (0.27 us of tensor time) up to 0.43 us.
 __device__ __forceinline__ bool elect_one() {
   uint32_t r;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
@@ -101,18 +100,13 @@ inline EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// (rows, cols) row-major bf16 matrix, rows `ld` elements apart (0: cols; a multiple of 8) -> tensor map with a
-// (box_rows x 64) box and 128-byte swizzle.  Boxes past the last row or column are filled with zeros.
-inline int make_map(CUtensorMap* map, const void* base, int rows, int cols, int box_rows, int ld = 0) {
+inline int encode_map(CUtensorMap* map, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims, const cuuint64_t* strides,
+                      const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) { set_last_error("cuTensorMapEncodeTiled is not available from the driver"); return NB_ERR_LAUNCH; }
-  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)(ld ? ld : cols) * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = fn(map, type, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     char msg[96];
     std::snprintf(msg, sizeof(msg), "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
@@ -120,6 +114,28 @@ inline int make_map(CUtensorMap* map, const void* base, int rows, int cols, int 
     return NB_ERR_LAUNCH;
   }
   return NB_OK;
+}
+
+// (rows, cols) row-major 16-bit matrix, rows `ld` elements apart (0: cols; a multiple of 8) -> tensor map with a
+// (box_rows x 64) box and 128-byte swizzle.  Boxes past the last row or column are filled with zeros.
+inline int make_map(CUtensorMap* map, const void* base, int rows, int cols, int box_rows, int ld = 0) {
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)(ld ? ld : cols) * 2};
+  const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
+  return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+// bf16 -> fp16, eight elements per thread, saturating to +-65504 (exact for magnitudes 6.1e-5 .. 65504).
+static __global__ void __launch_bounds__(256) bf16_to_f16_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, size_t n8) {
+  asm volatile("griddepcontrol.launch_dependents;");        // the GEMM behind it waits before it reads
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n8) return;
+  const uint4 v = in[i];
+  const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+  uint32_t r[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) r[j] = f32x2_to_f16x2_sat(__uint_as_float(u[j] << 16), __uint_as_float(u[j] & 0xFFFF0000u));
+  out[i] = make_uint4(r[0], r[1], r[2], r[3]);
 }
 
 // fp32 -> two fp16 terms per element, hi = fp16(x) (saturating) and lo = fp16(x - hi), written as rows 2i and
@@ -142,6 +158,5 @@ static __global__ void __launch_bounds__(256) f32_to_f16_pair_kernel(const float
   out[(size_t)(2 * row) * k8 + c] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
   out[(size_t)(2 * row + 1) * k8 + c] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
 }
-
 
 }  // namespace nb
