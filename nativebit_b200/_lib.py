@@ -58,6 +58,12 @@ _SIGNATURES = {
     "nb_allreduce": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_int, _c.c_void_p, _c.c_int, _c.c_int, _c.c_int, _c.c_uint32,
                                 _c.c_void_p, _c.c_void_p]),
     "nb_embed_rows": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_int, _c.c_int, _c.c_int, _c.c_void_p, _c.c_void_p]),
+    "nb_chain_terms_bytes": (_c.c_size_t, [_c.c_int, _c.c_int]),
+    "nb_chain_linear": (_c.c_int, [_c.c_void_p, _c.c_void_p]),
+    "nb_chain_embed": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_int, _c.c_int, _c.c_int, _c.c_void_p, _c.c_void_p, _c.c_void_p,
+                                  _c.c_void_p, _c.c_void_p]),
+    "nb_decode_attention_terms": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_int,
+                                             _c.c_int, _c.c_int, _c.c_int, _c.c_void_p, _c.c_int, _c.c_int, _c.c_void_p]),
     "nb_softcap_argmax": (_c.c_int, [_c.c_void_p, _c.c_int, _c.c_int, _c.c_int, _c.c_float, _c.c_void_p, _c.c_void_p, _c.c_void_p,
                                      _c.c_void_p]),
     "nb_gemv_fused": (_c.c_int, [_c.c_int, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_float, _c.c_void_p, _c.c_int, _c.c_void_p,
@@ -105,6 +111,13 @@ def _struct(name: str, pointers: str, floats: str, ints: str):
     """An argument block of nativebit_b200_layered.h: pointers first, then floats, then ints."""
     fields = [(n, _P) for n in pointers.split()] + [(n, _F) for n in floats.split()] + [(n, _I) for n in ints.split()]
     return type(name, (_c.Structure,), {"_fields_": fields})
+
+
+class ChainArgs(_c.Structure):
+    """nb_chain_args of nativebit_b200.h."""
+    _fields_ = ([(n, _P) for n in "w x_terms sq y y_terms residual next_weight sq_out status ahead".split()] + [("ahead_bytes", _c.c_int64), ("eps", _F)]
+                + [(n, _I) for n in "M N K bits mode sq_n split".split()])
+
 
 
 MatvecArgs = _struct("MatvecArgs", "w bias y x delta delta_w x_out norm_w", "eps alpha limit", "N K ldw act norm")

@@ -12,6 +12,7 @@
 #include <cfloat>
 #include <type_traits>
 
+#include "nb_chain.cuh"
 #include "nb_common.cuh"
 #include "nb_device.cuh"
 #include "nb_host.h"
@@ -140,30 +141,32 @@ __global__ void rope_kv_kernel(const float* __restrict__ qkv, const float* __res
   }
 }
 
-// Single-query attention for one (head, batch): scores over keys 0..pos, softmax, weighted sum of
-// values; out[b, out_offset + h*hd + d].  grid (H, B, S) in clusters of S CTAs along z: the CTAs of
-// a cluster split the keys of one head into S contiguous ranges (the whole GPU works on the 32
-// heads of a batch-1 step instead of 32 SMs), each forms the softmax numerator and denominator of
-// its range, and rank 0 merges them through distributed shared memory.  Inside a CTA a warp takes
-// 8 keys per iteration: for the scores four lanes share a key (16-byte loads, two shuffles), for
-// the values a lane owns four head dimensions of all 8 keys.  The values of the first iteration
-// are requested before the scores are computed, so a context of up to 64*S keys costs one memory
-// round trip.  head_dim a multiple of 4, <= 128.  Dynamic smem: see attn_smem_floats.
+// Single-query attention for one (head, batch): softmax over keys 0..pos, weighted sum of values; out[b, out_offset + h*hd + d].
+// grid (H, B, S) in clusters of S CTAs along z: the CTAs of a cluster split the keys of one head into S contiguous ranges (the
+// whole GPU works on the 32 heads of a batch-1 step instead of 32 SMs).  Inside a CTA a warp takes 8 keys per iteration and
+// keeps running maximum, denominator and numerator for itself: for the scores four lanes share a key (16-byte loads, two
+// shuffles), for the values a lane owns four head dimensions of all 8 keys.  Keys and values of the first iteration are
+// requested before the dependency wait, so a context of up to 64*S keys costs one memory round trip.  One barrier later a thread
+// per dimension merges the warps and pushes the CTA's result into rank 0's shared memory; behind the cluster's barrier rank 0
+// merges those from its own.  What bounds it is that chain of latencies: with three more block-wide barriers around the
+// softmax and rank 0 reading the others' results one remote load at a time, a step of the 2.2B decoder with 12 layers took 418 instead of 391 us.
+// head_dim a multiple of 4, <= 128.
 //
 // When `qkv` is given (B, 3*H*hd = [q|k|v]) the kernel first does the work of rope_kv_kernel for its
 // head: it rotates q and k by the position's angle, the CTA that owns key `pos` writes k and v into
 // the caches, and all attend with the rotated q, so the step needs one launch instead of two.
-constexpr int kAttnWarps = 8;
+constexpr int kAttnWarps = 8, kAttnMaxSplit = 8;
 constexpr int kAttnKeysPerIter = kAttnWarps * 8;
 static int attn_per_max(int ctx, int S) { return (((ctx + S - 1) / S) + 7) & ~7; }
-static size_t attn_smem_floats(int ctx, int hd, int S) { return (size_t)attn_per_max(ctx, S) + (size_t)(2 + kAttnWarps) * hd + 4; }
+static size_t attn_limit_floats(int ctx, int hd, int S) { return (size_t)attn_per_max(ctx, S) + (size_t)(2 + kAttnWarps) * hd + 4; }
+static size_t attn_smem_floats(int hd) { return (size_t)(1 + kAttnWarps) * hd + (size_t)kAttnMaxSplit * (hd + 4); }
 
 __global__ void __launch_bounds__(kAttnWarps * 32) decode_attention_kernel(
     const float* __restrict__ q, float* k_cache, float* v_cache, const long long* __restrict__ pos_ptr, float* __restrict__ out,
     int H, int hd, int ctx, int out_stride, int out_offset, const float* __restrict__ qkv, const float* __restrict__ cos2,
-    const float* __restrict__ sin2) {
-  extern __shared__ __align__(16) float sm[];  // scores of this CTA's keys | q | per-warp outputs | exchange (o, max, sum)
-  __shared__ float red[kAttnWarps];
+    const float* __restrict__ sin2, uint8_t* __restrict__ terms) {
+  extern __shared__ __align__(16) float sm[];  // q | per-warp numerators | rank 0: the CTAs' numerator, maximum, denominator
+  __shared__ float s_m[kAttnWarps], s_l[kAttnWarps];
   cg::cluster_group cluster = cg::this_cluster();
   const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -173,156 +176,146 @@ __global__ void __launch_bounds__(kAttnWarps * 32) decode_attention_kernel(
   // wait and arrive while the qkv matvec drains.  Only the row this step writes (position pos) is fetched after it.
   long long pos = *pos_ptr;
   if (pos < 0) return;  // the same for every CTA of the cluster
+  asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");     // this CTA runs: others may write to its shared memory
   if (pos >= ctx) pos = ctx - 1;
   const int n = (int)pos + 1, hd4 = hd >> 2;
   const int per = (((n + S - 1) / S) + 7) & ~7;
   const int k0 = rank * per;
   const int cnt = max(0, min(n, k0 + per) - k0);
-  float* sc = sm;
-  float* qs = sc + ((((ctx + S - 1) / S) + 7) & ~7);
+  float* qs = sm;
   float* part = qs + hd;
-  float* xch = part + kAttnWarps * hd;
+  float* slots = part + kAttnWarps * hd;
+  const int slot = hd + 4;
   const size_t head = ((size_t)b * H + h);
   float* kb = k_cache + head * ctx * hd;
   float* vb = v_cache + head * ctx * hd;
   const int kq = lane >> 2, t = lane & 3;
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 kfirst[8], vfirst[8];  // keys and values of iteration 0
-  {
-    const int jl = warp * 8 + kq;
-    const bool ld = jl < cnt && k0 + jl != (int)pos;
-    const float4* krow = reinterpret_cast<const float4*>(kb + (size_t)(k0 + jl) * hd);
+  float4 kv[8], vv[8];          // keys and values of an iteration
+  auto load = [&](int it, int skip) {
+    const int j0 = (it * kAttnWarps + warp) * 8;
+    const bool ld = j0 + kq < cnt && k0 + j0 + kq != skip;
+    const float4* krow = reinterpret_cast<const float4*>(kb + (size_t)(k0 + j0 + kq) * hd);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) kfirst[i] = (ld && t + 4 * i < hd4) ? krow[t + 4 * i] : zero4;
+    for (int i = 0; i < 8; ++i) kv[i] = (ld && t + 4 * i < hd4) ? krow[t + 4 * i] : zero4;
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int ju = warp * 8 + u;
-      vfirst[u] = (ju < cnt && k0 + ju != (int)pos && lane < hd4) ? *reinterpret_cast<const float4*>(vb + (size_t)(k0 + ju) * hd + 4 * lane)
+    for (int u = 0; u < 8; ++u)
+      vv[u] = (j0 + u < cnt && k0 + j0 + u != skip && lane < hd4) ? *reinterpret_cast<const float4*>(vb + (size_t)(k0 + j0 + u) * hd + 4 * lane)
                                                                    : zero4;
-    }
-  }
+  };
+  load(0, (int)pos);
   float c_pre = 0.f, s_pre = 0.f;  // this thread's entry of the rotary tables (head_dim <= 128 < threads per CTA)
   if (qkv && tid < hd) { c_pre = cos2[pos * hd + tid]; s_pre = sin2[pos * hd + tid]; }
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (qkv) {
-    const float* base = qkv + (size_t)b * 3 * H * hd;
-    const float* qh = base + h * hd;
-    const float* kh = base + H * hd + h * hd;
-    const float* vh = base + 2 * H * hd + h * hd;
-    const bool owner = pos >= k0 && pos < k0 + cnt;
-    for (int i = tid; i < hd; i += blockDim.x) {
-      const float c = c_pre, s = s_pre;
-      const int j = i ^ 1;
-      const float sign = (i & 1) ? 1.f : -1.f;   // rot = (-x2, x1) on interleaved pairs
-      qs[i] = (qh[i] * c + sign * qh[j] * s) * rsqrtf((float)hd);
-      if (owner) {
-        kb[(size_t)pos * hd + i] = kh[i] * c + sign * kh[j] * s;
-        vb[(size_t)pos * hd + i] = vh[i];
+  if (tid < hd) {
+    if (qkv) {
+      const float* qh = qkv + (size_t)b * 3 * H * hd + h * hd;
+      const float *kh = qh + H * hd, *vh = kh + H * hd;
+      const int j = tid ^ 1;
+      const float sign = (tid & 1) ? 1.f : -1.f;   // rot = (-x2, x1) on interleaved pairs
+      qs[tid] = (qh[tid] * c_pre + sign * qh[j] * s_pre) * rsqrtf((float)hd);
+      if (pos >= k0 && pos < k0 + cnt) {
+        kb[(size_t)pos * hd + tid] = kh[tid] * c_pre + sign * kh[j] * s_pre;
+        vb[(size_t)pos * hd + tid] = vh[tid];
       }
+    } else {
+      qs[tid] = q[head * hd + tid] * rsqrtf((float)hd);
     }
-  } else {
-    for (int i = tid; i < hd; i += blockDim.x) qs[i] = q[head * hd + i] * rsqrtf((float)hd);
   }
   __syncthreads();  // also orders the cache row written above before the reads below (same CTA)
 
   const int iters = (cnt + kAttnKeysPerIter - 1) / kAttnKeysPerIter;
   {  // the row written in this step (by this CTA above, or by the launch before): now it can be read
-    const int jl = warp * 8 + kq;
-    if (jl < cnt && k0 + jl == (int)pos) {
-      const float4* krow = reinterpret_cast<const float4*>(kb + (size_t)pos * hd);
+    const int jl = (int)pos - k0 - warp * 8;                 // its place among this warp's first keys
+    if (jl >= 0 && jl < 8 && (int)pos - k0 < cnt) {
+      if (kq == jl) {
+        const float4* krow = reinterpret_cast<const float4*>(kb + (size_t)pos * hd);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) kfirst[i] = (t + 4 * i < hd4) ? krow[t + 4 * i] : zero4;
-    }
+        for (int i = 0; i < 8; ++i) kv[i] = (t + 4 * i < hd4) ? krow[t + 4 * i] : zero4;
+      }
+      const float4 vp = lane < hd4 ? *reinterpret_cast<const float4*>(vb + (size_t)pos * hd + 4 * lane) : zero4;
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int ju = warp * 8 + u;
-      if (ju < cnt && k0 + ju == (int)pos && lane < hd4) vfirst[u] = *reinterpret_cast<const float4*>(vb + (size_t)pos * hd + 4 * lane);
+      for (int u = 0; u < 8; ++u)
+        if (u == jl) vv[u] = vp;
     }
   }
-  float mx = -FLT_MAX;
+  float mx = -FLT_MAX, sum = 0.f;
+  float4 acc = zero4;
+#pragma unroll 1
   for (int it = 0; it < iters; ++it) {
-    const int jl = (it * kAttnWarps + warp) * 8 + kq;
+    if (it > 0) load(it, -1);
+    const int j0 = (it * kAttnWarps + warp) * 8;
     float s = 0.f;
-    if (jl < cnt) {
-      const float4* krow = reinterpret_cast<const float4*>(kb + (size_t)(k0 + jl) * hd);
-      float4 kv[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) kv[i] = it == 0 ? kfirst[i] : ((t + 4 * i < hd4) ? krow[t + 4 * i] : zero4);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (t + 4 * i < hd4) {
-          const float4 qv = reinterpret_cast<const float4*>(qs)[t + 4 * i];
-          s += qv.x * kv[i].x + qv.y * kv[i].y + qv.z * kv[i].z + qv.w * kv[i].w;
-        }
+    for (int i = 0; i < 8; ++i) {
+      if (t + 4 * i < hd4) {
+        const float4 qv = reinterpret_cast<const float4*>(qs)[t + 4 * i];
+        s += qv.x * kv[i].x + qv.y * kv[i].y + qv.z * kv[i].z + qv.w * kv[i].w;
       }
     }
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     s += __shfl_xor_sync(0xffffffffu, s, 2);
-    if (jl < cnt) {
-      if (t == 0) sc[jl] = s;
-      mx = fmaxf(mx, s);
-    }
-  }
-  mx = warp_max(mx);
-  if (lane == 0) red[warp] = mx;
-  __syncthreads();
-  mx = red[0];
-#pragma unroll
-  for (int i = 1; i < kAttnWarps; ++i) mx = fmaxf(mx, red[i]);
-  __syncthreads();
-  float sum = 0.f;
-  for (int j = tid; j < cnt; j += blockDim.x) {
-    const float e = __expf(sc[j] - mx);
-    sc[j] = e;
-    sum += e;
-  }
-  sum = warp_sum(sum);
-  if (lane == 0) red[warp] = sum;
-  __syncthreads();
-  float tot = 0.f;
-#pragma unroll
-  for (int i = 0; i < kAttnWarps; ++i) tot += red[i];
-
-  float4 acc = zero4;
-  for (int it = 0; it < iters; ++it) {
-    const int j0 = (it * kAttnWarps + warp) * 8;
-    float4 vv[8];
+    const bool valid = j0 + kq < cnt;
+    if (!valid) s = -FLT_MAX;
+    float m_new = fmaxf(mx, s);
+    m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 4));
+    m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 8));
+    m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 16));
+    const float e = valid ? __expf(s - m_new) : 0.f;
+    const float keep = __expf(mx - m_new);
+    mx = m_new;
+    float e_sum = e;
+    e_sum += __shfl_xor_sync(0xffffffffu, e_sum, 4);
+    e_sum += __shfl_xor_sync(0xffffffffu, e_sum, 8);
+    e_sum += __shfl_xor_sync(0xffffffffu, e_sum, 16);
+    sum = sum * keep + e_sum;
+    acc.x *= keep; acc.y *= keep; acc.z *= keep; acc.w *= keep;
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      if (it == 0) vv[u] = vfirst[u];
-      else vv[u] = (j0 + u < cnt && lane < hd4) ? *reinterpret_cast<const float4*>(vb + (size_t)(k0 + j0 + u) * hd + 4 * lane) : zero4;
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const float pj = (j0 + u < cnt) ? sc[j0 + u] : 0.f;
-      acc.x += pj * vv[u].x; acc.y += pj * vv[u].y; acc.z += pj * vv[u].z; acc.w += pj * vv[u].w;
+      const float pj = __shfl_sync(0xffffffffu, e, 4 * u);
+      if (j0 + u < cnt) {       // (a row past the range is not looked at, whatever its memory holds)
+        acc.x += pj * vv[u].x; acc.y += pj * vv[u].y; acc.z += pj * vv[u].z; acc.w += pj * vv[u].w;
+      }
     }
   }
   if (lane < hd4) reinterpret_cast<float4*>(part + warp * hd)[lane] = acc;
+  if (lane == 0) { s_m[warp] = mx; s_l[warp] = sum; }
   __syncthreads();
-  for (int d = tid; d < hd; d += blockDim.x) {
-    float o = 0.f;
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  if (tid < hd) {               // a warp without keys has maximum -FLT_MAX: its weight is exp(-inf) = 0, or it has nothing to weigh
+    float m_all = s_m[0];
 #pragma unroll
-    for (int wi = 0; wi < kAttnWarps; ++wi) o += part[wi * hd + d];
-    xch[d] = o;
-  }
-  if (tid == 0) { xch[hd] = mx; xch[hd + 1] = tot; }
-  cluster.sync();
-  if (rank == 0) {
-    for (int d = tid; d < hd; d += blockDim.x) {
-      float m_all = -FLT_MAX;
-      for (int r = 0; r < S; ++r) m_all = fmaxf(m_all, cluster.map_shared_rank(xch, r)[hd]);
-      float num = 0.f, den = 0.f;
-      for (int r = 0; r < S; ++r) {  // a rank without keys has max -FLT_MAX: its weight is exp(-inf) = 0
-        const float* rx = cluster.map_shared_rank(xch, r);
-        const float w = __expf(rx[hd] - m_all);
-        num += w * rx[d];
-        den += w * rx[hd + 1];
-      }
-      out[(size_t)b * out_stride + out_offset + h * hd + d] = num / den;
+    for (int w = 1; w < kAttnWarps; ++w) m_all = fmaxf(m_all, s_m[w]);
+    float num = 0.f, den = 0.f;
+#pragma unroll
+    for (int w = 0; w < kAttnWarps; ++w) {
+      const float e = __expf(s_m[w] - m_all);
+      num += e * part[w * hd + tid];
+      den += e * s_l[w];
     }
+    float* dst = cluster.map_shared_rank(slots, 0) + rank * slot;
+    dst[tid] = num;
+    if (tid == 0) { dst[hd] = m_all; dst[hd + 1] = den; }
   }
-  cluster.sync();  // the exchange buffers stay alive until rank 0 has read them
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  if (rank == 0 && tid < hd) {
+    float m_all = -FLT_MAX;
+#pragma unroll
+    for (int r = 0; r < kAttnMaxSplit; ++r)
+      if (r < S) m_all = fmaxf(m_all, slots[r * slot + hd]);
+    float num = 0.f, den = 0.f;
+#pragma unroll
+    for (int r = 0; r < kAttnMaxSplit; ++r) {  // a rank without keys has max -FLT_MAX: its weight is exp(-inf) = 0
+      if (r < S) {
+        const float w = __expf(slots[r * slot + hd] - m_all);
+        num += w * slots[r * slot + tid];
+        den += w * slots[r * slot + hd + 1];
+      }
+    }
+    if (terms) store_chain_terms(terms, out_stride >> 7, b, out_offset + h * hd + tid, num / den);
+    else out[(size_t)b * out_stride + out_offset + h * hd + tid] = num / den;
+  }
 }
 
 // The same with one CTA per (head, batch), for calls whose heads alone fill the GPU (taken where the kernel above would split
@@ -340,7 +333,7 @@ static size_t wide_smem_floats(int hd) { return (size_t)kWideWarps * kWideD * 2 
 __global__ void __launch_bounds__(kWideWarps * 32) decode_attention_wide_kernel(
     const float* __restrict__ q, float* k_cache, float* v_cache, const long long* __restrict__ pos_ptr, float* __restrict__ out,
     int H, int hd, int ctx, int out_stride, int out_offset, const float* __restrict__ qkv, const float* __restrict__ cos2,
-    const float* __restrict__ sin2) {
+    const float* __restrict__ sin2, uint8_t* __restrict__ terms) {
   extern __shared__ __align__(16) float sm[];  // per warp kWideD stages of keys | values, then q | key | value of this step | outputs
   __shared__ float s_m[kWideWarps], s_l[kWideWarps];
   const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -474,7 +467,8 @@ __global__ void __launch_bounds__(kWideWarps * 32) decode_attention_wide_kernel(
       num += e * part[w * hd + tid];
       den += e * s_l[w];
     }
-    out[(size_t)b * out_stride + out_offset + h * hd + tid] = num / den;
+    if (terms) store_chain_terms(terms, out_stride >> 7, b, out_offset + h * hd + tid, num / den);
+    else out[(size_t)b * out_stride + out_offset + h * hd + tid] = num / den;
   }
 }
 
@@ -487,8 +481,7 @@ static int attn_split(int B, int H) {
 template <typename... Args>
 static int launch_attention(int B, int H, int hd, int ctx, cudaStream_t st, Args... args) {
   const int S = attn_split(B, H);
-  const size_t smem = attn_smem_floats(ctx, hd, S) * sizeof(float);
-  if (smem > 48 * 1024) return NB_ERR_SHAPE;      // the contexts that are taken do not depend on the kernel (this one could do more)
+  if (attn_limit_floats(ctx, hd, S) * sizeof(float) > 48 * 1024) return NB_ERR_SHAPE;      // the contexts that are taken stay what they were
   if (S <= 2) {     // more heads than SMs: no split is needed to occupy the GPU
     static bool done[64] = {};
     int dev = 0;
@@ -504,7 +497,7 @@ static int launch_attention(int B, int H, int hd, int ctx, cudaStream_t st, Args
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(H, B, S);
   cfg.blockDim = dim3(kAttnWarps * 32);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = attn_smem_floats(hd) * sizeof(float);
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1062,7 +1055,20 @@ extern "C" int nb_decode_attention_rope(const float* qkv, const float* cos2, con
   if ((uintptr_t)k_cache % 16 || (uintptr_t)v_cache % 16) return NB_ERR_ALIGN;
   if (int rc = check_device()) return rc;
   return launch_attention(B, H, hd, ctx, (cudaStream_t)stream, (const float*)nullptr, k_cache, v_cache,
-                          reinterpret_cast<const long long*>(pos), out, H, hd, ctx, out_stride, out_offset, qkv, cos2, sin2);
+                          reinterpret_cast<const long long*>(pos), out, H, hd, ctx, out_stride, out_offset, qkv, cos2, sin2, (uint8_t*)nullptr);
+}
+
+extern "C" int nb_decode_attention_terms(const float* qkv, const float* cos2, const float* sin2, const int64_t* pos, float* k_cache,
+                                         float* v_cache, int B, int H, int hd, int ctx, void* terms, int out_cols, int out_offset,
+                                         void* stream) {
+  if (!qkv || !cos2 || !sin2 || !k_cache || !v_cache || !pos || !terms || B < 1 || H < 1 || hd < 2 || (hd & 1) || ctx < 1 || out_offset < 0)
+    return NB_ERR_ARG;
+  if (hd > 128 || hd % 4 != 0 || out_cols % kBlock || out_offset + H * hd > out_cols) return NB_ERR_SHAPE;
+  if ((uintptr_t)k_cache % 16 || (uintptr_t)v_cache % 16 || (uintptr_t)terms % 16) return NB_ERR_ALIGN;
+  if (int rc = check_device()) return rc;
+  return launch_attention(B, H, hd, ctx, (cudaStream_t)stream, (const float*)nullptr, k_cache, v_cache,
+                          reinterpret_cast<const long long*>(pos), (float*)nullptr, H, hd, ctx, out_cols, out_offset, qkv, cos2, sin2,
+                          reinterpret_cast<uint8_t*>(terms));
 }
 
 extern "C" int nb_decode_attention(const float* q, const float* k_cache, const float* v_cache, const int64_t* pos, int B, int H,
@@ -1073,7 +1079,7 @@ extern "C" int nb_decode_attention(const float* q, const float* k_cache, const f
   if (int rc = check_device()) return rc;
   return launch_attention(B, H, hd, ctx, (cudaStream_t)stream, q, const_cast<float*>(k_cache), const_cast<float*>(v_cache),
                           reinterpret_cast<const long long*>(pos), out, H, hd, ctx, out_stride, out_offset, (const float*)nullptr,
-                          (const float*)nullptr, (const float*)nullptr);
+                          (const float*)nullptr, (const float*)nullptr, (uint8_t*)nullptr);
 }
 
 extern "C" int nb_prefill_attention(const float* qkv, int B, int T, int H, int hd, const float* cos2, const float* sin2, int pos0,

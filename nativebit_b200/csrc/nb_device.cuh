@@ -70,8 +70,7 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
 // selects between the two halves through a byte mask (0xFF where the index is >= 8) that a permute
 // of {0x00000000, 0xFFFFFFFF} produces from index >> 1.
 template <int BITS>
-__device__ __forceinline__ void lookup4(uint32_t sel, const uint32_t (&T)[BITS == 4 ? 8 : 4], uint32_t& r01, uint32_t& r23) {
-  uint32_t lo, hi;
+__device__ __forceinline__ void lookup_planes(uint32_t sel, const uint32_t (&T)[BITS == 4 ? 8 : 4], uint32_t& lo, uint32_t& hi) {
   if (BITS == 4) {
     const uint32_t s7 = sel & 0x7777u;
     const uint32_t m = prmt(0u, 0xFFFFFFFFu, (sel >> 1) & 0x7777u);
@@ -83,8 +82,44 @@ __device__ __forceinline__ void lookup4(uint32_t sel, const uint32_t (&T)[BITS =
     lo = prmt(T[0], T[1], sel);
     hi = prmt(T[2], T[3], sel);
   }
+}
+template <int BITS>
+__device__ __forceinline__ void lookup4(uint32_t sel, const uint32_t (&T)[BITS == 4 ? 8 : 4], uint32_t& r01, uint32_t& r23) {
+  uint32_t lo, hi;
+  lookup_planes<BITS>(sel, T, lo, hi);
   r01 = prmt(lo, hi, 0x5140);
   r23 = prmt(lo, hi, 0x7362);
+}
+
+// 256 and -256 as values that the compiler cannot see through, so that a multiply-add by them stays one.  Byte permutes, logic
+// and shifts share one pipe of 64 lanes per clock and SM, which bounds every kernel that looks weights up; multiply-adds run
+// beside it on another (measured on B200, lanes per clock and SM: permute, logic or shift 64, multiply-add 64, the two in turn
+// 130; the high half of a product 32, so right shifts stay shifts).  gridDim.z is 1 wherever this is used.
+struct ByteShift {
+  uint32_t up, down;
+};
+__device__ __forceinline__ ByteShift byte_shift() { return ByteShift{gridDim.z << 8, 0u - (gridDim.z << 8)}; }
+__device__ __forceinline__ uint32_t mad_lo(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t d;
+  asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+
+// Two bytes each of four weights, lo = (l0, l1, l2, l3) and hi = (h0, h1, h2, h3), -> the pairs (w0, w2) and (w1, w3) with one
+// permute and two multiply-adds: 256 hi + lo counts every byte where it belongs and those of w1 and w3 once more in the byte
+// above, which is 256 (w1, w3); the sums are exact modulo 2^32.
+__device__ __forceinline__ void interleave_pairs(uint32_t lo, uint32_t hi, const ByteShift& k, uint32_t& w02, uint32_t& w13) {
+  w13 = prmt(lo, hi, 0x7351);
+  w02 = mad_lo(w13, k.down, mad_lo(hi, k.up, lo));
+}
+
+// lookup4 with the weights of nibbles 0 and 2, then those of nibbles 1 and 3.
+template <int BITS>
+__device__ __forceinline__ void lookup4_pairs(uint32_t sel, const uint32_t (&T)[BITS == 4 ? 8 : 4], const ByteShift& k, uint32_t& w02,
+                                              uint32_t& w13) {
+  uint32_t lo, hi;
+  lookup_planes<BITS>(sel, T, lo, hi);
+  interleave_pairs(lo, hi, k, w02, w13);
 }
 
 __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
@@ -139,6 +174,39 @@ __device__ __forceinline__ void read_block(const uint8_t* blk, uint32_t (&w)[Fmt
     const uint4 v = *reinterpret_cast<const uint4*>(blk + 16 * i);
     w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
   }
+}
+
+// ---- a unit of the stream layout (nb_stream_pack): 16 rows x 128 weights ------------------------------------------
+// Lane (g, t) = (lane >> 2, lane & 3) owns weights 32t .. 32t + 31 of rows g and g + 8: four selector words per row, word j with
+// the indices of positions 8j .. 8j + 7, one per nibble, ready for the byte-permute lookups.  Behind the lanes' words the 16
+// rows' lookup tables.  (Packed indices, 1024 instead of 1280 bytes per unit at 3 bits, were measured: they cost a unit 18
+// operations per lane on the pipe that bounds its lookups, and 78 matvecs in one launch took 170 us for 165.)
+template <int BITS> struct StreamUnit {
+  static constexpr int kIdxBytes = 1024;                    // 32 lanes x 2 rows x 4 selector words
+  static constexpr int kTabBytes = BITS == 4 ? 32 : 16;     // one row's lookup table
+  static constexpr int kBytes = kIdxBytes + 16 * kTabBytes; // 1280 at 2 and 3 bits, 1536 at 4
+};
+
+// Selector words of row g (half 0) or g + 8 (half 1) of lane (g, t).
+__device__ __forceinline__ void unit_selectors(const uint8_t* ub, int lane, int half, uint32_t (&P)[4]) {
+  const uint4 v = *reinterpret_cast<const uint4*>(ub + half * 512 + lane * 16);
+  P[0] = v.x; P[1] = v.y; P[2] = v.z; P[3] = v.w;
+}
+// Row `row`'s lookup table.
+template <int BITS>
+__device__ __forceinline__ void unit_table(const uint8_t* ub, int row, uint32_t (&T)[BITS == 4 ? 8 : 4]) {
+  using U = StreamUnit<BITS>;
+#pragma unroll
+  for (int j = 0; j < U::kTabBytes / 16; ++j) {
+    const uint4 v = *reinterpret_cast<const uint4*>(ub + U::kIdxBytes + row * U::kTabBytes + 16 * j);
+    T[4 * j] = v.x; T[4 * j + 1] = v.y; T[4 * j + 2] = v.z; T[4 * j + 3] = v.w;
+  }
+}
+
+// 16 bytes of shared memory where `act`, else `v` stays what it is: lanes without data cost the load nothing.
+__device__ __forceinline__ void lds_if(uint4& v, const uint8_t* src, uint32_t act) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\t@p ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+               : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w) : "r"(smem_u32(src)), "r"(act));
 }
 
 __device__ __forceinline__ float load_x(const void* x, int dtype, size_t i) {

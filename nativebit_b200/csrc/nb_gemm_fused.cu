@@ -83,11 +83,6 @@ constexpr bool enough_stages() {
 }
 static_assert(enough_stages(), "stages per producer group");
 
-template <int BITS> struct FusedFmt {
-  static constexpr int kTabBytes = BITS == 4 ? 32 : 16;
-  static constexpr int kUnitBytes = 1024 + 16 * kTabBytes;   // the stream layout's unit (nb_stream.cu)
-};
-
 // k-steps of one of ks splits: whole k-blocks, as the raw weights arrive
 __host__ __device__ constexpr int split_steps(int KT, int ks) { return (KT / 2 + ks - 1) / ks * 2; }
 
@@ -100,7 +95,7 @@ template <int BITS>
 __global__ void __launch_bounds__(kFThreads, 1)
 gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, void* __restrict__ y, int y_dtype,
                   int M, int N, int K, int BN, int m_tiles, int w_tiles, int pair, int ks, float* __restrict__ partial, int* status) {
-  using F = FusedFmt<BITS>;
+  using F = StreamUnit<BITS>;
   constexpr int kT = BITS == 4 ? 8 : 4;
   const int S = fused_stages(BN), R = fused_raw_stages(BN);
   const int b_bytes = BN * kFK * 2;           // multiple of 1024 because BN is a multiple of 16
@@ -262,7 +257,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         for (int kb = k_lo >> 1; kb < k_hi >> 1; ++kb) {
           ok = bar_wait(&raw_empty[r], phase ^ 1, abort_flag, status);
           if (!ok) break;
-          bar_expect_tx(&raw_full[r], 8u * F::kUnitBytes);
+          bar_expect_tx(&raw_full[r], 8u * F::kBytes);
           tma_load_3d(sW + r * kFRawBytes, &map_w, &raw_full[r], 0, kb, rt0);
           if (++r == R) { r = 0; phase ^= 1; }
         }
@@ -274,7 +269,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     const int w = warp - kFProducerWarp0;
     const int grp = w / kFProducerWarps, rt0 = 2 * (w % kFProducerWarps);      // group `grp` fills the steps st with st % 4 == grp
     const int r16 = lane >> 1, q2 = lane & 1, g = r16 & 7, hrow = r16 >> 3;
-    const uint8_t* raw0 = sW + rt0 * F::kUnitBytes;
+    const uint8_t* raw0 = sW + rt0 * F::kBytes;
     // positions 64 * (grp & 1) .. + 63 of a k-block: this thread's lane group of the unit is 2 * (grp & 1) + q2
     const int sel_off = hrow * 512 + (g * 4 + 2 * (grp & 1) + q2) * 16, tab_off = 1024 + r16 * F::kTabBytes;
     // row r of a K-major tile with 128-byte swizzle: 16-byte chunk c sits at chunk c ^ (r & 7); a row tile is 2 KB
@@ -295,7 +290,7 @@ gemm_fused_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         uint4 out[2][4];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const uint8_t* u = raw0 + r * kFRawBytes + h * F::kUnitBytes;
+          const uint8_t* u = raw0 + r * kFRawBytes + h * F::kBytes;
           const uint4 sel = *reinterpret_cast<const uint4*>(u + sel_off);
           uint32_t T[kT];
 #pragma unroll
@@ -443,7 +438,7 @@ extern "C" int nb_gemm_prefill_fused(const void* x, int x_dtype, int M, const ui
   const int bn = plan.bn;
   CUtensorMap mx, mw;
   if (int rc = make_map(&mx, xh, rows, K, bn)) return rc;
-  if (int rc = make_map_units(&mw, w_stream, bits == 4 ? FusedFmt<4>::kUnitBytes : FusedFmt<3>::kUnitBytes, K / kBlock, (N + 15) / 16)) return rc;
+  if (int rc = make_map_units(&mw, w_stream, bits == 4 ? StreamUnit<4>::kBytes : StreamUnit<3>::kBytes, K / kBlock, (N + 15) / 16)) return rc;
   const int m_tiles = (rows + bn - 1) / bn, w_tiles = (N + kFM - 1) / kFM;
   int ks = plan.ks;
   if (ks > 1 && (N % 4 != 0 || (uintptr_t)y % 16)) ks = 1;       // the summing kernel writes four outputs at a time

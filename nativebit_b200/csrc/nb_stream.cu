@@ -100,16 +100,10 @@ constexpr int kStreamSmem = kOffDst + 256;
 static_assert(sizeof(StreamOp) == 160, "nb_stream_op layout");
 static_assert(kStreamSmem <= 224 * 1024, "shared memory budget");
 
-// A unit in the stream layout: the 32 lanes' selector words, then the 16 rows' lookup tables.  Lane
-// (g, t) owns weights 32t .. 32t+31 of the block in rows g and g+8: four words per row, word j = the
-// indices of positions 32t + 8j .. + 7, one per nibble in position order, ready for the byte-permute
-// lookups (the 3- and 2-bit fields are spread to nibbles when the copy is built, so the kernels spend
-// no instructions on it, and activations are used in their natural order).
-template <int BITS> struct UnitFmt {
+// A unit of the stream layout (StreamUnit, nb_device.cuh) as the source words of a lane and as a ring stage.
+template <int BITS> struct UnitFmt : StreamUnit<BITS> {
+  using StreamUnit<BITS>::kBytes;
   static constexpr int kW = Fmt<BITS>::kWords / 4;          // packed words of one lane's 32 indices in the source layout
-  static constexpr int kIdxBytes = 1024;                    // 32 lanes x 2 rows x 4 selector words
-  static constexpr int kTabBytes = BITS == 4 ? 32 : 16;     // one row's lookup table
-  static constexpr int kBytes = kIdxBytes + 16 * kTabBytes; // 1280 at 2 and 3 bits, 1536 at 4: one ring stage
   static constexpr int kStages = kRingBytes / (kSW * kBytes) < 16 ? kRingBytes / (kSW * kBytes) : 16;   // per warp: 6, 6, 5 with 16 warps
   // units a warp works on per loop iteration (one wait, one round of bookkeeping for all of them)
 #ifdef NB_STREAM_BATCH

@@ -348,6 +348,9 @@ def step(model: PackedGPT, x: torch.Tensor, caches):
     return logits[:, -1, :], caches
 
 
+CHAIN_MAX_ROWS = 16          # activation rows up to which a step's linears run on nb_chain_linear
+
+
 class DecodeSession(Session):
     """Greedy decoding of a PackedGPT with the whole step in one CUDA graph: token, position and caches live on the
     device, the next token is the argmax written back into the token buffer, so N steps are N graph
@@ -376,6 +379,11 @@ class DecodeSession(Session):
         # (nb_gemv_stream_rows): one pass over the weights for all rows, as many rows per launch as shared memory holds
         self.tile_rows = bool(fits and 2 <= batch_size <= 8 and fused and tile_gemv is not False
                               and getattr(model, "exchange", None) is None)
+        # the default for both on one GPU: a chain in which every launch hands the next its activations ready for the tensor cores
+        # (nb_chain_linear)
+        self.chain = bool(fits and fused and tile_gemv is not False and batch_size <= CHAIN_MAX_ROWS and model.tp_size == 1
+                          and getattr(model, "exchange", None) is None and model.embedding.dtype == torch.bfloat16
+                          and model.config.n_embd % 128 == 0 and all(b.gate_up.out_features % 256 == 0 for b in model.blocks))
         # stream=True (one sequence on one GPU): the whole step is ONE launch of the persistent kernel
         # (stream.py).  The default is the chain of fused kernels, which measures faster: inside one launch
         # every operation pays a device-wide flag wait and the staging of its activations in full.
@@ -403,6 +411,10 @@ class DecodeSession(Session):
             self.bgu = torch.zeros(B, blk.gate_up.out_features, **f32)
             self.bhm = torch.zeros(B, blk.down.in_features, **f32)
             self.bd = torch.zeros(B, cfg.n_embd, **f32)
+            if self.chain:                    # what the chain's launches exchange: rows as terms, partial sums of squares
+                self.cx, self.catt, self.ch = (ops.chain_terms(B, k, dev) for k in (cfg.n_embd, model.o_cols, blk.down.in_features))
+                self.csq = torch.zeros(B, cfg.n_embd // 16, **f32)
+                self.cstatus = torch.zeros(1, dtype=torch.int32, device=dev)
             self.bterms = torch.empty(2 * B * max(cfg.n_embd, blk.down.in_features) if B > 16 else 0, dtype=torch.float16, device=dev)
 
     def _terms_of(self, lin: PackedLinear) -> torch.Tensor | None:
@@ -424,6 +436,35 @@ class DecodeSession(Session):
             ops.gemv(x[r:r + 16], lin.packed_indices, lin.codebook, lin.bits, lin.block_size, lin.out_features,
                      lin.in_features, out=out[r:r + 16])
 
+    def _chain_layers(self) -> torch.Tensor:
+        """The layers of a step through nb_chain_linear, five launches each: q | k | v, attention, out_proj, gate and up, down.
+        Returns the residual stream behind the last layer."""
+        m, x, eps = self.model, self.bx, self.model.config.norm_eps
+        ops.chain_embed(m.embedding, self.token, m.blocks[0].ln1, x, self.cx, self.csq)
+
+        def weight(lin, mode):
+            return lin.stream_weight(1 if mode == ops.CHAIN_SWIGLU else 0)
+
+        def linear(mode, lin, x_terms, behind=None, **kw):
+            ops.chain_linear(mode, weight(lin, mode), lin.bits, self.B, lin.out_features, lin.in_features, x_terms, self.cstatus,
+                             ahead=behind, **kw)
+        # every launch brings the matrix two linears ahead into L2: one ahead is too late for gate and up (18 MB behind the 3 us of
+        # out_proj), and nothing reads memory while the attention runs
+        for i, blk in enumerate(m.blocks):
+            k_buf, v_buf, _ = self.caches[i]
+            nxt = m.blocks[i + 1] if i + 1 < len(m.blocks) else None
+            linear(ops.CHAIN_STORE, blk.qkv, self.cx, weight(blk.gate_up, ops.CHAIN_SWIGLU), sq=self.csq, eps=eps, y=self.bqkv)
+            ops.decode_attention_terms(self.bqkv, m.cos2, m.sin2, self.pos, k_buf, v_buf, self.catt, m.o_cols, m.o_col0)
+            linear(ops.CHAIN_RESIDUAL, blk.out_proj, self.catt, weight(blk.down, 0), residual=x, y_terms=self.cx, next_weight=blk.ln2,
+                   sq_out=self.csq)
+            linear(ops.CHAIN_SWIGLU, blk.gate_up, self.cx, nxt and weight(nxt.qkv, 0), sq=self.csq, eps=eps, y_terms=self.ch)
+            if nxt is not None:
+                linear(ops.CHAIN_RESIDUAL, blk.down, self.ch, weight(nxt.out_proj, 0), residual=x, y_terms=self.cx, next_weight=nxt.ln1,
+                       sq_out=self.csq)
+            else:
+                linear(ops.CHAIN_RESIDUAL, blk.down, self.ch, residual=x)
+        return x
+
     @torch.no_grad()
     def _step_body_fused(self):
         """The decode step on the fused kernels.  Up to 8 sequences: 5 launches per layer (residual add +
@@ -434,7 +475,10 @@ class DecodeSession(Session):
         fold = self.B <= 8
         xch = getattr(m, "exchange", None) if fold else None     # all-reduces folded into the GEMVs
         xa, xb = self.bx, self.bx2                                # residual stream, ping-pong
-        if m.embedding.dtype == torch.bfloat16:
+        chain = self.chain and self.swiglu_epilogue and not (self.single_term or self.residual_in_matvec)
+        if chain:
+            xa = self._chain_layers()
+        elif m.embedding.dtype == torch.bfloat16:
             ops.embed_rows(m.embedding, self.token, xa)
         else:
             xa.copy_(m.embedding[self.token[:, 0]])
@@ -508,7 +552,7 @@ class DecodeSession(Session):
                 self._linear_into(lin, x, out)
             return m._all_reduce(out)
 
-        for i, blk in enumerate(m.blocks):
+        for i, blk in enumerate(() if chain else m.blocks):
             k_buf, v_buf, _ = self.caches[i]
             norm_linear(blk.qkv, delta, blk.ln1, self.bqkv)
             ops.decode_attention_rope(self.bqkv, m.cos2, m.sin2, self.pos, k_buf, v_buf, self.batt, m.o_col0)
@@ -583,6 +627,8 @@ class DecodeSession(Session):
         tensor-parallel exchange that never arrived).  Reads device status words: synchronises."""
         if self.prog is not None and self.prog.status() != 0:
             raise RuntimeError("nb_stream_run: a bounded wait ran out (status NB_ERR_TIMEOUT in the program state)")
+        if getattr(self, "cstatus", None) is not None and int(self.cstatus.item()) != 0:
+            raise RuntimeError("nb_chain_linear: a bounded wait ran out (status NB_ERR_TIMEOUT)")
         held = list(self._scratch)               # what the graphs replay on, and the workspaces of the streams the steps ran on
         for st in ((self.stream, torch.cuda.current_stream(self.dev)) if self.use_graph else (torch.cuda.current_stream(self.dev),)):
             with torch.cuda.stream(st):

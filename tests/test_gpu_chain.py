@@ -1,0 +1,116 @@
+"""The decode chain's packed linears (nb_chain_linear, nb_chain_embed) against fp64 products of the oracle's dense weight."""
+import numpy as np
+import pytest
+import torch
+
+from nativebit_b200 import ops
+from nativebit_b200.stream import stream_pack
+from oracle import nb_oracle as o
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _matrix(n, k, bits, seed, row_mode=0):
+    packed, cb, _ = o.make_packed_linear(n, k, bits, seed=seed)
+    w = stream_pack(torch.from_numpy(packed).to(DEV), torch.from_numpy(cb).to(DEV), bits, n, k, row_mode)
+    return w, torch.from_numpy(o.dequant_packed(packed, cb.astype(np.float32), n, k, bits)).to(DEV).double()
+
+
+def _terms(x):
+    """(m, k) fp32 -> the layout of nb_chain_linear, written out from its description."""
+    m, k = x.shape
+    hi = x.clamp(-65504, 65504).half()
+    lo = (x - hi.float()).half()
+    out = torch.zeros(m, 2, k // 128, 4, 4, 8, dtype=torch.float16, device=DEV)      # row, term, block, segment, chunk, value
+    for s, v in enumerate((hi, lo)):
+        v = v.view(m, k // 128, 4, 4, 8)[..., [0, 2, 1, 3, 4, 6, 5, 7]]
+        for t in range(4):
+            for c in range(4):
+                out[:, s, :, t, c ^ t ^ s] = v[:, :, t, c]
+    return out.view(torch.uint8).reshape(-1)
+
+
+def _values(terms, m, k):
+    t = terms[:4 * m * k].view(torch.float16).view(m, 2, k // 128, 4, 4, 8).double()
+    out = torch.zeros(m, k // 128, 4, 4, 8, dtype=torch.float64, device=DEV)
+    for s in range(2):
+        for seg in range(4):
+            for c in range(4):
+                out[:, :, seg, c] += t[:, s, :, seg, c ^ seg ^ s]
+    return out[..., [0, 2, 1, 3, 4, 6, 5, 7]].view(m, k)
+
+
+def _close(got, want, rel):
+    assert torch.isfinite(got.double()).all()
+    err = (got.double() - want).norm() / want.norm()
+    assert err <= rel, float(err)
+
+
+# fp32 sums of products of 22-bit activations and exact weights: a few 2^-22 of the norm (2.4e-7 each)
+REL = 2e-6
+SHAPES = [(16, 128, 1), (40, 128, 3), (256, 384, 1), (2560, 2560, 1), (2560, 6912, 1), (2560, 6912, 2), (1000, 1024, 4), (7680, 2560, 5),
+          (2560, 6912, 8), (5632, 2048, 8), (512, 2560, 9), (2560, 6912, 16), (2560, 2560, 17), (3072, 1024, 32), (30000, 256, 1)]
+
+
+@pytest.mark.parametrize("n,k,m", SHAPES)
+@pytest.mark.parametrize("bits", [2, 3, 4])
+def test_chain_linear_stores_the_product(built_lib, n, k, m, bits):
+    w, dense = _matrix(n, k, bits, seed=n + k + m)
+    g = torch.Generator(device=DEV).manual_seed(m)
+    x = torch.randn(m, k, device=DEV, generator=g)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    want = x.double() @ dense.T
+    ran = 0
+    for split in (0, 1, 2, 4, 8):
+        y = torch.full((m, n), float("nan"), device=DEV)
+        try:
+            ops.chain_linear(ops.CHAIN_STORE, w, bits, m, n, k, _terms(x), status, y=y, split=split)
+        except RuntimeError as e:
+            assert split and "shape" in str(e)            # more CTAs than k-blocks, or the activations do not fit
+            continue
+        ran += 1
+        _close(y, want, REL)
+        again = torch.empty_like(y)
+        ops.chain_linear(ops.CHAIN_STORE, w, bits, m, n, k, _terms(x), status, y=again, split=split)
+        assert torch.equal(y, again)
+    assert ran >= 2 and int(status.item()) == 0
+
+
+@pytest.mark.parametrize("m,c,f", [(1, 256, 512), (3, 1024, 2816), (8, 2560, 6912), (20, 384, 640)])
+def test_chain_carries_norms_and_residuals(built_lib, m, c, f):
+    """embedding -> gate | up -> down -> a linear of the normed result."""
+    bits, eps = 3, 1e-6
+    g = torch.Generator(device=DEV).manual_seed(c)
+    table = torch.randn(50, c, device=DEV, generator=g).bfloat16()
+    token = torch.randint(0, 50, (m, 1), device=DEV, generator=g)
+    w1, w2 = (1 + 0.1 * torch.randn(c, device=DEV, generator=g) for _ in range(2))
+    gu, gu_dense = _matrix(2 * f, c, bits, 1, row_mode=1)
+    down, down_dense = _matrix(c, f, bits, 2)
+    last, last_dense = _matrix(400, c, bits, 3)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    x, sq = torch.empty(m, c, device=DEV), torch.empty(m, c // 16, device=DEV)
+    cx, ch = ops.chain_terms(m, c, DEV), ops.chain_terms(m, f, DEV)
+    ops.chain_embed(table, token, w1, x, cx, sq)
+    emb = table[token[:, 0]].double()
+    assert torch.equal(x.double(), emb)
+    _close(_values(cx, m, c), emb * w1.double(), REL)
+    _close(sq.double().sum(1), (emb * emb).sum(1), REL)
+
+    def rms(v, w):
+        return v / torch.sqrt((v * v).mean(-1, keepdim=True) + eps) * w.double()
+    ops.chain_linear(ops.CHAIN_SWIGLU, gu, bits, m, 2 * f, c, cx, status, sq=sq, eps=eps, y_terms=ch)
+    z = rms(emb, w1) @ gu_dense.T
+    h = torch.nn.functional.silu(z[:, :f]) * z[:, f:]
+    _close(_values(ch, m, f), h, 4 * REL)                 # + the fast exponential
+    ops.chain_linear(ops.CHAIN_RESIDUAL, down, bits, m, c, f, ch, status, residual=x, y_terms=cx, next_weight=w2, sq_out=sq)
+    r = emb + h @ down_dense.T
+    _close(x, r, 4 * REL)
+    _close(_values(cx, m, c), r * w2.double(), 4 * REL)
+    y = torch.empty(m, 400, device=DEV)
+    ops.chain_linear(ops.CHAIN_STORE, last, bits, m, 400, c, cx, status, sq=sq, eps=eps, y=y)
+    _close(y, rms(r, w2) @ last_dense.T, 8 * REL)
+    before = x.clone()
+    ops.chain_linear(ops.CHAIN_RESIDUAL, down, bits, m, c, f, ch, status, residual=x)          # nothing behind it
+    _close(x, before.double() + h @ down_dense.T, 4 * REL)
+    assert int(status.item()) == 0
