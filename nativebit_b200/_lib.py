@@ -6,10 +6,11 @@ non-zero status, a RuntimeError is raised.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 import re
 
-from .build import LIB_PATH, library_path
+from .build import BIND_PATH, LIB_PATH, library_path
 
 NB_F32, NB_F16, NB_BF16, NB_F16_TERMS = 0, 1, 2, 8
 
@@ -183,6 +184,21 @@ def lib() -> ctypes.CDLL:
     if _lib is None:
         _lib = _open(LIB_PATH, _SIGNATURES)
     return _lib
+
+
+_bind = None
+
+
+def bind():
+    """The native host side of PackedLinear's call (csrc/nb_bind.cpp)."""
+    global _bind
+    if _bind is None:
+        if not os.path.exists(BIND_PATH):
+            raise RuntimeError(f"{BIND_PATH} is missing: build it with `python -m nativebit_b200.build` (nativebit_b200 has no fallback path)")
+        spec = importlib.util.spec_from_file_location("nativebit_b200._bind", BIND_PATH)
+        _bind = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(_bind)
+    return _bind
 
 
 def layered_lib() -> ctypes.CDLL:

@@ -1,0 +1,93 @@
+// The host side of PackedLinear's call as one native function (a CPython module over torch's C++ tensors and the C ABI).  One
+// activation row through 2560 x 2560 is 4.9 us on the device and was 16.2 us of host code: 2.4 of them the launch, the rest views,
+// attribute and device look-ups, and fifteen arguments converted one by one.
+//
+// `linear` takes the calls it knows to be plain, and answers None to everything else (another device than the current one,
+// tensor subclasses, no rows, gaps between rows, a workspace that is missing or too small, any status but success): the
+// general path then does what it always did, its errors included.
+#include <ATen/core/Tensor.h>
+#include <ATen/ops/empty.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/nativebit_b200.h"
+
+namespace {
+
+constexpr int64_t kBlock = 128, kGemvRows = 16, kFusedRows = 1024;
+
+int tag(at::ScalarType t) {
+  return t == at::kFloat ? (int)NB_F32 : t == at::kHalf ? (int)NB_F16 : t == at::kBFloat16 ? (int)NB_BF16 : -1;
+}
+
+// workspaces[(device, stream)], or nullptr.
+const at::Tensor* workspace(PyObject* workspaces, int device, void* stream) {
+  PyObject* key = Py_BuildValue("(iK)", device, (unsigned long long)(uintptr_t)stream);
+  if (!key) return nullptr;
+  PyObject* ws = PyDict_GetItemWithError(workspaces, key);        // borrowed
+  Py_DECREF(key);
+  return ws && THPVariable_Check(ws) ? &THPVariable_Unpack(ws) : nullptr;
+}
+
+// linear(x, packed, codebook, w_stream or None, n, k, bits, ordered, gemv workspaces, prefill workspaces) -> y or None
+PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
+  HANDLE_TH_ERRORS
+  if (count != 10) {
+    PyErr_SetString(PyExc_TypeError, "linear takes ten arguments");
+    return nullptr;
+  }
+  if (!THPVariable_CheckExact(a[0]) || !THPVariable_CheckExact(a[1]) || !THPVariable_CheckExact(a[2]) || !PyDict_Check(a[8]) || !PyDict_Check(a[9]))
+    Py_RETURN_NONE;
+  const at::Tensor &x = THPVariable_Unpack(a[0]), &packed = THPVariable_Unpack(a[1]), &codebook = THPVariable_Unpack(a[2]);
+  const int64_t n = PyLong_AsLongLong(a[4]), k = PyLong_AsLongLong(a[5]);
+  const int bits = (int)PyLong_AsLong(a[6]), ordered = PyObject_IsTrue(a[7]);
+  if (PyErr_Occurred()) return nullptr;
+  const int xt = tag(x.scalar_type()), ct = tag(codebook.scalar_type());
+  if (xt < 0 || (ct != NB_F16 && ct != NB_F32) || !x.is_cuda() || x.layout() != at::kStrided || x.dim() < 1 || x.size(-1) != k || !x.is_contiguous() ||
+      n < 1 || k < 1 || n > INT32_MAX || k > INT32_MAX)
+    Py_RETURN_NONE;
+  const at::Device device = x.device();
+  const int64_t m = x.numel() / k;
+  if (m < 1 || m > kFusedRows || packed.device() != device || codebook.device() != device || device.index() != c10::cuda::current_device()) Py_RETURN_NONE;
+  void* const stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
+  at::DimVector shape(x.sizes());
+  shape.back() = n;
+  int rc = NB_ERR_ARG;
+  if (m <= kGemvRows) {
+    const at::Tensor* ws = workspace(a[8], device.index(), stream);
+    if (!ws) Py_RETURN_NONE;
+    at::Tensor y = at::empty(shape, x.options().requires_grad(false).memory_format(c10::MemoryFormat::Contiguous));
+    const void *xp = x.const_data_ptr(), *cp = codebook.const_data_ptr();
+    const uint8_t* pp = static_cast<const uint8_t*>(packed.const_data_ptr());
+    void *yp = y.mutable_data_ptr(), *wp = ws->mutable_data_ptr();
+    const size_t wn = ws->nbytes();
+    Py_BEGIN_ALLOW_THREADS
+    rc = (ordered ? nb_gemv_ordered : nb_gemv)(xp, xt, (int)m, pp, cp, ct, bits, kBlock, (int)n, (int)k, yp, xt, wp, wn, stream);
+    Py_END_ALLOW_THREADS
+    if (rc == NB_OK) return THPVariable_Wrap(std::move(y));
+  } else if (xt != NB_F16 && m * (xt == NB_F32 ? 2 : 1) <= kFusedRows && THPVariable_CheckExact(a[3])) {       // (that kernel writes bf16 or fp32)
+    const at::Tensor &w = THPVariable_Unpack(a[3]), *ws = workspace(a[9], device.index(), stream);
+    if (!ws || w.device() != device) Py_RETURN_NONE;
+    at::Tensor y = at::empty(shape, x.options().requires_grad(false).memory_format(c10::MemoryFormat::Contiguous));
+    const void* xp = x.const_data_ptr();
+    const uint8_t* pw = static_cast<const uint8_t*>(w.const_data_ptr());
+    void *yp = y.mutable_data_ptr(), *wp = ws->mutable_data_ptr();
+    const size_t wn = ws->nbytes();
+    Py_BEGIN_ALLOW_THREADS
+    rc = nb_gemm_prefill_fused(xp, xt, (int)m, pw, bits, (int)n, (int)k, yp, xt, wp, wn, stream);
+    Py_END_ALLOW_THREADS
+    if (rc == NB_OK) return THPVariable_Wrap(std::move(y));
+  }
+  if (PyErr_Occurred()) return nullptr;
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {{"linear", (PyCFunction)(void (*)(void))linear, METH_FASTCALL, nullptr}, {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_bind", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__bind(void) { return PyModule_Create(&module); }

@@ -13,7 +13,7 @@ import numpy as np
 import torch
 from torch.nn.modules import module as _module
 
-from . import ops
+from . import _lib, ops
 
 BS = 128      # weights per codebook block
 NE = 8        # codebook entries per block at 3 bits
@@ -70,6 +70,13 @@ class PackedLinear(torch.nn.Module):
         self._fresh = True
 
     def forward(self, x):
+        if self.block_size == BS and x.is_cuda:      # the plain calls: checks, result and launch in one native function
+            y = _lib.bind().linear(x, self.packed_indices, self.codebook, self.__dict__.get("_wstream"), self.out_features, self.in_features,
+                                   self.bits, self._fresh, ops._workspaces, ops._prefill_ws)
+            if y is not None:
+                if self._fresh and y.numel() <= GEMV_MAX_M * self.out_features:
+                    self._fresh = False
+                return y
         shape = x.shape
         x_flat = x.reshape(-1, self.in_features)
         if not x_flat.is_contiguous():
@@ -84,7 +91,8 @@ class PackedLinear(torch.nn.Module):
         elif m <= GEMV_MAX_M:
             y = ops.gemv(x_flat, self.packed_indices, self.codebook, self.bits, self.block_size,
                          self.out_features, self.in_features, ordered=self._fresh)
-            self._fresh = False
+            if self._fresh:
+                self._fresh = False
         else:
             y = self._forward_many(x_flat)
         return y.reshape(*shape[:-1], self.out_features)

@@ -1,0 +1,63 @@
+"""PackedLinear's native call against the general path: same results, same refusals."""
+import pytest
+import torch
+
+from nativebit_b200 import PackedLinear, _lib, ops
+
+
+def test_native_call_leaves_everything_else_to_the_general_path(built_lib):
+    call = _lib.bind().linear
+    x, p, c = torch.zeros(2, 128), torch.zeros(48, dtype=torch.uint8), torch.zeros(1, 8).half()
+    assert call(x, p, c, None, 1, 128, 3, True, {}, {}) is None                  # not on a GPU
+    assert call(x.int(), p, c, None, 1, 128, 3, True, {}, {}) is None
+    assert call(torch.nn.Parameter(x), p, c, None, 1, 128, 3, True, {}, {}) is None
+    assert call(None, p, c, None, 1, 128, 3, True, {}, {}) is None
+    with pytest.raises(TypeError):
+        call(x, p, c)
+    with pytest.raises(TypeError):
+        call(x, p, c, None, "n", 128, 3, True, {}, {})
+
+
+def _general(lin, x):
+    """The call without its native form."""
+    flat = x.reshape(-1, lin.in_features).contiguous()
+    if flat.shape[0] <= 16:
+        y = ops.gemv(flat, lin.packed_indices, lin.codebook, lin.bits, 128, lin.out_features, lin.in_features, ordered=True)
+    else:
+        y = lin._forward_many(flat)
+    return y.reshape(*x.shape[:-1], lin.out_features)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bits", [2, 3, 4])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_native_call_equals_the_general_path(built_lib, bits, dtype):
+    n, k = 272, 640
+    g = torch.Generator(device="cuda").manual_seed(bits)
+    idx = torch.randint(0, 1 << bits, (n * k,), dtype=torch.uint8, device="cuda", generator=g)
+    lin = PackedLinear(ops.pack(idx, bits), torch.randn(n * k // 128, 1 << bits, device="cuda", generator=g).half(), n, k, bits=bits)
+    big = torch.randn(700, 2 * k, device="cuda", generator=g).to(dtype)
+    forms = [big[0, :k], big[:1, :k], big[:16, :k].contiguous(), big[:16, :k], big[:17, :k].contiguous(), big[:17, :k], big[:600, k:].contiguous(),
+             big[:12, :k].reshape(3, 4, k), big[:40, :k].reshape(2, 20, k), big[:24, :k].view(4, 6, k).transpose(0, 1), big[:0, :k]]
+    for turn in range(2):                                   # the first calls make the workspaces and the stream-layout copy
+        for x in forms:
+            if x.shape[0] == 0:
+                with pytest.raises(RuntimeError):           # no rows: refused as before
+                    lin(x)
+                continue
+            y, want = lin(x), _general(lin, x)
+            assert y.shape == want.shape and y.dtype == want.dtype and y.is_contiguous() and not y.requires_grad
+            assert torch.equal(y, want)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for x in (forms[1], forms[4]):
+            assert torch.equal(lin(x), _general(lin, x))
+        with torch.cuda.graph(graph := torch.cuda.CUDAGraph(), stream=side):
+            y = lin(forms[2])
+        graph.replay()
+    side.synchronize()
+    assert torch.equal(y, _general(lin, forms[2]))
+    for wrong in (big[:4], big[:4, :k].double(), big[:4, :k].int()):
+        with pytest.raises(RuntimeError):
+            lin(wrong)
