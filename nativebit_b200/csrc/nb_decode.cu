@@ -766,25 +766,45 @@ static int prefill_attention_tile(int B, int T, int H, int hd, int pos0, cudaStr
 // in front and the soft-cap + arg-max behind it (inference/generate_torch.py:155-160 and :300-310): logits[v] =
 // cap * tanh(dot(table[v], norm(x + delta) * w) / cap).  HBM-bound (164 MB per token at V = 32000, C = 2560): CTA b
 // owns the table rows [V*b/G, V*(b+1)/G); a warp takes every tenth of them through its own ring of 16-byte
-// asynchronous copies (up to four slots of one row: three rows are in flight while one is multiplied, 150 KB per SM
+// asynchronous copies (four slots of one row at C = 2560: three rows are in flight while one is multiplied, 150 KB per SM
 // on the way — plain loads were sunk to their uses by the compiler, four in flight per lane) and multiplies them
 // with the activations staged once in shared memory as fp32 (bf16 x fp32 products are exact in fp32).  The
 // norm's scale is one factor on the dot products.  Every CTA leaves its best (value, index) as a candidate;
 // lm_head_finish_kernel picks the token (largest capped logit, lowest index among equals) and advances the
-// position.  C = 256 * NC: a lane owns eight values of every 256.
+// position.  C = 256 * NC: a lane owns eight values of every 256, whose activations it keeps in registers (read from shared
+// memory for every row they took twice the shared-memory cycles of the row itself).  32000 rows, three tables in turn, head and
+// finish, with four slots and activations in shared memory -> now (us): C = 1024 22.4 -> 17.9, 2048 33.8 -> 27.1, 2560 38.4 -> 32.6
+// (5.0 TB/s); in the step of a small model 32.5 -> 17.
 constexpr int kHeadWarps = 10;
 constexpr int kHeadThreads = kHeadWarps * 32;
 constexpr int kHeadMaxCtas = 1024;
 constexpr int kHeadMaxNC = 12;                               // C <= 3072
 constexpr size_t kHeadSmemBudget = 216 * 1024;               // activations + the warps' rings
+constexpr int kHeadMaxSlots = 10;                            // rows of one warp's ring
 
 __device__ __forceinline__ void head_cp_async16(void* dst, const void* src) {   // 16 bytes global -> shared, past L1
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 
+// All but the newest `n` requests have landed.
+__device__ __forceinline__ void head_wait(int n) {
+  switch (n) {
+    case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+    case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+    case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+    case 4: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+    case 5: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
+    case 6: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
+    case 7: asm volatile("cp.async.wait_group 7;" ::: "memory"); break;
+    case 8: asm volatile("cp.async.wait_group 8;" ::: "memory"); break;
+    default: asm volatile("cp.async.wait_group 9;" ::: "memory"); break;
+  }
+}
+
+template <int NC>
 __global__ void __launch_bounds__(kHeadThreads, 1) lm_head_kernel(const float* __restrict__ x, const float* __restrict__ delta,
                                                                   const float* __restrict__ w, float eps,
-                                                                  const __nv_bfloat16* __restrict__ table, int V, int NC, int slots,
+                                                                  const __nv_bfloat16* __restrict__ table, int V, int slots,
                                                                   float cap, float* __restrict__ logits_out,
                                                                   float* __restrict__ cand_val, int* __restrict__ cand_idx) {
   extern __shared__ __align__(16) uint8_t head_smem[];
@@ -792,7 +812,7 @@ __global__ void __launch_bounds__(kHeadThreads, 1) lm_head_kernel(const float* _
   __shared__ int s_ci[kHeadWarps];
   __shared__ float s_scale;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int C = NC * 256, row_bytes = C * 2;
+  constexpr int C = NC * 256, row_bytes = C * 2;
   float* hs = reinterpret_cast<float*>(head_smem);                                   // C floats
   uint8_t* ring = head_smem + (size_t)C * 4 + (size_t)warp * slots * row_bytes;     // [slots][row_bytes]
   const int G = gridDim.x, b = blockIdx.x;
@@ -804,6 +824,7 @@ __global__ void __launch_bounds__(kHeadThreads, 1) lm_head_kernel(const float* _
     if (r < row1) {
       const uint8_t* src = reinterpret_cast<const uint8_t*>(table) + (size_t)r * row_bytes;
       uint8_t* dst = ring + (size_t)rq_slot * row_bytes;
+#pragma unroll
       for (int j = 0; j < NC; ++j) head_cp_async16(dst + (j * 32 + lane) * 16, src + (j * 32 + lane) * 16);
     }
     ++rq;
@@ -837,22 +858,25 @@ __global__ void __launch_bounds__(kHeadThreads, 1) lm_head_kernel(const float* _
   }
   __syncthreads();
   const float scale = s_scale;
+  float4 xr[2 * NC];                                         // this lane's eight values of every 256
+#pragma unroll
+  for (int j = 0; j < NC; ++j) {
+    xr[2 * j] = *reinterpret_cast<const float4*>(hs + (j * 32 + lane) * 8);
+    xr[2 * j + 1] = *reinterpret_cast<const float4*>(hs + (j * 32 + lane) * 8 + 4);
+  }
   float best = -FLT_MAX;
   int best_i = 0x7fffffff;
   int use_slot = 0;
 #pragma unroll 1
   for (int r = row0 + warp; r < row1; r += kHeadWarps) {
     request();                                               // (past the end: an empty group)
-    if (slots == 4) asm volatile("cp.async.wait_group 3;" ::: "memory");
-    else if (slots == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
-    else asm volatile("cp.async.wait_group 1;" ::: "memory");
+    head_wait(slots - 1);
     __syncwarp();
     const uint8_t* pr = ring + (size_t)use_slot * row_bytes;
     float acc = 0.f;
-#pragma unroll 2
+#pragma unroll
     for (int j = 0; j < NC; ++j) {
-      const float4 x0 = *reinterpret_cast<const float4*>(hs + (j * 32 + lane) * 8);
-      const float4 x1 = *reinterpret_cast<const float4*>(hs + (j * 32 + lane) * 8 + 4);
+      const float4 x0 = xr[2 * j], x1 = xr[2 * j + 1];
       const uint4 t = *reinterpret_cast<const uint4*>(pr + (j * 32 + lane) * 16);
       // a word holds elements 2e (low half) and 2e + 1
       acc += __uint_as_float(t.x << 16) * x0.x + __uint_as_float(t.x & 0xffff0000u) * x0.y;
@@ -1111,6 +1135,24 @@ extern "C" int nb_prefill_attention(const float* qkv, int B, int T, int H, int h
 
 extern "C" size_t nb_lm_head_scratch_bytes(void) { return (size_t)kHeadMaxCtas * 8; }
 
+template <int NC>
+static int launch_head(const float* x, const float* delta, const float* w, float eps, const __nv_bfloat16* table, int V, float cap,
+                       float* logits_out, float* cv, int* ci, int G, cudaStream_t st) {
+  // ring slots per warp: as many rows in flight as the shared memory holds, which for narrow rows are many (C = 1024: ten slots
+  // instead of four)
+  constexpr size_t act = (size_t)NC * 256 * 4, row = (size_t)kHeadWarps * NC * 256 * 2;
+  constexpr int slots = (kHeadSmemBudget - act) / row < kHeadMaxSlots ? (int)((kHeadSmemBudget - act) / row) : kHeadMaxSlots;
+  static_assert(slots >= 2, "a row in flight while one is multiplied");
+  static bool done[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!done[dev & 63]) {
+    if (cudaError_t e = cudaFuncSetAttribute(lm_head_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHeadSmemBudget)) return record_cuda_error(e);
+    done[dev & 63] = true;
+  }
+  return launch_pdl(lm_head_kernel<NC>, dim3(G), dim3(kHeadThreads), act + slots * row, st, x, delta, w, eps, table, V, slots, cap, logits_out, cv, ci);
+}
+
 extern "C" int nb_lm_head(const float* x, const float* delta, const float* norm_weight, float eps, const void* table_bf16, int V, int C,
                           float cap, float* logits_out, int64_t* token, int64_t* pos, void* scratch, void* stream) {
   if (!x || !table_bf16 || !logits_out || !token || !scratch || V < 1 || C < 1 || !(cap > 0.f)) return NB_ERR_ARG;
@@ -1122,21 +1164,23 @@ extern "C" int nb_lm_head(const float* x, const float* delta, const float* norm_
   float* cv = reinterpret_cast<float*>(scratch);
   int* ci = reinterpret_cast<int*>(cv + kHeadMaxCtas);
   cudaStream_t st = (cudaStream_t)stream;
-  // ring slots per warp: as many rows in flight as the shared memory holds (4 at C = 2560, 3 at C = 3072)
-  const size_t ring_row = (size_t)kHeadWarps * C * 2;
-  const int slots = (int)std::min<size_t>(4, (kHeadSmemBudget - (size_t)C * 4) / ring_row);
-  if (slots < 2) return NB_ERR_SHAPE;
-  const size_t smem = (size_t)C * 4 + (size_t)slots * ring_row;
-  static bool attr_done[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!attr_done[dev & 63]) {
-    if (cudaError_t e = cudaFuncSetAttribute(lm_head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHeadSmemBudget)) return record_cuda_error(e);
-    attr_done[dev & 63] = true;
+  int rc = NB_OK;
+  const auto launch = [&](auto nc) { rc = launch_head<decltype(nc)::value>(x, delta, norm_weight, eps, reinterpret_cast<const __nv_bfloat16*>(table_bf16), V, cap, logits_out, cv, ci, G, st); };
+  switch (C / 256) {
+    case 1: launch(std::integral_constant<int, 1>{}); break;
+    case 2: launch(std::integral_constant<int, 2>{}); break;
+    case 3: launch(std::integral_constant<int, 3>{}); break;
+    case 4: launch(std::integral_constant<int, 4>{}); break;
+    case 5: launch(std::integral_constant<int, 5>{}); break;
+    case 6: launch(std::integral_constant<int, 6>{}); break;
+    case 7: launch(std::integral_constant<int, 7>{}); break;
+    case 8: launch(std::integral_constant<int, 8>{}); break;
+    case 9: launch(std::integral_constant<int, 9>{}); break;
+    case 10: launch(std::integral_constant<int, 10>{}); break;
+    case 11: launch(std::integral_constant<int, 11>{}); break;
+    default: launch(std::integral_constant<int, 12>{}); break;
   }
-  if (int rc = launch_pdl(lm_head_kernel, dim3(G), dim3(kHeadThreads), smem, st, x, delta, norm_weight, eps,
-                          reinterpret_cast<const __nv_bfloat16*>(table_bf16), V, C / 256, slots, cap, logits_out, cv, ci))
-    return rc;
+  if (rc) return rc;
   return launch_pdl(lm_head_finish_kernel, dim3(1), dim3(256), 0, st, (const float*)cv, (const int*)ci, G,
                     reinterpret_cast<long long*>(token), reinterpret_cast<long long*>(pos));
 }
