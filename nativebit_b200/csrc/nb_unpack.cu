@@ -112,8 +112,9 @@ __global__ void pack_kernel(const uint8_t* __restrict__ idx, int64_t count, int 
 }
 
 // ---- dequant ------------------------------------------------------------------------------
-// Fast path (fp16 codebook, block_size % 8 == 0, aligned): a thread dequantises the consecutive weights of ONE 16-byte
-// store, so that a warp's stores are one contiguous run (a thread with 32 weights of its own left every store 64 or 128
+// Fast path (fp16 codebook, block_size % 8 == 0, aligned): a thread dequantises the eight consecutive weights of ONE store of 16
+// bytes, 32 for fp32 (four per thread there built every table twice: 6912 x 2560 at 3 bits 19.5 -> 14.5 us, 6.4 TB/s with 32 bytes
+// per thread), so that a warp's stores are one contiguous run (a thread with 32 weights of its own left every store 64 or 128
 // bytes from its neighbour's: 12.1 us for 6912 x 2560 to fp16 and 34.7 us to fp32, which take 6.7 and 12.2 us at the copy
 // rate).  The 3- or 2-bit fields are spread to the nibbles of one selector word; the block's table, as byte planes, answers
 // four lookups with two byte permutes.  A thread takes PER stores a block stride apart and requests all inputs first: four where
@@ -138,14 +139,14 @@ template <int BITS> __device__ __forceinline__ uint32_t load_selectors(const uin
   return (v & 0x07070707u) | ((v & 0x38383838u) << 1); // three per nibble
 }
 
-// Four lookups (eight for 16-bit types) as one 16-byte store.
-template <int BITS> __device__ __forceinline__ void store16(__half* dst, uint32_t sel, const uint32_t (&T)[BITS == 4 ? 8 : 4]) {
+// Eight lookups as one store of 16 bytes, 32 for fp32.
+template <int BITS> __device__ __forceinline__ void store8(__half* dst, uint32_t sel, const uint32_t (&T)[BITS == 4 ? 8 : 4]) {
   uint32_t h[4];
   lookup4<BITS>(sel, T, h[0], h[1]);
   lookup4<BITS>(sel >> 16, T, h[2], h[3]);
   *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
 }
-template <int BITS> __device__ __forceinline__ void store16(__nv_bfloat16* dst, uint32_t sel, const uint32_t (&T)[BITS == 4 ? 8 : 4]) {
+template <int BITS> __device__ __forceinline__ void store8(__nv_bfloat16* dst, uint32_t sel, const uint32_t (&T)[BITS == 4 ? 8 : 4]) {
   uint32_t h[4];
   lookup4<BITS>(sel, T, h[0], h[1]);
   lookup4<BITS>(sel >> 16, T, h[2], h[3]);
@@ -157,11 +158,19 @@ template <int BITS> __device__ __forceinline__ void store16(__nv_bfloat16* dst, 
   }
   *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
 }
-template <int BITS> __device__ __forceinline__ void store16(float* dst, uint32_t sel, const uint32_t (&T)[BITS == 4 ? 8 : 4]) {
-  uint32_t h[2];
+template <int BITS> __device__ __forceinline__ void store8(float* dst, uint32_t sel, const uint32_t (&T)[BITS == 4 ? 8 : 4]) {
+  uint32_t h[4];
   lookup4<BITS>(sel, T, h[0], h[1]);
+  lookup4<BITS>(sel >> 16, T, h[2], h[3]);
   const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&h[0])), b = __half22float2(*reinterpret_cast<const __half2*>(&h[1]));
-  *reinterpret_cast<float4*>(dst) = make_float4(a.x, a.y, b.x, b.y);
+  const float2 c = __half22float2(*reinterpret_cast<const __half2*>(&h[2])), d = __half22float2(*reinterpret_cast<const __half2*>(&h[3]));
+  if ((uintptr_t)dst % 32 == 0) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(dst), "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y), "f"(d.x), "f"(d.y) : "memory");
+  } else {
+    reinterpret_cast<float4*>(dst)[0] = make_float4(a.x, a.y, b.x, b.y);
+    reinterpret_cast<float4*>(dst)[1] = make_float4(c.x, c.y, d.x, d.y);
+  }
 }
 
 template <int BITS, int PER, typename OutT>
@@ -169,19 +178,17 @@ __global__ void __launch_bounds__(kDqThreads) dequant16b_kernel(const uint32_t* 
                                                                int64_t n_stores, int64_t n_bytes, int64_t total, int block_size, int shift,
                                                                OutT* __restrict__ out) {
   constexpr int kT = BITS == 4 ? 8 : 4;
-  constexpr bool kHalves = sizeof(OutT) == 4;          // a store takes half of a chunk of eight
   const int64_t i0 = (int64_t)blockIdx.x * (kDqThreads * PER) + threadIdx.x;
   uint32_t sel[PER], e[PER][kT];
 #pragma unroll
   for (int u = 0; u < PER; ++u) {
-    const int64_t i = i0 + u * kDqThreads, c = kHalves ? i >> 1 : i;
+    const int64_t i = i0 + u * kDqThreads;
     sel[u] = 0;
 #pragma unroll
     for (int j = 0; j < kT; ++j) e[u][j] = 0;
     if (i < n_stores) {
-      sel[u] = load_selectors<BITS>(packed, c);
-      if (kHalves && (i & 1)) sel[u] >>= 16;
-      const int64_t block = block_of(c, block_size >> 3, shift);
+      sel[u] = load_selectors<BITS>(packed, i);
+      const int64_t block = block_of(i, block_size >> 3, shift);
       const uint8_t* row = reinterpret_cast<const uint8_t*>(codebook) + block * (2 << BITS);
       if (BITS == 2) {
         const uint2 v = *reinterpret_cast<const uint2*>(row);
@@ -210,10 +217,10 @@ __global__ void __launch_bounds__(kDqThreads) dequant16b_kernel(const uint32_t* 
         T[j + 2] = prmt(e[u][j], e[u][j + 1], 0x7531); T[j + 3] = prmt(e[u][j + 2], e[u][j + 3], 0x7531);
       }
     }
-    store16<BITS>(out + i * (16 / sizeof(OutT)), sel[u], T);
+    store8<BITS>(out + i * 8, sel[u], T);
   }
   // fewer than 32 weights behind the last whole packed word, one for each of the threads without a store
-  const int64_t one = n_stores * (16 / (int)sizeof(OutT)) + (i - n_stores);
+  const int64_t one = n_stores * 8 + (i - n_stores);
   if (i >= n_stores && i < i0 + PER * kDqThreads && one < total) {
     const uint32_t at = stream_index(reinterpret_cast<const uint8_t*>(packed), n_bytes, one, BITS);
     out[one] = (OutT)(float)codebook[block_of(one, block_size, -1) * (1 << BITS) + at];
@@ -254,6 +261,9 @@ __global__ void quantize_kernel(const float* __restrict__ w, int64_t total, int6
 // kernel at 92 us for 6912 x 2560 weights; what bounds this one is the argmin itself, three operations of the half-rate pipe
 // per entry and weight (floor 20 us).  (Four such runs per thread take 1 % longer there and 4.4 instead of 2.6 us for 100 x 100.)
 constexpr int kQThreads = 256;
+// from this many weights on the search is faster (us, every entry tried | search: 3 bits, 1 M weights 3.3 | 3.5, 2 M 5.1 | 4.5,
+// 17.7 M 32.3 | 20.3; 4 bits, 262 k 2.5 | 2.3, 524 k 3.3 | 2.7, 17.7 M 55.5 | 26.9; 2 bits 17.7 M 20.5 | 19.7, below slower)
+constexpr int64_t kQSearch3 = 1 << 21, kQSearch4 = 1 << 19;
 
 template <typename CbT, int NE> __device__ __forceinline__ void load_entries(const CbT* cb, float (&c)[NE]);
 template <> __device__ __forceinline__ void load_entries<float, 4>(const float* cb, float (&c)[4]) {
@@ -322,6 +332,111 @@ __global__ void __launch_bounds__(kQThreads) quantize4_kernel(const float* __res
   }
 }
 
+// The same with the indices packed, eight weights per thread, for large matrices.  Trying every entry is 48 instructions per weight
+// at 3 bits, and issuing them bounds the kernel above.  The exporter's codebooks are in ascending order, and there a binary
+// search in shared memory, three instructions a step, finds the entries on either side of a weight, one of which is the nearest.
+//   The answer has to be that of the trial of all entries in fp32, first minimum on ties: distances are rounded, so an entry
+// further away may round to the same distance as its neighbour and come first.  With entries in order, more than 2^-20 of their
+// range apart, and a weight below the last entry by any distance or above it by less than three ranges, the distances to tell
+// apart are at most 4 ranges, an ulp of which is at most 2^-21 ranges: entries on one side of the weight are then at different
+// distances.  A tie between the two sides goes to the lower one, as there.  Every other block or weight (codebooks
+// out of order, with equal, infinite or NaN entries; weights far above, infinite or NaN) is tried entry by entry.
+__device__ __forceinline__ float lds_f32(uint32_t at) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+  return v;
+}
+
+constexpr int kQRows = kQThreads * 8 / 32 + 1;               // codebooks that a CTA's 2048 weights may meet (blocks of 32 and more)
+
+template <int BITS>
+__global__ void __launch_bounds__(kQThreads) quantize8_pack_kernel(const float* __restrict__ w, int64_t total, int64_t padded,
+                                                                   const float* __restrict__ codebook, int block8, int shift,
+                                                                   uint32_t* __restrict__ out) {
+  constexpr int NE = 1 << BITS;
+  __shared__ __align__(16) float rows[kQRows][NE + 4];      // the entries, the last one once more
+  __shared__ float limits[kQRows];                           // weights below may be searched for
+  const int64_t i0 = (int64_t)blockIdx.x * kQThreads, i = i0 + threadIdx.x, units = padded >> 3;      // in units of eight weights
+  const bool in = i < units;
+  float v[8];
+  if (8 * i + 8 <= total) {
+    const float4 a = reinterpret_cast<const float4*>(w)[2 * i], b = reinterpret_cast<const float4*>(w)[2 * i + 1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = 8 * i + j < total ? w[8 * i + j] : 0.f;
+  }
+  const int64_t row0 = block_of(i0, block8, shift), last = block_of(min(i0 + kQThreads, units) - 1, block8, shift);
+  if ((int)threadIdx.x <= (int)(last - row0)) {
+    float c[NE];
+    load_entries<float, NE>(codebook + (row0 + threadIdx.x) * NE, c);
+    float gap = c[1] - c[0];
+    bool plain = c[0] < c[1];
+#pragma unroll
+    for (int e = 2; e < NE; ++e) {
+      gap = fminf(gap, c[e] - c[e - 1]);
+      plain = plain && c[e - 1] < c[e];                      // (false for NaN, which fminf drops)
+    }
+    const float range = c[NE - 1] - c[0];
+    limits[threadIdx.x] = plain && gap > range * 0x1p-20f && range < 8e37f ? c[NE - 1] + 3.f * range : -INFINITY;
+#pragma unroll
+    for (int e = 0; e < NE; e += 4) *reinterpret_cast<float4*>(&rows[threadIdx.x][e]) = make_float4(c[e], c[e + 1], c[e + 2], c[e + 3]);
+    rows[threadIdx.x][NE] = c[NE - 1];
+  }
+  __syncthreads();
+  uint32_t f = 0;
+  if (in) {
+    const int r = (int)(block_of(i, block8, shift) - row0);
+    const float *row = rows[r], limit = limits[r];
+    bool plain = true;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) plain = plain && v[j] < limit;
+    if (plain) {
+      // byte offsets of the entries found, summed at their places and freed of the row's own offset at the end
+      const uint32_t base = smem_u32(row);
+      constexpr int kGroup = BITS == 4 ? 4 : 8;              // weights whose sums fit 32 bits
+#pragma unroll
+      for (int h = 0; h < 8 / kGroup; ++h) {
+        uint32_t sum = 0, ones = 0;
+#pragma unroll
+        for (int q = 0; q < kGroup; ++q) {
+          const float x = v[h * kGroup + q];
+          uint32_t p = base;
+#pragma unroll
+          for (int half = NE / 2; half > 0; half >>= 1)
+            if (x >= lds_f32(p + 4 * half)) p += 4 * half;
+          if (fabsf(x - lds_f32(p + 4)) < fabsf(x - lds_f32(p))) p += 4;
+          sum += p << (BITS * q);
+          ones += 1u << (BITS * q);
+        }
+        f |= ((sum - base * ones) >> 2) << (16 * h);
+      }
+    } else {
+#pragma unroll 1
+      for (int j = 0; j < 8; ++j) {
+        float x = v[0];
+#pragma unroll
+        for (int q = 1; q < 8; ++q) x = q == j ? v[q] : x;
+        float best = fabsf(x - row[0]);
+        uint32_t arg = 0;
+#pragma unroll
+        for (int e = 1; e < NE; ++e) {
+          const float d = fabsf(x - row[e]);
+          if (d < best) { best = d; arg = e; }
+        }
+        f |= arg << (BITS * j);
+      }
+    }
+  }
+  if (BITS == 4) {
+    if (in) out[i] = f;
+  } else {                                                               // four lanes hold 96 bits
+    const uint32_t next = __shfl_down_sync(0xffffffffu, f, 1);
+    const int q = threadIdx.x & 3;
+    if (in && q < 3) out[(i >> 2) * 3 + q] = (f >> (8 * q)) | (next << (24 - 8 * q));
+  }
+}
+
 // Whether the four-wide kernels take these arguments: fp32 entries (the exporter's), 2 to 4 bits, four weights per load
 // and four indices per store (a packed word holds 32 indices of whole blocks).
 static bool quantize4_fits(const float* w, const void* codebook, int cb_dtype, int n_entries, int block_size, const void* out, bool pack) {
@@ -332,6 +447,14 @@ static bool quantize4_fits(const float* w, const void* codebook, int cb_dtype, i
 template <bool PACK>
 static int launch_quantize4(const float* w, int64_t total, int64_t padded, const float* codebook, int n_entries, int block_size, void* out,
                             cudaStream_t st) {
+  if (PACK && ((n_entries == 8 && padded >= kQSearch3) || (n_entries == 16 && padded >= kQSearch4))) {
+    const int block8 = block_size / 8, shift8 = shift_of(block8);
+    const unsigned g = (unsigned)((padded / 8 + kQThreads - 1) / kQThreads);
+    uint32_t* o8 = (uint32_t*)out;
+    if (n_entries == 8) quantize8_pack_kernel<3><<<g, kQThreads, 0, st>>>(w, total, padded, codebook, block8, shift8, o8);
+    else quantize8_pack_kernel<4><<<g, kQThreads, 0, st>>>(w, total, padded, codebook, block8, shift8, o8);
+    return check_launch();
+  }
   const int block4 = block_size / 4, shift = shift_of(block4);
   const unsigned grid = (unsigned)((padded / 4 + kQThreads - 1) / kQThreads);
   uint32_t* o = (uint32_t*)out;
@@ -348,7 +471,7 @@ static int dequant_dispatch(const uint8_t* packed, const void* codebook, int cb_
   const int64_t n_bytes = packed_bytes(n_blocks * block_size, bits);
   const bool aligned = ((uintptr_t)packed % 4 == 0) && ((uintptr_t)out % 16 == 0) && ((uintptr_t)codebook % 16 == 0);
   if (cb_dtype == NB_F16 && block_size % 8 == 0 && aligned) {
-    const int64_t stores = total / 32 * 32 / (int64_t)(16 / sizeof(OutT));      // whole packed words
+    const int64_t stores = total / 32 * 4;             // whole packed words
     if (stores > 0) {
       const int shift = shift_of(block_size / 8);
       const bool several = stores >= (int64_t)kDqRuns * kDqThreads * 4 * sm_count();

@@ -395,3 +395,36 @@ def test_quantize_pack_dequant_edges_of_the_wide_kernels(dev, bits, total, block
     want = torch.gather(half, 1, torch.from_numpy(ref.astype(np.int64)).to(dev).view(blocks, block)).view(-1)[:total].view(1, total)
     for dtype in (torch.float16, torch.bfloat16, torch.float32):
         assert torch.equal(ops.dequant(packed, half, bits, block, (1, total), dtype), want.to(dtype))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bits", [2, 3, 4])
+def test_quantize_pack_finds_the_first_nearest_entry(dev, bits):
+    """The search over ordered codebooks against the trial of every entry in fp32, where the two could part: ties, entries out of
+    order, equal, close together, infinite or NaN, weights on, between and far beyond the entries."""
+    e, block, rows = 1 << bits, 128, 4096                      # enough weights for the kernel that searches
+    g = torch.Generator().manual_seed(bits)
+    cb = (0.02 * torch.randn(rows, e, generator=g)).sort(dim=1).values
+    w = 0.02 * torch.randn(rows, block, generator=g)
+    cb[0] = torch.arange(e) - e // 2                           # weights half way between entries: the lower index
+    w[0] = (torch.arange(block) % (4 * e)) / 4 - e / 2 - 1
+    cb[1] = cb[1].flip(0)
+    cb[2, 1] = cb[2, 0]
+    cb[3] = 1.0 + torch.arange(e) * 2.0 ** -22                 # closer than the distances resolve
+    w[3] = 100 * torch.randn(block, generator=g)
+    cb[4, e - 1], cb[5, 0], cb[6, e // 2] = float("inf"), float("-inf"), float("nan")
+    w[7, ::7], w[7, 1::7], w[7, 2::7] = float("inf"), float("-inf"), float("nan")
+    w[8] = 1e6 * torch.randn(block, generator=g)               # the distances of several entries round to one value
+    cb[9] = torch.arange(e) * 1e-40
+    w[9] = 1e-40 * e * torch.rand(block, generator=g)
+    w[10] = cb[10][torch.arange(block) % e]
+    cb[11] = torch.linspace(-3e38, 3e38, e)
+    best, want = (w - cb[:, :1]).abs(), torch.zeros(rows, block, dtype=torch.uint8)
+    for i in range(1, e):
+        d = (w - cb[:, i:i + 1]).abs()
+        want[d < best] = i
+        best = torch.where(d < best, d, best)
+    from nativebit_b200 import ops
+    got = ops.unpack(ops.quantize_pack(w.reshape(-1).to(dev), cb.to(dev), block, bits), bits, rows * block).cpu().view(rows, block)
+    wrong = (got != want).nonzero()
+    assert len(wrong) == 0, (wrong[:5], got[got != want][:5], want[got != want][:5])
