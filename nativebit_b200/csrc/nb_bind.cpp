@@ -55,7 +55,22 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
   at::DimVector shape(x.sizes());
   shape.back() = n;
   int rc = NB_ERR_ARG;
-  if (m <= kGemvRows) {
+  if (m >= 2 && m <= kGemvRows && THPVariable_CheckExact(a[3])) {
+    const at::Tensor &w = THPVariable_Unpack(a[3]), *ws = workspace(a[9], device.index(), stream);
+    if (!ws || w.device() != device) Py_RETURN_NONE;
+    at::Tensor y = at::empty(shape, x.options().requires_grad(false).memory_format(c10::MemoryFormat::Contiguous));
+    nb_chain_args args = {};
+    args.w = static_cast<const uint8_t*>(w.const_data_ptr());
+    args.x = x.const_data_ptr();
+    args.y = y.mutable_data_ptr();
+    args.status = static_cast<int*>(ws->mutable_data_ptr());         // the workspace's head
+    args.M = (int)m; args.N = (int)n; args.K = (int)k; args.bits = bits;
+    args.x_dtype = args.y_dtype = xt;
+    Py_BEGIN_ALLOW_THREADS
+    rc = nb_chain_linear(&args, stream);
+    Py_END_ALLOW_THREADS
+    if (rc == NB_OK) return THPVariable_Wrap(std::move(y));
+  } else if (m == 1) {
     const at::Tensor* ws = workspace(a[8], device.index(), stream);
     if (!ws) Py_RETURN_NONE;
     at::Tensor y = at::empty(shape, x.options().requires_grad(false).memory_format(c10::MemoryFormat::Contiguous));

@@ -27,6 +27,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "nb_chain.cuh"
 #include "nb_common.cuh"
@@ -56,7 +57,7 @@ struct ChainParams {
   const uint8_t* w;           // stream layout
   const uint8_t* xt;          // activations as terms
   const float* ss;            // (M, ss_n) partial sums of squares of the rows in front of the norm (null: no norm)
-  float* y;                   // NB_CHAIN_STORE: (M, N)
+  void* y;                    // NB_CHAIN_STORE: (M, N) of type y_dtype
   uint8_t* yt;                // the other two: terms of the next linear's activations (null: none)
   float* res;                 // NB_CHAIN_RESIDUAL: (M, N), updated in place
   const float* w_next;        // ... the next norm's weight
@@ -64,6 +65,8 @@ struct ChainParams {
   const uint8_t* ahead;       // weights of the launch behind (null: none), `ahead_step` bytes per CTA
   int* status;
   unsigned ahead_bytes, ahead_step;
+  const void* x;              // plain activations (M, K) of type x_dtype instead of the terms (null: none)
+  int x_dtype, y_dtype;
   int N, bpr, M, mode, ss_n;
   float eps;
   int m_part, parts;          // activation rows per part of the launch, parts
@@ -111,9 +114,9 @@ __device__ __forceinline__ void st_cluster_f32(uint32_t local, uint32_t rank, fl
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
 }
 
-// Shared memory: the CTA's units, tile after tile | staged columns (2 m_part of kc_max * 256 bytes) | partial
+// Shared memory: the CTA's units, tile after tile | staged columns (XT m_part of kc_max * 256 bytes) | partial
 // results [own tile][CTA][J][row][16] of the tiles this CTA finishes.
-template <int BITS, int CG, bool kCluster>
+template <int BITS, int CG, int XT, bool kCluster>
 __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p) {
   constexpr int kUnit = StreamUnit<BITS>::kBytes;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -142,7 +145,7 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
   const int U = T * kc;                                     // units of this CTA, tile after tile
   const int ua = U * warp / kCW, ub = U * (warp + 1) / kCW; // this warp's run
   uint8_t* x_s = smem + (size_t)p.units * kUnit;
-  float* parts = reinterpret_cast<float*>(x_s + (size_t)2 * p.m_part * kc_max * 256);
+  float* parts = reinterpret_cast<float*>(x_s + (size_t)XT * p.m_part * kc_max * 256);
   const int own = (T + S - 1 - rank) >> lg;                 // tiles rank, rank + S, .. of the cluster's are finished here
   const int slot = 16 * m;
   const int i_first = div_rcp(ua, kc, rcp_kc), kk_first = ua - i_first * kc;
@@ -155,8 +158,47 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
   asm volatile("griddepcontrol.launch_dependents;");
 
   const uint8_t* xt = p.xt + ((size_t)(2 * row0) * p.bpr + k0) * 256;
-  const bool bulk = 2 * m * kc > kChainBulk;
-  if (bulk) {
+  const bool bulk = !p.x && 2 * m * kc > kChainBulk;
+  if (XT == 1 || p.x) {                                     // converted here; four pieces of eight values per thread on the way
+    const int chunks = kc * 16, total = m * chunks;         // of a row, of all
+    constexpr int kAhead = 4;
+    for (int i0 = tid; i0 < total; i0 += kAhead * kCThreads) {
+      float v[kAhead][8];
+      int col[kAhead], n[kAhead];
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        const int i = i0 + q * kCThreads, r = i / chunks;
+        col[q] = r;
+        n[q] = (i - r * chunks) * 8;
+        if (i < total) load_x8(p.x, p.x_dtype, ((size_t)(row0 + r) * p.bpr + k0) * kBlock + n[q], v[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        if (i0 + q * kCThreads < total) {
+          uint32_t hi[4];
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) hi[2 * h + e] = f32x2_to_f16x2_sat(v[q][4 * h + e], v[q][4 * h + e + 2]);     // in the order 0, 2, 1, 3
+          const int seg = n[q] >> 5 & 3, at = (n[q] >> 7) * 256 + seg * 64, c = XT * col[q];
+          *reinterpret_cast<uint4*>(x_s + (size_t)c * kc_max * 256 + at + (((n[q] >> 3 & 3) ^ seg ^ (c & 1)) << 4)) =
+              make_uint4(hi[0], hi[1], hi[2], hi[3]);
+          if (XT == 2) {
+            uint32_t lo[4];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi[2 * h + e]));
+                lo[2 * h + e] = f32x2_to_f16x2_sat(v[q][4 * h + e] - f.x, v[q][4 * h + e + 2] - f.y);
+              }
+            *reinterpret_cast<uint4*>(x_s + (size_t)(c + 1) * kc_max * 256 + at + (((n[q] >> 3 & 3) ^ seg ^ 1) << 4)) =
+                make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          }
+        }
+      }
+    }
+  } else if (bulk) {
     const uint32_t bytes = (uint32_t)kc * 256u;
     if (warp == 0) {
       if (lane == 0) mbar_arrive_expect_tx(&s_xbar, 2u * m * bytes);
@@ -204,8 +246,8 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
   // (m_part takes at least one row of the last group of columns; its lanes without a column keep zeros)
   const uint8_t* xc[CG];
 #pragma unroll
-  for (int j = 0; j < CG; ++j) xc[j] = x_s + (size_t)min(8 * j + g, 2 * m - 1) * kc_max * 256 + t * 64;
-  const uint32_t act = 8 * (CG - 1) + g < 2 * m;
+  for (int j = 0; j < CG; ++j) xc[j] = x_s + (size_t)min(8 * j + g, XT * m - 1) * kc_max * 256 + t * 64;
+  const uint32_t act = 8 * (CG - 1) + g < XT * m;
   uint4 x_last[1] = {make_uint4(0u, 0u, 0u, 0u)};
   constexpr int kAcc = CG == 1 ? 2 : CG;
   bool cluster_up = !kCluster;
@@ -231,27 +273,33 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
       for (int j = 0; j < CG; ++j) xp[j] += 256;
     }
     if (!cluster_up) { cluster_wait(); cluster_up = true; }
-    // lane (g, t): rows g and g + 8 of the tile, both terms of activation row 4j + t.  The warp that ends the tile leaves zeros in
-    // the places behind its own
+    // lane (g, t): rows g and g + 8 of the tile, columns 8j + 2t and 8j + 2t + 1: both terms of activation row 4j + t, or two rows.
+    // The warp that ends the tile leaves zeros in the places behind its own
     const uint32_t dst = smem_u32(parts + (size_t)(((i >> lg) * S + rank) * p.J) * slot);
     const int last_j = tile_end == (i + 1) * kc ? p.J - 1 : slot_j;
+    if (CG == 1)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) c[0][e] += c[kAcc - 1][e];
 #pragma unroll
     for (int j = 0; j < CG; ++j) {
-      const int mm = 4 * j + t;
-      if (mm < m) {
-        float va = CG == 1 ? (c[0][0] + c[kAcc - 1][0]) + (c[0][1] + c[kAcc - 1][1]) : c[j][0] + c[j][1];
-        float vb = CG == 1 ? (c[0][2] + c[kAcc - 1][2]) + (c[0][3] + c[kAcc - 1][3]) : c[j][2] + c[j][3];
+#pragma unroll
+      for (int o = 0; o < (XT == 2 ? 1 : 2); ++o) {
+        const int mm = XT == 2 ? 4 * j + t : 8 * j + 2 * t + o;
+        if (mm < m) {
+          float va = XT == 2 ? c[j][0] + c[j][1] : c[j][o];
+          float vb = XT == 2 ? c[j][2] + c[j][3] : c[j][2 + o];
 #pragma unroll 1
-        for (int q = slot_j; q <= last_j; ++q) {
-          const uint32_t at = dst + (uint32_t)(q * slot + mm * 16 + g) * 4u;
-          if (kCluster) {
-            st_cluster_f32(at, (uint32_t)(i & (S - 1)), va);
-            st_cluster_f32(at + 32u, (uint32_t)(i & (S - 1)), vb);
-          } else {
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(va) : "memory");
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + 32u), "f"(vb) : "memory");
+          for (int q = slot_j; q <= last_j; ++q) {
+            const uint32_t at = dst + (uint32_t)(q * slot + mm * 16 + g) * 4u;
+            if (kCluster) {
+              st_cluster_f32(at, (uint32_t)(i & (S - 1)), va);
+              st_cluster_f32(at + 32u, (uint32_t)(i & (S - 1)), vb);
+            } else {
+              asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(va) : "memory");
+              asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + 32u), "f"(vb) : "memory");
+            }
+            va = vb = 0.f;
           }
-          va = vb = 0.f;
         }
       }
     }
@@ -293,7 +341,7 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
     const float scale = p.ss ? s_scale[mm] : 1.f;
     if (p.mode == NB_CHAIN_STORE) {
       const int n = tile * 16 + row;
-      if (n < p.N) p.y[(size_t)b * p.N + n] = v * scale;
+      if (n < p.N) store_y(p.y, p.y_dtype, (size_t)b * p.N + n, v * scale);
     } else if (p.mode == NB_CHAIN_SWIGLU) {                 // rows 0 .. 7 of a tile are gate channels, 8 .. 15 the matching up channels
       v *= scale;
       v2 *= scale;
@@ -339,20 +387,21 @@ __global__ void __launch_bounds__(256) chain_embed_kernel(const __nv_bfloat16* _
 constexpr size_t kChainSmemMax = 227 * 1024 - 2048;
 
 struct ChainPlan {
-  int S, clusters, parts, m_part, launches, per_launch, units, J, cg;      // per_launch: row tiles
+  int S, clusters, parts, m_part, launches, per_launch, units, J, cg, terms;      // per_launch: row tiles
   size_t smem;
   double cost;
 };
 
 // Split over clusters of S CTAs; false if even one row tile does not fit.  As many launches as it takes for a CTA's units, its
 // share of the activations and the partial results to fit.
-static bool chain_plan(int N, int bpr, int M, int bits, int S, int max_clusters, ChainPlan& pl) {
+static bool chain_plan(int N, int bpr, int M, int terms, bool plain, int bits, int S, int max_clusters, ChainPlan& pl) {
   if (S > bpr) return false;
   const int n_tiles = (N + 15) / 16, unit = bits == 4 ? StreamUnit<4>::kBytes : StreamUnit<3>::kBytes;
   pl.S = S;
   pl.parts = (M + 15) / 16;
   pl.m_part = (M + pl.parts - 1) / pl.parts;
-  pl.cg = pl.m_part <= 4 ? 1 : pl.m_part <= 8 ? 2 : 4;
+  pl.terms = terms;
+  pl.cg = terms * pl.m_part <= 8 ? 1 : terms * pl.m_part <= 16 ? 2 : 4;
   const int room = std::max(1, max_clusters / pl.parts), kc_max = (bpr + S - 1) / S, kc_min = bpr / S;
   for (pl.launches = 1; pl.launches <= n_tiles; ++pl.launches) {
     pl.per_launch = (n_tiles + pl.launches - 1) / pl.launches;
@@ -363,10 +412,11 @@ static bool chain_plan(int N, int bpr, int M, int bits, int S, int max_clusters,
     // a tile of kc units meets at most kc warps, and two more than it has whole runs
     const int run = std::max(1, std::max(1, last / pl.clusters) * kc_min / kCW);
     pl.J = std::min(kc_max, kc_max / run + 2);
-    pl.smem = (size_t)pl.units * unit + (size_t)2 * pl.m_part * kc_max * 256 + (size_t)((T + S - 1) / S) * S * pl.J * 64 * pl.m_part;
+    pl.smem = (size_t)pl.units * unit + (size_t)terms * pl.m_part * kc_max * 256 + (size_t)((T + S - 1) / S) * S * pl.J * 64 * pl.m_part;
     if (T <= kChainTiles && pl.smem <= kChainSmemMax) {
-      // clocks: units at the rate of their lookups and MMAs, staged columns, launch and drain, a cluster's barriers
-      pl.cost = pl.launches * (pl.units * (60.0 + 9.0 * (pl.cg - 1)) + 2.0 * pl.m_part * kc_max * 256 / 64.0 + 4000.0 + (S > 1 ? 2500.0 : 0.0));
+      // clocks: units at the rate of their lookups and MMAs, staged columns (copied, or converted), launch and drain, a cluster's
+      // barriers; within 15 % of the best of the four splits over eight shapes and 1 to 16 rows
+      pl.cost = pl.launches * (pl.units * (60.0 + 9.0 * (pl.cg - 1)) + (double)terms * pl.m_part * kc_max * (plain ? 16.0 : 4.0) + 4000.0 + (S > 1 ? 2500.0 : 0.0));
       return true;
     }
     if (T == 1) return false;
@@ -374,13 +424,13 @@ static bool chain_plan(int N, int bpr, int M, int bits, int S, int max_clusters,
   return false;
 }
 
-template <int BITS, int CG, bool kCluster>
-static int chain_launch_as(const ChainPlan& pl, const ChainParams& p, cudaStream_t st) {
+template <int BITS, int CG, int XT, bool kCluster>
+static int chain_launch_as(const ChainPlan& pl, const ChainParams& p, bool ordered, cudaStream_t st) {
   static bool done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!done[dev & 63]) {
-    if (cudaError_t e = cudaFuncSetAttribute(chain_kernel<BITS, CG, kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmemMax))
+    if (cudaError_t e = cudaFuncSetAttribute(chain_kernel<BITS, CG, XT, kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmemMax))
       return record_cuda_error(e);
     done[dev & 63] = true;
   }
@@ -390,19 +440,30 @@ static int chain_launch_as(const ChainPlan& pl, const ChainParams& p, cudaStream
   cfg.dynamicSmemBytes = pl.smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = pl.S;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = kCluster ? 2 : 1;
-  return record_cuda_error(cudaLaunchKernelEx(&cfg, chain_kernel<BITS, CG, kCluster>, p));
+  if (!ordered) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (kCluster) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = pl.S;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
+  return record_cuda_error(cudaLaunchKernelEx(&cfg, chain_kernel<BITS, CG, XT, kCluster>, p));
 }
-template <int BITS, int CG>
-static int chain_launch(const ChainPlan& pl, const ChainParams& p, cudaStream_t st) {
-  return pl.S > 1 ? chain_launch_as<BITS, CG, true>(pl, p, st) : chain_launch_as<BITS, CG, false>(pl, p, st);
+template <int BITS>
+static int chain_launch(const ChainPlan& pl, const ChainParams& p, bool ordered, cudaStream_t st) {
+  const auto run = [&](auto cg, auto xt) {
+    constexpr int CG = decltype(cg)::value, XT = decltype(xt)::value;
+    return pl.S > 1 ? chain_launch_as<BITS, CG, XT, true>(pl, p, ordered, st) : chain_launch_as<BITS, CG, XT, false>(pl, p, ordered, st);
+  };
+  using std::integral_constant;
+  if (pl.terms == 1) return pl.cg == 1 ? run(integral_constant<int, 1>{}, integral_constant<int, 1>{}) : run(integral_constant<int, 2>{}, integral_constant<int, 1>{});
+  if (pl.cg == 1) return run(integral_constant<int, 1>{}, integral_constant<int, 2>{});
+  if (pl.cg == 2) return run(integral_constant<int, 2>{}, integral_constant<int, 2>{});
+  return run(integral_constant<int, 4>{}, integral_constant<int, 2>{});
 }
 
 // Clusters of S CTAs with a whole SM each that the device runs at once.
@@ -425,8 +486,8 @@ static int max_clusters(int S) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int got = 0;
-    if (cudaFuncSetAttribute(chain_kernel<3, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmemMax) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&got, chain_kernel<3, 1, true>, &cfg) != cudaSuccess || got < 1) {
+    if (cudaFuncSetAttribute(chain_kernel<3, 1, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmemMax) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&got, chain_kernel<3, 1, 2, true>, &cfg) != cudaSuccess || got < 1) {
       cudaGetLastError();
       got = 1;
     }
@@ -443,18 +504,20 @@ extern "C" size_t nb_chain_terms_bytes(int M, int K) { return M < 1 || K < kBloc
 
 extern "C" int nb_chain_linear(const nb_chain_args* a, void* stream) {
   constexpr long long kMost = 1ll << 26;                    // products of sizes below stay in 32 bits
-  if (!a || !a->w || !a->x_terms || !a->status || a->M < 1 || a->N < 1) return NB_ERR_ARG;
+  if (!a || !a->w || (a->x ? a->sq || a->mode != NB_CHAIN_STORE : !a->x_terms) || !a->status || a->M < 1 || a->N < 1) return NB_ERR_ARG;
   if (a->mode < NB_CHAIN_STORE || a->mode > NB_CHAIN_RESIDUAL) return NB_ERR_ARG;
   if (a->mode == NB_CHAIN_STORE ? !a->y : a->mode == NB_CHAIN_SWIGLU ? !a->y_terms : !a->residual) return NB_ERR_ARG;
   if (a->mode == NB_CHAIN_RESIDUAL && a->y_terms && (!a->next_weight || !a->sq_out)) return NB_ERR_ARG;
   if (a->sq && a->sq_n < 1) return NB_ERR_ARG;
+  if (a->x && (a->x_dtype < NB_F32 || a->x_dtype > NB_BF16)) return NB_ERR_ARG;
+  if (a->y_dtype < NB_F32 || a->y_dtype > NB_BF16) return NB_ERR_ARG;
   if (a->bits != 2 && a->bits != 3 && a->bits != 4) return NB_ERR_SHAPE;
   if (a->K < kBlock || a->K % kBlock) return NB_ERR_SHAPE;
   if (a->mode == NB_CHAIN_SWIGLU && a->N % (2 * kBlock)) return NB_ERR_SHAPE;
   if (a->mode == NB_CHAIN_RESIDUAL && a->N % kBlock) return NB_ERR_SHAPE;
   if (a->split < 0 || a->split > 8 || (a->split & (a->split - 1))) return NB_ERR_ARG;
   if ((long long)(a->N + 15) / 16 * (a->K / kBlock) > kMost || a->N > (1 << 24)) return NB_ERR_SHAPE;
-  if ((uintptr_t)a->w % 16 || (uintptr_t)a->x_terms % 16 || (uintptr_t)a->y_terms % 16 || (uintptr_t)a->ahead % 16 || a->ahead_bytes % 16)
+  if ((uintptr_t)a->w % 16 || (uintptr_t)a->x_terms % 16 || (uintptr_t)a->y_terms % 16 || (uintptr_t)a->ahead % 16 || a->ahead_bytes % 16 || (uintptr_t)a->x % 16)
     return NB_ERR_ALIGN;
   if (int rc = check_device()) return rc;
   const int bpr = a->K / kBlock;
@@ -462,12 +525,13 @@ extern "C" int nb_chain_linear(const nb_chain_args* a, void* stream) {
   best.cost = 1e30;
   for (int S : {1, 2, 4, 8}) {
     if (a->split && S != a->split) continue;
-    if (chain_plan(a->N, bpr, a->M, a->bits, S, max_clusters(S), pl) && pl.cost < best.cost) best = pl;
+    if (chain_plan(a->N, bpr, a->M, a->x && a->x_dtype != NB_F32 ? 1 : 2, a->x != nullptr, a->bits, S, max_clusters(S), pl) && pl.cost < best.cost) best = pl;
   }
   if (best.cost == 1e30) return NB_ERR_SHAPE;
   ChainParams p{};
   p.w = a->w; p.xt = reinterpret_cast<const uint8_t*>(a->x_terms); p.ss = a->sq; p.y = a->y; p.yt = reinterpret_cast<uint8_t*>(a->y_terms);
   p.res = a->residual; p.w_next = a->next_weight; p.ss_out = a->sq_out; p.status = a->status;
+  p.x = a->x; p.x_dtype = a->x_dtype; p.y_dtype = a->y_dtype;
   p.N = a->N; p.bpr = bpr; p.M = a->M; p.mode = a->mode; p.ss_n = a->sq_n; p.eps = a->eps;
   p.m_part = best.m_part; p.parts = best.parts; p.lg_split = best.S == 8 ? 3 : best.S >> 1; p.units = best.units; p.J = best.J;
   auto rcp = [](int v) { return (unsigned)((0x100000000ull + v - 1) / v); };
@@ -485,17 +549,7 @@ extern "C" int nb_chain_linear(const nb_chain_args* a, void* stream) {
     }
     int rc = NB_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    switch (a->bits * 8 + best.cg) {
-      case 17: rc = chain_launch<2, 1>(best, p, st); break;
-      case 18: rc = chain_launch<2, 2>(best, p, st); break;
-      case 20: rc = chain_launch<2, 4>(best, p, st); break;
-      case 25: rc = chain_launch<3, 1>(best, p, st); break;
-      case 26: rc = chain_launch<3, 2>(best, p, st); break;
-      case 28: rc = chain_launch<3, 4>(best, p, st); break;
-      case 33: rc = chain_launch<4, 1>(best, p, st); break;
-      case 34: rc = chain_launch<4, 2>(best, p, st); break;
-      default: rc = chain_launch<4, 4>(best, p, st); break;
-    }
+    rc = a->bits == 2 ? chain_launch<2>(best, p, a->ordered, st) : a->bits == 3 ? chain_launch<3>(best, p, a->ordered, st) : chain_launch<4>(best, p, a->ordered, st);
     if (rc) return rc;
   }
   return NB_OK;

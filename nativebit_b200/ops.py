@@ -503,6 +503,26 @@ def chain_linear(mode: int, w_stream: torch.Tensor, bits: int, m: int, n: int, k
         _lib.check(_lib.lib().nb_chain_linear(_c.byref(args), _stream()), "nb_chain_linear")
 
 
+def chain_rows(x: torch.Tensor, w_stream: torch.Tensor, bits: int, n: int, k: int, ordered: bool = False,
+               out: torch.Tensor | None = None) -> torch.Tensor | None:
+    """y (M, n) = x (M, k) @ W.T in x's type for a few rows of any float type against the stream-layout weights (nb_chain_linear);
+    None if the rows do not fit.  ordered: as for gemv, for weights that the launch before may have written."""
+    _need_cuda(x, w_stream)
+    if x.dim() != 2 or x.shape[1] != k or x.dtype not in _DTYPE:
+        raise RuntimeError(f"x must be a contiguous float (M, {k}) tensor; got {x.dtype} {tuple(x.shape)}")
+    if out is None:
+        out = torch.empty(x.shape[0], n, dtype=x.dtype, device=x.device)
+    with torch.cuda.device(x.device):
+        status = prefill_workspace(x.device, 256)            # its head
+        args = _lib.ChainArgs(w=w_stream.data_ptr(), y=out.data_ptr(), status=status.data_ptr(), M=x.shape[0], N=n, K=k, bits=bits,
+                              x_dtype=_DTYPE[x.dtype], y_dtype=_DTYPE[out.dtype], ordered=int(ordered), x=x.data_ptr())
+        rc = _lib.lib().nb_chain_linear(_c.byref(args), _stream())
+    if rc == 3:
+        return None
+    _lib.check(rc, "nb_chain_linear")
+    return out
+
+
 def chain_embed(table: torch.Tensor, token: torch.Tensor, weight: torch.Tensor, x: torch.Tensor, terms: torch.Tensor, sq: torch.Tensor) -> None:
     """x = table[token] (bf16 -> fp32), terms = x * weight, sq = its partial sums of squares (nb_chain_embed)."""
     _need_cuda(table, token, weight, x, terms, sq)

@@ -21,7 +21,12 @@ def test_native_call_leaves_everything_else_to_the_general_path(built_lib):
 def _general(lin, x):
     """The call without its native form."""
     flat = x.reshape(-1, lin.in_features).contiguous()
-    if flat.shape[0] <= 16:
+    if 2 <= flat.shape[0] <= 16:
+        y = ops.chain_rows(flat, lin.stream_weight(), lin.bits, lin.out_features, lin.in_features, ordered=True)
+        z = ops.gemv(flat, lin.packed_indices, lin.codebook, lin.bits, 128, lin.out_features, lin.in_features, ordered=True)
+        # the sums of two kernels in fp32, rounded: two results to either side of a tie are an ulp apart
+        assert (y.double() - z.double()).norm() <= {torch.float32: 2e-6, torch.float16: 2.0 ** -10, torch.bfloat16: 2.0 ** -7}[x.dtype] * z.double().norm()
+    elif flat.shape[0] == 1:
         y = ops.gemv(flat, lin.packed_indices, lin.codebook, lin.bits, 128, lin.out_features, lin.in_features, ordered=True)
     else:
         y = lin._forward_many(flat)
@@ -39,6 +44,9 @@ def test_native_call_equals_the_general_path(built_lib, bits, dtype):
     big = torch.randn(700, 2 * k, device="cuda", generator=g).to(dtype)
     forms = [big[0, :k], big[:1, :k], big[:16, :k].contiguous(), big[:16, :k], big[:17, :k].contiguous(), big[:17, :k], big[:600, k:].contiguous(),
              big[:12, :k].reshape(3, 4, k), big[:40, :k].reshape(2, 20, k), big[:24, :k].view(4, 6, k).transpose(0, 1), big[:0, :k]]
+    odd = torch.zeros(4 * k + 8, device="cuda", dtype=dtype)[1:4 * k + 1].view(4, k)                # not on a 16-byte boundary
+    odd.copy_(big[:4, :k])
+    assert torch.equal(lin(odd), ops.gemv(odd, lin.packed_indices, lin.codebook, bits, 128, n, k, ordered=True))
     for turn in range(2):                                   # the first calls make the workspaces and the stream-layout copy
         for x in forms:
             if x.shape[0] == 0:

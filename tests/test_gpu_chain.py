@@ -114,3 +114,19 @@ def test_chain_carries_norms_and_residuals(built_lib, m, c, f):
     ops.chain_linear(ops.CHAIN_RESIDUAL, down, bits, m, c, f, ch, status, residual=x)          # nothing behind it
     _close(x, before.double() + h @ down_dense.T, 4 * REL)
     assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("n,k,m", [(16, 128, 1), (1000, 1024, 9), (2560, 6912, 16), (5632, 2048, 11), (333, 2560, 13), (4096, 256, 33)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("bits", [2, 3, 4])
+def test_chain_rows_takes_plain_activations(built_lib, n, k, m, dtype, bits):
+    w, dense = _matrix(n, k, bits, seed=n + m)
+    x = torch.randn(m, k, device=DEV, generator=torch.Generator(device=DEV).manual_seed(k)).to(dtype)
+    want = x.double() @ dense.T
+    for ordered in (True, False):
+        y = ops.chain_rows(x, w, bits, n, k, ordered=ordered, out=torch.full((m, n), float("nan"), dtype=torch.float32, device=DEV))
+        _close(y, want, REL)
+    y = ops.chain_rows(x, w, bits, n, k)
+    assert y.dtype == dtype
+    # a rounding of the result to nearest is at most half an ulp (2^-11, 2^-8) of each value
+    _close(y, want, {torch.float32: REL, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[dtype])
