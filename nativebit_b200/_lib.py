@@ -60,6 +60,7 @@ _SIGNATURES = {
                                 _c.c_void_p, _c.c_void_p]),
     "nb_embed_rows": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_int, _c.c_int, _c.c_int, _c.c_void_p, _c.c_void_p]),
     "nb_chain_terms_bytes": (_c.c_size_t, [_c.c_int, _c.c_int]),
+    "nb_chain_takes": (_c.c_int, [_c.c_int] * 5),
     "nb_chain_linear": (_c.c_int, [_c.c_void_p, _c.c_void_p]),
     "nb_chain_embed": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_int, _c.c_int, _c.c_int, _c.c_void_p, _c.c_void_p, _c.c_void_p,
                                   _c.c_void_p, _c.c_void_p]),

@@ -55,7 +55,7 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
   at::DimVector shape(x.sizes());
   shape.back() = n;
   int rc = NB_ERR_ARG;
-  if (m >= 2 && m <= kGemvRows && THPVariable_CheckExact(a[3])) {
+  if (m >= 2 && THPVariable_CheckExact(a[3]) && (m <= kGemvRows || nb_chain_takes((int)m, (int)n, (int)k, bits, xt))) {
     const at::Tensor &w = THPVariable_Unpack(a[3]), *ws = workspace(a[9], device.index(), stream);
     if (!ws || w.device() != device) Py_RETURN_NONE;
     at::Tensor y = at::empty(shape, x.options().requires_grad(false).memory_format(c10::MemoryFormat::Contiguous));

@@ -502,6 +502,21 @@ using namespace nb;
 
 extern "C" size_t nb_chain_terms_bytes(int M, int K) { return M < 1 || K < kBlock || K % kBlock ? 0 : (size_t)M * K * 4; }
 
+// Whether nb_chain_linear is the faster one for more rows than its columns were made for.  Its MMAs and parts grow with the rows, the
+// tcgen05 kernel has its start, its k-steps and a sum over k splits whatever the rows are (fused | this, us, 3 bits, fp32 rows:
+// 3072 x 1024 17 rows 8.4 | 5.5, 64: 11.5 | 8.5; 2560 x 2560 32: 10.9 | 9.4, 48: 10.4 | 11.6; 6144 x 2048 17: 10.7 | 10.8; bf16 6144 x 2048 32:
+// 11.0 | 9.4, 48: 11.7 | 17.7; 7680 x 2560 17: 12.1 | 10.9, 24: 12.2 | 17.6): up to 400 M products in one launch.
+extern "C" int nb_chain_takes(int M, int N, int K, int bits, int x_dtype) {
+  if (M < 1 || N < 1 || K < kBlock || K % kBlock || (bits != 2 && bits != 3 && bits != 4) || M > 64) return 0;
+  const int terms = x_dtype == NB_F32 ? 2 : 1;
+  if ((double)M * terms * N * K > 400e6 || check_device() != NB_OK) return 0;
+  ChainPlan pl{}, best{};
+  best.cost = 1e30;
+  for (int S : {1, 2, 4, 8})
+    if (chain_plan(N, K / kBlock, M, terms, true, bits, S, max_clusters(S), pl) && pl.cost < best.cost) best = pl;
+  return best.cost < 1e30 && best.launches == 1;
+}
+
 extern "C" int nb_chain_linear(const nb_chain_args* a, void* stream) {
   constexpr long long kMost = 1ll << 26;                    // products of sizes below stay in 32 bits
   if (!a || !a->w || (a->x ? a->sq || a->mode != NB_CHAIN_STORE : !a->x_terms) || !a->status || a->M < 1 || a->N < 1) return NB_ERR_ARG;

@@ -348,7 +348,7 @@ def step(model: PackedGPT, x: torch.Tensor, caches):
     return logits[:, -1, :], caches
 
 
-CHAIN_MAX_ROWS = 16          # activation rows up to which a step's linears run on nb_chain_linear
+CHAIN_MAX_ROWS = 16          # activation rows up to which a step's linears run on nb_chain_linear whatever their sizes
 
 
 class DecodeSession(Session):
@@ -381,9 +381,11 @@ class DecodeSession(Session):
                               and getattr(model, "exchange", None) is None)
         # the default for both on one GPU: a chain in which every launch hands the next its activations ready for the tensor cores
         # (nb_chain_linear)
-        self.chain = bool(fits and fused and tile_gemv is not False and batch_size <= CHAIN_MAX_ROWS and model.tp_size == 1
+        self.chain = bool(fits and fused and tile_gemv is not False and model.tp_size == 1
                           and getattr(model, "exchange", None) is None and model.embedding.dtype == torch.bfloat16
-                          and model.config.n_embd % 128 == 0 and all(b.gate_up.out_features % 256 == 0 for b in model.blocks))
+                          and model.config.n_embd % 128 == 0 and all(b.gate_up.out_features % 256 == 0 for b in model.blocks)
+                          and (batch_size <= CHAIN_MAX_ROWS or all(ops.chain_takes(batch_size, l.out_features, l.in_features, l.bits, torch.float32)
+                                                                   for b in model.blocks for l in (b.qkv, b.out_proj, b.gate_up, b.down))))
         # stream=True (one sequence on one GPU): the whole step is ONE launch of the persistent kernel
         # (stream.py).  The default is the chain of fused kernels, which measures faster: inside one launch
         # every operation pays a device-wide flag wait and the staging of its activations in full.

@@ -503,6 +503,19 @@ def chain_linear(mode: int, w_stream: torch.Tensor, bits: int, m: int, n: int, k
         _lib.check(_lib.lib().nb_chain_linear(_c.byref(args), _stream()), "nb_chain_linear")
 
 
+_takes: dict = {}
+
+
+def chain_takes(m: int, n: int, k: int, bits: int, dtype: torch.dtype) -> bool:
+    """Whether m > 16 rows of this type are for chain_rows rather than gemm_prefill_fused (nb_chain_takes)."""
+    if m > 64:
+        return False
+    key = (m, n, k, bits, dtype)
+    if key not in _takes:
+        _takes[key] = bool(_lib.lib().nb_chain_takes(m, n, k, bits, _DTYPE[dtype]))
+    return _takes[key]
+
+
 def chain_rows(x: torch.Tensor, w_stream: torch.Tensor, bits: int, n: int, k: int, ordered: bool = False,
                out: torch.Tensor | None = None) -> torch.Tensor | None:
     """y (M, n) = x (M, k) @ W.T in x's type for a few rows of any float type against the stream-layout weights (nb_chain_linear);

@@ -124,6 +124,9 @@ class PackedLinear(torch.nn.Module):
         """M > 16 rows on the tcgen05 kernels (exact fp16 weights; bf16 and fp16 activations as given, fp32
         carried as two fp16 terms; fp32 accumulation; result in x's dtype): one pass over the packed weights,
         dequantised inside the kernel, up to FUSED_MAX_ROWS rows; dequantise-once + GEMM beyond."""
+        if x_flat.dtype in (torch.float32, torch.float16, torch.bfloat16) and self._few_enough(x_flat.shape[0], x_flat.dtype) and (
+                y := self._forward_few(x_flat)) is not None:
+            return y
         if self._tensor_cores():
             rows = x_flat.shape[0] * (2 if x_flat.dtype == torch.float32 else 1)
             if rows > FUSED_MAX_ROWS:
@@ -144,12 +147,16 @@ class PackedLinear(torch.nn.Module):
     def _tensor_cores(self) -> bool:
         return self.block_size == BS and self.in_features % BS == 0 and self.bits in (2, 3, 4)
 
+    def _few_enough(self, rows: int, dtype) -> bool:
+        """More than 16 rows, of a matrix so small that they are faster on the kernel for few rows."""
+        return self._tensor_cores() and ops.chain_takes(rows, self.out_features, self.in_features, self.bits, dtype)
+
     def takes_terms(self, rows: int) -> bool:
         """Whether a call would split this many fp32 rows into two fp16 terms itself and nobody else looks at them, so that
         `forward_terms` may take their place: no hooks, no forward of a subclass or of this instance."""
         seen = (self._forward_pre_hooks or self._forward_hooks or _module._global_forward_pre_hooks or _module._global_forward_hooks
                 or "forward" in self.__dict__ or type(self).forward is not PackedLinear.forward)
-        return rows > GEMV_MAX_M and self._tensor_cores() and not seen
+        return rows > GEMV_MAX_M and self._tensor_cores() and not self._few_enough(rows, torch.float32) and not seen
 
     def forward_terms(self, terms, out=None):
         """fp32 (M, out_features) of M fp32 rows given as their two fp16 terms, (2M, in_features); see ops.add_rmsnorm_terms."""
