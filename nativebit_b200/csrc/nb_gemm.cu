@@ -42,6 +42,7 @@
 
 #include "nb_common.cuh"
 #include "nb_host.h"
+#include "nb_launch.cuh"
 #include "nb_umma.cuh"
 #include "../../include/nativebit_b200_layered.h"
 
@@ -504,15 +505,17 @@ extern "C" int nb_gemm_prefill(const void* x, int x_dtype, int M, const uint8_t*
   if (int rc = nb_dequant(packed, codebook, cb_dtype, bits, block_size, N, K, w, NB_F16, stream)) return rc;
   if (x_dtype == NB_F16 || x_dtype == NB_F16_TERMS)
     return gemm_16bit(x, w, 1, M, N, K, y, y_dtype, reinterpret_cast<int*>(workspace), stream, x_dtype == NB_F16_TERMS);
+  // the conversion runs beside the dequantisation: it reads and writes nothing of its (a call with 2048 rows
+  // x 6912 x 2560 78.2 -> 75.2 us, together with the wider stores of nb_dequant)
   const size_t n8 = (size_t)M * K / 8;  // K % 64 == 0
+  const dim3 grid((unsigned)((n8 + 255) / 256)), block(256);
   if (x_dtype == NB_F32) {  // two fp16 terms per element; rows 2i and 2i + 1 of the kernel's result are one row of 2K here
-    f32_to_f16_pair_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(reinterpret_cast<const float4*>(x),
-                                                                                          reinterpret_cast<uint4*>(xh), M, K);
-    if (int rc = check_launch()) return rc;
+    if (int rc = launch_pdl(f32_to_f16_pair_kernel, grid, block, 0, (cudaStream_t)stream, reinterpret_cast<const float4*>(x),
+                            reinterpret_cast<uint4*>(xh), M, K))
+      return rc;
     return gemm_16bit(xh, w, 1, M, N, K, y, y_dtype, reinterpret_cast<int*>(workspace), stream, true);
   }
-  bf16_to_f16_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(reinterpret_cast<const uint4*>(x),
-                                                                                    reinterpret_cast<uint4*>(xh), n8);
-  if (int rc = check_launch()) return rc;
+  if (int rc = launch_pdl(bf16_to_f16_kernel, grid, block, 0, (cudaStream_t)stream, reinterpret_cast<const uint4*>(x), reinterpret_cast<uint4*>(xh), n8))
+    return rc;
   return gemm_16bit(xh, w, 1, M, N, K, y, y_dtype, reinterpret_cast<int*>(workspace), stream);
 }

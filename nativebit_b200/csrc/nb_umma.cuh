@@ -136,6 +136,8 @@ static __global__ void __launch_bounds__(256) bf16_to_f16_kernel(const uint4* __
 #pragma unroll
   for (int j = 0; j < 4; ++j) r[j] = f32x2_to_f16x2_sat(__uint_as_float(u[j] << 16), __uint_as_float(u[j] & 0xFFFF0000u));
   out[i] = make_uint4(r[0], r[1], r[2], r[3]);
+  // where this launch runs beside the dequantisation, its end has to mean that one's end as well: the GEMM waits for this one only
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // fp32 -> two fp16 terms per element, hi = fp16(x) (saturating) and lo = fp16(x - hi), written as rows 2i and
@@ -157,6 +159,7 @@ static __global__ void __launch_bounds__(256) f32_to_f16_pair_kernel(const float
   }
   out[(size_t)(2 * row) * k8 + c] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
   out[(size_t)(2 * row + 1) * k8 + c] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  asm volatile("griddepcontrol.wait;" ::: "memory");        // as above
 }
 
 }  // namespace nb

@@ -5,6 +5,7 @@
 // (nativebit/pack.py:21-41, 75-82, 97-116).
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
+#include <type_traits>
 #include <cuda_bf16.h>
 
 #include "nb_common.cuh"
@@ -113,8 +114,7 @@ __global__ void pack_kernel(const uint8_t* __restrict__ idx, int64_t count, int 
 
 // ---- dequant ------------------------------------------------------------------------------
 // Fast path (fp16 codebook, block_size % 8 == 0, aligned): a thread dequantises the eight consecutive weights of ONE store of 16
-// bytes, 32 for fp32 (four per thread there built every table twice: 6912 x 2560 at 3 bits 19.5 -> 14.5 us, 6.4 TB/s with 32 bytes
-// per thread), so that a warp's stores are one contiguous run (a thread with 32 weights of its own left every store 64 or 128
+// bytes, 32 for fp32 (four per thread there built every table twice: 6912 x 2560 at 3 bits 19.5 -> 14.5 us, 5.5 TB/s), so that a warp's stores are one contiguous run (a thread with 32 weights of its own left every store 64 or 128
 // bytes from its neighbour's: 12.1 us for 6912 x 2560 to fp16 and 34.7 us to fp32, which take 6.7 and 12.2 us at the copy
 // rate).  The 3- or 2-bit fields are spread to the nibbles of one selector word; the block's table, as byte planes, answers
 // four lookups with two byte permutes.  A thread takes PER stores a block stride apart and requests all inputs first: four where
@@ -173,22 +173,51 @@ template <int BITS> __device__ __forceinline__ void store8(float* dst, uint32_t 
   }
 }
 
-template <int BITS, int PER, typename OutT>
+// Sixteen lookups as one store of 32 bytes, where the address allows it.
+template <int BITS, typename T16> __device__ __forceinline__ void store_pair(T16* dst, uint32_t sel0, uint32_t sel1, const uint32_t (&T)[BITS == 4 ? 8 : 4]) {
+  if ((uintptr_t)dst % 32 != 0) {
+    store8<BITS>(dst, sel0, T);
+    store8<BITS>(dst + 8, sel1, T);
+    return;
+  }
+  uint32_t h[8];
+  lookup4<BITS>(sel0, T, h[0], h[1]);
+  lookup4<BITS>(sel0 >> 16, T, h[2], h[3]);
+  lookup4<BITS>(sel1, T, h[4], h[5]);
+  lookup4<BITS>(sel1 >> 16, T, h[6], h[7]);
+  if (std::is_same<T16, __nv_bfloat16>::value) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h[j]));
+      const __nv_bfloat162 b = __floats2bfloat162_rn(f.x, f.y);
+      h[j] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+  }
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"l"(dst), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]), "r"(h[4]), "r"(h[5]), "r"(h[6]), "r"(h[7]) : "memory");
+}
+
+// W: chunks of eight weights per store (2: 16-bit types in blocks of whole 16 weights, at 3 and 4 bits: 13824 x 2560 to fp16 20.2 -> 16.8
+// and 18.7 -> 15.2 us; at 2 bits, whose lookups and loads are few, 12.4 -> 14.4).
+template <int BITS, int PER, int W, typename OutT>
 __global__ void __launch_bounds__(kDqThreads) dequant16b_kernel(const uint32_t* __restrict__ packed, const __half* __restrict__ codebook,
                                                                int64_t n_stores, int64_t n_bytes, int64_t total, int block_size, int shift,
                                                                OutT* __restrict__ out) {
+  asm volatile("griddepcontrol.launch_dependents;");        // a conversion behind this may run beside it
   constexpr int kT = BITS == 4 ? 8 : 4;
   const int64_t i0 = (int64_t)blockIdx.x * (kDqThreads * PER) + threadIdx.x;
-  uint32_t sel[PER], e[PER][kT];
+  uint32_t sel[PER][W], e[PER][kT];
 #pragma unroll
   for (int u = 0; u < PER; ++u) {
     const int64_t i = i0 + u * kDqThreads;
-    sel[u] = 0;
+#pragma unroll
+    for (int q = 0; q < W; ++q) sel[u][q] = 0;
 #pragma unroll
     for (int j = 0; j < kT; ++j) e[u][j] = 0;
     if (i < n_stores) {
-      sel[u] = load_selectors<BITS>(packed, i);
-      const int64_t block = block_of(i, block_size >> 3, shift);
+#pragma unroll
+      for (int q = 0; q < W; ++q) sel[u][q] = load_selectors<BITS>(packed, W * i + q);
+      const int64_t block = block_of(i, block_size / (8 * W), shift);
       const uint8_t* row = reinterpret_cast<const uint8_t*>(codebook) + block * (2 << BITS);
       if (BITS == 2) {
         const uint2 v = *reinterpret_cast<const uint2*>(row);
@@ -217,10 +246,11 @@ __global__ void __launch_bounds__(kDqThreads) dequant16b_kernel(const uint32_t* 
         T[j + 2] = prmt(e[u][j], e[u][j + 1], 0x7531); T[j + 3] = prmt(e[u][j + 2], e[u][j + 3], 0x7531);
       }
     }
-    store8<BITS>(out + i * 8, sel[u], T);
+    if constexpr (W == 2) store_pair<BITS>(out + i * 16, sel[u][0], sel[u][1], T);
+    else store8<BITS>(out + i * 8, sel[u][0], T);
   }
   // fewer than 32 weights behind the last whole packed word, one for each of the threads without a store
-  const int64_t one = n_stores * 8 + (i - n_stores);
+  const int64_t one = n_stores * (8 * W) + (i - n_stores);
   if (i >= n_stores && i < i0 + PER * kDqThreads && one < total) {
     const uint32_t at = stream_index(reinterpret_cast<const uint8_t*>(packed), n_bytes, one, BITS);
     out[one] = (OutT)(float)codebook[block_of(one, block_size, -1) * (1 << BITS) + at];
@@ -471,9 +501,10 @@ static int dequant_dispatch(const uint8_t* packed, const void* codebook, int cb_
   const int64_t n_bytes = packed_bytes(n_blocks * block_size, bits);
   const bool aligned = ((uintptr_t)packed % 4 == 0) && ((uintptr_t)out % 16 == 0) && ((uintptr_t)codebook % 16 == 0);
   if (cb_dtype == NB_F16 && block_size % 8 == 0 && aligned) {
-    const int64_t stores = total / 32 * 4;             // whole packed words
-    if (stores > 0) {
-      const int shift = shift_of(block_size / 8);
+    const auto start = [&](auto width) {
+      constexpr int W = decltype(width)::value;
+      const int64_t stores = total / 32 * (4 / W);          // whole packed words
+      const int shift = shift_of(block_size / (8 * W));
       const bool several = stores >= (int64_t)kDqRuns * kDqThreads * 4 * sm_count();
       const int64_t per = kDqThreads * (several ? kDqRuns : 1);
       auto run = [&](auto kernel) {
@@ -481,9 +512,15 @@ static int dequant_dispatch(const uint8_t* packed, const void* codebook, int cb_
                                                                             block_size, shift, out);
         return check_launch();
       };
-      if (bits == 3) return several ? run(dequant16b_kernel<3, kDqRuns, OutT>) : run(dequant16b_kernel<3, 1, OutT>);
-      if (bits == 2) return several ? run(dequant16b_kernel<2, kDqRuns, OutT>) : run(dequant16b_kernel<2, 1, OutT>);
-      return several ? run(dequant16b_kernel<4, kDqRuns, OutT>) : run(dequant16b_kernel<4, 1, OutT>);
+      if (bits == 3) return several ? run(dequant16b_kernel<3, kDqRuns, W, OutT>) : run(dequant16b_kernel<3, 1, W, OutT>);
+      if (bits == 2) return several ? run(dequant16b_kernel<2, kDqRuns, W, OutT>) : run(dequant16b_kernel<2, 1, W, OutT>);
+      return several ? run(dequant16b_kernel<4, kDqRuns, W, OutT>) : run(dequant16b_kernel<4, 1, W, OutT>);
+    };
+    if (total >= 32) {
+      if constexpr (sizeof(OutT) == 2) {
+        if (bits != 2 && block_size % 16 == 0) return start(std::integral_constant<int, 2>{});
+      }
+      return start(std::integral_constant<int, 1>{});
     }
   }
   const unsigned grid = (unsigned)((total + 255) / 256);
