@@ -576,6 +576,10 @@ __device__ __forceinline__ void copy16_or_zero(float* dst, const float* src, boo
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
 }
 
+// What bounds it: two warps per scheduler that wait for their own loads; 58 % of the multiply-add pipe's slots are used at eight
+// prompts of 512 tokens, 32 heads of 80 (333 us).  Two steps of the scores' loop in one put the second one's loads ahead of the first one's sums:
+// one prompt of 512 tokens 58.7 -> 51.3 us, eight of 500 with 16 heads of 128 306 -> 296; with 64 queries of heads of 80 the registers for
+// that are not there (333 -> 341), so that form takes one.  Three CTAs of 48 or 32 queries per SM: 361, 348.
 template <int R, int PK, int NP>
 __global__ void __launch_bounds__(128, 2) prefill_attention_kernel(
     const float* __restrict__ qkv, const float* __restrict__ cos2, const float* __restrict__ sin2, const float* __restrict__ k_cache,
@@ -638,7 +642,8 @@ __global__ void __launch_bounds__(128, 2) prefill_attention_kernel(
         for (int i = 0; i < KI; ++i) sum[r][i] = 0ull;
       const float* qr = q_s + ty * R * hdp;
       const float* kr = k_s + tx * hdp;
-#pragma unroll 1
+      constexpr int kSteps = R == 8 && NP == 5 ? 1 : 2;
+#pragma unroll kSteps
       for (int d = 0; d < hd; d += 4) {
         ulonglong2 y[KI];
 #pragma unroll
