@@ -161,10 +161,12 @@ static int attn_per_max(int ctx, int S) { return (((ctx + S - 1) / S) + 7) & ~7;
 static size_t attn_limit_floats(int ctx, int hd, int S) { return (size_t)attn_per_max(ctx, S) + (size_t)(2 + kAttnWarps) * hd + 4; }
 static size_t attn_smem_floats(int hd) { return (size_t)(1 + kAttnWarps) * hd + (size_t)kAttnMaxSplit * (hd + 4); }
 
+// kTerms: `out` is the terms buffer of the chain's next launch, out_stride columns wide, not rows of floats.
+template <bool kTerms>
 __global__ void __launch_bounds__(kAttnWarps * 32) decode_attention_kernel(
     const float* __restrict__ q, float* k_cache, float* v_cache, const long long* __restrict__ pos_ptr, float* __restrict__ out,
     int H, int hd, int ctx, int out_stride, int out_offset, const float* __restrict__ qkv, const float* __restrict__ cos2,
-    const float* __restrict__ sin2, uint8_t* __restrict__ terms) {
+    const float* __restrict__ sin2) {
   extern __shared__ __align__(16) float sm[];  // q | per-warp numerators | rank 0: the CTAs' numerator, maximum, denominator
   __shared__ float s_m[kAttnWarps], s_l[kAttnWarps];
   cg::cluster_group cluster = cg::this_cluster();
@@ -313,7 +315,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) decode_attention_kernel(
         den += w * slots[r * slot + hd + 1];
       }
     }
-    if (terms) store_chain_terms(terms, out_stride >> 7, b, out_offset + h * hd + tid, num / den);
+    if (kTerms) store_chain_terms(reinterpret_cast<uint8_t*>(out), out_stride >> 7, b, out_offset + h * hd + tid, num / den);
     else out[(size_t)b * out_stride + out_offset + h * hd + tid] = num / den;
   }
 }
@@ -330,10 +332,11 @@ __global__ void __launch_bounds__(kAttnWarps * 32) decode_attention_kernel(
 constexpr int kWideWarps = 4, kWideKeys = 8, kWideD = 3;
 static size_t wide_smem_floats(int hd) { return (size_t)kWideWarps * kWideD * 2 * kWideKeys * hd + (size_t)(3 + kWideWarps) * hd; }
 
+template <bool kTerms>
 __global__ void __launch_bounds__(kWideWarps * 32) decode_attention_wide_kernel(
     const float* __restrict__ q, float* k_cache, float* v_cache, const long long* __restrict__ pos_ptr, float* __restrict__ out,
     int H, int hd, int ctx, int out_stride, int out_offset, const float* __restrict__ qkv, const float* __restrict__ cos2,
-    const float* __restrict__ sin2, uint8_t* __restrict__ terms) {
+    const float* __restrict__ sin2) {
   extern __shared__ __align__(16) float sm[];  // per warp kWideD stages of keys | values, then q | key | value of this step | outputs
   __shared__ float s_m[kWideWarps], s_l[kWideWarps];
   const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -467,7 +470,7 @@ __global__ void __launch_bounds__(kWideWarps * 32) decode_attention_wide_kernel(
       num += e * part[w * hd + tid];
       den += e * s_l[w];
     }
-    if (terms) store_chain_terms(terms, out_stride >> 7, b, out_offset + h * hd + tid, num / den);
+    if (kTerms) store_chain_terms(reinterpret_cast<uint8_t*>(out), out_stride >> 7, b, out_offset + h * hd + tid, num / den);
     else out[(size_t)b * out_stride + out_offset + h * hd + tid] = num / den;
   }
 }
@@ -478,7 +481,7 @@ static int attn_split(int B, int H) {
   return want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;
 }
 
-template <typename... Args>
+template <bool kTerms, typename... Args>
 static int launch_attention(int B, int H, int hd, int ctx, cudaStream_t st, Args... args) {
   const int S = attn_split(B, H);
   if (attn_limit_floats(ctx, hd, S) * sizeof(float) > 48 * 1024) return NB_ERR_SHAPE;      // the contexts that are taken stay what they were
@@ -487,12 +490,12 @@ static int launch_attention(int B, int H, int hd, int ctx, cudaStream_t st, Args
     int dev = 0;
     cudaGetDevice(&dev);
     if (!done[dev & 63]) {
-      if (cudaError_t e = cudaFuncSetAttribute(decode_attention_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      if (cudaError_t e = cudaFuncSetAttribute(decode_attention_wide_kernel<kTerms>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)(wide_smem_floats(128) * sizeof(float))))
         return record_cuda_error(e);
       done[dev & 63] = true;
     }
-    return launch_pdl(decode_attention_wide_kernel, dim3(H, B), dim3(kWideWarps * 32), wide_smem_floats(hd) * sizeof(float), st, args...);
+    return launch_pdl(decode_attention_wide_kernel<kTerms>, dim3(H, B), dim3(kWideWarps * 32), wide_smem_floats(hd) * sizeof(float), st, args...);
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(H, B, S);
@@ -508,7 +511,7 @@ static int launch_attention(int B, int H, int hd, int ctx, cudaStream_t st, Args
   attr[1].val.clusterDim.z = S;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return record_cuda_error(cudaLaunchKernelEx(&cfg, decode_attention_kernel, args...));
+  return record_cuda_error(cudaLaunchKernelEx(&cfg, decode_attention_kernel<kTerms>, args...));
 }
 
 // The pairs (x, y) and (z, w) turned by their angles.
@@ -1083,8 +1086,8 @@ extern "C" int nb_decode_attention_rope(const float* qkv, const float* cos2, con
   if (hd > 128 || hd % 4 != 0) return NB_ERR_SHAPE;
   if ((uintptr_t)k_cache % 16 || (uintptr_t)v_cache % 16) return NB_ERR_ALIGN;
   if (int rc = check_device()) return rc;
-  return launch_attention(B, H, hd, ctx, (cudaStream_t)stream, (const float*)nullptr, k_cache, v_cache,
-                          reinterpret_cast<const long long*>(pos), out, H, hd, ctx, out_stride, out_offset, qkv, cos2, sin2, (uint8_t*)nullptr);
+  return launch_attention<false>(B, H, hd, ctx, (cudaStream_t)stream, (const float*)nullptr, k_cache, v_cache,
+                                 reinterpret_cast<const long long*>(pos), out, H, hd, ctx, out_stride, out_offset, qkv, cos2, sin2);
 }
 
 extern "C" int nb_decode_attention_terms(const float* qkv, const float* cos2, const float* sin2, const int64_t* pos, float* k_cache,
@@ -1095,9 +1098,9 @@ extern "C" int nb_decode_attention_terms(const float* qkv, const float* cos2, co
   if (hd > 128 || hd % 4 != 0 || out_cols % kBlock || out_offset + H * hd > out_cols) return NB_ERR_SHAPE;
   if ((uintptr_t)k_cache % 16 || (uintptr_t)v_cache % 16 || (uintptr_t)terms % 16) return NB_ERR_ALIGN;
   if (int rc = check_device()) return rc;
-  return launch_attention(B, H, hd, ctx, (cudaStream_t)stream, (const float*)nullptr, k_cache, v_cache,
-                          reinterpret_cast<const long long*>(pos), (float*)nullptr, H, hd, ctx, out_cols, out_offset, qkv, cos2, sin2,
-                          reinterpret_cast<uint8_t*>(terms));
+  return launch_attention<true>(B, H, hd, ctx, (cudaStream_t)stream, (const float*)nullptr, k_cache, v_cache,
+                                reinterpret_cast<const long long*>(pos), reinterpret_cast<float*>(terms), H, hd, ctx, out_cols, out_offset,
+                                qkv, cos2, sin2);
 }
 
 extern "C" int nb_decode_attention(const float* q, const float* k_cache, const float* v_cache, const int64_t* pos, int B, int H,
@@ -1106,9 +1109,9 @@ extern "C" int nb_decode_attention(const float* q, const float* k_cache, const f
   if (hd > 128 || hd % 4 != 0) return NB_ERR_SHAPE;
   if ((uintptr_t)k_cache % 16 || (uintptr_t)v_cache % 16) return NB_ERR_ALIGN;
   if (int rc = check_device()) return rc;
-  return launch_attention(B, H, hd, ctx, (cudaStream_t)stream, q, const_cast<float*>(k_cache), const_cast<float*>(v_cache),
-                          reinterpret_cast<const long long*>(pos), out, H, hd, ctx, out_stride, out_offset, (const float*)nullptr,
-                          (const float*)nullptr, (const float*)nullptr, (uint8_t*)nullptr);
+  return launch_attention<false>(B, H, hd, ctx, (cudaStream_t)stream, q, const_cast<float*>(k_cache), const_cast<float*>(v_cache),
+                                 reinterpret_cast<const long long*>(pos), out, H, hd, ctx, out_stride, out_offset, (const float*)nullptr,
+                                 (const float*)nullptr, (const float*)nullptr);
 }
 
 extern "C" int nb_prefill_attention(const float* qkv, int B, int T, int H, int hd, const float* cos2, const float* sin2, int pos0,
