@@ -22,27 +22,37 @@ int tag(at::ScalarType t) {
   return t == at::kFloat ? (int)NB_F32 : t == at::kHalf ? (int)NB_F16 : t == at::kBFloat16 ? (int)NB_BF16 : -1;
 }
 
-// workspaces[(device, stream)], or nullptr.
-const at::Tensor* workspace(PyObject* workspaces, int device, void* stream) {
+// workspaces[(device, stream)], held for the call (another thread may replace the entry meanwhile), or an undefined tensor.
+at::Tensor workspace(PyObject* workspaces, int device, void* stream) {
   PyObject* key = Py_BuildValue("(iK)", device, (unsigned long long)(uintptr_t)stream);
-  if (!key) return nullptr;
+  if (!key) return {};
   PyObject* ws = PyDict_GetItemWithError(workspaces, key);        // borrowed
   Py_DECREF(key);
-  return ws && THPVariable_Check(ws) ? &THPVariable_Unpack(ws) : nullptr;
+  return ws && THPVariable_Check(ws) ? THPVariable_Unpack(ws) : at::Tensor();
 }
 
-// linear(x, packed, codebook, w_stream or None, n, k, bits, ordered, gemv workspaces, prefill workspaces) -> y or None
+// Whether a copy made of the tensors and versions in `of`, (packed, codebook, version, version), is one of these tensors as they are now.
+bool copy_of(PyObject* of, PyObject* packed, PyObject* codebook) {
+  if (!PyTuple_CheckExact(of) || PyTuple_GET_SIZE(of) != 4 || PyTuple_GET_ITEM(of, 0) != packed || PyTuple_GET_ITEM(of, 1) != codebook) return false;
+  for (int i = 0; i < 2; ++i) {
+    const at::Tensor& t = THPVariable_Unpack(PyTuple_GET_ITEM(of, i));
+    if (PyLong_AsLongLong(PyTuple_GET_ITEM(of, 2 + i)) != (t.is_inference() ? -1 : t._version())) return false;
+  }
+  return true;
+}
+
+// linear(x, packed, codebook, w_stream or None, what it was made of, n, k, bits, ordered, gemv workspaces, prefill workspaces) -> y or None
 PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
   HANDLE_TH_ERRORS
-  if (count != 10) {
-    PyErr_SetString(PyExc_TypeError, "linear takes ten arguments");
+  if (count != 11) {
+    PyErr_SetString(PyExc_TypeError, "linear takes eleven arguments");
     return nullptr;
   }
-  if (!THPVariable_CheckExact(a[0]) || !THPVariable_CheckExact(a[1]) || !THPVariable_CheckExact(a[2]) || !PyDict_Check(a[8]) || !PyDict_Check(a[9]))
+  if (!THPVariable_CheckExact(a[0]) || !THPVariable_CheckExact(a[1]) || !THPVariable_CheckExact(a[2]) || !PyDict_Check(a[9]) || !PyDict_Check(a[10]))
     Py_RETURN_NONE;
   const at::Tensor &x = THPVariable_Unpack(a[0]), &packed = THPVariable_Unpack(a[1]), &codebook = THPVariable_Unpack(a[2]);
-  const int64_t n = PyLong_AsLongLong(a[4]), k = PyLong_AsLongLong(a[5]);
-  const int bits = (int)PyLong_AsLong(a[6]), ordered = PyObject_IsTrue(a[7]);
+  const int64_t n = PyLong_AsLongLong(a[5]), k = PyLong_AsLongLong(a[6]);
+  const int bits = (int)PyLong_AsLong(a[7]), ordered = PyObject_IsTrue(a[8]);
   if (PyErr_Occurred()) return nullptr;
   const int xt = tag(x.scalar_type()), ct = tag(codebook.scalar_type());
   if (xt < 0 || (ct != NB_F16 && ct != NB_F32) || !x.is_cuda() || x.layout() != at::kStrided || x.dim() < 1 || x.size(-1) != k || !x.is_contiguous() ||
@@ -56,40 +66,41 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
   shape.back() = n;
   int rc = NB_ERR_ARG;
   if (m >= 2 && THPVariable_CheckExact(a[3]) && (m <= kGemvRows || nb_chain_takes((int)m, (int)n, (int)k, bits, xt))) {
-    const at::Tensor &w = THPVariable_Unpack(a[3]), *ws = workspace(a[9], device.index(), stream);
-    if (!ws || w.device() != device) Py_RETURN_NONE;
+    const at::Tensor &w = THPVariable_Unpack(a[3]), ws = workspace(a[10], device.index(), stream);
+    if (!ws.defined() || w.device() != device || !copy_of(a[4], a[1], a[2])) Py_RETURN_NONE;
     at::Tensor y = at::empty(shape, x.options().requires_grad(false).memory_format(c10::MemoryFormat::Contiguous));
     nb_chain_args args = {};
     args.w = static_cast<const uint8_t*>(w.const_data_ptr());
     args.x = x.const_data_ptr();
     args.y = y.mutable_data_ptr();
-    args.status = static_cast<int*>(ws->mutable_data_ptr());         // the workspace's head
+    args.status = static_cast<int*>(ws.mutable_data_ptr());         // the workspace's head
     args.M = (int)m; args.N = (int)n; args.K = (int)k; args.bits = bits;
     args.x_dtype = args.y_dtype = xt;
+    args.ordered = ordered;                                          // the copy of the weights may be as new as the launch before
     Py_BEGIN_ALLOW_THREADS
     rc = nb_chain_linear(&args, stream);
     Py_END_ALLOW_THREADS
     if (rc == NB_OK) return THPVariable_Wrap(std::move(y));
   } else if (m == 1) {
-    const at::Tensor* ws = workspace(a[8], device.index(), stream);
-    if (!ws) Py_RETURN_NONE;
+    const at::Tensor ws = workspace(a[9], device.index(), stream);
+    if (!ws.defined()) Py_RETURN_NONE;
     at::Tensor y = at::empty(shape, x.options().requires_grad(false).memory_format(c10::MemoryFormat::Contiguous));
     const void *xp = x.const_data_ptr(), *cp = codebook.const_data_ptr();
     const uint8_t* pp = static_cast<const uint8_t*>(packed.const_data_ptr());
-    void *yp = y.mutable_data_ptr(), *wp = ws->mutable_data_ptr();
-    const size_t wn = ws->nbytes();
+    void *yp = y.mutable_data_ptr(), *wp = ws.mutable_data_ptr();
+    const size_t wn = ws.nbytes();
     Py_BEGIN_ALLOW_THREADS
     rc = (ordered ? nb_gemv_ordered : nb_gemv)(xp, xt, (int)m, pp, cp, ct, bits, kBlock, (int)n, (int)k, yp, xt, wp, wn, stream);
     Py_END_ALLOW_THREADS
     if (rc == NB_OK) return THPVariable_Wrap(std::move(y));
   } else if (xt != NB_F16 && m * (xt == NB_F32 ? 2 : 1) <= kFusedRows && THPVariable_CheckExact(a[3])) {       // (that kernel writes bf16 or fp32)
-    const at::Tensor &w = THPVariable_Unpack(a[3]), *ws = workspace(a[9], device.index(), stream);
-    if (!ws || w.device() != device) Py_RETURN_NONE;
+    const at::Tensor &w = THPVariable_Unpack(a[3]), ws = workspace(a[10], device.index(), stream);
+    if (!ws.defined() || w.device() != device || !copy_of(a[4], a[1], a[2])) Py_RETURN_NONE;
     at::Tensor y = at::empty(shape, x.options().requires_grad(false).memory_format(c10::MemoryFormat::Contiguous));
     const void* xp = x.const_data_ptr();
     const uint8_t* pw = static_cast<const uint8_t*>(w.const_data_ptr());
-    void *yp = y.mutable_data_ptr(), *wp = ws->mutable_data_ptr();
-    const size_t wn = ws->nbytes();
+    void *yp = y.mutable_data_ptr(), *wp = ws.mutable_data_ptr();
+    const size_t wn = ws.nbytes();
     Py_BEGIN_ALLOW_THREADS
     rc = nb_gemm_prefill_fused(xp, xt, (int)m, pw, bits, (int)n, (int)k, yp, xt, wp, wn, stream);
     Py_END_ALLOW_THREADS

@@ -71,10 +71,10 @@ class PackedLinear(torch.nn.Module):
 
     def forward(self, x):
         if self.block_size == BS and x.is_cuda:      # the plain calls: checks, result and launch in one native function
-            y = _lib.bind().linear(x, self.packed_indices, self.codebook, self.__dict__.get("_wstream"), self.out_features, self.in_features,
-                                   self.bits, self._fresh, ops._workspaces, ops._prefill_ws)
+            y = _lib.bind().linear(x, self.packed_indices, self.codebook, self.__dict__.get("_wstream"), self.__dict__.get("_wstream_of"),
+                                   self.out_features, self.in_features, self.bits, self._fresh, ops._workspaces, ops._prefill_ws)
             if y is not None:
-                if self._fresh and y.numel() <= GEMV_MAX_M * self.out_features:
+                if self._fresh:
                     self._fresh = False
                 return y
         shape = x.shape
@@ -101,14 +101,22 @@ class PackedLinear(torch.nn.Module):
 
     def stream_weight(self, row_mode: int = 0):
         """Tile-major copy of the packed weight for the fused tensor-core kernel and the many-matrix / decode-chain
-        kernels (built on first use, kept with the module).  row_mode 1: this is a fused [gate | up] matrix and every
+        kernels (built on first use, kept with the module, made again after other weights were loaded).  row_mode 1: this is a fused [gate | up] matrix and every
         16-row tile holds 8 gate channels and the matching 8 up channels (for a SwiGLU epilogue)."""
         attr = "_wstream" if row_mode == 0 else "_wstream_rm1"
-        w = getattr(self, attr, None)
-        if w is None:
+        w, of = getattr(self, attr, None), self.__dict__.get(attr + "_of")
+        p, c = self.packed_indices, self.codebook
+        now = (p, c, -1 if p.is_inference() else p._version, -1 if c.is_inference() else c._version)
+        if w is None or of is not None and not (of[0] is p and of[1] is c and of[2:] == now[2:]):
             from .stream import stream_pack
-            w = stream_pack(self.packed_indices, self.codebook, self.bits, self.out_features, self.in_features, row_mode)
-            setattr(self, attr, w)
+            new = stream_pack(p, c, self.bits, self.out_features, self.in_features, row_mode)
+            if w is not None and w.device == new.device:
+                w.copy_(new)                # other weights were loaded: captured graphs hold this copy's address
+            else:
+                setattr(self, attr, new)
+                w = new
+            setattr(self, attr + "_of", now)
+            self._fresh = True              # the next launch must not start beside the packing
         return w
 
     def _forward_few(self, x_flat):
@@ -117,8 +125,11 @@ class PackedLinear(torch.nn.Module):
         16: 13.9 | 6.8; 1024 x 1024 bf16 16: 8.0 | 3.9.  One row (4.1 | 4.1) does not pay for a second copy of the weights."""
         if not self._tensor_cores() or x_flat.data_ptr() % 16:
             return None
-        fresh = getattr(self, "_wstream", None) is None
-        return ops.chain_rows(x_flat, self.stream_weight(), self.bits, self.out_features, self.in_features, ordered=fresh)
+        w = self.stream_weight()
+        y = ops.chain_rows(x_flat, w, self.bits, self.out_features, self.in_features, ordered=self._fresh)
+        if y is not None and self._fresh:
+            self._fresh = False
+        return y
 
     def _forward_many(self, x_flat):
         """M > 16 rows on the tcgen05 kernels (exact fp16 weights; bf16 and fp16 activations as given, fp32
@@ -165,10 +176,11 @@ class PackedLinear(torch.nn.Module):
         if terms.shape[0] > FUSED_MAX_ROWS:
             return ops.gemm_prefill(terms, self.packed_indices, self.codebook, self.bits, self.block_size, self.out_features, self.in_features,
                                     out_dtype=torch.float32, out=out, terms=True)
-        if getattr(self, "_wstream", None) is None:
-            self.stream_weight()
+        of = self.__dict__.get("_wstream_of")
+        w = self.stream_weight()
+        if self.__dict__.get("_wstream_of") is not of:
             terms = terms.clone()           # a launch between the packing and the GEMM, which starts beside the launch before it
-        return ops.gemm_prefill_fused(terms, self.stream_weight(), self.bits, self.out_features, self.in_features, out=out, terms=True)
+        return ops.gemm_prefill_fused(terms, w, self.bits, self.out_features, self.in_features, out=out, terms=True)
 
     def dequantized_weight(self, dtype=torch.float32):
         """The dense (out_features, in_features) weight; bit-exact gather of the codebook values."""

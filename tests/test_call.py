@@ -8,14 +8,14 @@ from nativebit_b200 import PackedLinear, _lib, ops
 def test_native_call_leaves_everything_else_to_the_general_path(built_lib):
     call = _lib.bind().linear
     x, p, c = torch.zeros(2, 128), torch.zeros(48, dtype=torch.uint8), torch.zeros(1, 8).half()
-    assert call(x, p, c, None, 1, 128, 3, True, {}, {}) is None                  # not on a GPU
-    assert call(x.int(), p, c, None, 1, 128, 3, True, {}, {}) is None
-    assert call(torch.nn.Parameter(x), p, c, None, 1, 128, 3, True, {}, {}) is None
-    assert call(None, p, c, None, 1, 128, 3, True, {}, {}) is None
+    assert call(x, p, c, None, None, 1, 128, 3, True, {}, {}) is None                  # not on a GPU
+    assert call(x.int(), p, c, None, None, 1, 128, 3, True, {}, {}) is None
+    assert call(torch.nn.Parameter(x), p, c, None, None, 1, 128, 3, True, {}, {}) is None
+    assert call(None, p, c, None, None, 1, 128, 3, True, {}, {}) is None
     with pytest.raises(TypeError):
         call(x, p, c)
     with pytest.raises(TypeError):
-        call(x, p, c, None, "n", 128, 3, True, {}, {})
+        call(x, p, c, None, None, "n", 128, 3, True, {}, {})
 
 
 def _general(lin, x):
@@ -69,3 +69,33 @@ def test_native_call_equals_the_general_path(built_lib, bits, dtype):
     for wrong in (big[:4], big[:4, :k].double(), big[:4, :k].int()):
         with pytest.raises(RuntimeError):
             lin(wrong)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 4, 16, 20, 300])
+def test_other_weights_are_what_the_next_call_multiplies(built_lib, rows):
+    n, k = 144, 256
+    g = torch.Generator(device="cuda").manual_seed(rows)
+
+    def weights():
+        idx = torch.randint(0, 8, (n * k,), dtype=torch.uint8, device="cuda", generator=g)
+        return ops.pack(idx, 3), torch.randn(n * k // 128, 8, device="cuda", generator=g).half()
+
+    first, second, third = weights(), weights(), weights()
+    lin = PackedLinear(first[0].clone(), first[1].clone(), n, k)
+    x = torch.randn(rows, k, device="cuda", generator=g)
+
+    def check(w):
+        for _ in range(3):
+            assert torch.equal(lin(x), PackedLinear(*w, n, k)(x))
+
+    lin.stream_weight()
+    check(first)
+    held = lin.stream_weight()
+    lin.load_state_dict({"packed_indices": second[0], "codebook": second[1]})
+    check(second)
+    lin.codebook = third[1]
+    check((second[0], third[1]))
+    lin.packed_indices = third[0]
+    check(third)
+    assert lin.stream_weight().data_ptr() == held.data_ptr()            # what a captured graph reads
