@@ -549,8 +549,8 @@ __global__ void __launch_bounds__(256) prompt_keys_kernel(const float* __restric
 // multiply-adds along the head dimension (12 loads per 64 of them at R = 8).  Values: the same thread owns its R queries x
 // 2 * NP head dimensions (pairs 16 apart) for every second four keys — eight lanes of a half-warp take the even fours, eight
 // the odd ones, and the halves meet once at the end — so the weights cross shared memory inside a half-warp only.
-// head_dim a multiple of 4, <= 128; NP pairs per thread cover 16 * NP >= head_dim.  Two CTAs share an SM: PK is 64 where
-// their tiles fit, else 32 (and for tiles of 16 queries, which are taken where 32 keys are all there are).
+// head_dim a multiple of 4, <= 128; NP pairs per thread cover 16 * NP >= head_dim.  Two CTAs share an SM.  PK is 64, and 32 for
+// tiles of 16 queries, which are taken where 32 keys are all there are.
 constexpr int prompt_pairs(int hd) { return hd <= 32 ? 2 : hd <= 64 ? 4 : hd <= 80 ? 5 : 8; }
 // Floats behind the values that the spare pairs of the last row read (and nobody uses): all 16 * NP dimensions of that row
 // end before the weights, which other warps are writing.
@@ -581,8 +581,8 @@ __device__ __forceinline__ void copy16_or_zero(float* dst, const float* src, boo
 
 // What bounds it: two warps per scheduler that wait for their own loads; 58 % of the multiply-add pipe's slots are used at eight
 // prompts of 512 tokens, 32 heads of 80 (333 us).  Two steps of the scores' loop in one put the second one's loads ahead of the first one's sums:
-// one prompt of 512 tokens 58.7 -> 51.3 us, eight of 500 with 16 heads of 128 306 -> 296; with 64 queries of heads of 80 the registers for
-// that are not there (333 -> 341), so that form takes one.  Three CTAs of 48 or 32 queries per SM: 361, 348.
+// one prompt of 512 tokens 58.7 -> 51.3 us, of 128 tokens 17.6 -> 15.7; with 64 queries of heads of 80 the registers for that are not
+// there (333 -> 341), so that form takes one.  Three CTAs of 48 or 32 queries per SM: 361, 348.
 template <int R, int PK, int NP>
 __global__ void __launch_bounds__(128, 2) prefill_attention_kernel(
     const float* __restrict__ qkv, const float* __restrict__ cos2, const float* __restrict__ sin2, const float* __restrict__ k_cache,
@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(128, 2) prefill_attention_kernel(
 
 template <int R, int NP, typename... Args>
 static int launch_prefill_attention(int B, int T, int H, int hd, cudaStream_t st, Args... args) {
-  constexpr int BQ = 8 * R, PK = R == 2 || (NP > 5 && R == 8) ? 32 : 64;
+  constexpr int BQ = 8 * R, PK = R == 2 ? 32 : 64;
   const size_t smem = (size_t)((BQ + 2 * PK) * (hd + 4) + kPromptSpare + BQ * (PK + 4)) * sizeof(float);      // <= 92 KB
   static bool attr_done[64] = {};
   int dev = 0;
@@ -762,12 +762,15 @@ static int launch_prefill_attention(int B, int T, int H, int hd, cudaStream_t st
 // Tiles of 64 queries stage every key half as often as tiles of 32; short or few prompts take the latter, which puts
 // twice as many SMs to work on them, and very short ones (one chunk of 32 keys in all) tiles of 16, whose padding and shared
 // memory are half of that again.  32 sequences x 32 heads of 80, 64 / 32 / 16 queries: 5 tokens 36.9 / 25.1 / 14.9 us,
-// 17 tokens 42.0 / 29.9 us; one sequence, 5 tokens 8.7 / 7.7 / 5.9 us.
+// 17 tokens 42.0 / 29.9 us; one sequence, 5 tokens 8.7 / 7.7 / 5.9 us.  Heads wider than 80 always take 32: with 64 only chunks of
+// 32 keys fit beside them.  64 | 32 queries: 8 x 500 tokens, 16 heads of 128 296 | 283, 1 x 4000, 8 of 128 1023 | 888, 16 x 200, 16 of
+// 128 171 | 139, 8 x 300, 8 of 88 68.7 | 55.1, 32 x 64, 8 of 128 25.2 | 25.2.
 template <int NP, typename... Args>
 static int prefill_attention_tile(int B, int T, int H, int hd, int pos0, cudaStream_t st, Args... args) {
   if (T <= 16 && pos0 + T <= 32) return launch_prefill_attention<2, NP>(B, T, H, hd, st, args...);
-  if (T <= 32 || (long long)B * H * ((T + 63) / 64) < 2 * sm_count()) return launch_prefill_attention<4, NP>(B, T, H, hd, st, args...);
-  return launch_prefill_attention<8, NP>(B, T, H, hd, st, args...);
+  if constexpr (NP <= 5)
+    if (T > 32 && (long long)B * H * ((T + 63) / 64) >= 2 * sm_count()) return launch_prefill_attention<8, NP>(B, T, H, hd, st, args...);
+  return launch_prefill_attention<4, NP>(B, T, H, hd, st, args...);
 }
 
 // The tied LM head of one sequence as a matvec over the bf16 embedding table, with the final residual add + RMSNorm
