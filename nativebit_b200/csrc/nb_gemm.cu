@@ -502,11 +502,13 @@ extern "C" int nb_gemm_prefill(const void* x, int x_dtype, int M, const uint8_t*
   if ((uintptr_t)x % 16) return NB_ERR_ALIGN;
   uint8_t* w = reinterpret_cast<uint8_t*>(workspace) + 256;
   uint8_t* xh = w + (((size_t)N * K * 2 + 255) & ~(size_t)255);
-  if (int rc = nb_dequant(packed, codebook, cb_dtype, bits, block_size, N, K, w, NB_F16, stream)) return rc;
-  if (x_dtype == NB_F16 || x_dtype == NB_F16_TERMS)
+  if (x_dtype == NB_F16 || x_dtype == NB_F16_TERMS) {
+    if (int rc = nb_dequant(packed, codebook, cb_dtype, bits, block_size, N, K, w, NB_F16, stream)) return rc;
     return gemm_16bit(x, w, 1, M, N, K, y, y_dtype, reinterpret_cast<int*>(workspace), stream, x_dtype == NB_F16_TERMS);
+  }
   // the conversion runs beside the dequantisation: it reads and writes nothing of its (a call with 2048 rows
   // x 6912 x 2560 78.2 -> 75.2 us, together with the wider stores of nb_dequant)
+  if (int rc = dequant_beside(packed, codebook, cb_dtype, bits, block_size, N, K, w, NB_F16, stream)) return rc;
   const size_t n8 = (size_t)M * K / 8;  // K % 64 == 0
   const dim3 grid((unsigned)((n8 + 255) / 256)), block(256);
   if (x_dtype == NB_F32) {  // two fp16 terms per element; rows 2i and 2i + 1 of the kernel's result are one row of 2K here

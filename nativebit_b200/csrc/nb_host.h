@@ -18,6 +18,10 @@ int check_device();
 // cudaGetLastError() after a launch -> status.
 int check_launch();
 
+// nb_dequant, but the launch behind it may run beside it: for one that neither reads the matrix nor ends before this has.
+int dequant_beside(const uint8_t* packed, const void* codebook, int cb_dtype, int bits, int block_size, int64_t n_rows, int64_t n_cols,
+                   void* w_out, int w_dtype, void* stream);
+
 // Number of SMs of the current device (cached per device).
 int sm_count();
 

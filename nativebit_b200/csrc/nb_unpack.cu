@@ -202,8 +202,8 @@ template <int BITS, typename T16> __device__ __forceinline__ void store_pair(T16
 template <int BITS, int PER, int W, typename OutT>
 __global__ void __launch_bounds__(kDqThreads) dequant16b_kernel(const uint32_t* __restrict__ packed, const __half* __restrict__ codebook,
                                                                int64_t n_stores, int64_t n_bytes, int64_t total, int block_size, int shift,
-                                                               OutT* __restrict__ out) {
-  asm volatile("griddepcontrol.launch_dependents;");        // a conversion behind this may run beside it
+                                                               OutT* __restrict__ out, bool beside) {
+  if (beside) asm volatile("griddepcontrol.launch_dependents;");
   constexpr int kT = BITS == 4 ? 8 : 4;
   const int64_t i0 = (int64_t)blockIdx.x * (kDqThreads * PER) + threadIdx.x;
   uint32_t sel[PER][W], e[PER][kT];
@@ -494,9 +494,11 @@ static int launch_quantize4(const float* w, int64_t total, int64_t padded, const
   return check_launch();
 }
 
+// beside: the launch behind may start before this one ends.  Only for a caller that knows that launch (dequant_beside): one that
+// reads the dequantised matrix ahead of its dependency wait, as the LM head reads its table, must not.
 template <typename OutT>
 static int dequant_dispatch(const uint8_t* packed, const void* codebook, int cb_dtype, int bits, int block_size,
-                            int64_t total, OutT* out, cudaStream_t st) {
+                            int64_t total, OutT* out, bool beside, cudaStream_t st) {
   const int64_t n_blocks = (total + block_size - 1) / block_size;
   const int64_t n_bytes = packed_bytes(n_blocks * block_size, bits);
   const bool aligned = ((uintptr_t)packed % 4 == 0) && ((uintptr_t)out % 16 == 0) && ((uintptr_t)codebook % 16 == 0);
@@ -509,7 +511,7 @@ static int dequant_dispatch(const uint8_t* packed, const void* codebook, int cb_
       const int64_t per = kDqThreads * (several ? kDqRuns : 1);
       auto run = [&](auto kernel) {
         kernel<<<(unsigned)((stores + 31 + per - 1) / per), kDqThreads, 0, st>>>((const uint32_t*)packed, (const __half*)codebook, stores, n_bytes, total,
-                                                                            block_size, shift, out);
+                                                                            block_size, shift, out, beside);
         return check_launch();
       };
       if (bits == 3) return several ? run(dequant16b_kernel<3, kDqRuns, W, OutT>) : run(dequant16b_kernel<3, 1, W, OutT>);
@@ -529,6 +531,27 @@ static int dequant_dispatch(const uint8_t* packed, const void* codebook, int cb_
   else
     dequant_generic_kernel<float, OutT><<<grid, 256, 0, st>>>(packed, n_bytes, (const float*)codebook, bits, block_size, total, out);
   return check_launch();
+}
+
+static int dequant_checked(const uint8_t* packed, const void* codebook, int cb_dtype, int bits, int block_size, int64_t n_rows,
+                           int64_t n_cols, void* w_out, int w_dtype, bool beside, void* stream) {
+  if (!packed || !codebook || !w_out || n_rows <= 0 || n_cols <= 0 || block_size <= 0) return NB_ERR_ARG;
+  if (bits != 2 && bits != 3 && bits != 4) return NB_ERR_ARG;
+  if (cb_dtype != NB_F16 && cb_dtype != NB_F32) return NB_ERR_ARG;
+  if (int rc = check_device()) return rc;
+  const int64_t total = n_rows * n_cols;
+  cudaStream_t st = (cudaStream_t)stream;
+  switch (w_dtype) {
+    case NB_F32: return dequant_dispatch<float>(packed, codebook, cb_dtype, bits, block_size, total, (float*)w_out, beside, st);
+    case NB_F16: return dequant_dispatch<__half>(packed, codebook, cb_dtype, bits, block_size, total, (__half*)w_out, beside, st);
+    case NB_BF16: return dequant_dispatch<__nv_bfloat16>(packed, codebook, cb_dtype, bits, block_size, total, (__nv_bfloat16*)w_out, beside, st);
+    default: return NB_ERR_ARG;
+  }
+}
+
+int dequant_beside(const uint8_t* packed, const void* codebook, int cb_dtype, int bits, int block_size, int64_t n_rows, int64_t n_cols,
+                   void* w_out, int w_dtype, void* stream) {
+  return dequant_checked(packed, codebook, cb_dtype, bits, block_size, n_rows, n_cols, w_out, w_dtype, true, stream);
 }
 
 }  // namespace nb
@@ -578,18 +601,7 @@ extern "C" int nb_pack(const uint8_t* idx, int bits, int64_t count, uint8_t* pac
 
 extern "C" int nb_dequant(const uint8_t* packed, const void* codebook, int cb_dtype, int bits, int block_size,
                           int64_t n_rows, int64_t n_cols, void* w_out, int w_dtype, void* stream) {
-  if (!packed || !codebook || !w_out || n_rows <= 0 || n_cols <= 0 || block_size <= 0) return NB_ERR_ARG;
-  if (bits != 2 && bits != 3 && bits != 4) return NB_ERR_ARG;
-  if (cb_dtype != NB_F16 && cb_dtype != NB_F32) return NB_ERR_ARG;
-  if (int rc = check_device()) return rc;
-  const int64_t total = n_rows * n_cols;
-  cudaStream_t st = (cudaStream_t)stream;
-  switch (w_dtype) {
-    case NB_F32: return dequant_dispatch<float>(packed, codebook, cb_dtype, bits, block_size, total, (float*)w_out, st);
-    case NB_F16: return dequant_dispatch<__half>(packed, codebook, cb_dtype, bits, block_size, total, (__half*)w_out, st);
-    case NB_BF16: return dequant_dispatch<__nv_bfloat16>(packed, codebook, cb_dtype, bits, block_size, total, (__nv_bfloat16*)w_out, st);
-    default: return NB_ERR_ARG;
-  }
+  return dequant_checked(packed, codebook, cb_dtype, bits, block_size, n_rows, n_cols, w_out, w_dtype, false, stream);
 }
 
 extern "C" int nb_quantize(const float* w, int64_t total, const void* codebook, int cb_dtype, int n_entries, int block_size,
