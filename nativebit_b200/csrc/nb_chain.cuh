@@ -13,10 +13,11 @@ __device__ __forceinline__ uint8_t* chain_term(uint8_t* terms, int bpr, int row,
   return terms + ((size_t)(2 * row + s) * bpr + (n >> 7)) * 256 + ((n >> 5) & 3) * 64 + ((((n >> 3) & 3) ^ ((n >> 5) & 3) ^ s) << 4) +
          ((n & 4) | (n & 1) << 1 | (n >> 1 & 1)) * 2;
 }
+// Saturating like every split into terms here, and NaN stays NaN in both: it has to come out of the products behind.
 __device__ __forceinline__ void store_chain_terms(uint8_t* terms, int bpr, int row, int n, float v) {
-  const __half hi = to_half_clamped(v);
+  const __half hi = to_half_sat(v);
   *reinterpret_cast<__half*>(chain_term(terms, bpr, row, 0, n)) = hi;
-  *reinterpret_cast<__half*>(chain_term(terms, bpr, row, 1, n)) = to_half_clamped(v - __half2float(hi));
+  *reinterpret_cast<__half*>(chain_term(terms, bpr, row, 1, n)) = to_half_sat(v - __half2float(hi));
 }
 
 }  // namespace nb

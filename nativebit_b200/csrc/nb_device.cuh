@@ -250,8 +250,9 @@ __device__ __forceinline__ uint32_t f32x2_to_f16x2_sat(float a, float b) {
   return d;
 }
 
-__device__ __forceinline__ __half to_half_clamped(float v) {
-  return __float2half_rn(fminf(fmaxf(v, -65504.f), 65504.f));
+// Round to nearest, saturating to +-65504; NaN stays NaN.
+__device__ __forceinline__ __half to_half_sat(float v) {
+  return __ushort_as_half((unsigned short)(f32x2_to_f16x2_sat(v, 0.f) & 0xFFFFu));
 }
 
 }  // namespace nb

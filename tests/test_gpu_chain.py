@@ -130,3 +130,44 @@ def test_chain_rows_takes_plain_activations(built_lib, n, k, m, dtype, bits):
     assert y.dtype == dtype
     # a rounding of the result to nearest is at most half an ulp (2^-11, 2^-8) of each value
     _close(y, want, {torch.float32: REL, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[dtype])
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), 1e5])
+def test_what_is_no_number_reaches_the_products_behind(built_lib, value):
+    """gate | up -> down and attention -> out_proj hand their rows over as terms: NaN arrives in every output of its row, what fp16
+    does not hold arrives as the largest two terms, and other rows are as they were."""
+    m, c, f, bits = 3, 256, 512, 3
+    g = torch.Generator(device=DEV).manual_seed(5)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    gu, gu_dense = _matrix(2 * f, c, bits, 1, row_mode=1)
+    down, dense = _matrix(c, f, bits, 2)
+    torch.cuda.synchronize()
+    x = torch.randn(m, c, device=DEV, generator=g)
+    x[1, 5] = value if value != value else 60000.0
+    h = ops.chain_terms(m, f, DEV)
+    ops.chain_linear(ops.CHAIN_SWIGLU, gu, bits, m, 2 * f, c, _terms(x), status, y_terms=h)
+    y = torch.zeros(m, c, device=DEV)
+    ops.chain_linear(ops.CHAIN_RESIDUAL, down, bits, m, c, f, h, status, residual=y)
+    z = x.double() @ gu_dense.T
+    want = (torch.nn.functional.silu(z[:, :f]) * z[:, f:]).clamp(-131008, 131008) @ dense.T
+    assert torch.equal(y.isnan(), torch.tensor([False, value != value, False], device=DEV)[:, None].expand(m, c))
+    _close(y[[0, 2]], want[[0, 2]], 4 * REL)
+    if value == value:                                   # beyond 65504 the second term is up to 65504 itself, with an error of up to 16
+        _close(y[1], want[1], 2.0 ** -12)
+
+    heads, hd, ctx = 2, 64, 16                           # 128 columns of attention in front of an out_proj
+    out, out_dense = _matrix(256, heads * hd, bits, 3)
+    torch.cuda.synchronize()
+    k, v = (torch.randn(m, heads, ctx, hd, device=DEV, generator=g) for _ in range(2))
+    v[1, :, 2] = value
+    cos2, sin2 = torch.ones(ctx, hd, device=DEV), torch.zeros(ctx, hd, device=DEV)
+    qkv, pos = torch.randn(m, 3 * heads * hd, device=DEV, generator=g), torch.tensor([7], device=DEV)
+    terms, plain = ops.chain_terms(m, heads * hd, DEV), torch.zeros(m, heads * hd, device=DEV)
+    ops.decode_attention_rope(qkv, cos2, sin2, pos, k, v, plain, 0)
+    ops.decode_attention_terms(qkv, cos2, sin2, pos, k, v, terms, heads * hd, 0)
+    y = torch.zeros(m, 256, device=DEV)
+    ops.chain_linear(ops.CHAIN_RESIDUAL, out, bits, m, 256, heads * hd, terms, status, residual=y)
+    assert torch.equal(y.isnan(), plain.isnan().any(1, keepdim=True).expand(m, 256))
+    _close(y[[0, 2]], plain[[0, 2]].double() @ out_dense.T, REL)
+    if value == value:
+        _close(y[1], plain[1].double().clamp(-131008, 131008) @ out_dense.T, 2.0 ** -12)
