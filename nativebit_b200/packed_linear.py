@@ -49,6 +49,57 @@ def dequant_matvec(x, indices, codebook, N, K, tile_n=TILE_N):
     return dequant_matvec_3bit(x, packed, codebook, N, K)
 
 
+COPIES = ("_wstream", "_wstream_rm1")          # by row mode
+
+
+def _version(t: torch.Tensor) -> int:
+    return -1 if t.is_inference() else t._version
+
+
+def capturing(device: torch.device) -> bool:
+    if device.type != "cuda":
+        return False
+    with torch.cuda.device(device):
+        return torch.cuda.is_current_stream_capturing()
+
+
+def make_copies(wanted) -> None:
+    """Makes the stream-layout copies (linear, row mode) that are missing or of other weights than the linear's present ones, and
+    waits for them: whatever thread or stream finds a copy, it is complete.  Copies that are made again stay at their place, which
+    captured graphs hold, after everything that was launched over them; both copies of a linear are made again together, so that
+    no step meets one of old and one of new weights."""
+    from .stream import stream_pack
+    todo: dict = {}
+    for lin, row_mode in wanted:
+        have, now = lin.__dict__, lin._copied_now()
+        for mode, name in enumerate(COPIES):
+            if (mode == row_mode or have.get(name) is not None) and not (now and have.get(name) is not None):
+                todo[id(lin), mode] = (lin, mode)
+    made, of = [], {}
+    for lin, mode in todo.values():
+        p, c = lin.packed_indices, lin.codebook
+        of.setdefault(lin, (p, c, _version(p), _version(c)))
+        made.append((lin, COPIES[mode], stream_pack(p, c, lin.bits, lin.out_features, lin.in_features, mode)))
+    for device in {w.device for _, _, w in made}:
+        _finish(device, any(w.device == device and lin.__dict__.get(name) is not None for lin, name, w in made))
+    for lin, name, w in made:
+        old = lin.__dict__.get(name)
+        if old is not None and old.device == w.device and old.shape == w.shape:
+            old.copy_(w)
+        else:
+            setattr(lin, name, w)
+    for device in {w.device for _, _, w in made}:
+        _finish(device, False)
+    for lin, key in of.items():
+        lin._wstream_of = key
+
+
+def _finish(device: torch.device, everything: bool) -> None:
+    """Waits for what the current stream, or the whole device, has been given."""
+    if device.type == "cuda":
+        torch.cuda.synchronize(device) if everything else torch.cuda.current_stream(device).synchronize()
+
+
 class PackedLinear(torch.nn.Module):
     """Drop-in for nn.Linear over NativeBit packed weights (inference/triton_kernel.py:223-286).
 
@@ -101,23 +152,27 @@ class PackedLinear(torch.nn.Module):
 
     def stream_weight(self, row_mode: int = 0):
         """Tile-major copy of the packed weight for the fused tensor-core kernel and the many-matrix / decode-chain
-        kernels (built on first use, kept with the module, made again after other weights were loaded).  row_mode 1: this is a fused [gate | up] matrix and every
-        16-row tile holds 8 gate channels and the matching 8 up channels (for a SwiGLU epilogue)."""
-        attr = "_wstream" if row_mode == 0 else "_wstream_rm1"
-        w, of = getattr(self, attr, None), self.__dict__.get(attr + "_of")
-        p, c = self.packed_indices, self.codebook
-        now = (p, c, -1 if p.is_inference() else p._version, -1 if c.is_inference() else c._version)
-        if w is None or of is not None and not (of[0] is p and of[1] is c and of[2:] == now[2:]):
+        kernels: made on first use, kept with the module at one place in memory, made again after other weights were loaded or
+        assigned (not after writes that PyTorch does not count: through `.data`, or to inference tensors).  row_mode 1: this is a fused
+        [gate | up] matrix and every 16-row tile holds 8 gate channels and the matching 8 up channels (for a SwiGLU epilogue)."""
+        w = self._copy(row_mode)
+        if w is None:                       # under capture: the graph's own copy, packed by every replay
             from .stream import stream_pack
-            new = stream_pack(p, c, self.bits, self.out_features, self.in_features, row_mode)
-            if w is not None and w.device == new.device:
-                w.copy_(new)                # other weights were loaded: captured graphs hold this copy's address
-            else:
-                setattr(self, attr, new)
-                w = new
-            setattr(self, attr + "_of", now)
-            self._fresh = True              # the next launch must not start beside the packing
+            w = stream_pack(self.packed_indices, self.codebook, self.bits, self.out_features, self.in_features, row_mode)
         return w
+
+    def _copy(self, row_mode: int = 0):
+        """stream_weight, but None under capture where the copy would have to be made."""
+        if not self._copied_now() or self.__dict__.get(COPIES[row_mode]) is None:
+            if capturing(self.packed_indices.device):
+                return None
+            make_copies([(self, row_mode)])
+        return self.__dict__[COPIES[row_mode]]
+
+    def _copied_now(self) -> bool:
+        """Whether the copies are of the weights as they are now."""
+        of = self.__dict__.get("_wstream_of")
+        return of is not None and of[0] is self.packed_indices and of[1] is self.codebook and of[2:] == (_version(of[0]), _version(of[1]))
 
     def _forward_few(self, x_flat):
         """2 to 16 rows against the stream-layout copy of the weights, None where that does not take them.  From a graph over cold
@@ -125,11 +180,8 @@ class PackedLinear(torch.nn.Module):
         16: 13.9 | 6.8; 1024 x 1024 bf16 16: 8.0 | 3.9.  One row (4.1 | 4.1) does not pay for a second copy of the weights."""
         if not self._tensor_cores() or x_flat.data_ptr() % 16:
             return None
-        w = self.stream_weight()
-        y = ops.chain_rows(x_flat, w, self.bits, self.out_features, self.in_features, ordered=self._fresh)
-        if y is not None and self._fresh:
-            self._fresh = False
-        return y
+        w = self._copy()
+        return None if w is None else ops.chain_rows(x_flat, w, self.bits, self.out_features, self.in_features)
 
     def _forward_many(self, x_flat):
         """M > 16 rows on the tcgen05 kernels (exact fp16 weights; bf16 and fp16 activations as given, fp32
@@ -140,7 +192,7 @@ class PackedLinear(torch.nn.Module):
             return y
         if self._tensor_cores():
             rows = x_flat.shape[0] * (2 if x_flat.dtype == torch.float32 else 1)
-            if rows > FUSED_MAX_ROWS:
+            if rows > FUSED_MAX_ROWS or (w := self._copy()) is None:
                 # long inputs: dequantising W once into a scratch copy (8.8 us for 6912 x 2560) and running the plain
                 # tensor-core kernel, against dequantising every weight tile once per 256 operand rows.  6912 x 2560, fused |
                 # two passes (us): bf16 512 rows 30.0 | 31.8, 1024 45 | 42, 2048 71 | 67; fp32 512 rows 37 | 44, 1024 59 | 68, 2048
@@ -148,7 +200,7 @@ class PackedLinear(torch.nn.Module):
                 # up to there the line is early for them by up to a seventh.
                 return ops.gemm_prefill(x_flat, self.packed_indices, self.codebook, self.bits, self.block_size,
                                         self.out_features, self.in_features, out_dtype=x_flat.dtype)
-            return ops.gemm_prefill_fused(x_flat, self.stream_weight(), self.bits, self.out_features, self.in_features,
+            return ops.gemm_prefill_fused(x_flat, w, self.bits, self.out_features, self.in_features,
                                           out_dtype=x_flat.dtype)
         wdt = x_flat.dtype if x_flat.dtype in (torch.float16, torch.bfloat16) else torch.float32
         w = ops.dequant(self.packed_indices, self.codebook, self.bits, self.block_size,
@@ -173,13 +225,9 @@ class PackedLinear(torch.nn.Module):
         """fp32 (M, out_features) of M fp32 rows given as their two fp16 terms, (2M, in_features); see ops.add_rmsnorm_terms."""
         if not self._tensor_cores():
             raise RuntimeError(f"forward_terms needs 2 to 4 bits, blocks of {BS} and a multiple of {BS} columns: {self.extra_repr()}")
-        if terms.shape[0] > FUSED_MAX_ROWS:
+        if terms.shape[0] > FUSED_MAX_ROWS or (w := self._copy()) is None:
             return ops.gemm_prefill(terms, self.packed_indices, self.codebook, self.bits, self.block_size, self.out_features, self.in_features,
                                     out_dtype=torch.float32, out=out, terms=True)
-        of = self.__dict__.get("_wstream_of")
-        w = self.stream_weight()
-        if self.__dict__.get("_wstream_of") is not of:
-            terms = terms.clone()           # a launch between the packing and the GEMM, which starts beside the launch before it
         return ops.gemm_prefill_fused(terms, w, self.bits, self.out_features, self.in_features, out=out, terms=True)
 
     def dequantized_weight(self, dtype=torch.float32):

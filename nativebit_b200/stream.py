@@ -64,6 +64,7 @@ def stream_pack(packed: torch.Tensor, codebook: torch.Tensor, bits: int, n: int,
     with torch.cuda.device(packed.device):
         _lib.check(l.nb_stream_pack(packed.data_ptr(), codebook.data_ptr(), _DT[codebook.dtype], bits, n, k, row_mode,
                                     out.data_ptr(), ops._stream()), "nb_stream_pack")
+        torch.zeros(1, device=packed.device)      # a launch in between: the kernels behind read weights ahead of the end of the launch in front
     return out
 
 
@@ -173,12 +174,13 @@ def stream_weights(model) -> list[dict]:
     cached = getattr(model, "_stream_weights", None)
     if cached is not None:
         return cached
+    from .packed_linear import make_copies
+    make_copies([(lin, int(lin is blk.gate_up)) for blk in model.blocks for lin in (blk.qkv, blk.out_proj, blk.gate_up, blk.down)])
     out = []
     for blk in model.blocks:
         d = {name: getattr(blk, name).stream_weight() for name in ("qkv", "out_proj", "down")}   # shared with the prefill kernel
         d["gate_up"] = blk.gate_up.stream_weight(1)
         out.append(d)
-    torch.cuda.synchronize(model.embedding.device)
     model._stream_weights = out
     return out
 
@@ -217,6 +219,8 @@ class MatvecGroup:
         if len(items) > int(l.nb_group_max_items()):
             raise RuntimeError(f"at most {int(l.nb_group_max_items())} matvecs per launch")
         bits = items[0][0].bits
+        from .packed_linear import make_copies
+        make_copies([(lin, 0) for lin, _, _ in items if lin.block_size == 128 and lin.bits == bits])
         arr = (GroupItem * len(items))()
         self.keep = []
         for i, (lin, x, out) in enumerate(items):

@@ -3,7 +3,7 @@ under capture."""
 import pytest
 import torch
 
-from nativebit_b200 import ops
+from nativebit_b200 import PackedLinear, ops
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -30,3 +30,52 @@ def test_a_table_dequantised_a_launch_ago_is_what_the_head_reads(built_lib):
         del table                                     # the next one takes its memory
         table = ops.dequant(packed, cb, 3, 128, (v, c), torch.bfloat16)
         assert torch.equal(head(table), want)
+
+
+def _weights(n, k, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return (ops.pack(torch.randint(0, 8, (n * k,), dtype=torch.uint8, device=DEV, generator=g), 3),
+            torch.randn(n * k // 128, 8, device=DEV, generator=g).half())
+
+
+@pytest.mark.parametrize("rows,n,k", [(4, 6912, 2560), (40, 1024, 1024), (100, 6912, 2560)])
+def test_a_linear_that_several_streams_ask_first(built_lib, rows, n, k):
+    """The first calls, one behind the other on two streams, then on both after other weights were loaded."""
+    torch.cuda.synchronize()
+    w, other = _weights(n, k, 1), _weights(n, k, 2)
+    x = torch.randn(rows, k, device=DEV, generator=torch.Generator(device=DEV).manual_seed(3))
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for load in (None, other):
+        want = PackedLinear(*(load or w), n, k)(x)
+        if load is None:
+            lin = PackedLinear(w[0].clone(), w[1].clone(), n, k)
+        else:
+            lin.load_state_dict({"packed_indices": load[0], "codebook": load[1]})
+        torch.cuda.synchronize()
+        got = []
+        for s in streams:
+            with torch.cuda.stream(s):
+                got.append(lin(x))
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, want) for y in got)
+
+
+@pytest.mark.parametrize("rows", [4, 40, 100])
+def test_a_linear_whose_first_call_of_many_rows_is_captured(built_lib, rows):
+    """The graph that would have to make the copy leaves none behind: calls before and after its replay are right, and so is it."""
+    n, k = 2560, 1024
+    w = _weights(n, k, 4)
+    g = torch.Generator(device=DEV).manual_seed(5)
+    x, big = torch.randn(rows, k, device=DEV, generator=g), torch.randn(300, k, device=DEV, generator=g)
+    want = PackedLinear(*w, n, k)(x).double()
+    lin = PackedLinear(*w, n, k)
+    lin(x[:1])
+    PackedLinear(*w, n, k)(big.repeat(4, 1))                  # the workspaces are there
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = lin(x)
+    assert not lin._copied_now() or rows <= 16
+    eager = lin(x)
+    graph.replay()
+    for got in (y, eager, lin(x)):                            # sums of other kernels in fp32: a few 2^-24 of the norm
+        assert (got.double() - want).norm() <= 2e-6 * want.norm()
