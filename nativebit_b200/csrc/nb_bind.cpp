@@ -33,12 +33,31 @@ at::Tensor workspace(PyObject* workspaces, int device, void* stream) {
 
 // Whether a copy made of the tensors and versions in `of`, (packed, codebook, version, version), is one of these tensors as they are now.
 bool copy_of(PyObject* of, PyObject* packed, PyObject* codebook) {
-  if (!PyTuple_CheckExact(of) || PyTuple_GET_SIZE(of) != 4 || PyTuple_GET_ITEM(of, 0) != packed || PyTuple_GET_ITEM(of, 1) != codebook) return false;
+  if (!packed || !codebook || !PyTuple_CheckExact(of) || PyTuple_GET_SIZE(of) != 4 ||
+      PyTuple_GET_ITEM(of, 0) != packed || PyTuple_GET_ITEM(of, 1) != codebook)
+    return false;
   for (int i = 0; i < 2; ++i) {
     const at::Tensor& t = THPVariable_Unpack(PyTuple_GET_ITEM(of, i));
     if (PyLong_AsLongLong(PyTuple_GET_ITEM(of, 2 + i)) != (t.is_inference() ? -1 : t._version())) return false;
   }
   return true;
+}
+
+// all_current([(a module's buffers, what its copy was made of), ..]) -> whether every copy is of the module's present weights
+PyObject* all_current(PyObject*, PyObject* list) {
+  HANDLE_TH_ERRORS
+  if (!PyList_Check(list)) {
+    PyErr_SetString(PyExc_TypeError, "all_current takes a list");
+    return nullptr;
+  }
+  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(list); ++i) {
+    PyObject* item = PyList_GET_ITEM(list, i);
+    if (!PyTuple_CheckExact(item) || PyTuple_GET_SIZE(item) != 2 || !PyDict_Check(PyTuple_GET_ITEM(item, 0))) Py_RETURN_FALSE;
+    PyObject* buffers = PyTuple_GET_ITEM(item, 0);
+    if (!copy_of(PyTuple_GET_ITEM(item, 1), PyDict_GetItemString(buffers, "packed_indices"), PyDict_GetItemString(buffers, "codebook"))) Py_RETURN_FALSE;
+  }
+  Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
 }
 
 // linear(x, packed, codebook, w_stream or None, what it was made of, n, k, bits, ordered, gemv workspaces, prefill workspaces) -> y or None
@@ -111,7 +130,8 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
   END_HANDLE_TH_ERRORS
 }
 
-PyMethodDef methods[] = {{"linear", (PyCFunction)(void (*)(void))linear, METH_FASTCALL, nullptr}, {nullptr, nullptr, 0, nullptr}};
+PyMethodDef methods[] = {{"linear", (PyCFunction)(void (*)(void))linear, METH_FASTCALL, nullptr}, {"all_current", all_current, METH_O, nullptr},
+                         {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_bind", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -24,8 +24,8 @@ import numpy as np
 import torch
 import torch.nn.functional as F
 
-from . import ops, synthetic, tp
-from .packed_linear import PackedLinear
+from . import _lib, ops, synthetic, tp
+from .packed_linear import COPIES, PackedLinear, capturing, make_copies
 from .session import Session
 
 
@@ -395,6 +395,7 @@ class DecodeSession(Session):
             if not _stream.stream_supported(model, batch_size):
                 raise RuntimeError("the one-launch decode step needs batch 1, one rank, bf16 embeddings and block-128 codebooks")
         self.prog = None
+        self._copied = []                     # (a linear's buffers, what its copies were made of), as of the last capture
         self.batch_gemm = batch_gemm          # kept for compatibility: batches above 16 rows always take the tensor-core kernel
         dev = self.dev
         self.caches = init_kv_cache(model, batch_size, dev)
@@ -438,6 +439,31 @@ class DecodeSession(Session):
             ops.gemv(x[r:r + 16], lin.packed_indices, lin.codebook, lin.bits, lin.block_size, lin.out_features,
                      lin.in_features, out=out[r:r + 16])
 
+    def _linears(self) -> list[tuple[PackedLinear, bool]]:
+        """The packed linears of the model, and whether they are gate and up."""
+        return [(lin, lin is blk.gate_up) for blk in self.model.blocks for lin in (blk.qkv, blk.out_proj, blk.gate_up, blk.down)
+                if isinstance(lin, PackedLinear)]
+
+    def _make_step_copies(self) -> None:
+        """What a step reads of the stream-layout copies, made in one go ahead of it."""
+        rows = self.tile_gemv or self.tile_rows or self.chain
+        gated = rows and self.swiglu_epilogue and (self.chain or getattr(self.model, "exchange", None) is None)
+        if (rows or self.B > 16) and not capturing(self.dev):
+            make_copies([(lin, int(gated and gate_up)) for lin, gate_up in self._linears() if lin.in_features % 128 == 0])
+
+    def _copied_linears(self) -> list[tuple[dict, tuple]]:
+        return [(lin._buffers, lin._wstream_of) for lin, _ in self._linears() if "_wstream_of" in lin.__dict__]
+
+    def _on_capture(self) -> None:
+        self._copied = self._copied_linears()
+
+    def _on_prompt(self) -> None:
+        """Captured prompts and steps replay over copies of the weights: where some are of weights that were replaced, all are made
+        again before either runs."""
+        if self._copied and not _lib.bind().all_current(self._copied) and not capturing(self.dev):
+            make_copies([(lin, mode) for lin, _ in self._linears() for mode, name in enumerate(COPIES) if name in lin.__dict__])
+            self._copied = self._copied_linears()
+
     def _chain_layers(self) -> torch.Tensor:
         """The layers of a step through nb_chain_linear, five launches each: q | k | v, attention, out_proj, gate and up, down.
         Returns the residual stream behind the last layer."""
@@ -474,6 +500,7 @@ class DecodeSession(Session):
         of three linears, a conversion in front of out_proj, a sum behind every linear whose k range is split)."""
         m, cfg = self.model, self.model.config
         eps = cfg.norm_eps
+        self._make_step_copies()
         fold = self.B <= 8
         xch = getattr(m, "exchange", None) if fold else None     # all-reduces folded into the GEMVs
         xa, xb = self.bx, self.bx2                                # residual stream, ping-pong

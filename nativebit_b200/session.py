@@ -45,6 +45,12 @@ class Session:
     def _on_reset(self) -> None:
         """Gives back what the finished sequences hold."""
 
+    def _on_prompt(self) -> None:
+        """In front of a prompt or a portion of one: other weights may have been loaded since the last."""
+
+    def _on_capture(self) -> None:
+        """Right after a capture."""
+
     def check(self) -> None:
         """Raises if a bounded wait inside one of the kernels ever ran out."""
 
@@ -68,6 +74,7 @@ class Session:
         if prompt.shape[1] > self.context_len:
             raise RuntimeError(f"prompt of {prompt.shape[1]} tokens exceeds the context of {self.context_len}")
         T = int(prompt.shape[1])
+        self._on_prompt()
         if not self.use_graph or not prompt.is_cuda:
             self._prefill_body(prompt)
         else:
@@ -85,6 +92,7 @@ class Session:
                     with torch.cuda.graph(g, stream=self.stream):
                         self._prefill_body(static_in)
                     self._keep_scratch()
+                    self._on_capture()
                 cur.wait_stream(self.stream)
                 self._prefill_graphs[T] = (g, static_in)
             else:
@@ -109,6 +117,7 @@ class Session:
             self.token.copy_(tokens)
             self.step()
             return self.logits[:, None, :].expand(-1, len(want), -1)
+        self._on_prompt()
         out = self._extend_body(tokens, want)
         self.pos_host += T
         self.pos.fill_(self.pos_host)
@@ -140,6 +149,7 @@ class Session:
                 with torch.cuda.graph(self.graph, stream=self.stream):
                     self._step_body()
                 self._keep_scratch()
+                self._on_capture()
                 # the capture does not execute: state is unchanged; stale cache slots past `pos` are masked
             torch.cuda.current_stream().wait_stream(self.stream)
         self.graph.replay()

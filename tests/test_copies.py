@@ -65,3 +65,23 @@ def test_a_graph_that_is_captured_makes_no_copy_for_others(packing, monkeypatch)
     w = lin.stream_weight()
     monkeypatch.setattr(packed_linear, "capturing", lambda device: True)
     assert lin._copy() is w
+
+
+def test_native_check_of_many_copies(packing, built_lib):
+    from nativebit_b200 import _lib
+    lins = [_linear(i) for i in range(3)]
+    make_copies([(lin, 0) for lin in lins])
+    held = [(lin._buffers, lin._wstream_of) for lin in lins]
+    assert _lib.bind().all_current(held) and _lib.bind().all_current([])
+    lins[1].packed_indices.add_(1)
+    assert not _lib.bind().all_current(held)
+    make_copies([(lin, 0) for lin in lins])
+    assert not _lib.bind().all_current(held)                                  # as of the old ones
+    held = [(lin._buffers, lin._wstream_of) for lin in lins]
+    assert _lib.bind().all_current(held)
+    lins[2].codebook = lins[2].codebook.clone()
+    assert not _lib.bind().all_current(held)
+    for wrong in ([1], [(1, 2)], [({}, ())], [({}, held[0][1])]):
+        assert not _lib.bind().all_current(wrong)
+    with pytest.raises(TypeError):
+        _lib.bind().all_current(None)

@@ -79,3 +79,30 @@ def test_a_linear_whose_first_call_of_many_rows_is_captured(built_lib, rows):
     graph.replay()
     for got in (y, eager, lin(x)):                            # sums of other kernels in fp32: a few 2^-24 of the norm
         assert (got.double() - want).norm() <= 2e-6 * want.norm()
+
+
+@pytest.mark.parametrize("batch", [1, 4])
+def test_sessions_follow_other_weights_from_the_next_prompt_on(built_lib, batch):
+    """After other weights were loaded under captured prompts and steps, a prompt of a known and one of a new length and the steps behind
+    them are those of a session made with these weights."""
+    from nativebit_b200 import generate as G
+    cfg = G.ModelConfig(vocab_size=512, n_layers=2, n_embd=256, n_head=4, ffn_hidden=512, context_len=64)
+    model, other = G.PackedGPT.random_init(cfg, seed=0), G.PackedGPT.random_init(cfg, seed=1)
+    g = torch.Generator(device=DEV).manual_seed(6)
+    prompts = [torch.randint(0, 512, (batch, t), device=DEV, generator=g) for t in (20, 20, 33)]
+
+    def run(session, prompt):
+        out = [session.prefill(prompt).clone()]
+        for _ in range(3):
+            session.token.fill_(7)
+            session.step()
+            out.append(session.logits.clone())
+        return torch.stack(out)
+
+    session = model.session(batch)
+    run(session, prompts[0])
+    model.load_state_dict(other.state_dict())
+    for prompt in prompts[1:]:
+        assert torch.equal(run(session, prompt), run(other.session(batch), prompt))
+    for a, b in zip(model.blocks, other.blocks):
+        assert torch.equal(a.gate_up.stream_weight(1), b.gate_up.stream_weight(1)) and torch.equal(a.qkv.stream_weight(), b.qkv.stream_weight())
