@@ -16,7 +16,8 @@
 //    of all of them and pushes its parts into the shared memory of the CTA that finishes the tile.
 //  * Column 2r + s of the MMAs carries term s of activation row r: one product covers four fp32 rows.
 // Decode step of the 2.2B decoder with 12 layers (us), matvecs that stage the rows themselves -> this: 1 sequence 437 -> 388, 2:
-// 539 -> 443, 8: 665 -> 510, 16 (a matvec over the packed bytes and launches between): 1523 -> 913.  17 and more rows stay on
+// 539 -> 443, 8: 665 -> 510, 16 (a matvec over the packed bytes and launches between): 1523 -> 934, whose rows are given plainly and normed before they are
+// split (857 with terms, which keep fewer bits of small rows).  17 and more rows stay on
 // the tcgen05 kernel (32: 1121, here 1460).  For one sequence a layer's 28 us are four times 1.3 us from the end of a launch
 // to the next one's first dependent instruction, 12.5 us of products (66 clocks per unit and SM against 54 without copies; down
 // projections wait for the 12 SMs with two tiles), 4.4 us of attention and the rest staging and sums.  Measured and not kept:
@@ -61,11 +62,12 @@ struct ChainParams {
   uint8_t* yt;                // the other two: terms of the next linear's activations (null: none)
   float* res;                 // NB_CHAIN_RESIDUAL: (M, N), updated in place
   const float* w_next;        // ... the next norm's weight
-  float* ss_out;              // ... (M, N / 16) partial sums of squares of the new rows
+  float* ss_out;              // ... (M, N / 16) partial sums of squares of the new rows (null: none)
   const uint8_t* ahead;       // weights of the launch behind (null: none), `ahead_step` bytes per CTA
   int* status;
   unsigned ahead_bytes, ahead_step;
   const void* x;              // plain activations (M, K) of type x_dtype instead of the terms (null: none)
+  const float* x_weight;      // ... with ss: the weight of their norm
   int x_dtype, y_dtype;
   int N, bpr, M, mode, ss_n;
   float eps;
@@ -112,6 +114,15 @@ __device__ __forceinline__ void st_cluster_f32(uint32_t local, uint32_t rank, fl
   uint32_t remote;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
+}
+
+// 1 / rms of row `r` from its partial sums, by a whole warp, in a fixed order: the same bits in every CTA.
+__device__ __forceinline__ float row_scale(const ChainParams& p, int r, int lane) {
+  const float* sq = p.ss + (size_t)r * p.ss_n;
+  float s = 0.f;
+#pragma unroll 6
+  for (int q = lane; q < p.ss_n; q += 32) s += __ldcg(sq + q);
+  return 1.0f / sqrtf(warp_sum(s) / (float)(p.bpr * kBlock) + p.eps);
 }
 
 // Shared memory: the CTA's units, tile after tile | staged columns (XT m_part of kc_max * 256 bytes) | partial
@@ -162,7 +173,8 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
   if (XT == 1 || p.x) {                                     // converted here; four pieces of eight values per thread on the way
     const int chunks = kc * 16, total = m * chunks;         // of a row, of all
     constexpr int kAhead = 4;
-    for (int i0 = tid; i0 < total; i0 += kAhead * kCThreads) {
+    for (int base = 0; base < total; base += kAhead * kCThreads) {
+      const int i0 = base + tid;
       float v[kAhead][8];
       int col[kAhead], n[kAhead];
 #pragma unroll
@@ -172,9 +184,28 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
         n[q] = (i - r * chunks) * 8;
         if (i < total) load_x8(p.x, p.x_dtype, ((size_t)(row0 + r) * p.bpr + k0) * kBlock + n[q], v[q]);
       }
+      if (XT == 2 && p.ss && base == 0) {                   // rows in front of their norm, whose scale arrives beside them
+        if (warp < m) {
+          const float s = row_scale(p, row0 + warp, lane);
+          if (lane == 0) s_scale[warp] = s;
+        }
+        __syncthreads();
+      }
 #pragma unroll
       for (int q = 0; q < kAhead; ++q) {
         if (i0 + q * kCThreads < total) {
+          if (XT == 2 && p.ss) {
+            float w[8];
+            const float* src = p.x_weight + k0 * kBlock + n[q];
+            if ((uintptr_t)p.x_weight % 16 == 0) {
+              load_x8(src, NB_F32, 0, w);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) w[e] = __ldg(src + e);
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[q][e] = v[q][e] * s_scale[col[q]] * w[e];
+          }
           uint32_t hi[4];
 #pragma unroll
           for (int h = 0; h < 2; ++h)
@@ -221,7 +252,7 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
   }
   // requested here, used behind the products: a row's partial sums of squares (one warp per row), residual values
   constexpr int kSq = 6;
-  const bool sq_mine = p.ss != nullptr && warp < m;
+  const bool sq_late = p.ss != nullptr && p.x == nullptr, sq_mine = sq_late && warp < m;
   const float* sq = p.ss + (size_t)(row0 + warp) * p.ss_n;
   float sqv[kSq];
 #pragma unroll
@@ -308,16 +339,12 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
     slot_j = 0;
   }
   if (sq_mine) {                                            // in a fixed order: the same bits in every CTA
-    for (int r = warp; r < m; r += kCW, sq += (size_t)kCW * p.ss_n) {
-      float s = 0.f;
-      if (r == warp) {
+    float s = 0.f;
 #pragma unroll
-        for (int q = 0; q < kSq; ++q) s += sqv[q];
-      }
-      for (int q = lane + (r == warp ? 32 * kSq : 0); q < p.ss_n; q += 32) s += __ldcg(sq + q);
-      s = warp_sum(s);
-      if (lane == 0) s_scale[r] = 1.0f / sqrtf(s / (float)(p.bpr * kBlock) + p.eps);
-    }
+    for (int q = 0; q < kSq; ++q) s += sqv[q];
+    for (int q = lane + 32 * kSq; q < p.ss_n; q += 32) s += __ldcg(sq + q);
+    s = warp_sum(s);
+    if (lane == 0) s_scale[warp] = 1.0f / sqrtf(s / (float)(p.bpr * kBlock) + p.eps);
   }
   if (kCluster) {
     if (!cluster_up) cluster_wait();
@@ -338,7 +365,7 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
       v += src[(size_t)q * slot];
       if (p.mode == NB_CHAIN_SWIGLU) v2 += src[(size_t)q * slot + 8];
     }
-    const float scale = p.ss ? s_scale[mm] : 1.f;
+    const float scale = sq_late ? s_scale[mm] : 1.f;
     if (p.mode == NB_CHAIN_STORE) {
       const int n = tile * 16 + row;
       if (n < p.N) store_y(p.y, p.y_dtype, (size_t)b * p.N + n, v * scale);
@@ -354,8 +381,8 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
       }
       v = v * scale + res;
       p.res[(size_t)b * p.N + n] = v;
-      if (p.yt) {
-        store_chain_terms(p.yt, p.N >> 7, b, n, v * wn);
+      if (p.yt) store_chain_terms(p.yt, p.N >> 7, b, n, v * wn);
+      if (p.ss_out) {
         float s = v * v;                                    // the tile's 16 rows are 16 neighbouring lanes
         const uint32_t half = 0xffffu << (lane & 16);
 #pragma unroll
@@ -366,7 +393,7 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
   }
 }
 
-// x (B, C) = the tokens' rows of a bf16 table, their terms times the norm weight `w`, and the sums of squares per 16 columns.
+// x (B, C) = the tokens' rows of a bf16 table, their terms times the norm weight `w` (null: no terms), and the sums of squares per 16 columns.
 __global__ void __launch_bounds__(256) chain_embed_kernel(const __nv_bfloat16* __restrict__ table, const long long* __restrict__ token,
                                                           const float* __restrict__ w, float* __restrict__ x, uint8_t* __restrict__ terms,
                                                           float* __restrict__ ss, int C, int V) {
@@ -377,7 +404,7 @@ __global__ void __launch_bounds__(256) chain_embed_kernel(const __nv_bfloat16* _
   tk = tk < 0 ? 0 : (tk >= V ? V - 1 : tk);
   const float v = __bfloat162float(table[(size_t)tk * C + n]);
   x[(size_t)b * C + n] = v;
-  store_chain_terms(terms, C >> 7, b, n, v * w[n]);
+  if (terms) store_chain_terms(terms, C >> 7, b, n, v * w[n]);
   float s = v * v;
 #pragma unroll
   for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -519,7 +546,7 @@ extern "C" int nb_chain_takes(int M, int N, int K, int bits, int x_dtype) {
 
 extern "C" int nb_chain_linear(const nb_chain_args* a, void* stream) {
   constexpr long long kMost = 1ll << 26;                    // products of sizes below stay in 32 bits
-  if (!a || !a->w || (a->x ? a->sq || a->mode != NB_CHAIN_STORE : !a->x_terms) || !a->status || a->M < 1 || a->N < 1) return NB_ERR_ARG;
+  if (!a || !a->w || (a->x ? a->sq && (!a->x_weight || a->x_dtype != NB_F32) : !a->x_terms) || !a->status || a->M < 1 || a->N < 1) return NB_ERR_ARG;
   if (a->mode < NB_CHAIN_STORE || a->mode > NB_CHAIN_RESIDUAL) return NB_ERR_ARG;
   if (a->mode == NB_CHAIN_STORE ? !a->y : a->mode == NB_CHAIN_SWIGLU ? !a->y_terms : !a->residual) return NB_ERR_ARG;
   if (a->mode == NB_CHAIN_RESIDUAL && a->y_terms && (!a->next_weight || !a->sq_out)) return NB_ERR_ARG;
@@ -546,7 +573,7 @@ extern "C" int nb_chain_linear(const nb_chain_args* a, void* stream) {
   ChainParams p{};
   p.w = a->w; p.xt = reinterpret_cast<const uint8_t*>(a->x_terms); p.ss = a->sq; p.y = a->y; p.yt = reinterpret_cast<uint8_t*>(a->y_terms);
   p.res = a->residual; p.w_next = a->next_weight; p.ss_out = a->sq_out; p.status = a->status;
-  p.x = a->x; p.x_dtype = a->x_dtype; p.y_dtype = a->y_dtype;
+  p.x = a->x; p.x_weight = a->x_weight; p.x_dtype = a->x_dtype; p.y_dtype = a->y_dtype;
   p.N = a->N; p.bpr = bpr; p.M = a->M; p.mode = a->mode; p.ss_n = a->sq_n; p.eps = a->eps;
   p.m_part = best.m_part; p.parts = best.parts; p.lg_split = best.S == 8 ? 3 : best.S >> 1; p.units = best.units; p.J = best.J;
   auto rcp = [](int v) { return (unsigned)((0x100000000ull + v - 1) / v); };
@@ -572,7 +599,7 @@ extern "C" int nb_chain_linear(const nb_chain_args* a, void* stream) {
 
 extern "C" int nb_chain_embed(const void* table_bf16, const int64_t* token, int B, int V, int C, const float* weight, float* x, void* terms,
                               float* sq, void* stream) {
-  if (!table_bf16 || !token || !weight || !x || !terms || !sq || B < 1 || V < 1 || C < 1) return NB_ERR_ARG;
+  if (!table_bf16 || !token || (terms && !weight) || !x || !sq || B < 1 || V < 1 || C < 1) return NB_ERR_ARG;
   if (C % kBlock || B > 65535) return NB_ERR_SHAPE;
   if ((uintptr_t)terms % 16) return NB_ERR_ALIGN;
   if (int rc = check_device()) return rc;

@@ -478,27 +478,31 @@ def chain_terms(m: int, k: int, device) -> torch.Tensor:
     return torch.zeros(int(_lib.lib().nb_chain_terms_bytes(m, k)), dtype=torch.uint8, device=device)
 
 
-def chain_linear(mode: int, w_stream: torch.Tensor, bits: int, m: int, n: int, k: int, x_terms: torch.Tensor, status: torch.Tensor,
+def chain_linear(mode: int, w_stream: torch.Tensor, bits: int, m: int, n: int, k: int, x_terms: torch.Tensor | None, status: torch.Tensor,
                  sq: torch.Tensor | None = None, eps: float = 0.0, y: torch.Tensor | None = None, y_terms: torch.Tensor | None = None,
                  residual: torch.Tensor | None = None, next_weight: torch.Tensor | None = None, sq_out: torch.Tensor | None = None,
-                 ahead: torch.Tensor | None = None, split: int = 0) -> None:
+                 ahead: torch.Tensor | None = None, split: int = 0, x: torch.Tensor | None = None, x_weight: torch.Tensor | None = None) -> None:
     """One packed linear of the decode chain (nb_chain_linear): m fp32 rows of k columns given as terms, sq (m, .) the partial sums
     of squares of the rows in front of their norm.  CHAIN_STORE: y (m, n).  CHAIN_SWIGLU: y_terms of n / 2 columns (w packed with
-    row_mode 1).  CHAIN_RESIDUAL: residual (m, n) += y, and with y_terms the terms and partial sums for the linear behind.
+    row_mode 1).  CHAIN_RESIDUAL: residual (m, n) += y, and with y_terms and sq_out the terms and partial sums for the linear behind.
+    x in place of x_terms: the rows themselves, fp32 (m, k); with sq they are normed, times x_weight (k), before they are split.
     ahead: the stream-layout weights of the linear behind, fetched into L2 meanwhile."""
-    _need_cuda(w_stream, x_terms, status)
+    _need_cuda(w_stream, status)
     n_out = n // 2 if mode == CHAIN_SWIGLU else n
     for name, t, size in (("sq", sq, None), ("y", y, m * n), ("residual", residual, m * n), ("next_weight", next_weight, n),
-                          ("sq_out", sq_out, m * (n // 16))):
+                          ("sq_out", sq_out, m * (n // 16)), ("x", x, m * k), ("x_weight", x_weight, k)):
         if t is not None and (t.dtype != torch.float32 or not t.is_cuda or not t.is_contiguous() or (size is not None and t.numel() != size)):
             raise RuntimeError(f"chain_linear: {name} must be a contiguous fp32 CUDA tensor" + (f" of {size} values" if size else ""))
     if sq is not None and (sq.numel() == 0 or sq.numel() % m):
         raise RuntimeError(f"chain_linear: sq must hold {m} rows of partial sums")
-    if x_terms.numel() < 4 * m * k or (y_terms is not None and (not y_terms.is_cuda or y_terms.numel() < 4 * m * n_out)):
+    if (x_terms is None) == (x is None):
+        raise RuntimeError("chain_linear: the rows are given as terms or plainly")
+    if x_terms is not None and (not x_terms.is_cuda or x_terms.numel() < 4 * m * k) or (y_terms is not None and (not y_terms.is_cuda or y_terms.numel() < 4 * m * n_out)):
         raise RuntimeError("chain_linear: a buffer of terms is too small")
     ptr = lambda t: None if t is None else t.data_ptr()
-    args = _lib.ChainArgs(w_stream.data_ptr(), x_terms.data_ptr(), ptr(sq), ptr(y), ptr(y_terms), ptr(residual), ptr(next_weight),
-                          ptr(sq_out), status.data_ptr(), ptr(ahead), 0 if ahead is None else ahead.numel(), float(eps), m, n, k, bits, mode, 0 if sq is None else sq.numel() // m, split)
+    args = _lib.ChainArgs(w_stream.data_ptr(), ptr(x_terms), ptr(sq), ptr(y), ptr(y_terms), ptr(residual), ptr(next_weight),
+                          ptr(sq_out), status.data_ptr(), ptr(ahead), 0 if ahead is None else ahead.numel(), float(eps), m, n, k, bits, mode,
+                          0 if sq is None else sq.numel() // m, split, x=ptr(x), x_weight=ptr(x_weight))
     with torch.cuda.device(w_stream.device):
         _lib.check(_lib.lib().nb_chain_linear(_c.byref(args), _stream()), "nb_chain_linear")
 
@@ -536,15 +540,17 @@ def chain_rows(x: torch.Tensor, w_stream: torch.Tensor, bits: int, n: int, k: in
     return out
 
 
-def chain_embed(table: torch.Tensor, token: torch.Tensor, weight: torch.Tensor, x: torch.Tensor, terms: torch.Tensor, sq: torch.Tensor) -> None:
-    """x = table[token] (bf16 -> fp32), terms = x * weight, sq = its partial sums of squares (nb_chain_embed)."""
-    _need_cuda(table, token, weight, x, terms, sq)
+def chain_embed(table: torch.Tensor, token: torch.Tensor, weight: torch.Tensor | None, x: torch.Tensor, terms: torch.Tensor | None,
+                sq: torch.Tensor) -> None:
+    """x = table[token] (bf16 -> fp32), terms = x * weight (None: not needed), sq = its partial sums of squares (nb_chain_embed)."""
+    _need_cuda(table, token, x, sq, *(() if terms is None else (weight, terms)))
     b, c = x.shape
-    if table.dtype != torch.bfloat16 or token.dtype != torch.int64 or token.numel() != b or terms.numel() < 4 * b * c or sq.numel() != b * (c // 16):
+    if (table.dtype != torch.bfloat16 or token.dtype != torch.int64 or token.numel() != b or (terms is not None and terms.numel() < 4 * b * c)
+            or sq.numel() != b * (c // 16)):
         raise RuntimeError("chain_embed: bad tensors")
     with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().nb_chain_embed(table.data_ptr(), token.data_ptr(), b, table.shape[0], c, weight.data_ptr(), x.data_ptr(),
-                                             terms.data_ptr(), sq.data_ptr(), _stream()), "nb_chain_embed")
+        _lib.check(_lib.lib().nb_chain_embed(table.data_ptr(), token.data_ptr(), b, table.shape[0], c, None if terms is None else weight.data_ptr(),
+                                             x.data_ptr(), None if terms is None else terms.data_ptr(), sq.data_ptr(), _stream()), "nb_chain_embed")
 
 
 def decode_attention_terms(qkv, cos2, sin2, pos, k_cache, v_cache, terms, out_cols: int, out_offset: int) -> None:
