@@ -61,6 +61,7 @@ _SIGNATURES = {
     "nb_embed_rows": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_int, _c.c_int, _c.c_int, _c.c_void_p, _c.c_void_p]),
     "nb_chain_terms_bytes": (_c.c_size_t, [_c.c_int, _c.c_int]),
     "nb_chain_takes": (_c.c_int, [_c.c_int] * 5),
+    "nb_chain_takes_packed": (_c.c_int, [_c.c_int] * 5),
     "nb_chain_linear": (_c.c_int, [_c.c_void_p, _c.c_void_p]),
     "nb_chain_embed": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_int, _c.c_int, _c.c_int, _c.c_void_p, _c.c_void_p, _c.c_void_p,
                                   _c.c_void_p, _c.c_void_p]),
@@ -118,7 +119,7 @@ def _struct(name: str, pointers: str, floats: str, ints: str):
 class ChainArgs(_c.Structure):
     """nb_chain_args of nativebit_b200.h."""
     _fields_ = ([(n, _P) for n in "w x_terms sq y y_terms residual next_weight sq_out status ahead".split()] + [("ahead_bytes", _c.c_int64), ("eps", _F)]
-                + [(n, _I) for n in "M N K bits mode sq_n split x_dtype y_dtype ordered".split()] + [(n, _P) for n in "x x_weight".split()])
+                + [(n, _I) for n in "M N K bits mode sq_n split x_dtype y_dtype ordered".split()] + [(n, _P) for n in "x x_weight codebook".split()] + [("codebook_dtype", _I)])
 
 
 MatvecArgs = _struct("MatvecArgs", "w bias y x delta delta_w x_out norm_w", "eps alpha limit", "N K ldw act norm")

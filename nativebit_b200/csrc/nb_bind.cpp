@@ -84,23 +84,32 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
   at::DimVector shape(x.sizes());
   shape.back() = n;
   int rc = NB_ERR_ARG;
-  if (m >= 2 && THPVariable_CheckExact(a[3]) && (m <= kGemvRows || nb_chain_takes((int)m, (int)n, (int)k, bits, xt))) {
-    const at::Tensor &w = THPVariable_Unpack(a[3]), ws = workspace(a[10], device.index(), stream);
-    if (!ws.defined() || w.device() != device || !copy_of(a[4], a[1], a[2])) Py_RETURN_NONE;
+  const bool few = nb_chain_takes_packed((int)m, (int)n, (int)k, bits, xt) != 0;     // over the packed bytes; more rows of a small matrix over its copy
+  if (few || (m > kGemvRows && THPVariable_CheckExact(a[3]) && nb_chain_takes((int)m, (int)n, (int)k, bits, xt))) {
+    const at::Tensor &w = THPVariable_Unpack(a[few ? 1 : 3]), ws = workspace(a[10], device.index(), stream);
+    if (!ws.defined()) Py_RETURN_NONE;
+    if (few ? packed.scalar_type() != at::kByte || !packed.is_contiguous() || !codebook.is_contiguous() ||
+                  packed.numel() < n * (k / 8) * bits || codebook.numel() != (n * (k / kBlock)) << bits
+            : w.device() != device || !copy_of(a[4], a[1], a[2]))
+      Py_RETURN_NONE;
     at::Tensor y = at::empty(shape, x.options().requires_grad(false).memory_format(c10::MemoryFormat::Contiguous));
     nb_chain_args args = {};
     args.w = static_cast<const uint8_t*>(w.const_data_ptr());
+    if (few) {
+      args.codebook = codebook.const_data_ptr();
+      args.codebook_dtype = ct;
+      args.ordered = ordered;
+    }
     args.x = x.const_data_ptr();
     args.y = y.mutable_data_ptr();
     args.status = static_cast<int*>(ws.mutable_data_ptr());         // the workspace's head
     args.M = (int)m; args.N = (int)n; args.K = (int)k; args.bits = bits;
     args.x_dtype = args.y_dtype = xt;
-    args.ordered = ordered;                                          // the copy of the weights may be as new as the launch before
     Py_BEGIN_ALLOW_THREADS
     rc = nb_chain_linear(&args, stream);
     Py_END_ALLOW_THREADS
     if (rc == NB_OK) return THPVariable_Wrap(std::move(y));
-  } else if (m == 1) {
+  } else if (m <= kGemvRows) {
     const at::Tensor ws = workspace(a[9], device.index(), stream);
     if (!ws.defined()) Py_RETURN_NONE;
     at::Tensor y = at::empty(shape, x.options().requires_grad(false).memory_format(c10::MemoryFormat::Contiguous));

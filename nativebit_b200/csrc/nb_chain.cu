@@ -14,6 +14,11 @@
 //    a tile meet in shared memory behind one barrier.
 //  * Where the staged rows do not fit beside the weights, a cluster of S CTAs shares its row tiles: every CTA takes K / S columns
 //    of all of them and pushes its parts into the shared memory of the CTA that finishes the tile.
+//  * Plain rows of up to 16 may come against the packed matrix itself (kRaw): what is written to it is what the next call reads, and
+//    nothing has to be made or kept beside it.  Unpacking costs a unit about 55 clocks more than the copy's selector words, and the
+//    products wait for all of a CTA's weights (2560 x 6912, 16 bf16 rows 11.4 us against 9.7 over the copy and 13.9 for nb_gemv;
+//    2560 x 2560, 8 rows 5.9, 5.0, 7.8; 13824 x 2560, 16 fp32 rows 24.6, 21.3, 35.9).  With a barrier per tile and an arrival per copying
+//    thread on it 12.7, 6.6.
 //  * Column 2r + s of the MMAs carries term s of activation row r: one product covers four fp32 rows.
 // Decode step of the 2.2B decoder with 12 layers (us), matvecs that stage the rows themselves -> this: 1 sequence 437 -> 388, 2:
 // 539 -> 443, 8: 665 -> 510, 16 (a matvec over the packed bytes and launches between): 1523 -> 934, whose rows are given plainly and normed before they are
@@ -55,7 +60,8 @@ __device__ __forceinline__ bool chain_wait(uint64_t* bar, uint32_t parity, int* 
 }
 
 struct ChainParams {
-  const uint8_t* w;           // stream layout
+  const uint8_t* w;           // stream layout, or with a codebook the packed rows themselves
+  const uint8_t* cb;          // the packed rows' codebooks (null: stream layout), cb_block bytes per block
   const uint8_t* xt;          // activations as terms
   const float* ss;            // (M, ss_n) partial sums of squares of the rows in front of the norm (null: no norm)
   void* y;                    // NB_CHAIN_STORE: (M, N) of type y_dtype
@@ -75,21 +81,61 @@ struct ChainParams {
   int clusters, lg_split;     // clusters of one part, of 2^lg_split CTAs each
   unsigned rcp_clusters, rcp_kc, rcp_kc1;     // ceil(2^32 / v) of the clusters, the smaller and the larger share of a row's blocks
   int tile0, n_tiles;         // row tiles of this launch
-  int units, J;               // room for units; partial results per tile and CTA
+  int w_bytes, J;             // room for weights; partial results per tile and CTA
+  int cb_dtype, cb_block, idx_stride, cb_stride;      // packed rows: bytes from row to row in shared memory
 };
 // v / d for v * d < 2^32 (d == 1 has no 32-bit reciprocal)
 __device__ __forceinline__ int div_rcp(int v, int d, unsigned rcp) { return d == 1 ? v : (int)__umulhi((unsigned)v, rcp); }
 
-// 16 rows x 128 weights against CG groups of eight columns.
-template <int BITS, int CG>
-__device__ __forceinline__ void chain_unit(const uint8_t* ub, const uint8_t* const (&x)[CG], int lane, const ByteShift& sm, uint32_t act, uint4 (&last)[1],
-                                           float (&c)[CG == 1 ? 2 : CG][4]) {
+// 32 packed indices -> four selector words, nibble i of word j the index at position 8j + i: the order of the stream layout.
+// Fields move apart half by half; what moves is picked by a mask and moved by a multiply-add.
+template <int BITS> __device__ __forceinline__ void packed_selectors(const uint8_t* src, uint32_t (&U)[4]) {
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(src);
+  if (BITS == 4) {
+    const uint4 v = *reinterpret_cast<const uint4*>(src);
+    U[0] = v.x; U[1] = v.y; U[2] = v.z; U[3] = v.w;
+  } else if (BITS == 3) {
+    const uint32_t w0 = w[0], w1 = w[1], w2 = w[2];
+    U[0] = w0 & 0xFFFFFFu;
+    U[1] = funnel_r(w0, w1, 24) & 0xFFFFFFu;
+    U[2] = funnel_r(w1, w2, 16) & 0xFFFFFFu;
+    U[3] = w2 >> 8;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      U[j] = mad_lo(U[j] & 0xFFF000u, 15u, U[j]);
+      U[j] = mad_lo(U[j] & 0x0FC00FC0u, 3u, U[j]);
+      U[j] += U[j] & 0x38383838u;
+    }
+  } else {
+    const uint2 v = *reinterpret_cast<const uint2*>(src);
+    U[0] = v.x & 0xFFFFu; U[1] = v.x >> 16; U[2] = v.y & 0xFFFFu; U[3] = v.y >> 16;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      U[j] = mad_lo(U[j] & 0xFF00u, 255u, U[j]);
+      U[j] = mad_lo(U[j] & 0x00F000F0u, 15u, U[j]);
+      U[j] = mad_lo(U[j] & 0x0C0C0C0Cu, 3u, U[j]);
+    }
+  }
+}
+
+// 16 rows x 128 weights against CG groups of eight columns.  kRaw: `ub` and `cb` are this lane's indices and codebook of row g, those
+// of row g + 8 eight strides on.
+template <int BITS, int CG, bool kRaw>
+__device__ __forceinline__ void chain_unit(const ChainParams& p, const uint8_t* ub, const uint8_t* cb, const uint8_t* const (&x)[CG], int lane,
+                                           const ByteShift& sm, uint32_t act, uint4 (&last)[1], float (&c)[CG == 1 ? 2 : CG][4]) {
   const int g = lane >> 2, t = lane & 3;
   uint32_t UA[4], UB[4], TA[BITS == 4 ? 8 : 4], TB[BITS == 4 ? 8 : 4];
-  unit_selectors(ub, lane, 0, UA);
-  unit_selectors(ub, lane, 1, UB);
-  unit_table<BITS>(ub, g, TA);
-  unit_table<BITS>(ub, g + 8, TB);
+  if (kRaw) {
+    packed_selectors<BITS>(ub, UA);
+    packed_selectors<BITS>(ub + 8 * p.idx_stride, UB);
+    make_table<BITS>(cb, p.cb_dtype, true, TA);
+    make_table<BITS>(cb + 8 * p.cb_stride, p.cb_dtype, true, TB);
+  } else {
+    unit_selectors(ub, lane, 0, UA);
+    unit_selectors(ub, lane, 1, UB);
+    unit_table<BITS>(ub, g, TA);
+    unit_table<BITS>(ub, g + 8, TB);
+  }
 #pragma unroll
   for (int uu = 0; uu < 4; ++uu) {
     uint4 xq[CG];
@@ -125,9 +171,9 @@ __device__ __forceinline__ float row_scale(const ChainParams& p, int r, int lane
   return 1.0f / sqrtf(warp_sum(s) / (float)(p.bpr * kBlock) + p.eps);
 }
 
-// Shared memory: the CTA's units, tile after tile | staged columns (XT m_part of kc_max * 256 bytes) | partial
+// Shared memory: the CTA's units, tile after tile (kRaw: a tile's 16 rows of indices, then of codebooks) | staged columns (XT m_part of kc_max * 256 bytes) | partial
 // results [own tile][CTA][J][row][16] of the tiles this CTA finishes.
-template <int BITS, int CG, int XT, bool kCluster>
+template <int BITS, int CG, int XT, bool kCluster, bool kRaw>
 __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p) {
   constexpr int kUnit = StreamUnit<BITS>::kBytes;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -142,20 +188,45 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
   // ---- the weights do not depend on the launch before: one copy per row tile
   if (tid == 0) {
     mbar_init(&s_xbar, 1);
-    for (int i = 0; i < T; ++i) mbar_init(&s_bar[i], 1);
+    for (int i = 0; !kRaw && i < T; ++i) mbar_init(&s_bar[i], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     const uint8_t* src = p.w + ((size_t)(p.tile0 + ci) * p.bpr + k0) * kUnit;
-    for (int i = 0; i < T; ++i) {
+    for (int i = 0; !kRaw && i < T; ++i) {
       mbar_arrive_expect_tx(&s_bar[i], (uint32_t)(kc * kUnit));
       bulk_g2s(smem + (size_t)i * kc * kUnit, src, (uint32_t)(kc * kUnit), &s_bar[i]);
       src += (size_t)p.clusters * p.bpr * kUnit;
     }
   }
+  const int tile_bytes = 16 * (p.idx_stride + p.cb_stride);
+  if (kRaw) {                                               // thread after thread takes the next piece of a row: indices, then codebooks
+    const int idx_pieces = kc * BITS, cb_piece = p.cb_block >= 16 ? 16 : 8, per_row = idx_pieces + kc * p.cb_block / cb_piece;
+    const int rows = kCThreads / per_row, rest = kCThreads - rows * per_row;
+    int r = tid / per_row, c = tid - r * per_row;
+    for (;;) {
+      if (c >= per_row) { c -= per_row; ++r; }
+      if (r >= 16 * T) break;
+      const int i = r >> 4, row = r & 15, tile = p.tile0 + ci + i * p.clusters;
+      const int n = p.mode == NB_CHAIN_SWIGLU ? tile * 8 + (row & 7) + (row & 8 ? p.N >> 1 : 0) : min(tile * 16 + row, p.N - 1);
+      const size_t block = (size_t)(n * p.bpr + k0);
+      uint8_t* dst = smem + i * tile_bytes;
+      if (c < idx_pieces) {
+        cp_async16(dst + row * p.idx_stride + 16 * c, p.w + block * (16 * BITS) + 16 * c);
+      } else {
+        dst += 16 * p.idx_stride + row * p.cb_stride + cb_piece * (c - idx_pieces);
+        const uint8_t* src = p.cb + block * p.cb_block + cb_piece * (c - idx_pieces);
+        if (cb_piece == 16) cp_async16(dst, src);
+        else cp_async8(dst, src);
+      }
+      r += rows;
+      c += rest;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
   const int row0 = part * p.m_part, m = min(p.m_part, p.M - row0);
   const unsigned rcp_kc = kc == kc_max ? p.rcp_kc1 : p.rcp_kc;
   const int U = T * kc;                                     // units of this CTA, tile after tile
   const int ua = U * warp / kCW, ub = U * (warp + 1) / kCW; // this warp's run
-  uint8_t* x_s = smem + (size_t)p.units * kUnit;
+  uint8_t* x_s = smem + p.w_bytes;
   float* parts = reinterpret_cast<float*>(x_s + (size_t)XT * p.m_part * kc_max * 256);
   const int own = (T + S - 1 - rank) >> lg;                 // tiles rank, rank + S, .. of the cluster's are finished here
   const int slot = 16 * m;
@@ -169,7 +240,7 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
   asm volatile("griddepcontrol.launch_dependents;");
 
   const uint8_t* xt = p.xt + ((size_t)(2 * row0) * p.bpr + k0) * 256;
-  const bool bulk = !p.x && 2 * m * kc > kChainBulk;
+  const bool bulk = !p.x && (kRaw || 2 * m * kc > kChainBulk);      // (a wait for 16-byte copies would be one for the weights')
   if (XT == 1 || p.x) {                                     // converted here; four pieces of eight values per thread on the way
     const int chunks = kc * 16, total = m * chunks;         // of a row, of all
     constexpr int kAhead = 4;
@@ -268,8 +339,9 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
   }
   if (bulk) {
     chain_wait(&s_xbar, 0, p.status);
-  } else {
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+  }
+  if (kRaw || !bulk) {                                      // (packed rows: one wait for all; an arrival per copying thread on a
+    asm volatile("cp.async.wait_group 0;" ::: "memory");    // barrier per tile is a shared-memory atomic each)
     __syncthreads();
   }
 
@@ -282,7 +354,7 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
   uint4 x_last[1] = {make_uint4(0u, 0u, 0u, 0u)};
   constexpr int kAcc = CG == 1 ? 2 : CG;
   bool cluster_up = !kCluster;
-  const uint8_t* up = smem + (size_t)ua * kUnit;
+  const uint8_t *up = smem + (size_t)ua * kUnit, *cp = nullptr;
   int u = ua, i = i_first, kk = kk_first, slot_j = j_first;
 #pragma unroll 1
   while (u < ub) {                                          // a tile's part of the run
@@ -295,11 +367,16 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
 #pragma unroll
     for (int j = 0; j < CG; ++j) xp[j] = xc[j] + kk * 256;
     const int tile_end = min(ub, u + kc - kk);
-    chain_wait(&s_bar[i], 0, p.status);
+    if (kRaw) {
+      up = smem + i * tile_bytes + g * p.idx_stride + (4 * kk + t) * (4 * BITS);
+      cp = smem + i * tile_bytes + 16 * p.idx_stride + g * p.cb_stride + kk * p.cb_block;
+    }
+    if (!kRaw) chain_wait(&s_bar[i], 0, p.status);
 #pragma unroll (CG == 1 ? 2 : 1)
     for (; u < tile_end; ++u) {
-      chain_unit<BITS, CG>(up, xp, lane, sm, act, x_last, c);
-      up += kUnit;
+      chain_unit<BITS, CG, kRaw>(p, up, cp, xp, lane, sm, act, x_last, c);
+      up += kRaw ? 16 * BITS : kUnit;
+      if (kRaw) cp += p.cb_block;
 #pragma unroll
       for (int j = 0; j < CG; ++j) xp[j] += 256;
     }
@@ -414,14 +491,16 @@ __global__ void __launch_bounds__(256) chain_embed_kernel(const __nv_bfloat16* _
 constexpr size_t kChainSmemMax = 227 * 1024 - 2048;
 
 struct ChainPlan {
-  int S, clusters, parts, m_part, launches, per_launch, units, J, cg, terms;      // per_launch: row tiles
+  int S, clusters, parts, m_part, launches, per_launch, w_bytes, J, cg, terms;      // per_launch: row tiles
+  int idx_stride, cb_stride;
   size_t smem;
   double cost;
 };
 
 // Split over clusters of S CTAs; false if even one row tile does not fit.  As many launches as it takes for a CTA's units, its
 // share of the activations and the partial results to fit.
-static bool chain_plan(int N, int bpr, int M, int terms, bool plain, int bits, int S, int max_clusters, ChainPlan& pl) {
+// cb_block: bytes of a block's codebook beside packed rows, 0 for the stream layout.
+static bool chain_plan(int N, int bpr, int M, int terms, bool plain, int bits, int cb_block, int S, int max_clusters, ChainPlan& pl) {
   if (S > bpr) return false;
   const int n_tiles = (N + 15) / 16, unit = bits == 4 ? StreamUnit<4>::kBytes : StreamUnit<3>::kBytes;
   pl.S = S;
@@ -430,20 +509,25 @@ static bool chain_plan(int N, int bpr, int M, int terms, bool plain, int bits, i
   pl.terms = terms;
   pl.cg = terms * pl.m_part <= 8 ? 1 : terms * pl.m_part <= 16 ? 2 : 4;
   const int room = std::max(1, max_clusters / pl.parts), kc_max = (bpr + S - 1) / S, kc_min = bpr / S;
+  // rows an odd number of 16 (3 bits), 32 (2) or 64 bytes (4) apart, codebooks of 16: the rows that are read together meet different banks
+  const int odd = bits == 3 ? 16 : bits == 2 ? 32 : 64;
+  pl.idx_stride = ((kc_max * 16 * bits + odd - 1) / odd | 1) * odd;
+  pl.cb_stride = ((kc_max * cb_block + 15) / 16 | 1) * 16;
+  const int tile_bytes = cb_block ? 16 * (pl.idx_stride + pl.cb_stride) : kc_max * unit;
   for (pl.launches = 1; pl.launches <= n_tiles; ++pl.launches) {
     pl.per_launch = (n_tiles + pl.launches - 1) / pl.launches;
     pl.clusters = std::min(pl.per_launch, room);
     const int T = (pl.per_launch + pl.clusters - 1) / pl.clusters, last = n_tiles - (pl.launches - 1) * pl.per_launch;
     if (last < 1) continue;
-    pl.units = T * kc_max;
+    pl.w_bytes = T * tile_bytes;
     // a tile of kc units meets at most kc warps, and two more than it has whole runs
     const int run = std::max(1, std::max(1, last / pl.clusters) * kc_min / kCW);
     pl.J = std::min(kc_max, kc_max / run + 2);
-    pl.smem = (size_t)pl.units * unit + (size_t)terms * pl.m_part * kc_max * 256 + (size_t)((T + S - 1) / S) * S * pl.J * 64 * pl.m_part;
+    pl.smem = (size_t)pl.w_bytes + (size_t)terms * pl.m_part * kc_max * 256 + (size_t)((T + S - 1) / S) * S * pl.J * 64 * pl.m_part;
     if (T <= kChainTiles && pl.smem <= kChainSmemMax) {
       // clocks: units at the rate of their lookups and MMAs, staged columns (copied, or converted), launch and drain, a cluster's
       // barriers; within 15 % of the best of the four splits over eight shapes and 1 to 16 rows
-      pl.cost = pl.launches * (pl.units * (60.0 + 9.0 * (pl.cg - 1)) + (double)terms * pl.m_part * kc_max * (plain ? 16.0 : 4.0) + 4000.0 + (S > 1 ? 2500.0 : 0.0));
+      pl.cost = pl.launches * (T * kc_max * ((cb_block ? 80.0 : 60.0) + 9.0 * (pl.cg - 1)) + (double)terms * pl.m_part * kc_max * (plain ? 16.0 : 4.0) + 4000.0 + (S > 1 ? 2500.0 : 0.0));
       return true;
     }
     if (T == 1) return false;
@@ -451,13 +535,13 @@ static bool chain_plan(int N, int bpr, int M, int terms, bool plain, int bits, i
   return false;
 }
 
-template <int BITS, int CG, int XT, bool kCluster>
+template <int BITS, int CG, int XT, bool kCluster, bool kRaw>
 static int chain_launch_as(const ChainPlan& pl, const ChainParams& p, bool ordered, cudaStream_t st) {
   static bool done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!done[dev & 63]) {
-    if (cudaError_t e = cudaFuncSetAttribute(chain_kernel<BITS, CG, XT, kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmemMax))
+    if (cudaError_t e = cudaFuncSetAttribute(chain_kernel<BITS, CG, XT, kCluster, kRaw>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmemMax))
       return record_cuda_error(e);
     done[dev & 63] = true;
   }
@@ -478,13 +562,13 @@ static int chain_launch_as(const ChainPlan& pl, const ChainParams& p, bool order
     attr[cfg.numAttrs].val.clusterDim.y = 1;
     attr[cfg.numAttrs++].val.clusterDim.z = 1;
   }
-  return record_cuda_error(cudaLaunchKernelEx(&cfg, chain_kernel<BITS, CG, XT, kCluster>, p));
+  return record_cuda_error(cudaLaunchKernelEx(&cfg, chain_kernel<BITS, CG, XT, kCluster, kRaw>, p));
 }
-template <int BITS>
+template <int BITS, bool kRaw>
 static int chain_launch(const ChainPlan& pl, const ChainParams& p, bool ordered, cudaStream_t st) {
   const auto run = [&](auto cg, auto xt) {
     constexpr int CG = decltype(cg)::value, XT = decltype(xt)::value;
-    return pl.S > 1 ? chain_launch_as<BITS, CG, XT, true>(pl, p, ordered, st) : chain_launch_as<BITS, CG, XT, false>(pl, p, ordered, st);
+    return pl.S > 1 ? chain_launch_as<BITS, CG, XT, true, kRaw>(pl, p, ordered, st) : chain_launch_as<BITS, CG, XT, false, kRaw>(pl, p, ordered, st);
   };
   using std::integral_constant;
   if (pl.terms == 1) return pl.cg == 1 ? run(integral_constant<int, 1>{}, integral_constant<int, 1>{}) : run(integral_constant<int, 2>{}, integral_constant<int, 1>{});
@@ -513,8 +597,8 @@ static int max_clusters(int S) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int got = 0;
-    if (cudaFuncSetAttribute(chain_kernel<3, 1, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmemMax) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&got, chain_kernel<3, 1, 2, true>, &cfg) != cudaSuccess || got < 1) {
+    if (cudaFuncSetAttribute(chain_kernel<3, 1, 2, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmemMax) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&got, chain_kernel<3, 1, 2, true, false>, &cfg) != cudaSuccess || got < 1) {
       cudaGetLastError();
       got = 1;
     }
@@ -540,8 +624,18 @@ extern "C" int nb_chain_takes(int M, int N, int K, int bits, int x_dtype) {
   ChainPlan pl{}, best{};
   best.cost = 1e30;
   for (int S : {1, 2, 4, 8})
-    if (chain_plan(N, K / kBlock, M, terms, true, bits, S, max_clusters(S), pl) && pl.cost < best.cost) best = pl;
+    if (chain_plan(N, K / kBlock, M, terms, true, bits, 0, S, max_clusters(S), pl) && pl.cost < best.cost) best = pl;
   return best.cost < 1e30 && best.launches == 1;
+}
+
+// Whether plain rows against the packed matrix are for nb_chain_linear rather than nb_gemv.  Where few 16-bit rows meet many short
+// rows of weights, every CTA of nb_gemv has whole rows, all CTAs run at once and its unpacking is the cheaper one (us, nb_gemv |
+// this, 3 bits, 2 and 4 rows: 5632 x 1024 3.5 | 4.1, 3.9 | 4.2; 6912 x 2560 6.0 | 7.7, 6.9 | 8.0; 9472 x 2560 6.6 | 8.2, 7.3 | 8.4; on the
+// other side of the line 4096 x 2560 5.7 | 5.7, 7.0 | 5.9; 6912 x 4096 11.6 | 9.3; 11008 x 2560 14.6 | 8.9; 6912 x 2560 with 5 rows 7.6 | 8.2, with
+// 8 9.4 | 8.6; at 2 bits 8192 x 2560 8.3 | 7.4).
+extern "C" int nb_chain_takes_packed(int M, int N, int K, int bits, int x_dtype) {
+  if (M < 2 || M > 16 || N < 1 || K < kBlock || K % kBlock || (bits != 2 && bits != 3 && bits != 4)) return 0;
+  return !(bits == 3 && x_dtype != NB_F32 && M <= 4 && N >= 5120 && K <= 2560 && (long long)N * K <= 25000000);
 }
 
 extern "C" int nb_chain_linear(const nb_chain_args* a, void* stream) {
@@ -559,23 +653,26 @@ extern "C" int nb_chain_linear(const nb_chain_args* a, void* stream) {
   if (a->mode == NB_CHAIN_RESIDUAL && a->N % kBlock) return NB_ERR_SHAPE;
   if (a->split < 0 || a->split > 8 || (a->split & (a->split - 1))) return NB_ERR_ARG;
   if ((long long)(a->N + 15) / 16 * (a->K / kBlock) > kMost || a->N > (1 << 24)) return NB_ERR_SHAPE;
-  if ((uintptr_t)a->w % 16 || (uintptr_t)a->x_terms % 16 || (uintptr_t)a->y_terms % 16 || (uintptr_t)a->ahead % 16 || a->ahead_bytes % 16 || (uintptr_t)a->x % 16)
+  if (a->codebook && a->codebook_dtype != NB_F16 && a->codebook_dtype != NB_F32) return NB_ERR_ARG;
+  if ((uintptr_t)a->w % 16 || (uintptr_t)a->codebook % 16 || (uintptr_t)a->x_terms % 16 || (uintptr_t)a->y_terms % 16 || (uintptr_t)a->ahead % 16 || a->ahead_bytes % 16 || (uintptr_t)a->x % 16)
     return NB_ERR_ALIGN;
   if (int rc = check_device()) return rc;
-  const int bpr = a->K / kBlock;
+  const int bpr = a->K / kBlock, cb_block = a->codebook ? (a->codebook_dtype == NB_F16 ? 2 : 4) << a->bits : 0;
   ChainPlan pl{}, best{};
   best.cost = 1e30;
   for (int S : {1, 2, 4, 8}) {
     if (a->split && S != a->split) continue;
-    if (chain_plan(a->N, bpr, a->M, a->x && a->x_dtype != NB_F32 ? 1 : 2, a->x != nullptr, a->bits, S, max_clusters(S), pl) && pl.cost < best.cost) best = pl;
+    if (chain_plan(a->N, bpr, a->M, a->x && a->x_dtype != NB_F32 ? 1 : 2, a->x != nullptr, a->bits, cb_block, S, max_clusters(S), pl) && pl.cost < best.cost) best = pl;
   }
   if (best.cost == 1e30) return NB_ERR_SHAPE;
   ChainParams p{};
+  p.cb = reinterpret_cast<const uint8_t*>(a->codebook); p.cb_dtype = a->codebook_dtype; p.cb_block = cb_block;
+  p.idx_stride = best.idx_stride; p.cb_stride = best.cb_stride;
   p.w = a->w; p.xt = reinterpret_cast<const uint8_t*>(a->x_terms); p.ss = a->sq; p.y = a->y; p.yt = reinterpret_cast<uint8_t*>(a->y_terms);
   p.res = a->residual; p.w_next = a->next_weight; p.ss_out = a->sq_out; p.status = a->status;
   p.x = a->x; p.x_weight = a->x_weight; p.x_dtype = a->x_dtype; p.y_dtype = a->y_dtype;
   p.N = a->N; p.bpr = bpr; p.M = a->M; p.mode = a->mode; p.ss_n = a->sq_n; p.eps = a->eps;
-  p.m_part = best.m_part; p.parts = best.parts; p.lg_split = best.S == 8 ? 3 : best.S >> 1; p.units = best.units; p.J = best.J;
+  p.m_part = best.m_part; p.parts = best.parts; p.lg_split = best.S == 8 ? 3 : best.S >> 1; p.w_bytes = best.w_bytes; p.J = best.J;
   auto rcp = [](int v) { return (unsigned)((0x100000000ull + v - 1) / v); };
   p.rcp_kc = rcp(std::max(1, bpr / best.S)); p.rcp_kc1 = rcp((bpr + best.S - 1) / best.S);
   const int n_tiles = (a->N + 15) / 16, most = best.clusters;
@@ -591,7 +688,12 @@ extern "C" int nb_chain_linear(const nb_chain_args* a, void* stream) {
     }
     int rc = NB_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    rc = a->bits == 2 ? chain_launch<2>(best, p, a->ordered, st) : a->bits == 3 ? chain_launch<3>(best, p, a->ordered, st) : chain_launch<4>(best, p, a->ordered, st);
+    const auto run = [&](auto raw) {
+      constexpr bool kRaw = decltype(raw)::value;
+      return a->bits == 2 ? chain_launch<2, kRaw>(best, p, a->ordered, st) : a->bits == 3 ? chain_launch<3, kRaw>(best, p, a->ordered, st)
+                                                                                         : chain_launch<4, kRaw>(best, p, a->ordered, st);
+    };
+    rc = a->codebook ? run(std::true_type{}) : run(std::false_type{});
     if (rc) return rc;
   }
   return NB_OK;

@@ -520,19 +520,32 @@ def chain_takes(m: int, n: int, k: int, bits: int, dtype: torch.dtype) -> bool:
     return _takes[key]
 
 
+def chain_takes_packed(m: int, n: int, k: int, bits: int, dtype: torch.dtype) -> bool:
+    """Whether 2 to 16 rows of this type against the packed bytes are for chain_rows rather than gemv (nb_chain_takes_packed)."""
+    return dtype in _DTYPE and bool(_lib.lib().nb_chain_takes_packed(m, n, k, bits, _DTYPE[dtype]))
+
+
 def chain_rows(x: torch.Tensor, w_stream: torch.Tensor, bits: int, n: int, k: int, ordered: bool = False,
-               out: torch.Tensor | None = None) -> torch.Tensor | None:
-    """y (M, n) = x (M, k) @ W.T in x's type for a few rows of any float type against the stream-layout weights (nb_chain_linear);
-    None if the rows do not fit.  ordered: as for gemv, for weights that the launch before may have written."""
+               out: torch.Tensor | None = None, codebook: torch.Tensor | None = None) -> torch.Tensor | None:
+    """y (M, n) = x (M, k) @ W.T in x's type for a few rows of any float type against the stream-layout weights, or with a codebook
+    against the packed bytes themselves (nb_chain_linear); None if the rows do not fit.  ordered: as for gemv, for weights that the
+    launch before may have written."""
     _need_cuda(x, w_stream)
     if x.dim() != 2 or x.shape[1] != k or x.dtype not in _DTYPE:
         raise RuntimeError(f"x must be a contiguous float (M, {k}) tensor; got {x.dtype} {tuple(x.shape)}")
+    if codebook is not None:
+        _need_cuda(codebook)
+        if (w_stream.dtype != torch.uint8 or w_stream.numel() < packed_nbytes(n * k, bits) or codebook.dtype not in (torch.float16, torch.float32)
+                or codebook.numel() != n * k // 128 << bits):
+            raise RuntimeError(f"chain_rows: packed bytes and codebooks of an ({n}, {k}) matrix at {bits} bits are needed")
     if out is None:
         out = torch.empty(x.shape[0], n, dtype=x.dtype, device=x.device)
     with torch.cuda.device(x.device):
         status = prefill_workspace(x.device, 256)            # its head
         args = _lib.ChainArgs(w=w_stream.data_ptr(), y=out.data_ptr(), status=status.data_ptr(), M=x.shape[0], N=n, K=k, bits=bits,
-                              x_dtype=_DTYPE[x.dtype], y_dtype=_DTYPE[out.dtype], ordered=int(ordered), x=x.data_ptr())
+                              x_dtype=_DTYPE[x.dtype], y_dtype=_DTYPE[out.dtype], ordered=int(ordered), x=x.data_ptr(),
+                              codebook=None if codebook is None else codebook.data_ptr(),
+                              codebook_dtype=0 if codebook is None else _DTYPE[codebook.dtype])
         rc = _lib.lib().nb_chain_linear(_c.byref(args), _stream())
     if rc == 3:
         return None

@@ -175,20 +175,22 @@ class PackedLinear(torch.nn.Module):
         return of is not None and of[0] is self.packed_indices and of[1] is self.codebook and of[2:] == (_version(of[0]), _version(of[1]))
 
     def _forward_few(self, x_flat):
-        """2 to 16 rows against the stream-layout copy of the weights, None where that does not take them.  From a graph over cold
-        weights, nb_gemv | this (us, 3 bits): 2560 x 6912 bf16 2 rows 8.7 | 6.3, 8: 11.8 | 6.8, 16: 13.9 | 10.1; 2560 x 2560 fp32 8: 11.6 | 6.0,
-        16: 13.9 | 6.8; 1024 x 1024 bf16 16: 8.0 | 3.9.  One row (4.1 | 4.1) does not pay for a second copy of the weights."""
-        if not self._tensor_cores() or x_flat.data_ptr() % 16:
+        """2 to 16 rows on the chain's kernel over the packed bytes, None where nb_gemv takes them."""
+        if not ops.chain_takes_packed(x_flat.shape[0], self.out_features, self.in_features, self.bits, x_flat.dtype) or x_flat.data_ptr() % 16 or self.packed_indices.data_ptr() % 16 or self.codebook.data_ptr() % 16:
             return None
-        w = self._copy()
-        return None if w is None else ops.chain_rows(x_flat, w, self.bits, self.out_features, self.in_features)
+        y = ops.chain_rows(x_flat, self.packed_indices, self.bits, self.out_features, self.in_features, ordered=self._fresh,
+                           codebook=self.codebook)
+        if y is not None and self._fresh:
+            self._fresh = False
+        return y
 
     def _forward_many(self, x_flat):
         """M > 16 rows on the tcgen05 kernels (exact fp16 weights; bf16 and fp16 activations as given, fp32
         carried as two fp16 terms; fp32 accumulation; result in x's dtype): one pass over the packed weights,
         dequantised inside the kernel, up to FUSED_MAX_ROWS rows; dequantise-once + GEMM beyond."""
-        if x_flat.dtype in (torch.float32, torch.float16, torch.bfloat16) and self._few_enough(x_flat.shape[0], x_flat.dtype) and (
-                y := self._forward_few(x_flat)) is not None:
+        if (x_flat.dtype in (torch.float32, torch.float16, torch.bfloat16) and x_flat.data_ptr() % 16 == 0
+                and self._few_enough(x_flat.shape[0], x_flat.dtype) and (w := self._copy()) is not None
+                and (y := ops.chain_rows(x_flat, w, self.bits, self.out_features, self.in_features)) is not None):
             return y
         if self._tensor_cores():
             rows = x_flat.shape[0] * (2 if x_flat.dtype == torch.float32 else 1)

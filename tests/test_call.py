@@ -99,3 +99,31 @@ def test_other_weights_are_what_the_next_call_multiplies(built_lib, rows):
     lin.packed_indices = third[0]
     check(third)
     assert lin.stream_weight().data_ptr() == held.data_ptr()            # what a captured graph reads
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 2, 16])
+def test_few_rows_multiply_the_packed_bytes_themselves(built_lib, rows):
+    """No copy that could be of other weights: writes that PyTorch does not count are followed as well, and nothing is kept."""
+    n, k = 144, 256
+    g = torch.Generator(device="cuda").manual_seed(rows)
+
+    def weights():
+        return ops.pack(torch.randint(0, 8, (n * k,), dtype=torch.uint8, device="cuda", generator=g), 3), torch.randn(n * k // 128, 8, device="cuda", generator=g).half()
+
+    w = [weights() for _ in range(3)]
+    x = torch.randn(rows, k, device="cuda", generator=g)
+    want = [PackedLinear(*v, n, k)(x) for v in w]
+    lin = PackedLinear(w[0][0].clone(), w[0][1].clone(), n, k)
+    assert torch.equal(lin(x), want[0]) and torch.equal(lin(x), want[0])
+    lin.packed_indices.data.copy_(w[1][0])
+    lin.codebook.data.copy_(w[1][1])
+    torch.cuda.synchronize()
+    assert torch.equal(lin(x), want[1])
+    with torch.inference_mode():
+        lin = PackedLinear(w[0][0].clone(), w[0][1].clone(), n, k)
+        assert lin.packed_indices.is_inference() and torch.equal(lin(x), want[0])
+        lin.load_state_dict({"packed_indices": w[2][0], "codebook": w[2][1]})
+        torch.cuda.synchronize()
+        assert torch.equal(lin(x), want[2])
+    assert not any("wstream" in name for name in lin.__dict__)

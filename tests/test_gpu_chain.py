@@ -171,3 +171,27 @@ def test_what_is_no_number_reaches_the_products_behind(built_lib, value):
     _close(y[[0, 2]], plain[[0, 2]].double() @ out_dense.T, REL)
     if value == value:
         _close(y[1], plain[1].double().clamp(-131008, 131008) @ out_dense.T, 2.0 ** -12)
+
+
+@pytest.mark.parametrize("n,k,m", [(16, 128, 2), (1000, 1024, 9), (2560, 6912, 16), (2560, 6912, 2), (5632, 2048, 11), (333, 2560, 13), (4096, 256, 33), (90000, 128, 16)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("bits", [2, 3, 4])
+def test_chain_rows_over_the_packed_bytes(built_lib, n, k, m, dtype, bits):
+    """The packed matrix itself in place of its stream-layout copy; codebooks of either type."""
+    packed, cb, _ = o.make_packed_linear(n, k, bits, seed=n + m)
+    dense = torch.from_numpy(o.dequant_packed(packed, cb.astype(np.float32), n, k, bits)).to(DEV).double()
+    p, cb = torch.from_numpy(packed).to(DEV), torch.from_numpy(cb).to(DEV)
+    x = torch.randn(m, k, device=DEV, generator=torch.Generator(device=DEV).manual_seed(k)).to(dtype)
+    want = x.double() @ dense.T
+    for codebook in (cb, cb.float()):
+        for ordered in (True, False):
+            y = ops.chain_rows(x, p, bits, n, k, ordered=ordered, out=torch.full((m, n), float("nan"), dtype=torch.float32, device=DEV), codebook=codebook)
+            _close(y, want, REL)
+            assert torch.equal(y, ops.chain_rows(x, p, bits, n, k, out=torch.empty_like(y), codebook=codebook))
+    y = ops.chain_rows(x, p, bits, n, k, codebook=cb)
+    assert y.dtype == dtype
+    _close(y, want, {torch.float32: REL, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[dtype])
+    with pytest.raises(RuntimeError):
+        ops.chain_rows(x, p[:-16], bits, n, k, codebook=cb)
+    with pytest.raises(RuntimeError):
+        ops.chain_rows(x, p, bits, n, k, codebook=cb[:-1])
