@@ -21,8 +21,8 @@
 //    thread on it 12.7, 6.6.
 //  * Column 2r + s of the MMAs carries term s of activation row r: one product covers four fp32 rows.
 // Decode step of the 2.2B decoder with 12 layers (us), matvecs that stage the rows themselves -> this: 1 sequence 437 -> 388, 2:
-// 539 -> 443, 8: 665 -> 510, 16 (a matvec over the packed bytes and launches between): 1523 -> 934, whose rows are given plainly and normed before they are
-// split (857 with terms, which keep fewer bits of small rows).  17 and more rows stay on
+// 539 -> 443, 8: 665 -> 510, 16 (a matvec over the packed bytes and launches between): 1523 -> 943 over the packed matrix, rows
+// given plainly and normed before they are split (934 over the copy; 865 with terms, which keep fewer bits of small rows).  17 and more rows stay on
 // the tcgen05 kernel (32: 1121, here 1460).  For one sequence a layer's 28 us are four times 1.3 us from the end of a launch
 // to the next one's first dependent instruction, 12.5 us of products (66 clocks per unit and SM against 54 without copies; down
 // projections wait for the 12 SMs with two tiles), 4.4 us of attention and the rest staging and sums.  Measured and not kept:

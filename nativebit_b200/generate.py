@@ -385,8 +385,13 @@ class DecodeSession(Session):
         self.chain = bool(fits and fused and tile_gemv is not False and model.tp_size == 1
                           and getattr(model, "exchange", None) is None and model.embedding.dtype == torch.bfloat16
                           and model.config.n_embd % 128 == 0 and all(b.gate_up.out_features % 256 == 0 for b in model.blocks)
+                          and (not CHAIN_TERM_ROWS < batch_size <= CHAIN_MAX_ROWS
+                               or all(t.data_ptr() % 16 == 0 for b in model.blocks for l in (b.qkv, b.out_proj, b.gate_up, b.down)
+                                      for t in (l.packed_indices, l.codebook)))
                           and (batch_size <= CHAIN_MAX_ROWS or all(ops.chain_takes(batch_size, l.out_features, l.in_features, l.bits, torch.float32)
                                                                    for b in model.blocks for l in (b.qkv, b.out_proj, b.gate_up, b.down))))
+        # 9 .. 16 sequences: over the packed bytes, which need no copy and follow whatever is written to them
+        self.chain_packed = self.chain and CHAIN_TERM_ROWS < batch_size <= CHAIN_MAX_ROWS
         # stream=True (one sequence on one GPU): the whole step is ONE launch of the persistent kernel
         # (stream.py).  The default is the chain of fused kernels, which measures faster: inside one launch
         # every operation pays a device-wide flag wait and the staging of its activations in full.
@@ -396,7 +401,7 @@ class DecodeSession(Session):
             if not _stream.stream_supported(model, batch_size):
                 raise RuntimeError("the one-launch decode step needs batch 1, one rank, bf16 embeddings and block-128 codebooks")
         self.prog = None
-        self._copied = []                     # (a linear's buffers, what its copies were made of), as of the last capture
+        self._captured = []                   # the weights at the last capture, see _weights
         self.batch_gemm = batch_gemm          # kept for compatibility: batches above 16 rows always take the tensor-core kernel
         dev = self.dev
         self.caches = init_kv_cache(model, batch_size, dev)
@@ -447,23 +452,30 @@ class DecodeSession(Session):
 
     def _make_step_copies(self) -> None:
         """What a step reads of the stream-layout copies, made in one go ahead of it."""
-        rows = self.tile_gemv or self.tile_rows or self.chain
+        rows = self.tile_gemv or self.tile_rows or (self.chain and not self.chain_packed)
         gated = rows and self.swiglu_epilogue and (self.chain or getattr(self.model, "exchange", None) is None)
         if (rows or self.B > 16) and not capturing(self.dev):
             make_copies([(lin, int(gated and gate_up)) for lin, gate_up in self._linears() if lin.in_features % 128 == 0])
 
-    def _copied_linears(self) -> list[tuple[dict, tuple]]:
-        return [(lin._buffers, lin._wstream_of) for lin, _ in self._linears() if "_wstream_of" in lin.__dict__]
+    def _weights(self) -> list[tuple[dict, tuple]]:
+        """Every linear's buffers, and the tensors and versions that its copies were made of, or that it has now."""
+        return [(lin._buffers, lin.__dict__.get("_wstream_of") or lin.weights_now()) for lin, _ in self._linears()]
 
     def _on_capture(self) -> None:
-        self._copied = self._copied_linears()
+        self._captured = self._weights()
 
     def _on_prompt(self) -> None:
-        """Captured prompts and steps replay over copies of the weights: where some are of weights that were replaced, all are made
-        again before either runs."""
-        if self._copied and not _lib.bind().all_current(self._copied) and not capturing(self.dev):
-            make_copies([(lin, mode) for lin, _ in self._linears() for mode, name in enumerate(COPIES) if name in lin.__dict__])
-            self._copied = self._copied_linears()
+        """Captured prompts and steps replay over copies of the weights and over the packed bytes: where a linear has other weights
+        than at the last capture, all copies are made again before either runs, and what was captured over tensors that others have
+        replaced is captured again."""
+        if not self._captured or _lib.bind().all_current(self._captured) or capturing(self.dev):
+            return
+        make_copies([(lin, mode) for lin, _ in self._linears() for mode, name in enumerate(COPIES) if name in lin.__dict__])
+        if any(buffers.get("packed_indices") is not of[0] or buffers.get("codebook") is not of[1] for buffers, of in self._captured):
+            torch.cuda.synchronize(self.dev)
+            self.graph = None
+            self._prefill_graphs.clear()
+        self._captured = self._weights()
 
     def _chain_layers(self) -> torch.Tensor:
         """The layers of a step through nb_chain_linear, five launches each: q | k | v, attention, out_proj, gate and up, down.
@@ -472,17 +484,17 @@ class DecodeSession(Session):
         Up to CHAIN_TERM_ROWS sequences a launch leaves the residual stream's rows, times the next norm's weight, as terms, and the norm's
         scale is a factor on the sums behind: the terms of small rows keep fewer bits (a relative 4.5e-8 at rms 1, 9e-7 at 0.02).  More
         sequences are normed where they are split, 4.5e-8 whatever the stream's size: 16 of the 2.2B shape with 12 layers take 934 us
-        a step for it, 857 with terms."""
+        a step for it, 865 with terms.  9 to 16 read the packed bytes: 943, and nothing to follow when these are written to."""
         m, x, eps = self.model, self.bx, self.model.config.norm_eps
         normed = self.B > CHAIN_TERM_ROWS
         ops.chain_embed(m.embedding, self.token, m.blocks[0].ln1, x, None if normed else self.cx, self.csq)
 
         def weight(lin, mode):
-            return lin.stream_weight(1 if mode == ops.CHAIN_SWIGLU else 0)
+            return lin.packed_indices if self.chain_packed else lin.stream_weight(1 if mode == ops.CHAIN_SWIGLU else 0)
 
         def linear(mode, lin, x_terms, behind=None, **kw):
             ops.chain_linear(mode, weight(lin, mode), lin.bits, self.B, lin.out_features, lin.in_features, x_terms, self.cstatus,
-                             ahead=behind, **kw)
+                             ahead=behind, codebook=lin.codebook if self.chain_packed else None, **kw)
 
         def norm_linear(mode, lin, norm, behind, **kw):
             rows = dict(x=x, x_weight=norm) if normed else {}

@@ -481,12 +481,14 @@ def chain_terms(m: int, k: int, device) -> torch.Tensor:
 def chain_linear(mode: int, w_stream: torch.Tensor, bits: int, m: int, n: int, k: int, x_terms: torch.Tensor | None, status: torch.Tensor,
                  sq: torch.Tensor | None = None, eps: float = 0.0, y: torch.Tensor | None = None, y_terms: torch.Tensor | None = None,
                  residual: torch.Tensor | None = None, next_weight: torch.Tensor | None = None, sq_out: torch.Tensor | None = None,
-                 ahead: torch.Tensor | None = None, split: int = 0, x: torch.Tensor | None = None, x_weight: torch.Tensor | None = None) -> None:
+                 ahead: torch.Tensor | None = None, split: int = 0, x: torch.Tensor | None = None, x_weight: torch.Tensor | None = None,
+                 codebook: torch.Tensor | None = None) -> None:
     """One packed linear of the decode chain (nb_chain_linear): m fp32 rows of k columns given as terms, sq (m, .) the partial sums
     of squares of the rows in front of their norm.  CHAIN_STORE: y (m, n).  CHAIN_SWIGLU: y_terms of n / 2 columns (w packed with
     row_mode 1).  CHAIN_RESIDUAL: residual (m, n) += y, and with y_terms and sq_out the terms and partial sums for the linear behind.
     x in place of x_terms: the rows themselves, fp32 (m, k); with sq they are normed, times x_weight (k), before they are split.
-    ahead: the stream-layout weights of the linear behind, fetched into L2 meanwhile."""
+    codebook: w_stream is the packed matrix itself, gate and up the halves of its rows.
+    ahead: the weights of the linear behind, fetched into L2 meanwhile."""
     _need_cuda(w_stream, status)
     n_out = n // 2 if mode == CHAIN_SWIGLU else n
     for name, t, size in (("sq", sq, None), ("y", y, m * n), ("residual", residual, m * n), ("next_weight", next_weight, n),
@@ -502,7 +504,8 @@ def chain_linear(mode: int, w_stream: torch.Tensor, bits: int, m: int, n: int, k
     ptr = lambda t: None if t is None else t.data_ptr()
     args = _lib.ChainArgs(w_stream.data_ptr(), ptr(x_terms), ptr(sq), ptr(y), ptr(y_terms), ptr(residual), ptr(next_weight),
                           ptr(sq_out), status.data_ptr(), ptr(ahead), 0 if ahead is None else ahead.numel(), float(eps), m, n, k, bits, mode,
-                          0 if sq is None else sq.numel() // m, split, x=ptr(x), x_weight=ptr(x_weight))
+                          0 if sq is None else sq.numel() // m, split, x=ptr(x), x_weight=ptr(x_weight), codebook=ptr(codebook),
+                          codebook_dtype=0 if codebook is None else _DTYPE[codebook.dtype])
     with torch.cuda.device(w_stream.device):
         _lib.check(_lib.lib().nb_chain_linear(_c.byref(args), _stream()), "nb_chain_linear")
 

@@ -77,8 +77,7 @@ def make_copies(wanted) -> None:
                 todo[id(lin), mode] = (lin, mode)
     made, of = [], {}
     for lin, mode in todo.values():
-        p, c = lin.packed_indices, lin.codebook
-        of.setdefault(lin, (p, c, _version(p), _version(c)))
+        p, c, *_ = of.setdefault(lin, lin.weights_now())
         made.append((lin, COPIES[mode], stream_pack(p, c, lin.bits, lin.out_features, lin.in_features, mode)))
     for device in {w.device for _, _, w in made}:
         _finish(device, any(w.device == device and lin.__dict__.get(name) is not None for lin, name, w in made))
@@ -168,6 +167,11 @@ class PackedLinear(torch.nn.Module):
                 return None
             make_copies([(self, row_mode)])
         return self.__dict__[COPIES[row_mode]]
+
+    def weights_now(self) -> tuple:
+        """The tensors and versions that a copy made now is of."""
+        p, c = self.packed_indices, self.codebook
+        return p, c, _version(p), _version(c)
 
     def _copied_now(self) -> bool:
         """Whether the copies are of the weights as they are now."""

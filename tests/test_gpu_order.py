@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from nativebit_b200 import PackedLinear, ops
+from nativebit_b200 import generate as G
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -81,28 +82,65 @@ def test_a_linear_whose_first_call_of_many_rows_is_captured(built_lib, rows):
         assert (got.double() - want).norm() <= 2e-6 * want.norm()
 
 
-@pytest.mark.parametrize("batch", [1, 4])
-def test_sessions_follow_other_weights_from_the_next_prompt_on(built_lib, batch):
-    """After other weights were loaded under captured prompts and steps, a prompt of a known and one of a new length and the steps behind
-    them are those of a session made with these weights."""
-    from nativebit_b200 import generate as G
+def _run(session, prompt, steps=3):
+    """The logits of a prompt and of the steps behind it over given tokens."""
+    out = [session.prefill(prompt).clone()]
+    for _ in range(steps):
+        session.token.fill_(7)
+        session.step()
+        out.append(session.logits.clone())
+    return torch.stack(out)
+
+
+def _two_models():
     cfg = G.ModelConfig(vocab_size=512, n_layers=2, n_embd=256, n_head=4, ffn_hidden=512, context_len=64)
-    model, other = G.PackedGPT.random_init(cfg, seed=0), G.PackedGPT.random_init(cfg, seed=1)
+    return G.PackedGPT.random_init(cfg, seed=0), G.PackedGPT.random_init(cfg, seed=1)
+
+
+@pytest.mark.parametrize("batch", [1, 4, 12, 40])
+def test_sessions_follow_other_weights_from_the_next_prompt_on(built_lib, batch):
+    """After other weights were loaded under captured prompts and steps, or took the place of the tensors, a prompt of a known and one
+    of a new length and the steps behind them are those of a session made with these weights."""
+    model, other = _two_models()
+    third = G.PackedGPT.random_init(model.config, seed=2)
     g = torch.Generator(device=DEV).manual_seed(6)
     prompts = [torch.randint(0, 512, (batch, t), device=DEV, generator=g) for t in (20, 20, 33)]
-
-    def run(session, prompt):
-        out = [session.prefill(prompt).clone()]
-        for _ in range(3):
-            session.token.fill_(7)
-            session.step()
-            out.append(session.logits.clone())
-        return torch.stack(out)
-
     session = model.session(batch)
-    run(session, prompts[0])
+    _run(session, prompts[0])
     model.load_state_dict(other.state_dict())
     for prompt in prompts[1:]:
-        assert torch.equal(run(session, prompt), run(other.session(batch), prompt))
-    for a, b in zip(model.blocks, other.blocks):
+        assert torch.equal(_run(session, prompt), _run(other.session(batch), prompt))
+    for a, b in zip(model.blocks, third.blocks):
+        for name in ("qkv", "out_proj", "gate_up", "down"):
+            getattr(a, name).packed_indices, getattr(a, name).codebook = getattr(b, name).packed_indices, getattr(b, name).codebook
+    model.embedding.copy_(third.embedding)
+    for prompt in prompts[1:]:
+        assert torch.equal(_run(session, prompt), _run(third.session(batch), prompt))
+    for a, b in zip(model.blocks, third.blocks):
         assert torch.equal(a.gate_up.stream_weight(1), b.gate_up.stream_weight(1)) and torch.equal(a.qkv.stream_weight(), b.qkv.stream_weight())
+
+
+@pytest.mark.parametrize("batch", [9, 16])
+def test_captured_steps_over_the_packed_bytes_follow_what_is_written_to_them(built_lib, batch):
+    """Nine to sixteen sequences: a step that was captured before other weights were written in place, counted or not, multiplies them."""
+    model, other = _two_models()
+    session = model.session(batch)
+    assert session.chain_packed
+    prompt = torch.randint(0, 512, (batch, 1), device=DEV)
+    _run(session, prompt)
+    for blk, src in zip(model.blocks, other.blocks):
+        for name in ("qkv", "out_proj", "gate_up", "down"):
+            getattr(blk, name).packed_indices.data.copy_(getattr(src, name).packed_indices)
+            getattr(blk, name).codebook.data.copy_(getattr(src, name).codebook)
+    torch.cuda.synchronize()
+    want = other.session(batch)
+    for s in (session, want):
+        s.reset()
+        s.token.fill_(3)
+        for k, v, _ in s.caches:
+            k.zero_(), v.zero_()
+    model.embedding.copy_(other.embedding)
+    for _ in range(3):
+        session.step(), want.step()
+        assert torch.equal(session.logits, want.logits)
+    assert not any("_wstream" in lin.__dict__ for blk in model.blocks for lin in (blk.qkv, blk.out_proj, blk.gate_up, blk.down))
