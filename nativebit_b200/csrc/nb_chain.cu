@@ -615,12 +615,13 @@ extern "C" size_t nb_chain_terms_bytes(int M, int K) { return M < 1 || K < kBloc
 
 // Whether nb_chain_linear is the faster one for more rows than its columns were made for.  Its MMAs and parts grow with the rows, the
 // tcgen05 kernel has its start, its k-steps and a sum over k splits whatever the rows are (fused | this, us, 3 bits, fp32 rows:
-// 3072 x 1024 17 rows 8.4 | 5.5, 64: 11.5 | 8.5; 2560 x 2560 32: 10.9 | 9.4, 48: 10.4 | 11.6; 6144 x 2048 17: 10.7 | 10.8; bf16 6144 x 2048 32:
-// 11.0 | 9.4, 48: 11.7 | 17.7; 7680 x 2560 17: 12.1 | 10.9, 24: 12.2 | 17.6): up to 400 M products in one launch.
+// 3072 x 1024 40 rows 11.1 | 7.2, 64: 12.0 | 8.6; 2560 x 2560 32: 11.6 | 9.4, 40: 10.8 | 11.2; 6144 x 2048 17: 11.8 | 10.9, 20: 11.8 | 11.5;
+// bf16 6144 x 2048 32: 12.1 | 9.5; 7680 x 2560 20: 13.4 | 11.7, 24, which takes two launches: 13.4 | 17.4): up to 510 M products in one
+// launch (453 - 503 M: 13824 x 512 32 rows 9.2 | 9.4, 1000 x 4096 56: 12.0 | 10.0, 4096 x 2048 28: 11.1 | 10.9).
 extern "C" int nb_chain_takes(int M, int N, int K, int bits, int x_dtype) {
   if (M < 1 || N < 1 || K < kBlock || K % kBlock || (bits != 2 && bits != 3 && bits != 4) || M > 64) return 0;
   const int terms = x_dtype == NB_F32 ? 2 : 1;
-  if ((double)M * terms * N * K > 400e6 || check_device() != NB_OK) return 0;
+  if ((double)M * terms * N * K > 510e6 || check_device() != NB_OK) return 0;
   ChainPlan pl{}, best{};
   best.cost = 1e30;
   for (int S : {1, 2, 4, 8})

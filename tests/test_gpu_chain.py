@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 import torch
 
-from nativebit_b200 import ops
+from nativebit_b200 import PackedLinear, ops
 from nativebit_b200.stream import stream_pack
 from oracle import nb_oracle as o
 
@@ -195,3 +195,17 @@ def test_chain_rows_over_the_packed_bytes(built_lib, n, k, m, dtype, bits):
         ops.chain_rows(x, p[:-16], bits, n, k, codebook=cb)
     with pytest.raises(RuntimeError):
         ops.chain_rows(x, p, bits, n, k, codebook=cb[:-1])
+
+
+@pytest.mark.parametrize("m,n,k,dtype,takes", [(64, 3072, 1024, torch.float32, True), (32, 6144, 2048, torch.bfloat16, True), (32, 2560, 2560, torch.float32, True),
+                                               (64, 2560, 2560, torch.bfloat16, True), (40, 2560, 2560, torch.float32, False),
+                                               (48, 6144, 2048, torch.bfloat16, False), (24, 7680, 2560, torch.float32, False), (65, 256, 256, torch.float32, False)])
+def test_rows_that_are_faster_here_come_here(built_lib, m, n, k, dtype, takes):
+    """The line between this kernel and the tcgen05 one, and that a call of PackedLinear on either side of it is right."""
+    assert ops.chain_takes(m, n, k, 3, dtype) == takes
+    packed, cb, _ = o.make_packed_linear(n, k, 3, seed=m)
+    lin = PackedLinear(torch.from_numpy(packed).to(DEV), torch.from_numpy(cb).to(DEV), n, k)
+    x = torch.randn(m, k, device=DEV, generator=torch.Generator(device=DEV).manual_seed(k)).to(dtype)
+    want = x.double() @ lin.dequantized_weight().double().T
+    for _ in range(2):                                     # the general path, then the native call
+        _close(lin(x), want, {torch.float32: 10 * REL, torch.bfloat16: 2.0 ** -8}[dtype])       # (the GEMM's tolerance elsewhere is 2e-5 of max |y|)
