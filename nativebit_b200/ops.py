@@ -478,6 +478,12 @@ def chain_terms(m: int, k: int, device) -> torch.Tensor:
     return torch.zeros(int(_lib.lib().nb_chain_terms_bytes(m, k)), dtype=torch.uint8, device=device)
 
 
+def _check_packed(name: str, packed: torch.Tensor, codebook: torch.Tensor, n: int, k: int, bits: int) -> None:
+    if (packed.dtype != torch.uint8 or packed.numel() < packed_nbytes(n * k, bits) or codebook.dtype not in (torch.float16, torch.float32)
+            or codebook.numel() != n * k // 128 << bits):
+        raise RuntimeError(f"{name}: packed bytes and codebooks of an ({n}, {k}) matrix at {bits} bits are needed")
+
+
 def chain_linear(mode: int, w_stream: torch.Tensor, bits: int, m: int, n: int, k: int, x_terms: torch.Tensor | None, status: torch.Tensor,
                  sq: torch.Tensor | None = None, eps: float = 0.0, y: torch.Tensor | None = None, y_terms: torch.Tensor | None = None,
                  residual: torch.Tensor | None = None, next_weight: torch.Tensor | None = None, sq_out: torch.Tensor | None = None,
@@ -489,8 +495,14 @@ def chain_linear(mode: int, w_stream: torch.Tensor, bits: int, m: int, n: int, k
     x in place of x_terms: the rows themselves, fp32 (m, k); with sq they are normed, times x_weight (k), before they are split.
     codebook: w_stream is the packed matrix itself, gate and up the halves of its rows.
     ahead: the weights of the linear behind, fetched into L2 meanwhile."""
-    _need_cuda(w_stream, status)
+    _need_cuda(w_stream, status, *(t for t in (x_terms, y_terms, ahead, codebook) if t is not None))
     n_out = n // 2 if mode == CHAIN_SWIGLU else n
+    if codebook is not None:
+        _check_packed("chain_linear", w_stream, codebook, n, k, bits)
+    elif w_stream.dtype != torch.uint8 or w_stream.numel() < int(_lib.lib().nb_stream_packed_bytes(n, k, bits)):
+        raise RuntimeError(f"chain_linear: the stream-layout bytes of an ({n}, {k}) matrix at {bits} bits are needed")
+    if status.dtype != torch.int32 or status.numel() < 1 or (ahead is not None and ahead.dtype != torch.uint8):
+        raise RuntimeError("chain_linear: status must be int32, ahead uint8")
     for name, t, size in (("sq", sq, None), ("y", y, m * n), ("residual", residual, m * n), ("next_weight", next_weight, n),
                           ("sq_out", sq_out, m * (n // 16)), ("x", x, m * k), ("x_weight", x_weight, k)):
         if t is not None and (t.dtype != torch.float32 or not t.is_cuda or not t.is_contiguous() or (size is not None and t.numel() != size)):
@@ -499,8 +511,9 @@ def chain_linear(mode: int, w_stream: torch.Tensor, bits: int, m: int, n: int, k
         raise RuntimeError(f"chain_linear: sq must hold {m} rows of partial sums")
     if (x_terms is None) == (x is None):
         raise RuntimeError("chain_linear: the rows are given as terms or plainly")
-    if x_terms is not None and (not x_terms.is_cuda or x_terms.numel() < 4 * m * k) or (y_terms is not None and (not y_terms.is_cuda or y_terms.numel() < 4 * m * n_out)):
-        raise RuntimeError("chain_linear: a buffer of terms is too small")
+    for t, size in ((x_terms, 4 * m * k), (y_terms, 4 * m * n_out)):
+        if t is not None and (t.dtype != torch.uint8 or t.numel() < size):
+            raise RuntimeError(f"chain_linear: a buffer of terms must be {size} bytes (chain_terms)")
     ptr = lambda t: None if t is None else t.data_ptr()
     args = _lib.ChainArgs(w_stream.data_ptr(), ptr(x_terms), ptr(sq), ptr(y), ptr(y_terms), ptr(residual), ptr(next_weight),
                           ptr(sq_out), status.data_ptr(), ptr(ahead), 0 if ahead is None else ahead.numel(), float(eps), m, n, k, bits, mode,
@@ -538,9 +551,9 @@ def chain_rows(x: torch.Tensor, w_stream: torch.Tensor, bits: int, n: int, k: in
         raise RuntimeError(f"x must be a contiguous float (M, {k}) tensor; got {x.dtype} {tuple(x.shape)}")
     if codebook is not None:
         _need_cuda(codebook)
-        if (w_stream.dtype != torch.uint8 or w_stream.numel() < packed_nbytes(n * k, bits) or codebook.dtype not in (torch.float16, torch.float32)
-                or codebook.numel() != n * k // 128 << bits):
-            raise RuntimeError(f"chain_rows: packed bytes and codebooks of an ({n}, {k}) matrix at {bits} bits are needed")
+        _check_packed("chain_rows", w_stream, codebook, n, k, bits)
+    elif w_stream.dtype != torch.uint8 or w_stream.numel() < int(_lib.lib().nb_stream_packed_bytes(n, k, bits)):
+        raise RuntimeError(f"chain_rows: the stream-layout bytes of an ({n}, {k}) matrix at {bits} bits are needed")
     if out is None:
         out = torch.empty(x.shape[0], n, dtype=x.dtype, device=x.device)
     with torch.cuda.device(x.device):
@@ -559,10 +572,13 @@ def chain_rows(x: torch.Tensor, w_stream: torch.Tensor, bits: int, n: int, k: in
 def chain_embed(table: torch.Tensor, token: torch.Tensor, weight: torch.Tensor | None, x: torch.Tensor, terms: torch.Tensor | None,
                 sq: torch.Tensor) -> None:
     """x = table[token] (bf16 -> fp32), terms = x * weight (None: not needed), sq = its partial sums of squares (nb_chain_embed)."""
+    if terms is not None and weight is None:
+        raise RuntimeError("chain_embed: terms need the norm's weight")
     _need_cuda(table, token, x, sq, *(() if terms is None else (weight, terms)))
     b, c = x.shape
-    if (table.dtype != torch.bfloat16 or token.dtype != torch.int64 or token.numel() != b or (terms is not None and terms.numel() < 4 * b * c)
-            or sq.numel() != b * (c // 16)):
+    if (table.dtype != torch.bfloat16 or table.dim() != 2 or table.shape[1] != c or token.dtype != torch.int64 or token.numel() != b
+            or x.dtype != torch.float32 or sq.dtype != torch.float32 or sq.numel() != b * (c // 16)
+            or (terms is not None and (terms.dtype != torch.uint8 or terms.numel() < 4 * b * c or weight.dtype != torch.float32 or weight.numel() != c))):
         raise RuntimeError("chain_embed: bad tensors")
     with torch.cuda.device(x.device):
         _lib.check(_lib.lib().nb_chain_embed(table.data_ptr(), token.data_ptr(), b, table.shape[0], c, None if terms is None else weight.data_ptr(),
@@ -571,9 +587,13 @@ def chain_embed(table: torch.Tensor, token: torch.Tensor, weight: torch.Tensor |
 
 def decode_attention_terms(qkv, cos2, sin2, pos, k_cache, v_cache, terms, out_cols: int, out_offset: int) -> None:
     """decode_attention_rope with its result as terms of rows of out_cols columns."""
+    _need_cuda(qkv, cos2, sin2, pos, k_cache, v_cache, terms)
     b, h, ctx, hd = k_cache.shape
-    if terms.numel() < 4 * b * out_cols:
-        raise RuntimeError("decode_attention_terms: the buffer of terms is too small")
+    if (any(t.dtype != torch.float32 for t in (qkv, cos2, sin2, k_cache, v_cache)) or v_cache.shape != k_cache.shape or qkv.numel() != 3 * b * h * hd
+            or min(cos2.numel(), sin2.numel()) < ctx * hd or pos.dtype != torch.int64 or pos.numel() < 1):
+        raise RuntimeError("decode_attention_terms: bad tensors")
+    if terms.dtype != torch.uint8 or terms.numel() < 4 * b * out_cols:
+        raise RuntimeError(f"decode_attention_terms: the buffer of terms must be {4 * b * out_cols} bytes (chain_terms)")
     _lib.check(_lib.lib().nb_decode_attention_terms(qkv.data_ptr(), cos2.data_ptr(), sin2.data_ptr(), pos.data_ptr(), k_cache.data_ptr(),
                                                     v_cache.data_ptr(), b, h, hd, ctx, terms.data_ptr(), out_cols, out_offset, _stream()),
                "nb_decode_attention_terms")

@@ -209,3 +209,52 @@ def test_rows_that_are_faster_here_come_here(built_lib, m, n, k, dtype, takes):
     want = x.double() @ lin.dequantized_weight().double().T
     for _ in range(2):                                     # the general path, then the native call
         _close(lin(x), want, {torch.float32: 10 * REL, torch.bfloat16: 2.0 ** -8}[dtype])       # (the GEMM's tolerance elsewhere is 2e-5 of max |y|)
+
+
+def test_the_wrappers_refuse_what_does_not_fit(built_lib):
+    """Sizes and types of every tensor are checked before a launch."""
+    n, k, m, bits = 256, 128, 2, 3
+    w, _ = _matrix(n, k, bits, 1)
+    packed, cb, _ = o.make_packed_linear(n, k, bits, seed=1)
+    packed, cb = torch.from_numpy(packed).to(DEV), torch.from_numpy(cb).to(DEV)
+    f32 = dict(device=DEV, dtype=torch.float32)
+    status, x, y = torch.zeros(1, dtype=torch.int32, device=DEV), torch.randn(m, k, **f32), torch.empty(m, n, **f32)
+    sq, terms = torch.ones(m, k // 16, **f32), _terms(x)
+
+    def linear(w=w, x_terms=terms, status=status, **kw):
+        ops.chain_linear(ops.CHAIN_STORE, w, bits, m, n, k, x_terms, status, **{"y": y, **kw})
+    linear()
+    linear(x_terms=None, x=x, sq=sq, x_weight=torch.ones(k, **f32))
+    linear(w=packed, codebook=cb)
+    for bad in (dict(w=w[:-16]), dict(w=w.view(torch.int8)), dict(x_terms=terms[:-2]), dict(x_terms=terms.view(torch.float16)), dict(status=status.long()),
+                dict(x_terms=None), dict(x=x), dict(x_terms=None, x=x[:, :-1]), dict(x_terms=None, x=x.half()), dict(sq=sq[0, :3]),
+                dict(x_terms=None, x=x, sq=sq), dict(x_terms=None, x=x, sq=sq, x_weight=torch.ones(k - 1, **f32)), dict(w=packed[:-1], codebook=cb),
+                dict(w=packed, codebook=cb[1:]), dict(w=packed, codebook=cb.double()), dict(y=y[:1]), dict(y=y.half()), dict(ahead=w.view(torch.int32)),
+                dict(w=w.cpu()), dict(y_terms=terms.cpu())):
+        with pytest.raises(RuntimeError):
+            linear(**bad)
+    for bad in ((w[:-16], None), (packed, cb[1:]), (packed[:-1], cb), (w.view(torch.int8), None)):
+        with pytest.raises(RuntimeError):
+            ops.chain_rows(x, bad[0], bits, n, k, codebook=bad[1])
+
+    table, token = torch.randn(9, k, device=DEV).bfloat16(), torch.zeros(m, 1, dtype=torch.long, device=DEV)
+    good = dict(table=table, token=token, weight=torch.ones(k, **f32), x=x, terms=terms, sq=sq)
+    ops.chain_embed(**good)
+    ops.chain_embed(**{**good, "weight": None, "terms": None})
+    for bad in (dict(weight=torch.ones(k, device=DEV).half()), dict(weight=torch.ones(k - 1, **f32)), dict(table=table.float()), dict(table=table[:, 1:].contiguous()),
+                dict(token=token.int()), dict(terms=terms[:-2]), dict(terms=terms.view(torch.float16)), dict(sq=sq[:1]), dict(x=x.half()), dict(sq=sq.half())):
+        with pytest.raises(RuntimeError):
+            ops.chain_embed(**{**good, **bad})
+
+    heads, hd, ctx = 2, 64, 8
+    good = dict(qkv=torch.randn(m, 3 * heads * hd, **f32), cos2=torch.ones(ctx, hd, **f32), sin2=torch.zeros(ctx, hd, **f32),
+                pos=torch.zeros(1, dtype=torch.long, device=DEV), k_cache=torch.zeros(m, heads, ctx, hd, **f32), v_cache=torch.zeros(m, heads, ctx, hd, **f32),
+                terms=ops.chain_terms(m, heads * hd, DEV), out_cols=heads * hd, out_offset=0)
+    ops.decode_attention_terms(**good)
+    for name, bad in (("qkv", good["qkv"][:, 1:].contiguous()), ("qkv", good["qkv"].half()), ("cos2", good["cos2"][:-1]), ("sin2", good["sin2"].double()),
+                      ("pos", good["pos"].int()), ("k_cache", good["k_cache"].half()), ("v_cache", good["v_cache"][:, :, :-1].contiguous()),
+                      ("k_cache", good["k_cache"].transpose(1, 2)), ("terms", good["terms"][:-2]), ("terms", good["terms"].view(torch.float16)),
+                      ("qkv", good["qkv"].cpu())):
+        with pytest.raises(RuntimeError):
+            ops.decode_attention_terms(**{**good, name: bad})
+    torch.cuda.synchronize()
