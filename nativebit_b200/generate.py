@@ -360,7 +360,8 @@ class DecodeSession(Session):
     (inference/generate_torch.py:91-97)."""
 
     def __init__(self, model: PackedGPT, batch_size: int = 1, use_graph: bool = True, fused: bool = True,
-                 batch_gemm: bool = False, stream: bool | None = None, tile_gemv: bool | None = None, hand_head: bool = True):
+                 batch_gemm: bool = False, stream: bool | None = None, tile_gemv: bool | None = None, hand_head: bool = True,
+                 chain: bool | None = None):
         super().__init__(model, batch_size, model.context_len, model.config.vocab_size, model.embedding.device, use_graph)
         self.hand_head = hand_head            # False: the LM head of a single sequence stays a library GEMM (comparison)
         self.residual_in_matvec = False       # True: out_proj and down add into the residual stream themselves (flag 4 of
@@ -381,8 +382,8 @@ class DecodeSession(Session):
         self.tile_rows = bool(fits and 2 <= batch_size <= 8 and fused and tile_gemv is not False
                               and getattr(model, "exchange", None) is None)
         # the default for both on one GPU: a chain in which every launch hands the next its activations ready for the tensor cores
-        # (nb_chain_linear)
-        self.chain = bool(fits and fused and tile_gemv is not False and model.tp_size == 1
+        # (nb_chain_linear); chain=False keeps the kernels above, chain=True refuses a model that has to use them
+        self.chain = bool(chain is not False and fits and fused and tile_gemv is not False and model.tp_size == 1
                           and getattr(model, "exchange", None) is None and model.embedding.dtype == torch.bfloat16
                           and model.config.n_embd % 128 == 0 and all(b.gate_up.out_features % 256 == 0 for b in model.blocks)
                           and (not CHAIN_TERM_ROWS < batch_size <= CHAIN_MAX_ROWS
@@ -390,6 +391,8 @@ class DecodeSession(Session):
                                       for t in (l.packed_indices, l.codebook)))
                           and (batch_size <= CHAIN_MAX_ROWS or all(ops.chain_takes(batch_size, l.out_features, l.in_features, l.bits, torch.float32)
                                                                    for b in model.blocks for l in (b.qkv, b.out_proj, b.gate_up, b.down))))
+        if chain and not self.chain:
+            raise RuntimeError("the chain of packed linears needs one rank, a bf16 table, whole blocks of 128 and few rows or small matrices")
         # 9 .. 16 sequences: over the packed bytes, which need no copy and follow whatever is written to them
         self.chain_packed = self.chain and CHAIN_TERM_ROWS < batch_size <= CHAIN_MAX_ROWS
         # stream=True (one sequence on one GPU): the whole step is ONE launch of the persistent kernel

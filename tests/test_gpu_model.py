@@ -419,7 +419,7 @@ def test_captured_steps_outlive_a_longer_prompt(built_lib, B):
     cfg = G.ModelConfig(vocab_size=512, n_layers=2, n_embd=512, n_head=4, ffn_hidden=6912, context_len=256)
     model = G.PackedGPT.random_init(cfg, seed=5, device=dev)
     toks = torch.randint(0, cfg.vocab_size, (B, 130), generator=torch.Generator().manual_seed(B)).to(dev)
-    a, b = G.DecodeSession(model, B), G.DecodeSession(model, B, use_graph=False)
+    a, b = G.DecodeSession(model, B, chain=False), G.DecodeSession(model, B, use_graph=False, chain=False)
     for s in (a, b):
         s.prefill(toks[:, :3])
         s.step()
@@ -470,7 +470,8 @@ def test_prompt_calls_the_linears_that_others_look_at(built_lib):
     assert torch.equal(logits(model), want)
 
 
-def test_norm_weights_at_any_place_of_a_buffer(built_lib):
+@pytest.mark.parametrize("chain", [False, True])
+def test_norm_weights_at_any_place_of_a_buffer(built_lib, chain):
     """Norm weights that are views at odd places of one buffer: prompts and steps of more than 16 rows give the same logits as with
     weights of their own."""
     from nativebit_b200 import generate as G
@@ -488,7 +489,7 @@ def test_norm_weights_at_any_place_of_a_buffer(built_lib):
                     w = torch.cat((buf[:at], w))[at:]
                     assert w.data_ptr() % 16
                 setattr(blk, name, w)
-        s = G.DecodeSession(model, 20, use_graph=False)
+        s = G.DecodeSession(model, 20, use_graph=False, chain=chain)
         first = s.prefill(toks).clone()
         s.step()
         got.append((first, s.logits.clone()))

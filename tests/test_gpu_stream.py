@@ -328,17 +328,17 @@ def test_decode_step_on_the_stream_layout_equals_the_workspace_kernels(built_lib
     cfg = G.ModelConfig(vocab_size=512, n_layers=3, n_embd=512, n_head=4, ffn_hidden=1408, context_len=64)
     model = G.PackedGPT.random_init(cfg, seed=5, device=dev)
     prompt = torch.randint(0, cfg.vocab_size, (1, 7), generator=torch.Generator().manual_seed(1)).to(dev)
-    a = G.DecodeSession(model, 1, use_graph=False, tile_gemv=True)
+    a = G.DecodeSession(model, 1, use_graph=False, tile_gemv=True, chain=False)
     b = G.DecodeSession(model, 1, use_graph=False, tile_gemv=False)
-    assert a.tile_gemv and not b.tile_gemv
+    assert a.tile_gemv and not b.tile_gemv and not a.chain and not b.chain
     a.prefill(prompt); b.prefill(prompt)
     for _ in range(12):
         a.step(); b.step()
         assert torch.equal(a.token, b.token)
         assert (a.logits - b.logits).abs().max() <= 1e-4 * b.logits.abs().max()
-    g = G.DecodeSession(model, 1, use_graph=True, tile_gemv=True)
+    g = G.DecodeSession(model, 1, use_graph=True, tile_gemv=True, chain=False)
     toks_g = g.generate(prompt, 12)
-    toks_e = G.DecodeSession(model, 1, use_graph=False, tile_gemv=True).generate(prompt, 12)
+    toks_e = G.DecodeSession(model, 1, use_graph=False, tile_gemv=True, chain=False).generate(prompt, 12)
     assert torch.equal(toks_g, toks_e)
 
 
@@ -352,16 +352,16 @@ def test_batched_decode_step_on_the_rows_kernel_equals_the_workspace_kernels(bui
     cfg = G.ModelConfig(vocab_size=512, n_layers=3, n_embd=512, n_head=4, ffn_hidden=1408, context_len=64)
     model = G.PackedGPT.random_init(cfg, seed=5, device=dev)
     prompt = torch.randint(0, cfg.vocab_size, (B, 7), generator=torch.Generator().manual_seed(B)).to(dev)
-    a = G.DecodeSession(model, B, use_graph=False)
+    a = G.DecodeSession(model, B, use_graph=False, chain=False)
     b = G.DecodeSession(model, B, use_graph=False, tile_gemv=False)
-    assert a.tile_rows and not b.tile_rows
+    assert a.tile_rows and not b.tile_rows and not a.chain and not b.chain
     a.prefill(prompt); b.prefill(prompt)
     for _ in range(10):
         a.step(); b.step()
         assert torch.equal(a.token, b.token)
         assert (a.logits - b.logits).abs().max() <= 1e-4 * b.logits.abs().max()
-    toks_g = G.DecodeSession(model, B, use_graph=True).generate(prompt, 10)
-    toks_e = G.DecodeSession(model, B, use_graph=False).generate(prompt, 10)
+    toks_g = G.DecodeSession(model, B, use_graph=True, chain=False).generate(prompt, 10)
+    toks_e = G.DecodeSession(model, B, use_graph=False, chain=False).generate(prompt, 10)
     assert torch.equal(toks_g, toks_e)
 
 
@@ -375,7 +375,7 @@ def test_batched_step_with_a_wide_down_projection(built_lib, B, tensor_cores):
     assert (B > 2 * ops.gemv_stream_max_rows(cfg.bits, cfg.ffn_hidden)) == tensor_cores
     model = G.PackedGPT.random_init(cfg, seed=5, device=dev)
     prompt = torch.randint(0, cfg.vocab_size, (B, 7), generator=torch.Generator().manual_seed(B)).to(dev)
-    a, g = G.DecodeSession(model, B, use_graph=False), G.DecodeSession(model, B)
+    a, g = G.DecodeSession(model, B, use_graph=False, chain=False), G.DecodeSession(model, B, chain=False)
     b = G.DecodeSession(model, B, use_graph=False, tile_gemv=False)
     for s in (a, g, b):
         s.prefill(prompt)
