@@ -402,7 +402,9 @@ def test_quantize_pack_dequant_edges_of_the_wide_kernels(dev, bits, total, block
 def test_quantize_pack_finds_the_first_nearest_entry(dev, bits):
     """The search over ordered codebooks against the trial of every entry in fp32, where the two could part: ties, entries out of
     order, equal, close together, infinite or NaN, weights on, between and far beyond the entries."""
-    e, block, rows = 1 << bits, 128, 4096                      # enough weights for the kernel that searches
+    e, block = 1 << bits, 160                                  # (160: no power of two)
+    rows = -(-(1 << 21) // block)                              # enough weights for the kernel that searches at 3 and at 4 bits
+    total = rows * block - 37                                  # the last block ends inside
     g = torch.Generator().manual_seed(bits)
     cb = (0.02 * torch.randn(rows, e, generator=g)).sort(dim=1).values
     w = 0.02 * torch.randn(rows, block, generator=g)
@@ -419,12 +421,13 @@ def test_quantize_pack_finds_the_first_nearest_entry(dev, bits):
     w[9] = 1e-40 * e * torch.rand(block, generator=g)
     w[10] = cb[10][torch.arange(block) % e]
     cb[11] = torch.linspace(-3e38, 3e38, e)
+    w.view(-1)[total:] = 0                                     # what fills the last block
     best, want = (w - cb[:, :1]).abs(), torch.zeros(rows, block, dtype=torch.uint8)
     for i in range(1, e):
         d = (w - cb[:, i:i + 1]).abs()
         want[d < best] = i
         best = torch.where(d < best, d, best)
     from nativebit_b200 import ops
-    got = ops.unpack(ops.quantize_pack(w.reshape(-1).to(dev), cb.to(dev), block, bits), bits, rows * block).cpu().view(rows, block)
+    got = ops.unpack(ops.quantize_pack(w.reshape(-1)[:total].to(dev), cb.to(dev), block, bits), bits, rows * block).cpu().view(rows, block)
     wrong = (got != want).nonzero()
     assert len(wrong) == 0, (wrong[:5], got[got != want][:5], want[got != want][:5])
