@@ -16,14 +16,14 @@
 //    of all of them and pushes its parts into the shared memory of the CTA that finishes the tile.
 //  * Plain rows of up to 16 may come against the packed matrix itself (kRaw): what is written to it is what the next call reads, and
 //    nothing has to be made or kept beside it.  Unpacking costs a unit about 55 clocks more than the copy's selector words, and the
-//    products wait for all of a CTA's weights (2560 x 6912, 16 bf16 rows 11.4 us against 9.7 over the copy and 13.9 for nb_gemv;
-//    2560 x 2560, 8 rows 5.9, 5.0, 7.8; 13824 x 2560, 16 fp32 rows 24.6, 21.3, 35.9).  With a barrier per tile and an arrival per copying
+//    products wait for all of a CTA's weights (2560 x 6912, 16 bf16 rows 11.3 us against 9.5 over the copy and 13.9 for nb_gemv;
+//    2560 x 2560, 8 rows 5.8, 4.8, 7.8; 13824 x 2560, 16 fp32 rows 24.6, 21.3, 35.9).  With a barrier per tile and an arrival per copying
 //    thread on it 12.7, 6.6.
 //  * Column 2r + s of the MMAs carries term s of activation row r: one product covers four fp32 rows.
-// Decode step of the 2.2B decoder with 12 layers (us), matvecs that stage the rows themselves -> this: 1 sequence 437 -> 388, 2:
-// 539 -> 443, 8: 665 -> 510, 16 (a matvec over the packed bytes and launches between): 1523 -> 943 over the packed matrix, rows
-// given plainly and normed before they are split (934 over the copy; 865 with terms, which keep fewer bits of small rows).  17 and more rows stay on
-// the tcgen05 kernel (32: 1121, here 1460).  For one sequence a layer's 28 us are four times 1.3 us from the end of a launch
+// Decode step of the 2.2B decoder with 12 layers (us), matvecs that stage the rows themselves -> this: 1 sequence 437 -> 384, 2:
+// 539 -> 448, 8: 665 -> 498, 16 (a matvec over the packed bytes and launches between): 1523 -> 943 over the packed matrix, rows
+// given plainly and normed before they are split (934 over the copy; 865 with terms, which keep fewer bits of small rows).  17 and
+// more rows stay on the tcgen05 kernel (32: 1121, here 1460).  For one sequence a layer's 28 us are four times 1.3 us from the end of a launch
 // to the next one's first dependent instruction, 12.5 us of products (66 clocks per unit and SM against 54 without copies; down
 // projections wait for the 12 SMs with two tiles), 4.4 us of attention and the rest staging and sums.  Measured and not kept:
 // 12 or 16 warps so that the next launch's CTA is resident early (391 -> 421, 442), clusters of 2 or 4 for balance (no
@@ -60,20 +60,18 @@ __device__ __forceinline__ bool chain_wait(uint64_t* bar, uint32_t parity, int* 
 }
 
 struct ChainParams {
-  const uint8_t* w;           // stream layout, or with a codebook the packed rows themselves
-  const uint8_t* cb;          // the packed rows' codebooks (null: stream layout), cb_block bytes per block
+  const uint8_t* w;           // stream layout, or (kRaw) the packed rows themselves
   const uint8_t* xt;          // activations as terms
   const float* ss;            // (M, ss_n) partial sums of squares of the rows in front of the norm (null: no norm)
   void* y;                    // NB_CHAIN_STORE: (M, N) of type y_dtype
   uint8_t* yt;                // the other two: terms of the next linear's activations (null: none)
   float* res;                 // NB_CHAIN_RESIDUAL: (M, N), updated in place
-  const float* w_next;        // ... the next norm's weight
+  const float* w_next;        // ... the next norm's weight; with x and ss that of the norm of the rows themselves
   float* ss_out;              // ... (M, N / 16) partial sums of squares of the new rows (null: none)
   const uint8_t* ahead;       // weights of the launch behind (null: none), `ahead_step` bytes per CTA
   int* status;
   unsigned ahead_bytes, ahead_step;
   const void* x;              // plain activations (M, K) of type x_dtype instead of the terms (null: none)
-  const float* x_weight;      // ... with ss: the weight of their norm
   int x_dtype, y_dtype;
   int N, bpr, M, mode, ss_n;
   float eps;
@@ -82,8 +80,15 @@ struct ChainParams {
   unsigned rcp_clusters, rcp_kc, rcp_kc1;     // ceil(2^32 / v) of the clusters, the smaller and the larger share of a row's blocks
   int tile0, n_tiles;         // row tiles of this launch
   int w_bytes, J;             // room for weights; partial results per tile and CTA
-  int cb_dtype, cb_block, idx_stride, cb_stride;      // packed rows: bytes from row to row in shared memory
 };
+// What only packed rows need; the other kernels' launches do not carry it.
+struct ChainRaw {
+  const uint8_t* cb;          // codebooks of type cb_dtype, cb_block bytes per block
+  int cb_dtype, cb_block;
+  int idx_stride, cb_stride;  // bytes from row to row in shared memory
+};
+struct ChainCopy {};
+template <bool kRaw> using ChainLayout = std::conditional_t<kRaw, ChainRaw, ChainCopy>;
 // v / d for v * d < 2^32 (d == 1 has no 32-bit reciprocal)
 __device__ __forceinline__ int div_rcp(int v, int d, unsigned rcp) { return d == 1 ? v : (int)__umulhi((unsigned)v, rcp); }
 
@@ -121,15 +126,15 @@ template <int BITS> __device__ __forceinline__ void packed_selectors(const uint8
 // 16 rows x 128 weights against CG groups of eight columns.  kRaw: `ub` and `cb` are this lane's indices and codebook of row g, those
 // of row g + 8 eight strides on.
 template <int BITS, int CG, bool kRaw>
-__device__ __forceinline__ void chain_unit(const ChainParams& p, const uint8_t* ub, const uint8_t* cb, const uint8_t* const (&x)[CG], int lane,
+__device__ __forceinline__ void chain_unit(const ChainLayout<kRaw>& raw, const uint8_t* ub, const uint8_t* cb, const uint8_t* const (&x)[CG], int lane,
                                            const ByteShift& sm, uint32_t act, uint4 (&last)[1], float (&c)[CG == 1 ? 2 : CG][4]) {
   const int g = lane >> 2, t = lane & 3;
   uint32_t UA[4], UB[4], TA[BITS == 4 ? 8 : 4], TB[BITS == 4 ? 8 : 4];
-  if (kRaw) {
+  if constexpr (kRaw) {
     packed_selectors<BITS>(ub, UA);
-    packed_selectors<BITS>(ub + 8 * p.idx_stride, UB);
-    make_table<BITS>(cb, p.cb_dtype, true, TA);
-    make_table<BITS>(cb + 8 * p.cb_stride, p.cb_dtype, true, TB);
+    packed_selectors<BITS>(ub + 8 * raw.idx_stride, UB);
+    make_table<BITS>(cb, raw.cb_dtype, true, TA);
+    make_table<BITS>(cb + 8 * raw.cb_stride, raw.cb_dtype, true, TB);
   } else {
     unit_selectors(ub, lane, 0, UA);
     unit_selectors(ub, lane, 1, UB);
@@ -173,8 +178,10 @@ __device__ __forceinline__ float row_scale(const ChainParams& p, int r, int lane
 
 // Shared memory: the CTA's units, tile after tile (kRaw: a tile's 16 rows of indices, then of codebooks) | staged columns (XT m_part of kc_max * 256 bytes) | partial
 // results [own tile][CTA][J][row][16] of the tiles this CTA finishes.
-template <int BITS, int CG, int XT, bool kCluster, bool kRaw>
-__global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p) {
+// kPlain: plain activations.  (As a run-time choice the code that converts and norms them, and the packed rows' parameters in every
+// launch, cost launches whose rows are terms 0.2 us each: a step of the 2.2B decoder with 12 layers 398 us, now 384.)
+template <int BITS, int CG, int XT, bool kCluster, bool kRaw, bool kPlain>
+__global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p, const ChainLayout<kRaw> raw) {
   constexpr int kUnit = StreamUnit<BITS>::kBytes;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ uint64_t s_bar[kChainTiles], s_xbar;
@@ -197,9 +204,8 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
       src += (size_t)p.clusters * p.bpr * kUnit;
     }
   }
-  const int tile_bytes = 16 * (p.idx_stride + p.cb_stride);
-  if (kRaw) {                                               // thread after thread takes the next piece of a row: indices, then codebooks
-    const int idx_pieces = kc * BITS, cb_piece = p.cb_block >= 16 ? 16 : 8, per_row = idx_pieces + kc * p.cb_block / cb_piece;
+  if constexpr (kRaw) {                                     // thread after thread takes the next piece of a row: indices, then codebooks
+    const int idx_pieces = kc * BITS, cb_piece = raw.cb_block >= 16 ? 16 : 8, per_row = idx_pieces + kc * raw.cb_block / cb_piece;
     const int rows = kCThreads / per_row, rest = kCThreads - rows * per_row;
     int r = tid / per_row, c = tid - r * per_row;
     for (;;) {
@@ -208,12 +214,12 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
       const int i = r >> 4, row = r & 15, tile = p.tile0 + ci + i * p.clusters;
       const int n = p.mode == NB_CHAIN_SWIGLU ? tile * 8 + (row & 7) + (row & 8 ? p.N >> 1 : 0) : min(tile * 16 + row, p.N - 1);
       const size_t block = (size_t)(n * p.bpr + k0);
-      uint8_t* dst = smem + i * tile_bytes;
+      uint8_t* dst = smem + i * 16 * (raw.idx_stride + raw.cb_stride);
       if (c < idx_pieces) {
-        cp_async16(dst + row * p.idx_stride + 16 * c, p.w + block * (16 * BITS) + 16 * c);
+        cp_async16(dst + row * raw.idx_stride + 16 * c, p.w + block * (16 * BITS) + 16 * c);
       } else {
-        dst += 16 * p.idx_stride + row * p.cb_stride + cb_piece * (c - idx_pieces);
-        const uint8_t* src = p.cb + block * p.cb_block + cb_piece * (c - idx_pieces);
+        dst += 16 * raw.idx_stride + row * raw.cb_stride + cb_piece * (c - idx_pieces);
+        const uint8_t* src = raw.cb + block * raw.cb_block + cb_piece * (c - idx_pieces);
         if (cb_piece == 16) cp_async16(dst, src);
         else cp_async8(dst, src);
       }
@@ -240,8 +246,8 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
   asm volatile("griddepcontrol.launch_dependents;");
 
   const uint8_t* xt = p.xt + ((size_t)(2 * row0) * p.bpr + k0) * 256;
-  const bool bulk = !p.x && (kRaw || 2 * m * kc > kChainBulk);      // (a wait for 16-byte copies would be one for the weights')
-  if (XT == 1 || p.x) {                                     // converted here; four pieces of eight values per thread on the way
+  const bool bulk = !kPlain && (kRaw || 2 * m * kc > kChainBulk);      // (a wait for 16-byte copies would be one for the weights')
+  if (kPlain) {                                             // converted here; four pieces of eight values per thread on the way
     const int chunks = kc * 16, total = m * chunks;         // of a row, of all
     constexpr int kAhead = 4;
     for (int base = 0; base < total; base += kAhead * kCThreads) {
@@ -267,8 +273,8 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
         if (i0 + q * kCThreads < total) {
           if (XT == 2 && p.ss) {
             float w[8];
-            const float* src = p.x_weight + k0 * kBlock + n[q];
-            if ((uintptr_t)p.x_weight % 16 == 0) {
+            const float* src = p.w_next + k0 * kBlock + n[q];
+            if ((uintptr_t)p.w_next % 16 == 0) {
               load_x8(src, NB_F32, 0, w);
             } else {
 #pragma unroll
@@ -323,7 +329,7 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
   }
   // requested here, used behind the products: a row's partial sums of squares (one warp per row), residual values
   constexpr int kSq = 6;
-  const bool sq_late = p.ss != nullptr && p.x == nullptr, sq_mine = sq_late && warp < m;
+  const bool sq_late = !kPlain && p.ss != nullptr, sq_mine = sq_late && warp < m;
   const float* sq = p.ss + (size_t)(row0 + warp) * p.ss_n;
   float sqv[kSq];
 #pragma unroll
@@ -367,16 +373,17 @@ __global__ void __launch_bounds__(kCThreads, 1) chain_kernel(const ChainParams p
 #pragma unroll
     for (int j = 0; j < CG; ++j) xp[j] = xc[j] + kk * 256;
     const int tile_end = min(ub, u + kc - kk);
-    if (kRaw) {
-      up = smem + i * tile_bytes + g * p.idx_stride + (4 * kk + t) * (4 * BITS);
-      cp = smem + i * tile_bytes + 16 * p.idx_stride + g * p.cb_stride + kk * p.cb_block;
+    if constexpr (kRaw) {
+      const uint8_t* tile = smem + i * 16 * (raw.idx_stride + raw.cb_stride);
+      up = tile + g * raw.idx_stride + (4 * kk + t) * (4 * BITS);
+      cp = tile + 16 * raw.idx_stride + g * raw.cb_stride + kk * raw.cb_block;
     }
     if (!kRaw) chain_wait(&s_bar[i], 0, p.status);
 #pragma unroll (CG == 1 ? 2 : 1)
     for (; u < tile_end; ++u) {
-      chain_unit<BITS, CG, kRaw>(p, up, cp, xp, lane, sm, act, x_last, c);
+      chain_unit<BITS, CG, kRaw>(raw, up, cp, xp, lane, sm, act, x_last, c);
       up += kRaw ? 16 * BITS : kUnit;
-      if (kRaw) cp += p.cb_block;
+      if constexpr (kRaw) cp += raw.cb_block;
 #pragma unroll
       for (int j = 0; j < CG; ++j) xp[j] += 256;
     }
@@ -535,13 +542,13 @@ static bool chain_plan(int N, int bpr, int M, int terms, bool plain, int bits, i
   return false;
 }
 
-template <int BITS, int CG, int XT, bool kCluster, bool kRaw>
-static int chain_launch_as(const ChainPlan& pl, const ChainParams& p, bool ordered, cudaStream_t st) {
+template <int BITS, int CG, int XT, bool kCluster, bool kRaw, bool kPlain>
+static int chain_launch_as(const ChainPlan& pl, const ChainParams& p, const ChainLayout<kRaw>& raw, bool ordered, cudaStream_t st) {
   static bool done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!done[dev & 63]) {
-    if (cudaError_t e = cudaFuncSetAttribute(chain_kernel<BITS, CG, XT, kCluster, kRaw>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmemMax))
+    if (cudaError_t e = cudaFuncSetAttribute(chain_kernel<BITS, CG, XT, kCluster, kRaw, kPlain>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmemMax))
       return record_cuda_error(e);
     done[dev & 63] = true;
   }
@@ -562,19 +569,26 @@ static int chain_launch_as(const ChainPlan& pl, const ChainParams& p, bool order
     attr[cfg.numAttrs].val.clusterDim.y = 1;
     attr[cfg.numAttrs++].val.clusterDim.z = 1;
   }
-  return record_cuda_error(cudaLaunchKernelEx(&cfg, chain_kernel<BITS, CG, XT, kCluster, kRaw>, p));
+  return record_cuda_error(cudaLaunchKernelEx(&cfg, chain_kernel<BITS, CG, XT, kCluster, kRaw, kPlain>, p, raw));
 }
 template <int BITS, bool kRaw>
-static int chain_launch(const ChainPlan& pl, const ChainParams& p, bool ordered, cudaStream_t st) {
-  const auto run = [&](auto cg, auto xt) {
+static int chain_launch(const ChainPlan& pl, const ChainParams& p, const ChainLayout<kRaw>& raw, bool ordered, cudaStream_t st) {
+  const auto run = [&](auto cg, auto xt, auto plain) {
     constexpr int CG = decltype(cg)::value, XT = decltype(xt)::value;
-    return pl.S > 1 ? chain_launch_as<BITS, CG, XT, true, kRaw>(pl, p, ordered, st) : chain_launch_as<BITS, CG, XT, false, kRaw>(pl, p, ordered, st);
+    constexpr bool kPlain = decltype(plain)::value;
+    return pl.S > 1 ? chain_launch_as<BITS, CG, XT, true, kRaw, kPlain>(pl, p, raw, ordered, st)
+                    : chain_launch_as<BITS, CG, XT, false, kRaw, kPlain>(pl, p, raw, ordered, st);
   };
-  using std::integral_constant;
-  if (pl.terms == 1) return pl.cg == 1 ? run(integral_constant<int, 1>{}, integral_constant<int, 1>{}) : run(integral_constant<int, 2>{}, integral_constant<int, 1>{});
-  if (pl.cg == 1) return run(integral_constant<int, 1>{}, integral_constant<int, 2>{});
-  if (pl.cg == 2) return run(integral_constant<int, 2>{}, integral_constant<int, 2>{});
-  return run(integral_constant<int, 4>{}, integral_constant<int, 2>{});
+  const std::integral_constant<int, 1> one{};
+  const std::integral_constant<int, 2> two{};
+  const std::integral_constant<int, 4> four{};
+  if (pl.terms == 1) return pl.cg == 1 ? run(one, one, std::true_type{}) : run(two, one, std::true_type{});
+  if (p.x) return pl.cg == 1 ? run(one, two, std::true_type{}) : pl.cg == 2 ? run(two, two, std::true_type{}) : run(four, two, std::true_type{});
+  if constexpr (!kRaw) {                                    // (terms against packed rows: steps of 9 to 16 sequences)
+    if (pl.cg == 1) return run(one, two, std::false_type{});
+    if (pl.cg == 2) return run(two, two, std::false_type{});
+  }
+  return run(four, two, std::false_type{});
 }
 
 // Clusters of S CTAs with a whole SM each that the device runs at once.
@@ -597,8 +611,8 @@ static int max_clusters(int S) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int got = 0;
-    if (cudaFuncSetAttribute(chain_kernel<3, 1, 2, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmemMax) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&got, chain_kernel<3, 1, 2, true, false>, &cfg) != cudaSuccess || got < 1) {
+    if (cudaFuncSetAttribute(chain_kernel<3, 1, 2, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmemMax) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&got, chain_kernel<3, 1, 2, true, false, false>, &cfg) != cudaSuccess || got < 1) {
       cudaGetLastError();
       got = 1;
     }
@@ -641,7 +655,7 @@ extern "C" int nb_chain_takes_packed(int M, int N, int K, int bits, int x_dtype)
 
 extern "C" int nb_chain_linear(const nb_chain_args* a, void* stream) {
   constexpr long long kMost = 1ll << 26;                    // products of sizes below stay in 32 bits
-  if (!a || !a->w || (a->x ? a->sq && (!a->x_weight || a->x_dtype != NB_F32) : !a->x_terms) || !a->status || a->M < 1 || a->N < 1) return NB_ERR_ARG;
+  if (!a || !a->w || (a->x ? a->sq && (!a->x_weight || a->x_dtype != NB_F32 || a->mode == NB_CHAIN_RESIDUAL) : !a->x_terms) || !a->status || a->M < 1 || a->N < 1) return NB_ERR_ARG;
   if (a->mode < NB_CHAIN_STORE || a->mode > NB_CHAIN_RESIDUAL) return NB_ERR_ARG;
   if (a->mode == NB_CHAIN_STORE ? !a->y : a->mode == NB_CHAIN_SWIGLU ? !a->y_terms : !a->residual) return NB_ERR_ARG;
   if (a->mode == NB_CHAIN_RESIDUAL && a->y_terms && (!a->next_weight || !a->sq_out)) return NB_ERR_ARG;
@@ -667,11 +681,10 @@ extern "C" int nb_chain_linear(const nb_chain_args* a, void* stream) {
   }
   if (best.cost == 1e30) return NB_ERR_SHAPE;
   ChainParams p{};
-  p.cb = reinterpret_cast<const uint8_t*>(a->codebook); p.cb_dtype = a->codebook_dtype; p.cb_block = cb_block;
-  p.idx_stride = best.idx_stride; p.cb_stride = best.cb_stride;
+  const ChainRaw raw{reinterpret_cast<const uint8_t*>(a->codebook), a->codebook_dtype, cb_block, best.idx_stride, best.cb_stride};
   p.w = a->w; p.xt = reinterpret_cast<const uint8_t*>(a->x_terms); p.ss = a->sq; p.y = a->y; p.yt = reinterpret_cast<uint8_t*>(a->y_terms);
-  p.res = a->residual; p.w_next = a->next_weight; p.ss_out = a->sq_out; p.status = a->status;
-  p.x = a->x; p.x_weight = a->x_weight; p.x_dtype = a->x_dtype; p.y_dtype = a->y_dtype;
+  p.res = a->residual; p.w_next = a->x && a->sq ? a->x_weight : a->next_weight; p.ss_out = a->sq_out; p.status = a->status;
+  p.x = a->x; p.x_dtype = a->x_dtype; p.y_dtype = a->y_dtype;
   p.N = a->N; p.bpr = bpr; p.M = a->M; p.mode = a->mode; p.ss_n = a->sq_n; p.eps = a->eps;
   p.m_part = best.m_part; p.parts = best.parts; p.lg_split = best.S == 8 ? 3 : best.S >> 1; p.w_bytes = best.w_bytes; p.J = best.J;
   auto rcp = [](int v) { return (unsigned)((0x100000000ull + v - 1) / v); };
@@ -689,12 +702,12 @@ extern "C" int nb_chain_linear(const nb_chain_args* a, void* stream) {
     }
     int rc = NB_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    const auto run = [&](auto raw) {
-      constexpr bool kRaw = decltype(raw)::value;
-      return a->bits == 2 ? chain_launch<2, kRaw>(best, p, a->ordered, st) : a->bits == 3 ? chain_launch<3, kRaw>(best, p, a->ordered, st)
-                                                                                         : chain_launch<4, kRaw>(best, p, a->ordered, st);
+    const auto run = [&](auto packed, const auto& layout) {
+      constexpr bool kRaw = decltype(packed)::value;
+      return a->bits == 2 ? chain_launch<2, kRaw>(best, p, layout, a->ordered, st) : a->bits == 3 ? chain_launch<3, kRaw>(best, p, layout, a->ordered, st)
+                                                                                                 : chain_launch<4, kRaw>(best, p, layout, a->ordered, st);
     };
-    rc = a->codebook ? run(std::true_type{}) : run(std::false_type{});
+    rc = a->codebook ? run(std::true_type{}, raw) : run(std::false_type{}, ChainCopy{});
     if (rc) return rc;
   }
   return NB_OK;
