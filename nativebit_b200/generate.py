@@ -25,7 +25,7 @@ import torch
 import torch.nn.functional as F
 
 from . import _lib, ops, synthetic, tp
-from .packed_linear import COPIES, PackedLinear, capturing, make_copies
+from .packed_linear import COPIES, FUSED_MAX_ROWS, GEMV_MAX_M, PackedLinear, capturing, make_copies
 from .session import Session
 
 
@@ -458,7 +458,7 @@ class DecodeSession(Session):
         rows = self.tile_gemv or self.tile_rows or (self.chain and not self.chain_packed)
         gated = rows and self.swiglu_epilogue and (self.chain or getattr(self.model, "exchange", None) is None)
         if (rows or self.B > 16) and not capturing(self.dev):
-            make_copies([(lin, int(gated and gate_up)) for lin, gate_up in self._linears() if lin.in_features % 128 == 0])
+            make_copies([(lin, int(gated and gate_up)) for lin, gate_up in self._linears() if lin._tensor_cores()])
 
     def _weights(self) -> list[tuple[dict, tuple]]:
         """Every linear's buffers, and the tensors and versions that its copies were made of, or that it has now."""
@@ -641,6 +641,8 @@ class DecodeSession(Session):
         ops.softcap_argmax(logits, cfg.logit_cap, self.logits, self.token, self.pos)
 
     def _prefill_body(self, prompt: torch.Tensor) -> None:
+        if GEMV_MAX_M < prompt.numel() <= FUSED_MAX_ROWS // 2 and not capturing(self.dev):      # rows that are multiplied over the copies
+            make_copies([(lin, 0) for lin, _ in self._linears() if lin._tensor_cores()])
         caches = [(k, v, 0) for k, v, _ in self.caches]
         logits, _ = self.model(prompt, kv_caches=caches, last_only=True)      # the caches are written in place
         self.pos.fill_(prompt.shape[1])
