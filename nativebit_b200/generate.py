@@ -521,9 +521,9 @@ class DecodeSession(Session):
 
     @torch.no_grad()
     def _step_body_fused(self):
-        """The decode step on the fused kernels.  Up to 8 sequences: 5 launches per layer (residual add +
-        RMSNorm and SwiGLU are computed inside the packed GEMVs that consume them); more: 7 to 12 (a norm or SwiGLU in front
-        of three linears, a conversion in front of out_proj, a sum behind every linear whose k range is split)."""
+        """The decode step on the fused kernels.  The chain (`_chain_layers`): 5 launches per layer.  Without it, up to 8 sequences: 5 as
+        well (residual add + RMSNorm and SwiGLU are computed inside the packed GEMVs that consume them); more: 7 to 12 (a norm or SwiGLU
+        in front of three linears, a conversion in front of out_proj, a sum behind every linear whose k range is split)."""
         m, cfg = self.model, self.model.config
         eps = cfg.norm_eps
         self._make_step_copies()

@@ -104,7 +104,8 @@ class PackedLinear(torch.nn.Module):
 
     Buffers keep the reference's names: `packed_indices` (flat uint8 in the nativebit/pack.py
     layout) and `codebook` ((num_blocks, 2**bits), fp16 or fp32).  forward accepts any leading
-    dims; the result has x's dtype.
+    dims; the result has x's dtype.  Calls of up to 16 rows and of more than 1024 (512 of fp32) multiply these
+    buffers; those between keep a tile-major copy of them (stream_weight), which the first such call makes and waits for.
     """
 
     def __init__(self, packed_indices, codebook, out_features, in_features, bits: int = 3, block_size: int = BS):
