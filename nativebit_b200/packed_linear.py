@@ -84,7 +84,8 @@ def make_copies(wanted) -> None:
     for lin, name, w in made:
         old = lin.__dict__.get(name)
         if old is not None and old.device == w.device and old.shape == w.shape:
-            old.copy_(w)
+            with torch.inference_mode():        # either may be an inference tensor
+                old.copy_(w)
         else:
             setattr(lin, name, w)
     for device in {w.device for _, _, w in made}:

@@ -54,6 +54,19 @@ def test_both_copies_follow_other_weights_at_their_place(packing):
     assert places == (plain.data_ptr(), gated.data_ptr())
 
 
+@pytest.mark.parametrize("first", [True, False])
+def test_copies_are_made_again_inside_and_outside_of_inference_mode(packing, first):
+    """A copy that was made under inference mode is an inference tensor, which nothing outside of it may write to."""
+    lin, second = _linear(0), _linear(1)
+    with torch.inference_mode(first):
+        w = lin.stream_weight()
+    lin.load_state_dict(second.state_dict())
+    with torch.inference_mode(not first):
+        assert lin.stream_weight() is w and _is_of(w, second, 0)
+        lin.packed_indices.add_(1)
+        assert _is_of(lin.stream_weight(), lin, 0)
+
+
 def test_a_graph_that_is_captured_makes_no_copy_for_others(packing, monkeypatch):
     lin = _linear(0)
     monkeypatch.setattr(packed_linear, "capturing", lambda device: True)
