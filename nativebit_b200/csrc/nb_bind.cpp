@@ -43,6 +43,26 @@ bool copy_of(PyObject* of, PyObject* packed, PyObject* codebook) {
   return true;
 }
 
+// The weights of the last launch over the packed bytes, [packed, codebook, version, version] or [] (or just whether to order it): whether
+// these are others.
+bool unseen(PyObject* seen, PyObject* packed, PyObject* codebook) {
+  if (!PyList_CheckExact(seen)) return PyObject_IsTrue(seen) == 1;
+  if (PyList_GET_SIZE(seen) != 4 || PyList_GET_ITEM(seen, 0) != packed || PyList_GET_ITEM(seen, 1) != codebook) return true;
+  for (int i = 0; i < 2; ++i) {
+    const at::Tensor& t = THPVariable_Unpack(i ? codebook : packed);
+    if (PyLong_AsLongLong(PyList_GET_ITEM(seen, 2 + i)) != (t.is_inference() ? -1 : t._version())) return true;
+  }
+  return false;
+}
+void note_seen(PyObject* seen, PyObject* packed, PyObject* codebook) {
+  if (!PyList_CheckExact(seen)) return;
+  const at::Tensor &p = THPVariable_Unpack(packed), &c = THPVariable_Unpack(codebook);
+  PyObject* now = Py_BuildValue("[OOLL]", packed, codebook, (long long)(p.is_inference() ? -1 : p._version()),
+                                (long long)(c.is_inference() ? -1 : c._version()));
+  if (now) PyList_SetSlice(seen, 0, PyList_GET_SIZE(seen), now);
+  Py_XDECREF(now);
+}
+
 // all_current([(a module's buffers, what its copy was made of), ..]) -> whether every copy is of the module's present weights
 PyObject* all_current(PyObject*, PyObject* list) {
   HANDLE_TH_ERRORS
@@ -60,7 +80,8 @@ PyObject* all_current(PyObject*, PyObject* list) {
   END_HANDLE_TH_ERRORS
 }
 
-// linear(x, packed, codebook, w_stream or None, what it was made of, n, k, bits, ordered, gemv workspaces, prefill workspaces) -> y or None
+// linear(x, packed, codebook, w_stream or None, what it was made of, n, k, bits, seen (`unseen`), gemv workspaces, prefill
+// workspaces) -> y or None
 PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
   HANDLE_TH_ERRORS
   if (count != 11) {
@@ -71,7 +92,7 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
     Py_RETURN_NONE;
   const at::Tensor &x = THPVariable_Unpack(a[0]), &packed = THPVariable_Unpack(a[1]), &codebook = THPVariable_Unpack(a[2]);
   const int64_t n = PyLong_AsLongLong(a[5]), k = PyLong_AsLongLong(a[6]);
-  const int bits = (int)PyLong_AsLong(a[7]), ordered = PyObject_IsTrue(a[8]);
+  const int bits = (int)PyLong_AsLong(a[7]);
   if (PyErr_Occurred()) return nullptr;
   const int xt = tag(x.scalar_type()), ct = tag(codebook.scalar_type());
   if (xt < 0 || (ct != NB_F16 && ct != NB_F32) || !x.is_cuda() || x.layout() != at::kStrided || x.dim() < 1 || x.size(-1) != k || !x.is_contiguous() ||
@@ -84,6 +105,7 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
   at::DimVector shape(x.sizes());
   shape.back() = n;
   int rc = NB_ERR_ARG;
+  const bool ordered = m <= kGemvRows && unseen(a[8], a[1], a[2]);
   const bool few = nb_chain_takes_packed((int)m, (int)n, (int)k, bits, xt) != 0;     // over the packed bytes; more rows of a small matrix over its copy
   if (few || (m > kGemvRows && THPVariable_CheckExact(a[3]) && nb_chain_takes((int)m, (int)n, (int)k, bits, xt))) {
     const at::Tensor &w = THPVariable_Unpack(a[few ? 1 : 3]), ws = workspace(a[10], device.index(), stream);
@@ -108,7 +130,10 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
     Py_BEGIN_ALLOW_THREADS
     rc = nb_chain_linear(&args, stream);
     Py_END_ALLOW_THREADS
-    if (rc == NB_OK) return THPVariable_Wrap(std::move(y));
+    if (rc == NB_OK) {
+      if (few && ordered) note_seen(a[8], a[1], a[2]);
+      return THPVariable_Wrap(std::move(y));
+    }
   } else if (m <= kGemvRows) {
     const at::Tensor ws = workspace(a[9], device.index(), stream);
     if (!ws.defined()) Py_RETURN_NONE;
@@ -120,7 +145,10 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
     Py_BEGIN_ALLOW_THREADS
     rc = (ordered ? nb_gemv_ordered : nb_gemv)(xp, xt, (int)m, pp, cp, ct, bits, kBlock, (int)n, (int)k, yp, xt, wp, wn, stream);
     Py_END_ALLOW_THREADS
-    if (rc == NB_OK) return THPVariable_Wrap(std::move(y));
+    if (rc == NB_OK) {
+      if (ordered) note_seen(a[8], a[1], a[2]);
+      return THPVariable_Wrap(std::move(y));
+    }
   } else if (xt != NB_F16 && m * (xt == NB_F32 ? 2 : 1) <= kFusedRows && THPVariable_CheckExact(a[3])) {       // (that kernel writes bf16 or fp32)
     const at::Tensor &w = THPVariable_Unpack(a[3]), ws = workspace(a[10], device.index(), stream);
     if (!ws.defined() || w.device() != device || !copy_of(a[4], a[1], a[2])) Py_RETURN_NONE;

@@ -117,17 +117,15 @@ class PackedLinear(torch.nn.Module):
         self.in_features = int(in_features)
         self.bits = int(bits)
         self.block_size = int(block_size)
-        # The buffers may have been written by kernels still in flight (from_packed / pack_linear pack on
-        # the device): the first fused launch is fully stream-ordered, later ones may start early.
-        self._fresh = True
+        # The buffers may have been written by kernels still in flight (from_packed / pack_linear pack on the device, weights are
+        # loaded): the first launch over other weights than these is fully stream-ordered, later ones may start early.
+        self._seen = []
 
     def forward(self, x):
         if self.block_size == BS and x.is_cuda:      # the plain calls: checks, result and launch in one native function
             y = _lib.bind().linear(x, self.packed_indices, self.codebook, self.__dict__.get("_wstream"), self.__dict__.get("_wstream_of"),
-                                   self.out_features, self.in_features, self.bits, self._fresh, ops._workspaces, ops._prefill_ws)
+                                   self.out_features, self.in_features, self.bits, self._seen, ops._workspaces, ops._prefill_ws)
             if y is not None:
-                if self._fresh:
-                    self._fresh = False
                 return y
         shape = x.shape
         x_flat = x.reshape(-1, self.in_features)
@@ -144,9 +142,7 @@ class PackedLinear(torch.nn.Module):
             pass
         elif m <= GEMV_MAX_M:
             y = ops.gemv(x_flat, self.packed_indices, self.codebook, self.bits, self.block_size,
-                         self.out_features, self.in_features, ordered=self._fresh)
-            if self._fresh:
-                self._fresh = False
+                         self.out_features, self.in_features, ordered=self._unseen())
         else:
             y = self._forward_many(x_flat)
         return y.reshape(*shape[:-1], self.out_features)
@@ -170,6 +166,14 @@ class PackedLinear(torch.nn.Module):
             make_copies([(self, row_mode)])
         return self.__dict__[COPIES[row_mode]]
 
+    def _unseen(self) -> bool:
+        """Whether the launch that follows is the first over the packed bytes as they are now."""
+        now, seen = self.weights_now(), self._seen
+        if len(seen) == 4 and seen[0] is now[0] and seen[1] is now[1] and (seen[2], seen[3]) == now[2:]:
+            return False
+        seen[:] = now
+        return True
+
     def weights_now(self) -> tuple:
         """The tensors and versions that a copy made now is of."""
         p, c = self.packed_indices, self.codebook
@@ -184,10 +188,10 @@ class PackedLinear(torch.nn.Module):
         """2 to 16 rows on the chain's kernel over the packed bytes, None where nb_gemv takes them."""
         if not ops.chain_takes_packed(x_flat.shape[0], self.out_features, self.in_features, self.bits, x_flat.dtype) or x_flat.data_ptr() % 16 or self.packed_indices.data_ptr() % 16 or self.codebook.data_ptr() % 16:
             return None
-        y = ops.chain_rows(x_flat, self.packed_indices, self.bits, self.out_features, self.in_features, ordered=self._fresh,
+        y = ops.chain_rows(x_flat, self.packed_indices, self.bits, self.out_features, self.in_features, ordered=self._unseen(),
                            codebook=self.codebook)
-        if y is not None and self._fresh:
-            self._fresh = False
+        if y is None:
+            self._seen.clear()              # nothing was launched
         return y
 
     def _forward_many(self, x_flat):

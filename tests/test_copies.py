@@ -98,3 +98,13 @@ def test_native_check_of_many_copies(packing, built_lib):
         assert not _lib.bind().all_current(wrong)
     with pytest.raises(TypeError):
         _lib.bind().all_current(None)
+
+
+def test_the_first_launch_over_other_weights_is_ordered():
+    """Behind a load of other weights a launch over the packed bytes may not start beside the launch that writes them."""
+    lin, other = _linear(0), _linear(1)
+    assert lin._unseen() and not lin._unseen()
+    lin.load_state_dict(other.state_dict())
+    assert lin._unseen() and not lin._unseen()
+    lin.codebook = other.codebook
+    assert lin._unseen() and not lin._unseen()
