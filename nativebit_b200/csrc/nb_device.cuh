@@ -97,7 +97,7 @@ __device__ __forceinline__ void lookup4(uint32_t sel, const uint32_t (&T)[BITS =
 // 256 and -256 as values that the compiler cannot see through, so that a multiply-add by them stays one.  Byte permutes, logic
 // and shifts share one pipe of 64 lanes per clock and SM, which bounds every kernel that looks weights up; multiply-adds run
 // beside it on another (measured on B200, lanes per clock and SM: permute, logic or shift 64, multiply-add 64, the two in turn
-// 130; the high half of a product 32, so right shifts stay shifts).  gridDim.z is 1 wherever this is used.
+// 124; the high half of a product 32, so right shifts stay shifts).  gridDim.z is 1 wherever this is used.
 struct ByteShift {
   uint32_t up, down;
 };
