@@ -78,17 +78,19 @@ def make_copies(wanted) -> None:
     made, of = [], {}
     for lin, mode in todo.values():
         p, c, *_ = of.setdefault(lin, lin.weights_now())
-        made.append((lin, COPIES[mode], stream_pack(p, c, lin.bits, lin.out_features, lin.in_features, mode)))
+        made.append((lin, COPIES[mode], stream_pack(p, c, lin.bits, lin.out_features, lin.in_features, mode, apart=False)))
     for device in {w.device for _, _, w in made}:
         _finish(device, any(w.device == device and lin.__dict__.get(name) is not None for lin, name, w in made))
+    again = set()
     for lin, name, w in made:
         old = lin.__dict__.get(name)
         if old is not None and old.device == w.device and old.shape == w.shape:
             with torch.inference_mode():        # either may be an inference tensor
                 old.copy_(w)
+            again.add(w.device)
         else:
             setattr(lin, name, w)
-    for device in {w.device for _, _, w in made}:
+    for device in again:
         _finish(device, False)
     for lin, key in of.items():
         lin._wstream_of = key

@@ -51,9 +51,12 @@ def n_slots(n: int, k: int) -> int:
     return int(_lib.lib().nb_stream_slots(n, k, n_ctas()))
 
 
-def stream_pack(packed: torch.Tensor, codebook: torch.Tensor, bits: int, n: int, k: int, row_mode: int = 0) -> torch.Tensor:
+def stream_pack(packed: torch.Tensor, codebook: torch.Tensor, bits: int, n: int, k: int, row_mode: int = 0,
+                apart: bool = True) -> torch.Tensor:
     """Tile-major copy of a packed (n, k) matrix for the persistent kernel.  row_mode 1: a fused
-    [gate | up] matrix whose gate and up rows are interleaved in groups of 8 (SwiGLU epilogue)."""
+    [gate | up] matrix whose gate and up rows are interleaved in groups of 8 (SwiGLU epilogue).  apart: a launch goes between the packing
+    and what follows it on the stream, as kernels read weights ahead of the end of the launch in front of them; not needed where the
+    packing is waited for."""
     if not (packed.is_cuda and codebook.is_cuda):
         raise RuntimeError("stream_pack needs CUDA tensors")
     l = _lib.lib()
@@ -64,7 +67,8 @@ def stream_pack(packed: torch.Tensor, codebook: torch.Tensor, bits: int, n: int,
     with torch.cuda.device(packed.device):
         _lib.check(l.nb_stream_pack(packed.data_ptr(), codebook.data_ptr(), _DT[codebook.dtype], bits, n, k, row_mode,
                                     out.data_ptr(), ops._stream()), "nb_stream_pack")
-        torch.zeros(1, device=packed.device)      # a launch in between: the kernels behind read weights ahead of the end of the launch in front
+        if apart:
+            torch.zeros(1, device=packed.device)
     return out
 
 

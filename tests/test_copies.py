@@ -12,7 +12,7 @@ def packing(monkeypatch):
     """Packs by copying, and notes the order of packings and waits."""
     log = []
 
-    def pack(p, c, bits, n, k, row_mode=0):
+    def pack(p, c, bits, n, k, row_mode=0, apart=True):
         log.append(("pack", row_mode))
         return torch.cat((p, c.view(torch.uint8).reshape(-1), torch.tensor([row_mode], dtype=torch.uint8)))
     monkeypatch.setattr(stream, "stream_pack", pack)
