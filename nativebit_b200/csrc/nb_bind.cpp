@@ -70,11 +70,15 @@ PyObject* all_current(PyObject*, PyObject* list) {
     PyErr_SetString(PyExc_TypeError, "all_current takes a list");
     return nullptr;
   }
+  static PyObject *const packed = PyUnicode_InternFromString("packed_indices"), *const codebook = PyUnicode_InternFromString("codebook");
   for (Py_ssize_t i = 0; i < PyList_GET_SIZE(list); ++i) {
     PyObject* item = PyList_GET_ITEM(list, i);
     if (!PyTuple_CheckExact(item) || PyTuple_GET_SIZE(item) != 2 || !PyDict_Check(PyTuple_GET_ITEM(item, 0))) Py_RETURN_FALSE;
     PyObject* buffers = PyTuple_GET_ITEM(item, 0);
-    if (!copy_of(PyTuple_GET_ITEM(item, 1), PyDict_GetItemString(buffers, "packed_indices"), PyDict_GetItemString(buffers, "codebook"))) Py_RETURN_FALSE;
+    if (!copy_of(PyTuple_GET_ITEM(item, 1), PyDict_GetItemWithError(buffers, packed), PyDict_GetItemWithError(buffers, codebook))) {
+      if (PyErr_Occurred()) return nullptr;
+      Py_RETURN_FALSE;
+    }
   }
   Py_RETURN_TRUE;
   END_HANDLE_TH_ERRORS

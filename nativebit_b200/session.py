@@ -45,8 +45,8 @@ class Session:
     def _on_reset(self) -> None:
         """Gives back what the finished sequences hold."""
 
-    def _on_prompt(self) -> None:
-        """In front of a prompt or a portion of one: other weights may have been loaded since the last."""
+    def _on_run(self) -> None:
+        """In front of a prompt, a portion of one or a step: other weights may have been loaded since the last."""
 
     def _on_capture(self) -> None:
         """Right after a capture."""
@@ -74,7 +74,7 @@ class Session:
         if prompt.shape[1] > self.context_len:
             raise RuntimeError(f"prompt of {prompt.shape[1]} tokens exceeds the context of {self.context_len}")
         T = int(prompt.shape[1])
-        self._on_prompt()
+        self._on_run()
         if not self.use_graph or not prompt.is_cuda:
             self._prefill_body(prompt)
         else:
@@ -117,7 +117,7 @@ class Session:
             self.token.copy_(tokens)
             self.step()
             return self.logits[:, None, :].expand(-1, len(want), -1)
-        self._on_prompt()
+        self._on_run()
         out = self._extend_body(tokens, want)
         self.pos_host += T
         self.pos.fill_(self.pos_host)
@@ -133,6 +133,7 @@ class Session:
             self._step_body()
             self.pos_host += 1
             return
+        self._on_run()
         if self.graph is None:
             # the warm-up and the capture run on the session's stream: it must first see what the caller's
             # stream has written (prefill: caches, position, first token)

@@ -116,6 +116,17 @@ def test_sessions_follow_other_weights_from_the_next_prompt_on(built_lib, batch)
     model.embedding.copy_(third.embedding)
     for prompt in prompts[1:]:
         assert torch.equal(_run(session, prompt), _run(third.session(batch), prompt))
+    a, b = other.session(batch), third.session(batch)       # in the middle of a sequence: the next step
+    for s in (a, b):
+        _run(s, prompts[0])
+    for (k, v, _), (k2, v2, _) in zip(a.caches, b.caches):
+        k2.copy_(k), v2.copy_(v)
+    other.load_state_dict(third.state_dict())
+    for _ in range(2):
+        for s in (a, b):
+            s.token.fill_(5)
+            s.step()
+        assert torch.equal(a.logits, b.logits)
     for a, b in zip(model.blocks, third.blocks):
         assert torch.equal(a.gate_up.stream_weight(1), b.gate_up.stream_weight(1)) and torch.equal(a.qkv.stream_weight(), b.qkv.stream_weight())
 
